@@ -449,6 +449,18 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void* tmap,
       "l"(tmap), "r"(bar_cluster), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void* tmap, uint32_t bar_cluster, int x, int y,
+                                                 int z, int w) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
+      "l"(tmap), "r"(bar_cluster), "r"(x), "r"(y), "r"(z), "r"(w)
+      : "memory");
+}
+// Programmatic dependent launch: wait for the kernel this one was launched behind (complete, its
+// writes visible) / let the kernel launched behind this one start.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Bounded wait on a barrier that a thread of the OTHER CTA of the cluster arrives on.
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, const AbortCtl& ctl, int code) {
   auto probe = [&]() {
