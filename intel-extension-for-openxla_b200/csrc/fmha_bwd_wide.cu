@@ -38,8 +38,7 @@ constexpr int kSlabBytes = 128;    // one swizzle span: 64 16-bit elements
 constexpr int kMaxSlabs = 4;       // head size <= 256
 constexpr int kBoxBytes = 128 * kSlabBytes;   // 128 rows x 128 bytes
 constexpr int kHalfBox = 64 * kSlabBytes;     // 64 rows x 128 bytes
-// P and dS of the heads of one group: half of it is touched under a causal mask.  The L2 holds 126 MB.
-constexpr size_t kGroupBudget = static_cast<size_t>(128) << 20;
+constexpr size_t kGroupBudget = static_cast<size_t>(192) << 20;   // scratch per group of heads (see heads_per_group)
 // The gradient tiles of a group are dealt to this many launches of wide_grads_kernel that run side by
 // side (see launch_bwd_wide).
 constexpr int kGradSlices = 6;
@@ -366,6 +365,7 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
           }
         };
+        const bool stored = warp_row < args.F && key0 < args.T;      // (warp-uniform) the box meets the plane
         const bool masked = key0 + 64 > args.T || (args.causal && key0 + 63 > warp_row);
         if (masked) make_p(std::true_type{}); else make_p(std::false_type{});
         // the box holds the previous tile's dS until its store has read it
@@ -384,7 +384,7 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         ptx::fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
+        if (lane == 0 && stored) {
           ptx::tma_store_3d(&tmap_p, box, key0, warp_row, run.head);
           ptx::bulk_commit_group();
         }
@@ -413,7 +413,7 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         stage_half_row(box, lane, 1, w[1]);
         ptx::fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
+        if (lane == 0 && stored) {
           ptx::tma_store_3d(&tmap_ds, box, key0, warp_row, run.head);
           ptx::bulk_commit_group();
         }
@@ -714,15 +714,14 @@ wide_grads_kernel(const __grid_constant__ GradMaps maps, const __grid_constant__
 
 // ------------------------------------------------------------------------------------- host side
 
-int64_t padded_rows(int F) { return static_cast<int64_t>(F + kRowBlock - 1) / kRowBlock * kRowBlock; }
-int64_t padded_keys(int T) { return static_cast<int64_t>(T + kKeyTile - 1) / kKeyTile * kKeyTile; }
+int64_t plane_pitch(int T) { return (static_cast<int64_t>(T) + 7) / 8 * 8; }   // keys of a plane's row: 16-byte rows
 
+// Heads of one batch that are taken together, and the scratch that the entry point asks for: 6 bytes per
+// query-key pair of a group, of which the planes of P and dS use 4.
 int heads_per_group(const Problem& p) {
-  const size_t per_head = static_cast<size_t>(padded_rows(p.F)) * padded_keys(p.T) * 4;   // P and dS
-  const int n = std::max(p.N, 1);
-  const int fit = static_cast<int>(std::min<size_t>(std::max<size_t>(kGroupBudget / std::max<size_t>(per_head, 1), 1), n));
-  const int groups = (n + fit - 1) / fit;
-  return (n + groups - 1) / groups;       // groups of (almost) one size
+  const size_t per_head = static_cast<size_t>(p.F) * plane_pitch(p.T) * 6;
+  if (per_head == 0) return 1;
+  return static_cast<int>(std::min<size_t>(std::max<size_t>(kGroupBudget / per_head, 1), static_cast<size_t>(std::max(p.N, 1))));
 }
 
 template <typename Kernel, typename... Args>
@@ -752,7 +751,7 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
   const Problem& p = bp.fwd;
   const CUtensorMapDataType dt = kBf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const int group = heads_per_group(p);
-  const int64_t rows = padded_rows(p.F), keys = padded_keys(p.T);
+  const int64_t rows = p.F, keys = plane_pitch(p.T);   // stores are clipped there, loads read zeros beyond
   uint16_t* plane_p = static_cast<uint16_t*>(scratch);
   uint16_t* plane_ds = plane_p + static_cast<int64_t>(group) * rows * keys;
 
@@ -817,8 +816,8 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
   ScoreArgs sa{};
   sa.N = p.N; sa.F = p.F; sa.T = p.T;
   sa.f_pad = f_pad;
-  sa.nq = static_cast<int>(rows / kRowBlock);
-  sa.nk = static_cast<int>(keys / kKeyTile);
+  sa.nq = (p.F + kRowBlock - 1) / kRowBlock;
+  sa.nk = (p.T + kKeyTile - 1) / kKeyTile;
   sa.slabs = (p.H + 63) / 64;
   sa.causal = p.causal ? 1 : 0;
   sa.tiles_per_head = 0;
@@ -890,7 +889,8 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
 }  // namespace
 
 size_t bwd_wide_scratch_bytes(const Problem& p) {
-  return static_cast<size_t>(heads_per_group(p)) * padded_rows(p.F) * padded_keys(p.T) * 4;
+  const size_t scores = static_cast<size_t>(heads_per_group(p)) * p.F * plane_pitch(p.T);
+  return (scores * 4 + 255) / 256 * 256 + (scores * 2 + 255) / 256 * 256;
 }
 
 // Per group of heads: one launch of the score kernel over all SM pairs, then the gradient tiles dealt
