@@ -1,6 +1,7 @@
 // Attention entry point: the host logic of RunFusedMHA
 // (xla/service/gpu/xetla_gpu_fused_mha_runner.cc:45-149) — dropout rejection, stride checks,
 // dimension derivation — in front of the two kernels.
+#include <algorithm>
 #include <cmath>
 
 #include "fmha_sm100.h"
@@ -84,7 +85,9 @@ size_t ixk_fmha_fwd_workspace_bytes(const ixk_fmha_desc* desc) {
   if (ixk::make_problem(desc, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, &p, false) != IXK_OK) return 0;
   if (p.B == 0 || p.N == 0 || p.F == 0 || p.T == 0) return 0;
   if (!ixk::use_decode(p)) return 0;
-  return ixk::fmha::decode_workspace_bytes(p, ixk::fmha::decode_splits(p, 148));
+  // With scratch for the split-key kernel only, that one runs.
+  return std::max(ixk::fmha::decode_workspace_bytes(p, ixk::fmha::decode_splits(p, 148)),
+                  ixk::fmha::decode_mma_workspace_bytes(p, 148));
 }
 
 int ixk_fmha_fwd(const ixk_fmha_desc* desc, const void* q, const void* k, const void* v, const void* bias,
@@ -106,7 +109,15 @@ int ixk_fmha_fwd(const ixk_fmha_desc* desc, const void* q, const void* k, const 
   ixk::DeviceInfo dev;
   if ((rc = ixk::get_device_info(&dev)) != IXK_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-  if (ixk::use_decode(p)) return ixk::fmha::launch_decode(p, dev, workspace, workspace_bytes, stream);
+  if (ixk::use_decode(p)) {
+    const size_t split_key_need = ixk::fmha::decode_workspace_bytes(p, ixk::fmha::decode_splits(p, dev.sm_count));
+    if (workspace_bytes >= split_key_need && ixk::fmha::decode_mma_applies(p, dev, workspace, workspace_bytes)) {
+      rc = ixk::fmha::launch_decode_mma(p, dev, workspace, stream);
+      if (rc != IXK_UNIMPLEMENTED) return rc;
+      ixk::clear_error();
+    }
+    return ixk::fmha::launch_decode(p, dev, workspace, workspace_bytes, stream);
+  }
   return ixk::fmha::launch_prefill(p, dev, stream);
 }
 

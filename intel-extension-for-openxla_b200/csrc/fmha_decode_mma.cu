@@ -1,0 +1,677 @@
+// Attention for 2..16 query rows against a long key/value cache, all rows in one pass over the cache.
+//
+// The step is a stream of K and V from HBM; what the split-key kernel of fmha_decode_sm100.cu does per
+// row on the FMA pipe (a dot product, its shuffles, an accumulator) bounds it by instruction issue from
+// two rows on, so there the cache is streamed ceil(F / 2) times.  Here the rows are the N side of small
+// tensor-core products whose M side is the cache:
+//   S^T [keys, rows] = K . Q^T         A = K as it lies in memory, B = Q (registers)
+//   O^T [head, rows] += V^T . P^T      A = V^T (transposing fragment loads), B = P
+// 8 rows cost one instruction per 16 x 16 block of K or V, 16 rows two: at head size 256 about a fifth
+// of the cycles that HBM takes to deliver the block.  (mma.sync and not tcgen05: with 8 rows the
+// product is 3 % of what the tensor core could do in the time; what counts is that nothing has to
+// travel through tensor memory between the two products.)
+//
+//   CTAs      persistent, one per SM; the (batch, head) units are cut into tiles of keys, the tiles
+//             numbered through, and every CTA takes an equal, contiguous range
+//   warp 8    TMA producer: K and V of a tile into one slot of a ring of up to 192 KB
+//   warps 0-7 16 keys of a tile each (so that a tile goes to 2 or 4 warps and the ring's slots are
+//             worked on side by side), every warp with its own running maximum, sum and O^T; merged
+//             through shared memory where a unit ends
+// A unit that a range boundary cuts leaves unnormalised partials (O, maximum, sum) in scratch, which
+// fmha_decode_mma_combine_kernel merges.
+//
+// P keeps its 32 bits: it is multiplied as the sum of two 16-bit numbers (hi + lo, 16 mantissa bits in
+// bf16, 21 in fp16), and all sums are fp32.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "fmha_sm100.h"
+#include "ptx.cuh"
+
+namespace ixk {
+namespace fmha {
+
+namespace {
+
+constexpr int kWarps = 8;                         // compute warps; one more for the loads
+constexpr int kThreads = (kWarps + 1) * 32;
+constexpr int kMinKeysPerCta = 128;               // below that the merge costs more than the streaming saves
+constexpr size_t kMaxPartialBytes = IXK_STATIC_SCRATCH_BYTES;  // also the scratch of ixk_fmha_fwd_static_scratch
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kLn2 = 0.6931471805599453f;
+
+// wait sites reported in the device status word
+enum : int { kSiteEmpty = 0x61, kSiteFull = 0x62 };
+
+constexpr int gcd(int a, int b) { return b == 0 ? a : gcd(b, a % b); }
+constexpr int lcm(int a, int b) { return a / gcd(a, b) * b; }
+
+template <int kSlabs, int kNT>
+struct Cfg {
+  static constexpr int kKeys = kSlabs > 2 ? 32 : 64;             // keys of a tile
+  static constexpr int kBoxBytes = kKeys * 128;                  // 64 head elements of them
+  static constexpr int kTileBytes = kSlabs * kBoxBytes;          // K or V
+  static constexpr int kStageBytes = 2 * kTileBytes;
+  static constexpr int kRows = kNT * 8;
+  static constexpr int kHPad = kSlabs * 64;
+  static constexpr int kMergeBytes = kWarps / 2 * kRows * kHPad * 4;
+  static constexpr int kTailBytes = 2048;                        // barriers, maxima and sums
+  // Q as B fragments takes kSlabs * kNT * 8 registers; beside the O^T of two blocks of rows and three or
+  // four slabs it would spill, and is read from shared memory for every 16 keys instead
+  static constexpr bool kQShared = kNT == 2 && kSlabs >= 3;
+  static constexpr int kQBytes = kQShared ? kRows * kHPad * 2 : 0;
+  static constexpr int kFit = (232448 - 1024 - kMergeBytes - kTailBytes - kQBytes) / kStageBytes;
+  static constexpr int kStages = kFit < 16 ? kFit : 16;
+  static constexpr int kWarpsPerTile = kKeys / 16;
+  static constexpr int kGroups = kWarps / kWarpsPerTile;         // tiles worked on side by side
+  // A tile's barriers: the tile's number modulo this, so that each is used by one slot and one group of
+  // warps only.  (Barriers per slot would not do: a group comes back to a slot after other groups' turns,
+  // and a wait by parity cannot tell their phases from its own.)
+  static constexpr int kBars = lcm(kStages, kGroups);
+  static constexpr int kSmemBytes = kStages * kStageBytes + kMergeBytes + kQBytes + kTailBytes + 1024;
+  static_assert(kSmemBytes <= 232448, "shared memory budget");
+  static_assert(kStages >= kGroups, "every group of warps needs a slot of its own");
+  static_assert(2 * kWarps * kRows * 4 + 16 * kBars + 8 <= kTailBytes, "tail");
+};
+
+struct Args {
+  int B, N, H, F, T;
+  int causal;
+  float scale_log2;
+  int tiles_per_unit, total_tiles;
+  const uint16_t* q;
+  const uint16_t* bias;
+  uint16_t* out;
+  float* lse;
+  float* partial;   // [2 * grid][F][H + 2]: the unit a CTA's range starts inside of, and the one it starts
+  int k_head_mul, k_batch_mul, v_head_mul, v_batch_mul;   // 0: one K / V for all heads / batches
+  int64_t q_strides[3], o_strides[3], bias_strides[3];
+  int* status_word;
+};
+
+__host__ __device__ __forceinline__ int range_begin(int total, int cta, int ctas) {
+  return static_cast<int>(static_cast<int64_t>(total) * cta / ctas);
+}
+
+template <bool kBf16>
+__device__ __forceinline__ float to_f32(uint16_t h) {
+  return kBf16 ? __uint_as_float(static_cast<uint32_t>(h) << 16) : __half2float(__ushort_as_half(h));
+}
+template <bool kBf16>
+__device__ __forceinline__ uint16_t from_f32(float x) {
+  return kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(x)) : __half_as_ushort(__float2half_rn(x));
+}
+
+// Two probabilities as hi + lo pairs.  hi is the largest 16-bit number strictly below p (0 for p = 0),
+// so that lo > 0 wherever p > 0: with lo = 0 an infinite V would turn p * inf into inf + 0 * inf = NaN.
+template <bool kBf16>
+__device__ __forceinline__ void split_pair(float p0, float p1, uint32_t& hi, uint32_t& lo) {
+  const float b0 = p0 > 0.0f ? __uint_as_float(__float_as_uint(p0) - 1u) : p0;   // (NaN stays NaN)
+  const float b1 = p1 > 0.0f ? __uint_as_float(__float_as_uint(p1) - 1u) : p1;
+  if constexpr (kBf16) {
+    const float h0 = __uint_as_float(__float_as_uint(b0) & 0xffff0000u);
+    const float h1 = __uint_as_float(__float_as_uint(b1) & 0xffff0000u);
+    hi = __byte_perm(__float_as_uint(b0), __float_as_uint(b1), 0x7632);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(p0 - h0, p1 - h1);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+  } else {
+    const __half h0 = __float2half_rz(b0), h1 = __float2half_rz(b1);
+    hi = static_cast<uint32_t>(__half_as_ushort(h0)) | (static_cast<uint32_t>(__half_as_ushort(h1)) << 16);
+    const __half2 l = __floats2half2_rn(p0 - __half2float(h0), p1 - __half2float(h1));
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+  }
+}
+
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+template <bool kBf16>
+__device__ __forceinline__ void mma_16x8x16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (kBf16)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int kSlabs, int kNT, bool kBf16>
+__global__ void __launch_bounds__(kThreads, 1)
+fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                       const __grid_constant__ Args a) {
+  using C = Cfg<kSlabs, kNT>;
+  constexpr int kSteps = kSlabs * 4;              // 16 head elements each
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_gen = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
+  float* merge = reinterpret_cast<float*>(smem_gen + C::kStages * C::kStageBytes);   // [4][head][rows]
+  uint8_t* q_rows = smem_gen + C::kStages * C::kStageBytes + C::kMergeBytes;            // [rows][head], 16-byte pieces swizzled
+  uint8_t* tail = q_rows + C::kQBytes;
+  float* sm_m = reinterpret_cast<float*>(tail);                  // [8 warps][rows]
+  float* sm_l = sm_m + kWarps * C::kRows;
+  // barriers (8 bytes each)
+  const uint32_t bars = smem_base + C::kStages * C::kStageBytes + C::kMergeBytes + C::kQBytes + 2 * kWarps * C::kRows * 4;
+  auto full = [&](int i) { return bars + 8u * i; };
+  auto empty = [&](int i) { return bars + 8u * (C::kBars + i); };
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 2 * kWarps * C::kRows * 4 + 16 * C::kBars);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  ptx::AbortCtl ctl{abort_flag, a.status_word};
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < C::kBars; ++i) {
+      ptx::mbar_init(full(i), 1);
+      ptx::mbar_init(empty(i), C::kWarpsPerTile);
+    }
+    ptx::fence_mbar_init();
+    ptx::prefetch_tmap(&tmap_k);
+    ptx::prefetch_tmap(&tmap_v);
+  }
+  __syncthreads();
+  ptx::grid_dependency_trigger();   // the combine kernel may be set up meanwhile; it waits for this grid's end
+
+  const int t_begin = range_begin(a.total_tiles, blockIdx.x, gridDim.x);
+  const int t_end = range_begin(a.total_tiles, blockIdx.x + 1, gridDim.x);
+
+  if (warp == kWarps) {
+    // ------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      int unit = t_begin / a.tiles_per_unit;
+      int in_unit = t_begin - unit * a.tiles_per_unit;
+      for (int seq = 0; seq < t_end - t_begin; ++seq) {
+        const int head = unit % a.N, batch = unit / a.N;
+        const int before = seq - C::kStages;      // the tile that had the slot
+        if (before >= 0 &&
+            !ptx::mbar_wait(empty(before % C::kBars), static_cast<uint32_t>(before / C::kBars) & 1u, ctl, kSiteEmpty))
+          break;
+        const uint32_t bar = full(seq % C::kBars);
+        ptx::mbar_expect_tx(bar, C::kStageBytes);
+        const uint32_t dst = smem_base + seq % C::kStages * C::kStageBytes;
+#pragma unroll
+        for (int s = 0; s < kSlabs; ++s)
+          ptx::tma_load_4d(dst + s * C::kBoxBytes, &tmap_k, bar, s * 64, in_unit * C::kKeys, head * a.k_head_mul,
+                           batch * a.k_batch_mul);
+#pragma unroll
+        for (int s = 0; s < kSlabs; ++s)
+          ptx::tma_load_4d(dst + C::kTileBytes + s * C::kBoxBytes, &tmap_v, bar, s * 64, in_unit * C::kKeys,
+                           head * a.v_head_mul, batch * a.v_batch_mul);
+        if (++in_unit == a.tiles_per_unit) {
+          in_unit = 0;
+          ++unit;
+        }
+      }
+    }
+  } else {
+    const int g = lane >> 2, c = lane & 3;        // fragment row / column-pair index
+    const int group = warp / C::kWarpsPerTile;
+    const int key_row = (warp % C::kWarpsPerTile) * 16;
+    // ldmatrix row addresses of this lane (row of the box, 16-byte column before the swizzle)
+    const int k_row = key_row + (lane & 7) + ((lane >> 3) & 1) * 8;
+    const int k_col = lane >> 4;
+    const int v_row = key_row + (lane & 7) + (lane >> 4) * 8;
+    const int v_col = (lane >> 3) & 1;
+    bool alive = true;
+
+    for (int t = t_begin; t < t_end;) {
+      // ---- one unit's part of the range (the loop is the same for all eight warps, barriers included)
+      const int unit = t / a.tiles_per_unit;
+      const int head = unit % a.N, batch = unit / a.N;
+      const int unit_t0 = unit * a.tiles_per_unit;
+      const int seg_end = min(t_end, unit_t0 + a.tiles_per_unit);
+
+      const uint16_t* q_base = a.q + batch * a.q_strides[0] + head * a.q_strides[1];
+      [[maybe_unused]] uint32_t qf[C::kQShared ? 1 : kSteps][kNT][2];
+      if constexpr (C::kQShared) {
+        // (every warp is past the previous unit's last tile: it has gone through that unit's merge)
+        for (int i = threadIdx.x; i < C::kRows * kSlabs * 8; i += kWarps * 32) {
+          const int f = i / (kSlabs * 8), piece = i % (kSlabs * 8);
+          uint4 w = make_uint4(0u, 0u, 0u, 0u);
+          if (f < a.F && piece * 8 < a.H) w = __ldg(reinterpret_cast<const uint4*>(q_base + f * a.q_strides[2] + piece * 8));
+          *reinterpret_cast<uint4*>(q_rows + f * C::kHPad * 2 + ((piece ^ (f & 7)) << 4)) = w;
+        }
+        ptx::named_barrier_sync(1, kWarps * 32);
+      } else {
+#pragma unroll
+        for (int nt = 0; nt < kNT; ++nt) {
+          const int f = nt * 8 + g;
+          const uint16_t* qrow = q_base + f * a.q_strides[2];
+#pragma unroll
+          for (int ks = 0; ks < kSteps; ++ks) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const int d = ks * 16 + i * 8 + 2 * c;
+              qf[ks][nt][i] = (f < a.F && d < a.H) ? __ldg(reinterpret_cast<const uint32_t*>(qrow + d)) : 0u;   // H is a multiple of 8
+            }
+          }
+        }
+      }
+      const uint16_t* bias_row[kNT][2];
+#pragma unroll
+      for (int nt = 0; nt < kNT; ++nt) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int fr = nt * 8 + 2 * c + i;
+          bias_row[nt][i] = (a.bias != nullptr && fr < a.F)
+                                ? a.bias + batch * a.bias_strides[0] + head * a.bias_strides[1] + fr * a.bias_strides[2]
+                                : nullptr;
+        }
+      }
+      float o[kSteps][kNT][4];
+      float m_run[kNT][2], l_run[kNT][2];
+#pragma unroll
+      for (int nt = 0; nt < kNT; ++nt) {
+        m_run[nt][0] = m_run[nt][1] = -INFINITY;
+        l_run[nt][0] = l_run[nt][1] = 0.0f;
+#pragma unroll
+        for (int mt = 0; mt < kSteps; ++mt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) o[mt][nt][i] = 0.0f;
+      }
+
+      // ---- this warp's tiles: every kGroups-th of the CTA's sequence
+      int seq = t - t_begin;
+      seq += (group - seq % C::kGroups + C::kGroups) % C::kGroups;
+      for (; alive && t_begin + seq < seg_end; seq += C::kGroups) {
+        const int slot = seq % C::kStages;
+        const int key0 = (t_begin + seq - unit_t0) * C::kKeys + key_row;   // first of this warp's 16 keys
+        float bias_v[kNT][4];
+#pragma unroll
+        for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) bias_v[nt][i] = 0.0f;
+        if (a.bias != nullptr) {
+#pragma unroll
+          for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int key = key0 + g + (i >> 1) * 8;
+              if (bias_row[nt][i & 1] != nullptr && key < a.T) bias_v[nt][i] = to_f32<kBf16>(__ldg(bias_row[nt][i & 1] + key));
+            }
+        }
+        const int bar = seq % C::kBars;
+        if (!ptx::mbar_wait(full(bar), static_cast<uint32_t>(seq / C::kBars) & 1u, ctl, kSiteFull)) {
+          alive = false;
+          break;
+        }
+        const uint32_t k_tile = smem_base + slot * C::kStageBytes;
+        const uint32_t v_tile = k_tile + C::kTileBytes;
+        // S^T: two accumulators per block of rows keep the chains short
+        float acc[2][kNT][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][nt][e] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < kSteps; ++ks) {
+          uint32_t af[4];
+          ldmatrix_x4(k_tile + (ks >> 2) * C::kBoxBytes + k_row * 128 + (((2 * (ks & 3) + k_col) ^ (k_row & 7)) << 4), af);
+          if constexpr (C::kQShared) {
+            uint32_t qb[4];     // b0, b1 of rows 0-7, b0, b1 of rows 8-15
+            const int row = (lane & 7) + (lane >> 4) * 8;
+            ldmatrix_x4(ptx::smem_u32(q_rows) + row * C::kHPad * 2 + (((2 * ks + ((lane >> 3) & 1)) ^ (row & 7)) << 4), qb);
+            mma_16x8x16<kBf16>(acc[ks & 1][0], af, qb[0], qb[1]);
+            mma_16x8x16<kBf16>(acc[ks & 1][kNT - 1], af, qb[2], qb[3]);
+          } else {
+#pragma unroll
+            for (int nt = 0; nt < kNT; ++nt) mma_16x8x16<kBf16>(acc[ks & 1][nt], af, qf[ks][nt][0], qf[ks][nt][1]);
+          }
+        }
+        const bool edge = a.causal || key0 + 16 > a.T;   // (warp-uniform)
+        uint32_t p_hi[kNT][2], p_lo[kNT][2];
+#pragma unroll
+        for (int nt = 0; nt < kNT; ++nt) {
+          float x[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            x[i] = (acc[0][nt][i] + acc[1][nt][i]) * a.scale_log2;
+            if (a.bias != nullptr) x[i] = fmaf(bias_v[nt][i], kLog2e, x[i]);
+            if (edge) {
+              const int key = key0 + g + (i >> 1) * 8;
+              if (key >= a.T || (a.causal && key > nt * 8 + 2 * c + (i & 1))) x[i] = -INFINITY;
+            }
+          }
+          float mx[2] = {fmaxf(x[0], x[2]), fmaxf(x[1], x[3])};
+#pragma unroll
+          for (int off = 4; off < 32; off <<= 1) {
+            mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], off));
+            mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], off));
+          }
+          const bool raised = mx[0] > m_run[nt][0] || mx[1] > m_run[nt][1];
+          if (__any_sync(0xffffffffu, raised)) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const float m_new = fmaxf(m_run[nt][i], mx[i]);
+              const float corr = m_new == -INFINITY ? 1.0f : ptx::ex2_approx(m_run[nt][i] - m_new);   // 0 from -inf
+              m_run[nt][i] = m_new;
+              l_run[nt][i] *= corr;
+#pragma unroll
+              for (int mt = 0; mt < kSteps; ++mt) {
+                o[mt][nt][i] *= corr;
+                o[mt][nt][i + 2] *= corr;
+              }
+            }
+          }
+          float p[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float m = m_run[nt][i & 1];
+            p[i] = ptx::ex2_approx(x[i] - (m == -INFINITY ? 0.0f : m));   // 0 for masked / absent keys
+            l_run[nt][i & 1] += p[i];
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {   // keys g (+ 8): [key][row] blocks turned into B fragments
+            uint32_t hi, lo;
+            split_pair<kBf16>(p[2 * i], p[2 * i + 1], hi, lo);
+            p_hi[nt][i] = transpose_8x8(hi);
+            p_lo[nt][i] = transpose_8x8(lo);
+          }
+        }
+#pragma unroll
+        for (int mt = 0; mt < kSteps; ++mt) {
+          uint32_t af[4];
+          ldmatrix_x4_trans(v_tile + (mt >> 2) * C::kBoxBytes + v_row * 128 + (((2 * (mt & 3) + v_col) ^ (v_row & 7)) << 4), af);
+#pragma unroll
+          for (int nt = 0; nt < kNT; ++nt) {
+            mma_16x8x16<kBf16>(o[mt][nt], af, p_hi[nt][0], p_hi[nt][1]);
+            mma_16x8x16<kBf16>(o[mt][nt], af, p_lo[nt][0], p_lo[nt][1]);
+          }
+        }
+        ptx::fence_proxy_async_smem();   // these reads come before the slot's next TMA write
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(empty(bar));
+      }
+
+      // ---- merge the eight warps: the upper four into the lower four, then all threads over the rest
+      auto put = [&](int w4) {
+#pragma unroll
+        for (int nt = 0; nt < kNT; ++nt) {
+#pragma unroll
+          for (int mt = 0; mt < kSteps; ++mt) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              float* dst = merge + ((w4 * C::kHPad + mt * 16 + g + i * 8) * kNT + nt) * 8 + 2 * c;
+              *reinterpret_cast<float2*>(dst) = make_float2(o[mt][nt][2 * i], o[mt][nt][2 * i + 1]);
+            }
+          }
+        }
+      };
+#pragma unroll
+      for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int off = 4; off < 32; off <<= 1) l_run[nt][i] += __shfl_xor_sync(0xffffffffu, l_run[nt][i], off);
+      auto put_stats = [&]() {
+        if (g == 0) {
+#pragma unroll
+          for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              sm_m[warp * C::kRows + nt * 8 + 2 * c + i] = m_run[nt][i];
+              sm_l[warp * C::kRows + nt * 8 + 2 * c + i] = l_run[nt][i];
+            }
+        }
+      };
+      ptx::named_barrier_sync(1, kWarps * 32);    // the previous unit's merge has been read
+      if (warp >= 4) {
+        put(warp - 4);
+        put_stats();
+      }
+      ptx::named_barrier_sync(1, kWarps * 32);
+      if (warp < 4) {
+#pragma unroll
+        for (int nt = 0; nt < kNT; ++nt) {
+          float cs[2], co[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int r = nt * 8 + 2 * c + i;
+            const float m_o = sm_m[(warp + 4) * C::kRows + r], l_o = sm_l[(warp + 4) * C::kRows + r];
+            const float m_new = fmaxf(m_run[nt][i], m_o);
+            cs[i] = m_run[nt][i] == -INFINITY ? 0.0f : ptx::ex2_approx(m_run[nt][i] - m_new);
+            co[i] = m_o == -INFINITY ? 0.0f : ptx::ex2_approx(m_o - m_new);
+            l_run[nt][i] = l_run[nt][i] * cs[i] + l_o * co[i];
+            m_run[nt][i] = m_new;
+          }
+#pragma unroll
+          for (int mt = 0; mt < kSteps; ++mt) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const float2 v =
+                  *reinterpret_cast<const float2*>(merge + ((warp * C::kHPad + mt * 16 + g + i * 8) * kNT + nt) * 8 + 2 * c);
+              o[mt][nt][2 * i] = o[mt][nt][2 * i] * cs[0] + v.x * co[0];
+              o[mt][nt][2 * i + 1] = o[mt][nt][2 * i + 1] * cs[1] + v.y * co[1];
+            }
+          }
+        }
+        put(warp);       // (each warp overwrites what it alone has read)
+        put_stats();
+      }
+      ptx::named_barrier_sync(1, kWarps * 32);
+      const bool whole = t == unit_t0 && seg_end == unit_t0 + a.tiles_per_unit;
+      float* part = a.partial + (static_cast<int64_t>(blockIdx.x) * 2 + (t == unit_t0 ? 1 : 0)) * a.F * (a.H + 2);
+      for (int f = 0; f < a.F; ++f) {
+        float m_all = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) m_all = fmaxf(m_all, sm_m[w * C::kRows + f]);
+        float l_all = 0.0f, cw[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const float m_w = sm_m[w * C::kRows + f];
+          cw[w] = m_w == -INFINITY ? 0.0f : ptx::ex2_approx(m_w - m_all);
+          l_all += sm_l[w * C::kRows + f] * cw[w];
+        }
+        const int d = threadIdx.x;
+        if (d < a.H) {
+          float v = 0.0f;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) v += merge[(w * C::kHPad + d) * C::kRows + f] * cw[w];
+          if (whole)
+            a.out[batch * a.o_strides[0] + head * a.o_strides[1] + f * a.o_strides[2] + d] = from_f32<kBf16>(v / l_all);
+          else
+            part[f * (a.H + 2) + d] = v;
+        }
+        if (threadIdx.x == 0) {
+          if (whole) {
+            if (a.lse != nullptr) a.lse[static_cast<int64_t>(unit) * a.F + f] = (m_all + log2f(l_all)) * kLn2;
+          } else {
+            part[f * (a.H + 2) + a.H] = m_all;
+            part[f * (a.H + 2) + a.H + 1] = l_all;
+          }
+        }
+      }
+      t = seg_end;
+    }
+  }
+  if (*abort_flag != 0) __nanosleep(2000000);
+}
+
+// One CTA per (range boundary, row): the first boundary inside a unit merges the unit's partials.
+template <bool kBf16>
+__global__ void __launch_bounds__(256)
+fmha_decode_mma_combine_kernel(const __grid_constant__ Args a, int ctas) {
+  ptx::grid_dependency_wait();
+  const int cta = blockIdx.x + 1;
+  const int f = blockIdx.y;
+  const int cut = range_begin(a.total_tiles, cta, ctas);
+  const int unit = cut / a.tiles_per_unit;
+  const int unit_t0 = unit * a.tiles_per_unit;
+  if (cut == unit_t0 || range_begin(a.total_tiles, cta - 1, ctas) > unit_t0) return;
+  int last = cta;   // the CTA that finishes the unit
+  while (last + 1 < ctas && range_begin(a.total_tiles, last + 1, ctas) < unit_t0 + a.tiles_per_unit) ++last;
+  const int64_t pitch = static_cast<int64_t>(a.F) * (a.H + 2);
+  const float* row = a.partial + f * (a.H + 2);
+  auto part = [&](int c) { return row + (2 * c + (c == cta - 1 ? 1 : 0)) * pitch; };
+  float m_all = -INFINITY;
+  for (int c = cta - 1; c <= last; ++c) m_all = fmaxf(m_all, part(c)[a.H]);
+  float l_all = 0.0f, o = 0.0f;
+  const int d = threadIdx.x;
+#pragma unroll 4
+  for (int c = cta - 1; c <= last; ++c) {
+    const float* pc = part(c);
+    const float m = pc[a.H];
+    const float coef = m == -INFINITY ? 0.0f : ptx::ex2_approx(m - m_all);
+    l_all += pc[a.H + 1] * coef;
+    if (d < a.H) o += pc[d] * coef;
+  }
+  const int head = unit % a.N, batch = unit / a.N;
+  if (d < a.H) a.out[batch * a.o_strides[0] + head * a.o_strides[1] + f * a.o_strides[2] + d] = from_f32<kBf16>(o / l_all);
+  if (d == 0 && a.lse != nullptr) a.lse[static_cast<int64_t>(unit) * a.F + f] = (m_all + log2f(l_all)) * kLn2;
+}
+
+int slabs_of(int H) { return (H + 63) / 64; }
+
+struct Plan {
+  int tiles_per_unit = 0, total_tiles = 0, ctas = 0;
+  bool cut = false;   // some unit is shared by several CTAs
+};
+bool make_plan(const Problem& p, int sm_count, Plan* plan) {
+  const int keys = slabs_of(p.H) > 2 ? 32 : 64;
+  const int64_t per_unit = (static_cast<int64_t>(p.T) + keys - 1) / keys;
+  const int64_t total = per_unit * p.B * p.N;
+  // Two rows of a short cache stay with the split-key kernel: a unit's merge is paid for few keys
+  // (B64 N16 H256, 33 keys: 31 us there, 36 us here; at 200 keys and B4 it is 22 and 19).
+  if (p.F < 2 || p.F > kDecodeMaxQueries || (p.F == 2 && p.T <= kMinKeysPerCta) || total <= 0 || total > 0x7fffffff) return false;
+  const int64_t cta_partials = 2 * static_cast<int64_t>(p.F) * (p.H + 2) * static_cast<int64_t>(sizeof(float));
+  const int64_t fit = static_cast<int64_t>(kMaxPartialBytes) / cta_partials;
+  const int64_t useful = (total * keys + kMinKeysPerCta - 1) / kMinKeysPerCta;
+  plan->tiles_per_unit = static_cast<int>(per_unit);
+  plan->total_tiles = static_cast<int>(total);
+  plan->ctas = static_cast<int>(std::max<int64_t>(std::min({static_cast<int64_t>(sm_count), useful, total, fit}), 1));
+  plan->cut = false;
+  for (int c = 1; c < plan->ctas; ++c)
+    if (range_begin(plan->total_tiles, c, plan->ctas) % plan->tiles_per_unit != 0) plan->cut = true;
+  return true;
+}
+size_t partial_bytes(const Problem& p, const Plan& plan) {
+  return plan.cut ? static_cast<size_t>(plan.ctas) * 2 * p.F * (p.H + 2) * sizeof(float) : 0;
+}
+
+template <int kSlabs, int kNT, bool kBf16>
+int launch_typed(const CUtensorMap& tk, const CUtensorMap& tv, const Args& a, const Plan& plan, const DeviceInfo& dev,
+                 cudaStream_t stream) {
+  using C = Cfg<kSlabs, kNT>;
+  auto* fn = &fmha_decode_mma_kernel<kSlabs, kNT, kBf16>;
+  static thread_local int configured_device = -1;
+  if (configured_device != dev.device) {
+    IXK_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+    configured_device = dev.device;
+  }
+  fn<<<plan.ctas, kThreads, C::kSmemBytes, stream>>>(tk, tv, a);
+  IXK_CUDA_OK(cudaGetLastError());
+  count_launch();
+  if (plan.cut) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(plan.ctas - 1, a.F, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    IXK_CUDA_OK(cudaLaunchKernelEx(&cfg, &fmha_decode_mma_combine_kernel<kBf16>, a, plan.ctas));
+    count_launch();
+  }
+  return IXK_OK;
+}
+
+}  // namespace
+
+size_t decode_mma_workspace_bytes(const Problem& p, int sm_count) {
+  Plan plan;
+  return make_plan(p, sm_count, &plan) ? partial_bytes(p, plan) : 0;
+}
+
+bool decode_mma_applies(const Problem& p, const DeviceInfo& dev, const void* workspace, size_t workspace_bytes) {
+  Plan plan;
+  if (!make_plan(p, dev.sm_count, &plan)) return false;
+  const size_t need = partial_bytes(p, plan);
+  return need == 0 || (workspace != nullptr && workspace_bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0);
+}
+
+int launch_decode_mma(const Problem& p, const DeviceInfo& dev, void* workspace, cudaStream_t stream) {
+  Plan plan;
+  if (!make_plan(p, dev.sm_count, &plan)) return fail(IXK_UNIMPLEMENTED, "decode problem outside the tensor-core kernel's range");
+  const int slabs = slabs_of(p.H);
+  auto make_map = [&](CUtensorMap* out, const void* base, const int64_t* strides) -> int {
+    TmapSpec s{};
+    s.dtype = p.dtype == IXK_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    s.rank = 4;
+    s.swizzle128 = true;
+    s.dims[0] = p.H;
+    s.dims[1] = p.T;
+    s.dims[2] = strides[1] == 0 ? 1 : p.N;
+    s.dims[3] = strides[0] == 0 ? 1 : p.B;
+    // extent-1 dimensions still need a legal stride; any 16-byte multiple will do
+    auto stride_bytes = [&](int64_t st, uint64_t fallback) -> uint64_t { return st > 0 ? static_cast<uint64_t>(st) * 2 : fallback; };
+    const uint64_t pitch = stride_bytes(strides[2], static_cast<uint64_t>(p.H) * 2);
+    s.strides_bytes[0] = pitch;
+    s.strides_bytes[1] = stride_bytes(strides[1], pitch * p.T);
+    s.strides_bytes[2] = stride_bytes(strides[0], pitch * p.T * p.N);
+    s.box[0] = 64;
+    s.box[1] = slabs > 2 ? 32 : 64;
+    s.box[2] = s.box[3] = 1;
+    return encode_tmap(out, base, s);
+  };
+  CUtensorMap tk, tv;
+  if (make_map(&tk, p.k, p.k_strides) != IXK_OK || make_map(&tv, p.v, p.v_strides) != IXK_OK) return IXK_UNIMPLEMENTED;
+  Args a{};
+  a.B = p.B; a.N = p.N; a.H = p.H; a.F = p.F; a.T = p.T;
+  a.causal = p.causal ? 1 : 0;
+  a.scale_log2 = p.head_scale * kLog2e;
+  a.tiles_per_unit = plan.tiles_per_unit;
+  a.total_tiles = plan.total_tiles;
+  a.q = static_cast<const uint16_t*>(p.q);
+  a.bias = static_cast<const uint16_t*>(p.bias);
+  a.out = static_cast<uint16_t*>(p.out);
+  a.lse = p.lse;
+  a.partial = static_cast<float*>(workspace);
+  a.k_head_mul = p.k_strides[1] == 0 ? 0 : 1;
+  a.k_batch_mul = p.k_strides[0] == 0 ? 0 : 1;
+  a.v_head_mul = p.v_strides[1] == 0 ? 0 : 1;
+  a.v_batch_mul = p.v_strides[0] == 0 ? 0 : 1;
+  for (int i = 0; i < 3; ++i) {
+    a.q_strides[i] = p.q_strides[i];
+    a.o_strides[i] = p.o_strides[i];
+    a.bias_strides[i] = p.bias_strides[i];
+  }
+  a.status_word = dev.status_word;
+  auto go = [&](auto slabs_tag) {
+    constexpr int kSlabs = decltype(slabs_tag)::value;
+    if (p.dtype == IXK_BF16)
+      return p.F <= 8 ? launch_typed<kSlabs, 1, true>(tk, tv, a, plan, dev, stream)
+                      : launch_typed<kSlabs, 2, true>(tk, tv, a, plan, dev, stream);
+    return p.F <= 8 ? launch_typed<kSlabs, 1, false>(tk, tv, a, plan, dev, stream)
+                    : launch_typed<kSlabs, 2, false>(tk, tv, a, plan, dev, stream);
+  };
+  switch (slabs) {
+    case 1: return go(std::integral_constant<int, 1>{});
+    case 2: return go(std::integral_constant<int, 2>{});
+    case 3: return go(std::integral_constant<int, 3>{});
+    default: return go(std::integral_constant<int, 4>{});
+  }
+}
+
+}  // namespace fmha
+}  // namespace ixk

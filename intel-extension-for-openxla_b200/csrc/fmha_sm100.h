@@ -39,6 +39,13 @@ size_t decode_workspace_bytes(const Problem& p, int splits);
 int launch_decode(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes,
                   cudaStream_t stream);
 
+// ---- one-pass decode kernel for several query rows (fmha_decode_mma.cu)
+// Scratch it wants (0 where it does not apply), whether it can take a call with the scratch given, and
+// the launch, which answers IXK_UNIMPLEMENTED for K / V views that no tensor map describes.
+size_t decode_mma_workspace_bytes(const Problem& p, int sm_count);
+bool decode_mma_applies(const Problem& p, const DeviceInfo& dev, const void* workspace, size_t workspace_bytes);
+int launch_decode_mma(const Problem& p, const DeviceInfo& dev, void* workspace, cudaStream_t stream);
+
 // ---- tcgen05 backward kernels (fmha_bwd_sm100.cu)
 // `fwd` carries q, k, v, bias, the forward's output (`out`, read only) and row statistic (`lse`).
 struct BwdProblem {

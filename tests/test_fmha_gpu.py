@@ -271,3 +271,58 @@ def test_rejections(pkg, cuda):
     with pytest.raises(pkg.IxkError) as e:
         run(pkg, q, q, q)
     assert e.value.status == pkg.IXK_UNIMPLEMENTED          # head_size % 8
+
+
+# Several query rows in one pass over the cache (fmha_decode_mma.cu): tiles of 64 keys (32 above head
+# size 128) in slices of 16, blocks of 8 rows, head slabs of 64, ranges of tiles cut anywhere in a unit.
+MULTI_ROW_CASES = [
+    # B, N, F, T, H, dtype, causal, bias
+    (1, 1, 2, 1, 8, "bf16", False, False),          # one key, one 16-byte row
+    (2, 3, 7, 17, 64, "fp16", False, False),        # one key past a slice, a row short of a block
+    (3, 5, 8, 65, 72, "bf16", False, True),         # one key past a tile, a slab of 8 elements
+    (1, 2, 9, 63, 136, "fp16", True, False),        # second block of rows; causal: 9 of 63 keys seen
+    (37, 4, 3, 95, 192, "bf16", False, False),      # three slabs, units of three tiles
+    (150, 1, 4, 33, 256, "bf16", False, False),     # more units than CTAs: ranges that cover whole units
+    (1, 1, 16, 9000, 256, "bf16", False, False),    # one unit cut into many ranges, full blocks of rows
+    (7, 11, 5, 777, 128, "fp16", False, True),      # ranges that start and end inside units
+    # enough tiles per CTA that its ring of slots and its barriers are used several times over
+    (40, 10, 4, 250, 256, "bf16", False, False),
+    (40, 10, 11, 250, 256, "fp16", False, False),
+    (40, 10, 9, 250, 192, "bf16", False, False),
+    (50, 16, 2, 600, 128, "bf16", False, False),
+    (90, 16, 3, 300, 64, "fp16", False, False),
+]
+
+
+@pytest.mark.parametrize("case", MULTI_ROW_CASES, ids=lambda c: "B{}N{}F{}T{}H{}{}c{}b{}".format(*c))
+def test_decode_several_rows(pkg, orc, cuda, case):
+    B, N, F, T, H, dt, causal, use_bias = case
+    dtype = torch.bfloat16 if dt == "bf16" else torch.float16
+    g = torch.Generator().manual_seed(T + H)
+    q = torch.randn(B, N, F, H, generator=g).to(dtype).to(cuda)
+    k, v = (torch.randn(B, T, N, H, generator=g).to(dtype).to(cuda).permute(0, 2, 1, 3) for _ in range(2))
+    bias = torch.randn(1, N, F, T, generator=g).to(dtype).to(cuda) if use_bias else None
+    if use_bias:
+        bias[..., 0] = torch.finfo(dtype).min       # a mask made of the type's lowest value
+        bias[:, :, -1, : T // 2] = float("-inf")
+    o, lse = run(pkg, q, k, v, bias, causal, lse=True)
+    want, want_lse = orc.fmha_forward(f32(q), f32(k), f32(v), None if bias is None else f32(bias), head_scale=H ** -0.5,
+                                      causal=causal, dtype=orc.BF16 if dt == "bf16" else orc.F16, round_p=False)
+    # P is carried in 16 (bf16) or more bits and every sum in fp32: what is left is the one rounding of
+    # the result, which two correct sums may take to neighbouring values, one ulp = 2^-7 or 2^-10 apart
+    ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
+    orc.check_close(f32(o), want, rtol=ulp, atol=1e-4, what=str(case))
+    orc.check_close(f32(lse), want_lse, rtol=1e-5, atol=1e-4, what=f"lse {case}")
+
+
+def test_decode_several_rows_infinite_values(pkg, cuda):
+    """An infinite V element makes its output column infinite (never NaN) for every row that sees the key."""
+    B, N, F, T, H = 1, 2, 4, 300, 128
+    g = torch.Generator().manual_seed(5)
+    q = torch.randn(B, N, F, H, generator=g).bfloat16().to(cuda)
+    k, v = (torch.randn(B, N, T, H, generator=g).bfloat16().to(cuda) for _ in range(2))
+    v[:, :, 33, 7] = float("inf")
+    o, _ = run(pkg, q, k, v)
+    assert torch.all(torch.isposinf(o[..., 7]))
+    o[..., 7] = 0
+    assert torch.all(torch.isfinite(o))
