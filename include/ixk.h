@@ -235,8 +235,10 @@ typedef struct ixk_fmha_desc {
  * rounds P to the storage type (fmha_forward.h:364-382); results agree within the 2e-2 the
  * parity tests allow, F16 and the decode path round to nearest.  lse (may be NULL) receives
  * m + ln(l) per row — the reference's "activation" output when is_training
- * (fmha_forward.h:433-450).  workspace must hold ixk_fmha_fwd_workspace_bytes(desc)
- * bytes (non-zero only for the split-key decode path, F <= 16). */
+ * (fmha_forward.h:433-450).  workspace should hold ixk_fmha_fwd_workspace_bytes(desc) bytes.
+ * The decode path (F <= 16) cannot do without the part of it that its key splits need and answers
+ * IXK_WORKSPACE_TOO_SMALL; a prefill that leaves the GPU partly idle uses it to split its work along
+ * the keys, and runs unsplit without it. */
 int ixk_fmha_fwd(const ixk_fmha_desc* desc, const void* q, const void* k,
                  const void* v, const void* bias, void* out, float* lse,
                  void* workspace, size_t workspace_bytes, void* cuda_stream);
@@ -252,7 +254,7 @@ size_t ixk_fmha_fwd_workspace_bytes(const ixk_fmha_desc* desc);
  * keeps its partial results in an array of IXK_STATIC_SCRATCH_BYTES that is part of the library's
  * device image (each GPU that loads libixk.so holds that much memory until the process exits).
  * The call allocates nothing and frees nothing.
- *   - A problem whose ixk_fmha_fwd_workspace_bytes(desc) exceeds IXK_STATIC_SCRATCH_BYTES is
+ *   - A problem whose key splits need more than IXK_STATIC_SCRATCH_BYTES is
  *     refused with IXK_WORKSPACE_TOO_SMALL and nothing is launched; use ixk_fmha_fwd then.
  *   - The first call on each device looks up the array's device address.  The call itself
  *     allocates nothing, but with CUDA's lazy module loading it can be the moment at which the

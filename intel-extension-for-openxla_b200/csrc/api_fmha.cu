@@ -78,13 +78,23 @@ bool use_decode(const fmha::Problem& p) { return p.F <= fmha::kDecodeMaxQueries;
 }  // namespace
 }  // namespace ixk
 
+namespace ixk {
+// The part of ixk_fmha_fwd_workspace_bytes that a call cannot do without.
+size_t fmha_required_workspace_bytes(const ixk_fmha_desc* desc) {
+  fmha::Problem p;
+  if (make_problem(desc, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, &p, false) != IXK_OK) return 0;
+  if (p.B == 0 || p.N == 0 || p.F == 0 || p.T == 0 || !use_decode(p)) return 0;
+  return fmha::decode_workspace_bytes(p, fmha::decode_splits(p, 148));
+}
+}  // namespace ixk
+
 extern "C" {
 
 size_t ixk_fmha_fwd_workspace_bytes(const ixk_fmha_desc* desc) {
   ixk::fmha::Problem p;
   if (ixk::make_problem(desc, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, &p, false) != IXK_OK) return 0;
   if (p.B == 0 || p.N == 0 || p.F == 0 || p.T == 0) return 0;
-  if (!ixk::use_decode(p)) return 0;
+  if (!ixk::use_decode(p)) return ixk::fmha::prefill_workspace_bytes(p, 148);
   // With scratch for the split-key kernel only, that one runs.
   return std::max(ixk::fmha::decode_workspace_bytes(p, ixk::fmha::decode_splits(p, 148)),
                   ixk::fmha::decode_mma_workspace_bytes(p, 148));
@@ -118,7 +128,7 @@ int ixk_fmha_fwd(const ixk_fmha_desc* desc, const void* q, const void* k, const 
     }
     return ixk::fmha::launch_decode(p, dev, workspace, workspace_bytes, stream);
   }
-  return ixk::fmha::launch_prefill(p, dev, stream);
+  return ixk::fmha::launch_prefill(p, dev, workspace, workspace_bytes, stream);
 }
 
 size_t ixk_fmha_bwd_workspace_bytes(const ixk_fmha_bwd_desc* desc) {

@@ -14,7 +14,7 @@
 //                                      O_t += P_t.V_j   (A = P from TMEM, B = V from shared memory)
 //   warps 12-15   epilogue: O / row sum out of TMEM, one rounding, stores (both tiles); the softmax
 //                 warps hand over 1 / row sum and go straight on to the next work item
-// The two softmax warpgroups take 184 registers per thread (a whole row of S lives in registers),
+// The two softmax warpgroups take 192 registers per thread (a whole row of S lives in registers),
 // the control and epilogue warpgroups give their share up (setmaxnreg).
 //
 // CTAs are persistent: each walks a static list of (batch, head, query block) work items, heaviest
@@ -57,10 +57,10 @@ constexpr int kProducerWarp = 8;
 constexpr int kMmaWarp = 9;
 constexpr int kParts = 4;  // pieces in which a block of P is handed to the MMA issuer (1, 2 or 4)
 constexpr int kEpilogueWarp = 12;  // first warp of the epilogue warpgroup
-// per-thread register budgets after re-partitioning: 256 x 184 + 128 x 56 + 128 x 88 = 65536
-constexpr int kSoftmaxRegs = 184;
-constexpr int kControlRegs = 56;
-constexpr int kEpilogueRegs = 88;
+// per-thread register budgets after re-partitioning: 256 x 192 + 128 x 48 + 128 x 80 = 65536
+constexpr int kSoftmaxRegs = 192;
+constexpr int kControlRegs = 48;
+constexpr int kEpilogueRegs = 80;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kTruncInflate = 1.0028179f;     // 1 + 2^-8 * (1 / (2 ln 2)): mean relative loss of bf16 truncation
@@ -112,6 +112,11 @@ struct KernelArgs {
   // 1 otherwise: multiplies the head / batch coordinate of the K and V loads
   int k_head_mul, k_batch_mul, v_head_mul, v_batch_mul;
   int use_schedule;  // the CTAs walk the host-made work list instead of the dealing formula
+  // Work units from num_direct on are parts of split_len key blocks of an item; they leave unnormalised
+  // results in the scratch below, which fmha_prefill_combine_kernel merges.  (num_items counts units.)
+  int num_direct, split_len;
+  float* part_o;      // [part][row of the item][kHeadDim]
+  float2* part_stat;  // [part][row of the item]: running maximum (log2 domain) and row sum
 };
 
 __device__ __forceinline__ uint32_t pack2(float lo, float hi, bool bf16) {
@@ -135,7 +140,9 @@ struct Item {
   int q0, head, batch;
   int nblk0, nblk1;  // key blocks of query tile 0 / 1 (scalars: a runtime index would put an array in local memory)
   int nblk_max;
-  int reversed;  // key blocks are walked from the diagonal down to block 0 (causal)
+  int reversed;  // key blocks are walked from the diagonal down to block `lo` (causal)
+  int lo;        // first key block (0 unless the item is split)
+  int part;      // index among the split parts, -1 for a whole item
   __device__ __forceinline__ int nblk(int t) const { return t == 0 ? nblk0 : nblk1; }
   // The item takes nblk_max steps; tile t takes part in nblk(t) consecutive ones: the first
   // nblk(t) in forward order, the last nblk(t) in reversed order (every tile ends on block 0).
@@ -143,10 +150,49 @@ struct Item {
   __device__ __forceinline__ bool active(int t, int step) const {
     return step >= first(t) && step < first(t) + nblk(t);
   }
-  __device__ __forceinline__ int key_block(int step) const { return reversed ? nblk_max - 1 - step : step; }
+  __device__ __forceinline__ int key_block(int step) const { return lo + (reversed ? nblk_max - 1 - step : step); }
 };
 
+// Key blocks that the query tile starting at row0 visits.
+__host__ __device__ __forceinline__ int tile_blocks(const KernelArgs& args, int row0) {
+  const int all = (args.T + kBlockKV - 1) / kBlockKV;
+  if (!args.causal) return all;
+  const int seen = (row0 + kBlockQ - 1) / kBlockKV + 1;
+  return seen < all ? seen : all;
+}
+// ... and the item of query block qb (its last tile with rows sees the most keys).
 template <int kQTiles>
+__host__ __device__ __forceinline__ int item_blocks(const KernelArgs& args, int qb) {
+  int row0 = (qb * kQTiles + kQTiles - 1) * kBlockQ;
+  if (kQTiles == 2 && row0 >= args.F) row0 -= kBlockQ;
+  return tile_blocks(args, row0);
+}
+
+// The idx-th split part.  Non-causal: the parts of an item are neighbours.  Causal (every item is split):
+// part by part over all (batch, head) pairs, query blocks from the last one down.
+struct SplitPart {
+  int pair, qb, part;
+};
+template <int kQTiles>
+__device__ __forceinline__ SplitPart split_part(const KernelArgs& args, int idx) {
+  SplitPart sp;
+  if (args.causal) {
+    const int pairs = args.N * args.B;
+    sp.part = idx / pairs;
+    sp.pair = idx - sp.part * pairs;
+    sp.qb = args.num_qblocks - 1;
+    for (int n; sp.part >= (n = (item_blocks<kQTiles>(args, sp.qb) + args.split_len - 1) / args.split_len); --sp.qb) sp.part -= n;
+  } else {
+    const int per_item = (tile_blocks(args, 0) + args.split_len - 1) / args.split_len;
+    const int item = args.num_direct + idx / per_item;
+    sp.part = idx % per_item;
+    sp.pair = item / args.num_qblocks;
+    sp.qb = item - sp.pair * args.num_qblocks;
+  }
+  return sp;
+}
+
+template <int kQTiles, bool kSplit>
 __device__ __forceinline__ Item get_item(const KernelArgs& args, int w) {
   // Causal: items are ordered heaviest first (the last query block sees the most keys), query
   // block by query block over all (batch, head) pairs, which the alternating deal below balances.
@@ -158,7 +204,16 @@ __device__ __forceinline__ Item get_item(const KernelArgs& args, int w) {
   const int pairs = args.N * args.B;
   Item it;
   int qb;
-  if (args.causal) {
+  it.lo = 0;
+  it.part = -1;
+  if (kSplit && w >= args.num_direct) {
+    const SplitPart sp = split_part<kQTiles>(args, w - args.num_direct);
+    it.part = w - args.num_direct;
+    it.lo = sp.part * args.split_len;
+    it.head = sp.pair % args.N;
+    it.batch = sp.pair / args.N;
+    qb = sp.qb;
+  } else if (args.causal) {
     const int rank = w / pairs;
     const int rest = w - rank * pairs;
     it.head = rest % args.N;
@@ -171,14 +226,13 @@ __device__ __forceinline__ Item get_item(const KernelArgs& args, int w) {
     it.batch = pair / args.N;
   }
   it.q0 = qb * (kBlockQ * kQTiles);
-  const int kv_blocks_all = (args.T + kBlockKV - 1) / kBlockKV;
   it.nblk0 = it.nblk1 = 0;
 #pragma unroll
   for (int t = 0; t < kQTiles; ++t) {
     const int row0 = it.q0 + t * kBlockQ;
     if (row0 < args.F) {
-      int n = kv_blocks_all;
-      if (args.causal) n = min(n, (row0 + kBlockQ - 1) / kBlockKV + 1);
+      int n = tile_blocks(args, row0);
+      if (kSplit && it.part >= 0) n = max(0, min(n - it.lo, args.split_len));
       if (t == 0) it.nblk0 = n; else it.nblk1 = n;
     }
   }
@@ -255,7 +309,7 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_
       : "memory");
 }
 
-template <int kHeadDim, int kQTiles, int kPolyOf4, bool kBias>
+template <int kHeadDim, int kQTiles, int kPolyOf4, bool kBias, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 1)
 fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_bias,
@@ -335,6 +389,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  if (kSplit) ptx::grid_dependency_trigger();   // (the combine kernel waits for this grid's end)
 
   if (warp == kProducerWarp) {
     // ------------------------------------------------------------------ TMA producer
@@ -345,7 +400,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       bool alive = true;
       uint32_t it = 0;
       for (int w = item_of(args, sched, 0); w < args.num_items && alive; w = item_of(args, sched, ++it)) {
-        const Item item = get_item<kQTiles>(args, w);
+        const Item item = get_item<kQTiles, kSplit>(args, w);
         // Q of tile t, once the tile's last S of the previous item has been issued.  A tile with
         // no rows in this item still completes its phase, so that parities follow the item count.
         auto load_q = [&](int t) {
@@ -476,7 +531,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         return alive;
       };
       for (int w = item_of(args, sched, 0); w < args.num_items && alive; w = item_of(args, sched, ++it), q_par ^= 1u) {
-        const Item item = get_item<kQTiles>(args, w);
+        const Item item = get_item<kQTiles, kSplit>(args, w);
         const int nblk_max = item.nblk_max;
         const int first0 = item.first(0), end0 = first0 + item.nblk0;
         const int first1 = item.first(1), end1 = first1 + item.nblk1;
@@ -586,7 +641,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     bool alive = true;
     uint32_t it = 0;
     for (int w = item_of(args, sched, 0); w < args.num_items && alive; w = item_of(args, sched, ++it)) {
-      const Item item = get_item<kQTiles>(args, w);
+      const Item item = get_item<kQTiles, kSplit>(args, w);
       for (int tt = 0; tt < kQTiles && alive; ++tt) {
         const int t = item.reversed ? kQTiles - 1 - tt : tt;  // the tile that started first is served first
         if (item.nblk(t) == 0) continue;
@@ -615,7 +670,22 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             wv[i] = pack2(__uint_as_float(o[2 * i]) * inv_l, __uint_as_float(o[2 * i + 1]) * inv_l, bf16);
         };
         constexpr int kOChunks = kHeadDim / 32;
-        if (C::kStageBytes > 0 && args.out_tma) {
+        if (kSplit && item.part >= 0) {   // part of a split item: fp32, as it is
+          float* dst = args.part_o + ((static_cast<int64_t>(item.part) * kQTiles + t) * kBlockQ + row_in_tile) * kHeadDim;
+#pragma unroll 1
+          for (int c = 0; c < kOChunks; ++c) {
+            uint32_t o[32];
+            ptx::tmem_ld_32x32(o_addr + c * 32, o);
+            ptx::tmem_ld_wait();
+            if (c == kOChunks - 1) {
+              ptx::tc_fence_before_sync();
+              ptx::mbar_arrive(o_free(t));
+            }
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+              reinterpret_cast<uint4*>(dst + c * 32)[g] = make_uint4(o[4 * g], o[4 * g + 1], o[4 * g + 2], o[4 * g + 3]);
+          }
+        } else if (C::kStageBytes > 0 && args.out_tma) {
           const uint32_t stage = stage_smem + t * kChunkBytes;
           const uint32_t my_row = stage + row_in_tile * 128;
           auto rendezvous = [&]() {
@@ -703,7 +773,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       bool alive = true;
       uint32_t it = 0;
       for (int w = item_of(args, sched, 0); w < args.num_items && alive; w = item_of(args, sched, ++it)) {
-        const Item item = get_item<kQTiles>(args, w);
+        const Item item = get_item<kQTiles, kSplit>(args, w);
         const int my_blocks = item.nblk(t);
         if (my_blocks == 0) continue;
         const int q0 = item.q0, head = item.head, batch = item.batch;
@@ -715,7 +785,9 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                      static_cast<int64_t>(f) * args.bias_strides[2];
         float m_run = -INFINITY;
         float l_run = 0.0f;
-        for (int j = 0; j < my_blocks; ++j) {
+        const int kv_step = item.reversed ? -kBlockKV : kBlockKV;
+        int kv0 = (item.lo + (item.reversed ? my_blocks - 1 : 0)) * kBlockKV;
+        for (int j = 0; j < my_blocks; ++j, kv0 += kv_step) {
           // The bias tile of this block is in shared memory before the scores are ready: its first
           // box (keys 0-63) goes into registers while S is still on its way.
           [[maybe_unused]] uint4 bw[kBiasPrefetch];
@@ -741,7 +813,6 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 #pragma unroll
           for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32(s_addr + c * 32, r[c]);
           ptx::tmem_ld_wait();
-          const int kv0 = (item.reversed ? my_blocks - 1 - j : j) * kBlockKV;
           // Scores enter the exponential as x = r * mult - m.  Fast path: r is the raw Q.K^T and
           // mult = head_scale * log2(e) (> 0, so the row maximum can be taken on r).  With a
           // non-positive scale, r is first rewritten as the full log2-domain score and mult = 1.
@@ -934,9 +1005,14 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           break;
         }
         ++n_o;
-        inv_l_slot[t * kBlockQ + row_in_tile] = (bf16 ? kTruncInflate : 1.0f) / l_run;  // the row sum carries the truncation bias
+        const bool whole = !kSplit || w < args.num_direct;
+        if (!whole) {
+          args.part_stat[(static_cast<int64_t>(w - args.num_direct) * kQTiles + t) * kBlockQ + row_in_tile] = make_float2(m_run, l_run);
+        } else {
+          inv_l_slot[t * kBlockQ + row_in_tile] = (bf16 ? kTruncInflate : 1.0f) / l_run;  // the row sum carries the truncation bias
+        }
         ptx::mbar_arrive(stats_full(t));  // (release: the store above is visible to whoever sees the phase)
-        if (args.lse != nullptr && row_ok) {
+        if (args.lse != nullptr && row_ok && whole) {
           const int64_t idx = (static_cast<int64_t>(batch) * args.N + head) * args.F + f;
           args.lse[idx] = (m_run + log2f(l_run) - (bf16 ? kTruncBiasLog2 : 0.0f)) * kLn2;
         }
@@ -951,6 +1027,104 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc(tmem_base, 512);
   }
+}
+
+// One warp per query row of the split items.
+template <int kHeadDim, int kQTiles>
+__global__ void __launch_bounds__(256)
+fmha_prefill_combine_kernel(const __grid_constant__ KernelArgs args, int first_item, int num_base_items) {
+  ptx::grid_dependency_wait();
+  const int lane = threadIdx.x & 31;
+  constexpr int kRows = kQTiles * kBlockQ;
+  const int64_t r = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const int item = first_item + static_cast<int>(r / kRows);
+  if (item >= num_base_items) return;
+  const int row = static_cast<int>(r % kRows);
+  const int pair = item / args.num_qblocks, qb = item - pair * args.num_qblocks;
+  const int f = qb * kRows + row;
+  if (f >= args.F) return;
+  const int head = pair % args.N, batch = pair / args.N;
+  const int len = args.split_len;
+  const int parts = (tile_blocks(args, f - row % kBlockQ) + len - 1) / len;   // of this row's tile
+  int64_t first, step;                                                        // its parts among all parts
+  if (args.causal) {
+    int before = 0;
+    for (int b = args.num_qblocks - 1; b > qb; --b) before += (item_blocks<kQTiles>(args, b) + len - 1) / len;
+    step = static_cast<int64_t>(args.N) * args.B;
+    first = before * step + pair;
+  } else {
+    step = 1;
+    first = static_cast<int64_t>(item - first_item) * parts;
+  }
+  float m = -INFINITY;
+  for (int p = 0; p < parts; ++p) m = fmaxf(m, args.part_stat[(first + p * step) * kRows + row].x);
+  float l = 0.0f, o[kHeadDim / 32];
+#pragma unroll
+  for (int i = 0; i < kHeadDim / 32; ++i) o[i] = 0.0f;
+#pragma unroll 2
+  for (int p = 0; p < parts; ++p) {
+    const int64_t at = (first + p * step) * kRows + row;
+    const float2 st = args.part_stat[at];
+    const float c = st.x == -INFINITY ? 0.0f : ptx::ex2_approx(st.x - m);
+    l = fmaf(st.y, c, l);
+#pragma unroll
+    for (int i = 0; i < kHeadDim / 32; ++i) o[i] = fmaf(args.part_o[at * kHeadDim + i * 32 + lane], c, o[i]);
+  }
+  const bool bf16 = args.is_bf16 != 0;
+  const float inv = (bf16 ? kTruncInflate : 1.0f) / l;
+  uint16_t* orow = args.out + batch * args.o_strides[0] + head * args.o_strides[1] + static_cast<int64_t>(f) * args.o_strides[2];
+#pragma unroll
+  for (int i = 0; i < kHeadDim / 32; ++i) {
+    const int d = i * 32 + lane;
+    if (d < args.H) orow[d] = static_cast<uint16_t>(pack2(o[i] * inv, 0.0f, bf16) & 0xffffu);
+  }
+  if (lane == 0 && args.lse != nullptr)
+    args.lse[(static_cast<int64_t>(batch) * args.N + head) * args.F + f] = (m + log2f(l) - (bf16 ? kTruncBiasLog2 : 0.0f)) * kLn2;
+}
+
+// Which items are split along the keys.  A CTA takes one item at a time, so a launch ends with a round in
+// which some CTAs have no item left, and a small problem is all such a round:
+//   non-causal   the items beyond the last full round, into as many parts as the idle CTAs can take
+//   causal       only where there is not one item per CTA, all items, into parts of one length
+//                (with more items the work list balances them)
+// The merge costs a launch and a pass over the partials, about 4 us; a key block costs a CTA about 1.9 us:
+// a split has to take at least kMinStepsSaved blocks off the longest CTA.
+constexpr int kMinStepsSaved = 4;
+struct SplitPlan {
+  int num_direct = 0, split_len = 0, parts = 0;   // parts == 0: no split
+};
+template <int kQTiles>
+SplitPlan split_plan(const KernelArgs& a, int64_t items, int sms) {
+  SplitPlan plan;
+  if (a.causal) {
+    if (items >= sms) return plan;
+    const int longest = item_blocks<kQTiles>(a, a.num_qblocks - 1);
+    for (int len = 2; longest - len >= kMinStepsSaved; ++len) {
+      int64_t parts = 0;
+      for (int qb = 0; qb < a.num_qblocks; ++qb) parts += (item_blocks<kQTiles>(a, qb) + len - 1) / len;
+      parts *= static_cast<int64_t>(a.N) * a.B;
+      if (parts <= sms) {
+        plan.split_len = len;
+        plan.parts = static_cast<int>(parts);
+        return plan;
+      }
+    }
+    return plan;
+  }
+  const int tail = static_cast<int>(items % sms);
+  if (tail == 0) return plan;
+  const int blocks = tile_blocks(a, 0);
+  const int want = std::min(sms / tail, std::max(blocks / 2, 1));
+  const int len = (blocks + want - 1) / want;
+  if (blocks - len < kMinStepsSaved) return plan;
+  plan.num_direct = static_cast<int>(items - tail);
+  plan.split_len = len;
+  plan.parts = tail * ((blocks + len - 1) / len);
+  return plan;
+}
+template <int kHeadDim, int kQTiles>
+size_t split_bytes(const SplitPlan& plan) {
+  return static_cast<size_t>(plan.parts) * kQTiles * kBlockQ * (kHeadDim + 2) * sizeof(float);
 }
 
 // Work list for a causal launch.  Items are taken in an order made for L2 — the (batch, head)
@@ -1000,7 +1174,7 @@ bool build_schedule(const KernelArgs& a, int grid, Schedule* out) {
 }
 
 template <int kHeadDim, int kQTiles, int kPolyOf4, bool kBias>
-int launch_cfg(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
+int launch_cfg(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   using C = Cfg<kHeadDim, kQTiles, kBias>;
   const CUtensorMapDataType dt = p.dtype == IXK_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   // A head / batch dimension with stride 0 (one K or V shared by all heads or batches) is encoded
@@ -1091,17 +1265,28 @@ int launch_cfg(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
   a.out_vec_ok = out_vec ? 1 : 0;
   a.out_tma = out_tma ? 1 : 0;
 
-  auto* fn = &fmha_prefill_kernel<kHeadDim, kQTiles, kPolyOf4, kBias>;
+  auto* whole_kernel = &fmha_prefill_kernel<kHeadDim, kQTiles, kPolyOf4, kBias, false>;
+  auto* split_kernel = &fmha_prefill_kernel<kHeadDim, kQTiles, kPolyOf4, kBias, kPolyOf4 == 0>;   // (the tuning variants never split)
   static thread_local int configured_device = -1;
   if (configured_device != dev.device) {
-    IXK_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+    IXK_CUDA_OK(cudaFuncSetAttribute(whole_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+    IXK_CUDA_OK(cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
     configured_device = dev.device;
   }
   const int rows_per_item = kBlockQ * kQTiles;
   a.num_qblocks = (p.F + rows_per_item - 1) / rows_per_item;
   const int64_t items = static_cast<int64_t>(a.num_qblocks) * p.N * p.B;
   if (items > 0x7fffffff) return fail(IXK_UNIMPLEMENTED, "too many (batch, head, query block) work items");
-  a.num_items = static_cast<int>(items);
+  const int base_items = static_cast<int>(items);
+  SplitPlan split = split_plan<kQTiles>(a, items, dev.sm_count);
+  if (kPolyOf4 != 0 || workspace == nullptr || workspace_bytes < split_bytes<kHeadDim, kQTiles>(split) ||
+      (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0)
+    split.parts = 0;
+  a.num_direct = split.parts > 0 ? split.num_direct : base_items;
+  a.split_len = split.split_len;
+  a.num_items = a.num_direct + split.parts;
+  a.part_o = static_cast<float*>(workspace);
+  a.part_stat = reinterpret_cast<float2*>(a.part_o + static_cast<size_t>(split.parts) * kQTiles * kBlockQ * kHeadDim);
   int grid = a.num_items < dev.sm_count ? a.num_items : dev.sm_count;
   // (5 KB: kept off the stack.  The list depends on the shape only, so a thread that launches the
   // same problem again, as a layer or a benchmark loop does, reuses the one it has.)
@@ -1109,15 +1294,42 @@ int launch_cfg(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
   static thread_local int sched_key[6] = {-1, -1, -1, -1, -1, -1};
   static thread_local bool sched_ok = false;
   const int key[6] = {a.B, a.N, a.F, a.T, a.causal, grid};
-  if (!std::equal(key, key + 6, sched_key)) {
+  if (split.parts == 0 && !std::equal(key, key + 6, sched_key)) {
     sched_ok = build_schedule<kQTiles>(a, grid, &sched);
     std::copy(key, key + 6, sched_key);
   }
-  a.use_schedule = sched_ok ? 1 : 0;
-  fn<<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, tbias, to, a, sched);
+  a.use_schedule = split.parts == 0 && sched_ok ? 1 : 0;
+  (split.parts > 0 ? split_kernel : whole_kernel)<<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, tbias, to, a, sched);
   IXK_CUDA_OK(cudaGetLastError());
   count_launch();
+  if (split.parts > 0) {
+    const int64_t rows = static_cast<int64_t>(base_items - a.num_direct) * rows_per_item;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>((rows + 7) / 8), 1, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    IXK_CUDA_OK(cudaLaunchKernelEx(&cfg, &fmha_prefill_combine_kernel<kHeadDim, kQTiles>, a, static_cast<int>(a.num_direct), base_items));
+    count_launch();
+  }
   return IXK_OK;
+}
+
+template <int kHeadDim, int kQTiles>
+size_t split_bytes_for(const Problem& p, int sms) {
+  KernelArgs a{};
+  a.B = p.B;
+  a.N = p.N;
+  a.F = p.F;
+  a.T = p.T;
+  a.causal = p.causal ? 1 : 0;
+  a.num_qblocks = (p.F + kBlockQ * kQTiles - 1) / (kBlockQ * kQTiles);
+  const int64_t items = static_cast<int64_t>(a.num_qblocks) * p.N * p.B;
+  return items > 0x7fffffff ? 0 : split_bytes<kHeadDim, kQTiles>(split_plan<kQTiles>(a, items, sms));
 }
 
 }  // namespace
@@ -1132,30 +1344,38 @@ bool bias_fits_tma(const Problem& p) {
 }
 
 template <int kHeadDim, int kQTiles, int kPolyOf4>
-int launch_bias(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
-  if (bias_fits_tma(p)) return launch_cfg<kHeadDim, kQTiles, kPolyOf4, true>(p, dev, stream);
-  return launch_cfg<kHeadDim, kQTiles, kPolyOf4, false>(p, dev, stream);
+int launch_bias(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  if (bias_fits_tma(p)) return launch_cfg<kHeadDim, kQTiles, kPolyOf4, true>(p, dev, workspace, workspace_bytes, stream);
+  return launch_cfg<kHeadDim, kQTiles, kPolyOf4, false>(p, dev, workspace, workspace_bytes, stream);
 }
 
-int launch_prefill(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
+// Scratch a launch can make use of (none is needed: without it no item is split).
+size_t prefill_workspace_bytes(const Problem& p, int sms) {
+  if (p.H <= 64) return p.F > kBlockQ ? split_bytes_for<64, 2>(p, sms) : split_bytes_for<64, 1>(p, sms);
+  if (p.H <= 128) return p.F > kBlockQ ? split_bytes_for<128, 2>(p, sms) : split_bytes_for<128, 1>(p, sms);
+  return split_bytes_for<256, 1>(p, sms);
+}
+
+int launch_prefill(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   // Head-size buckets follow the reference's policy pick (fmha_forward.h:621-646): <=64, <=128, <=256.
   constexpr int kPoly = 0;  // pairs of every four whose 2^x runs on the FMA pipe instead of the special-function unit
-  if (p.H <= 64) return p.F > kBlockQ ? launch_bias<64, 2, kPoly>(p, dev, stream) : launch_bias<64, 1, kPoly>(p, dev, stream);
+  if (p.H <= 64)
+    return p.F > kBlockQ ? launch_bias<64, 2, kPoly>(p, dev, workspace, workspace_bytes, stream)
+                         : launch_bias<64, 1, kPoly>(p, dev, workspace, workspace_bytes, stream);
   if (p.H <= 128) {
-    if (p.F <= kBlockQ) return launch_bias<128, 1, kPoly>(p, dev, stream);
+    if (p.F <= kBlockQ) return launch_bias<128, 1, kPoly>(p, dev, workspace, workspace_bytes, stream);
     // Tuning override for the main configuration: IXK_FMHA_POLY = 0..2.
     if (const char* env = std::getenv("IXK_FMHA_POLY")) {
       switch (std::atoi(env)) {
-        case 1: return launch_cfg<128, 2, 1, false>(p, dev, stream);
-        case 2: return launch_cfg<128, 2, 2, false>(p, dev, stream);
+        case 1: return launch_cfg<128, 2, 1, false>(p, dev, workspace, workspace_bytes, stream);
+        case 2: return launch_cfg<128, 2, 2, false>(p, dev, workspace, workspace_bytes, stream);
         default: break;
       }
     }
-    return launch_bias<128, 2, kPoly>(p, dev, stream);
+    return launch_bias<128, 2, kPoly>(p, dev, workspace, workspace_bytes, stream);
   }
-  return launch_bias<256, 1, kPoly>(p, dev, stream);
+  return launch_bias<256, 1, kPoly>(p, dev, workspace, workspace_bytes, stream);
 }
 
 }  // namespace fmha
 }  // namespace ixk
-

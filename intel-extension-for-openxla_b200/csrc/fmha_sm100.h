@@ -29,7 +29,10 @@ struct Problem {
 constexpr int kDecodeMaxQueries = 16;
 
 // ---- tcgen05 prefill kernel (fmha_prefill_sm100.cu)
-int launch_prefill(const Problem& p, const DeviceInfo& dev, cudaStream_t stream);
+// Scratch it can make use of (partial results where a problem is split along the keys); a call with less
+// runs unsplit.
+size_t prefill_workspace_bytes(const Problem& p, int sm_count);
+int launch_prefill(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 
 // ---- split-key decode kernel (fmha_decode_sm100.cu)
 // Number of key splits chosen for a problem, and the scratch it needs:

@@ -11,7 +11,8 @@
 // is a fixed array that lives in the library's device image: every GPU that loads libixk.so
 // carries IXK_STATIC_SCRATCH_BYTES of it until the process exits.  The entry point forwards to
 // the ordinary ixk_fmha_fwd with that array as the workspace, so results are identical to a
-// call that passes its own workspace.
+// call that passes its own workspace of that size.  (Calls that only profit from scratch, such as
+// a prefill that is split along the keys, run without it: they share nothing with each other.)
 #include <mutex>
 
 #include "host_common.h"
@@ -62,7 +63,7 @@ int ixk_fmha_fwd_static_scratch(const ixk_fmha_desc* desc, const void* q, const 
   IXK_API_RANGE("ixk_fmha_fwd_static_scratch");
   ixk::clear_error();
   if (desc == nullptr) return ixk::fail(IXK_INVALID_ARGUMENT, "desc is NULL");
-  const size_t need = ixk_fmha_fwd_workspace_bytes(desc);
+  const size_t need = ixk::fmha_required_workspace_bytes(desc);
   if (need > kScratchBytes)
     return ixk::fail(IXK_WORKSPACE_TOO_SMALL,
                      "this problem needs " + std::to_string(need) + " bytes of scratch but the built-in scratch holds " +

@@ -64,6 +64,8 @@ struct TmapSpec {
 };
 int encode_tmap(CUtensorMap* out, const void* base, const TmapSpec& spec);
 
+size_t fmha_required_workspace_bytes(const ixk_fmha_desc* desc);
+
 namespace comm {
 // Where a rank's scattered output goes: dest[o] = slot `rank` of the `world` slots ([rows / world]
 // rows of row_bytes each) that start at slots_offset in rank o's exchange buffer.  Checks that the

@@ -326,3 +326,52 @@ def test_decode_several_rows_infinite_values(pkg, cuda):
     assert torch.all(torch.isposinf(o[..., 7]))
     o[..., 7] = 0
     assert torch.all(torch.isfinite(o))
+
+
+# Prefill split along the keys (fmha_prefill_combine_kernel): a launch whose last round, or whose only
+# round, leaves CTAs without an item.
+SPLIT_CASES = [
+    # B, N, F, T, H, dtype, causal, bias, layout
+    (1, 2, 300, 1100, 128, "bf16", False, False, "bsnh"),     # a ragged second tile, a short last part
+    (1, 3, 128, 1000, 64, "fp16", False, True, "bnsh"),       # one tile per item, bias through TMA
+    (2, 1, 257, 900, 256, "bf16", False, False, "bnsh"),      # last item of one row
+    (19, 8, 200, 1500, 64, "bf16", False, False, "bsnh"),      # whole items in a full round, four split ones behind it
+    (1, 2, 1300, 1300, 128, "bf16", True, False, "bsnh"),     # causal: parts with work for the second tile only
+    (1, 1, 2049, 2049, 40, "fp16", True, False, "bnsh"),
+    (1, 2, 700, 1900, 256, "bf16", True, True, "bnsh"),       # more keys than queries; bias and mask
+    (1, 1, 1500, 900, 96, "bf16", True, False, "bnsh"),       # fewer keys than queries
+]
+
+
+@pytest.mark.parametrize("case", SPLIT_CASES, ids=lambda c: "B{}N{}F{}T{}H{}{}c{}b{}{}".format(*c))
+def test_prefill_split_along_the_keys(pkg, orc, cuda, case):
+    import ctypes
+    B, N, F, T, H, dt, causal, use_bias, layout = case
+    dtype = torch.bfloat16 if dt == "bf16" else torch.float16
+    g = torch.Generator().manual_seed(F + H)
+
+    def heads(S):
+        t = torch.randn((B, S, N, H) if layout == "bsnh" else (B, N, S, H), generator=g).to(dtype).to(cuda)
+        return t.permute(0, 2, 1, 3) if layout == "bsnh" else t
+    q, k, v = heads(F), heads(T), heads(T)
+    bias = None
+    if use_bias:
+        bias = torch.randn(B, 1, F, (T + 7) // 8 * 8, generator=g).to(dtype).to(cuda)[..., :T]
+        bias[..., : T // 3] = torch.finfo(dtype).min        # whole parts masked by the type's lowest value
+        bias[:, :, 5, 1:] = float("-inf")                   # a row with one key left, at the type's lowest value
+    launches = pkg.launch_count()
+    o, lse = run(pkg, q, k, v, bias, causal, lse=True)
+    assert pkg.launch_count() - launches == 2               # the split is taken
+    d = pkg._fmha_desc(q, k, v, bias, o, H ** -0.5, causal, 0.0)
+    o1, lse1 = torch.empty_like(o), torch.empty_like(lse)   # the same call without scratch runs unsplit
+    assert pkg.load_library().ixk_fmha_fwd(ctypes.byref(d), q.data_ptr(), k.data_ptr(), v.data_ptr(),
+                                           None if bias is None else bias.data_ptr(), o1.data_ptr(), lse1.data_ptr(), None, 0,
+                                           torch.cuda.current_stream().cuda_stream) == pkg.IXK_OK
+    assert pkg.launch_count() - launches == 3
+    want, want_lse = orc.fmha_forward(f32(q), f32(k), f32(v), None if bias is None else f32(bias), head_scale=H ** -0.5,
+                                      causal=causal, dtype=orc.BF16 if dt == "bf16" else orc.F16, round_p=False)
+    # (rows that see nothing but the type's lowest value overflow to -inf in base 2 and have no result)
+    keep = np.isfinite(want_lse) & (want_lse > -1e4)
+    for got, got_lse in ((o, lse), (o1, lse1)):
+        orc.check_close(f32(got)[keep], want[keep], rtol=2e-2, atol=2e-2 if dtype == torch.bfloat16 else 5e-3, what=str(case))
+        orc.check_close(f32(got_lse)[keep], want_lse[keep], rtol=2e-3, atol=2e-3, what=f"lse {case}")
