@@ -42,6 +42,17 @@ constexpr size_t kGroupBudget = static_cast<size_t>(192) << 20;   // scratch per
 // The gradient tiles of a group are dealt to this many launches of wide_grads_kernel that run side by
 // side (see launch_bwd_wide).
 constexpr int kGradSlices = 6;
+constexpr int kHeadChunk = 4;      // heads whose gradient tiles are sorted together
+
+// Where a block of 256 query rows lies in a plane.  Unfolded: at its own rows.  Under a causal mask block
+// qb has keys in its first 256 (qb + 1) columns only, so blocks qb and nq - 1 - qb can share one band of
+// 256 rows and 256 (nq + 1) columns, which nearly halves the plane.
+struct Fold {
+  int on, nq;
+  __host__ __device__ __forceinline__ bool second(int qb) const { return on != 0 && qb >= (nq + 1) / 2; }
+  __host__ __device__ __forceinline__ int band(int qb) const { return second(qb) ? nq - 1 - qb : qb; }
+  __host__ __device__ __forceinline__ int column(int qb) const { return second(qb) ? kRowBlock * (nq - qb) : 0; }
+};
 
 // wait sites reported in the device status word
 enum : int { kSiteScoreQ = 0x51, kSiteScoreKv = 0x52, kSiteScoreAcc = 0x53, kSiteScoreFull = 0x54, kSiteScoreOut = 0x55,
@@ -105,6 +116,7 @@ struct ScoreArgs {
   int total_tiles;
   int slabs;                   // ceil(H / 64)
   int causal;
+  Fold fold;
   uint32_t idesc;
   float scale_log2;
   const float* neg_lse2;
@@ -304,6 +316,8 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     for (int t = t_begin; t < t_end && alive;) {
       const Run run = run_at(args, t, t_end);
       const int bn = args.bn0 + run.head;
+      const int2 plane = make_int2(args.fold.column(run.qb),
+                                   args.fold.band(run.qb) * kRowBlock + static_cast<int>(rank) * 128 + quarter * 32);
       const int warp_row = run.qb * kRowBlock + static_cast<int>(rank) * 128 + quarter * 32;
       const int f = warp_row + lane;
       const bool row_ok = f < args.F;
@@ -365,7 +379,7 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
           }
         };
-        const bool stored = warp_row < args.F && key0 < args.T;      // (warp-uniform) the box meets the plane
+        const bool stored = args.fold.on || (warp_row < args.F && key0 < args.T);   // (warp-uniform) the box meets the plane
         const bool masked = key0 + 64 > args.T || (args.causal && key0 + 63 > warp_row);
         if (masked) make_p(std::true_type{}); else make_p(std::false_type{});
         // the box holds the previous tile's dS until its store has read it
@@ -384,8 +398,8 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         ptx::fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && stored) {
-          ptx::tma_store_3d(&tmap_p, box, key0, warp_row, run.head);
+        if (lane == 0) {
+          if (stored) ptx::tma_store_3d(&tmap_p, box, key0 + plane.x, plane.y, run.head);
           ptx::bulk_commit_group();
         }
         ptx::tmem_ld_32x32(acc + 128 + 32, dp[1]);
@@ -413,8 +427,8 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         stage_half_row(box, lane, 1, w[1]);
         ptx::fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && stored) {
-          ptx::tma_store_3d(&tmap_ds, box, key0, warp_row, run.head);
+        if (lane == 0) {
+          if (stored) ptx::tma_store_3d(&tmap_ds, box, key0 + plane.x, plane.y, run.head);
           ptx::bulk_commit_group();
         }
       }
@@ -456,6 +470,8 @@ struct GradArgs {
   int nq, nk2, ranks;          // 256-row blocks of queries / keys, and the larger of the two
   int f_lim, t_lim;            // F and T rounded up to a slab
   int causal;
+  Fold fold;
+  int chunk;                   // heads whose tiles are sorted together
   int slice, num_slices;       // this launch takes tiles slice, slice + num_slices, ...
   int wait_first;              // the first slice of a group waits for the scores, the others follow it
   uint32_t idesc_t, idesc_n;   // A with its rows contiguous (dV, dK) / with K contiguous (dQ)
@@ -475,11 +491,14 @@ struct GradTile {
 };
 __device__ __forceinline__ GradTile grad_tile(const GradArgs& a, int u) {
   GradTile g;
-  const int per_rank = 3 * a.heads;
-  const int rank = u / per_rank;
-  const int rest = u - rank * per_rank;
-  g.product = rest / a.heads;
-  g.head = rest - g.product * a.heads;
+  const int chunk = u / (3 * a.chunk * a.ranks);
+  const int chunk_heads = min(a.chunk, a.heads - chunk * a.chunk);
+  const int per_rank = 3 * chunk_heads;
+  const int in_chunk = u - chunk * (3 * a.chunk * a.ranks);
+  const int rank = in_chunk / per_rank;
+  const int rest = in_chunk - rank * per_rank;
+  g.product = rest / chunk_heads;
+  g.head = a.heads - 1 - chunk * a.chunk - (rest - g.product * chunk_heads);   // the scores written last are read first
   if (g.product == kProductDq) {
     g.block = a.nq - 1 - rank;            // the last query block meets the most keys
     g.k0 = 0;
@@ -580,11 +599,15 @@ wide_grads_kernel(const __grid_constant__ GradMaps maps, const __grid_constant__
         const int k = g.k0 + s * 64;
         if (ptx::elect_one()) {
           if (rank == 0) ptx::mbar_expect_tx(full_bar(st), 2 * C::kStageBytes);
+          const int qb = g.product == kProductDq ? g.block : k / kRowBlock;
+          const int x0 = args.fold.column(qb);
+          const int y0 = args.fold.band(qb) * kRowBlock;
           if (g.product == kProductDq) {
-            ptx::tma_load_3d_pair(a_dst, ma, bar, k, m0, g.head);
+            ptx::tma_load_3d_pair(a_dst, ma, bar, x0 + k, y0 + static_cast<int>(rank) * 128, g.head);
           } else {
-            ptx::tma_load_3d_pair(a_dst, ma, bar, m0, k, g.head);
-            ptx::tma_load_3d_pair(a_dst + kHalfBox, ma, bar, m0 + 64, k, g.head);
+            const int y = y0 + k % kRowBlock;
+            ptx::tma_load_3d_pair(a_dst, ma, bar, x0 + m0, y, g.head);
+            ptx::tma_load_3d_pair(a_dst + kHalfBox, ma, bar, x0 + m0 + 64, y, g.head);
           }
           ptx::tma_load_4d_pair(b_dst, mb, bar, static_cast<int>(rank) * 128, k, n, b);
           ptx::tma_load_4d_pair(b_dst + kHalfBox, mb, bar, static_cast<int>(rank) * 128 + 64, k, n, b);
@@ -724,6 +747,49 @@ int heads_per_group(const Problem& p) {
   return static_cast<int>(std::min<size_t>(std::max<size_t>(kGroupBudget / per_head, 1), static_cast<size_t>(std::max(p.N, 1))));
 }
 
+size_t scratch_bytes(const Problem& p) {
+  const size_t scores = static_cast<size_t>(heads_per_group(p)) * p.F * plane_pitch(p.T);
+  return (scores * 4 + 255) / 256 * 256 + (scores * 2 + 255) / 256 * 256;
+}
+
+struct Plan {
+  int group;          // heads of a group
+  int slices;         // launches of the gradient kernel per group
+  int chunk;
+  Fold fold;
+  int64_t rows, keys; // extents of a plane: stores are clipped there, loads read zeros beyond
+};
+Plan make_plan(const Problem& p, int pairs) {
+  Plan plan{};
+  plan.rows = p.F;
+  plan.keys = plane_pitch(p.T);
+  plan.group = heads_per_group(p);
+  plan.slices = kGradSlices;
+  plan.chunk = plan.group;
+  const int nq = (p.F + kRowBlock - 1) / kRowBlock, nk2 = (p.T + kRowBlock - 1) / kRowBlock;
+  plan.fold = Fold{0, nq};
+  const int64_t tiles = static_cast<int64_t>(3) * std::max(nq, nk2) * plan.group;
+  if (p.B == 1 || tiles <= pairs) return plan;
+  // Several batch elements, each with more gradient tiles than SM pairs: one launch of each kernel per
+  // group, the planes folded where that makes them smaller, and groups as large as the scratch holds, over
+  // batches as well as heads.  Every group costs about 18 us beside its work (ramp-up and the last round
+  // of both kernels).  (A single batch element keeps the groups and the seven launches of each that
+  // ixk_launch_count has always shown for it.)
+  plan.slices = 1;
+  const int64_t folded_rows = static_cast<int64_t>(kRowBlock) * ((nq + 1) / 2), folded_keys = static_cast<int64_t>(kRowBlock) * (nq + 1);
+  if (p.causal && folded_rows * folded_keys < plan.rows * plan.keys) {
+    plan.fold.on = 1;
+    plan.rows = folded_rows;
+    plan.keys = folded_keys;
+  }
+  const int64_t heads = static_cast<int64_t>(p.B) * p.N;
+  const int64_t fit = std::min<int64_t>(static_cast<int64_t>(scratch_bytes(p)) / (plan.rows * plan.keys * 4), heads);
+  const int64_t groups = (heads + fit - 1) / fit;
+  plan.group = static_cast<int>((heads + groups - 1) / groups);       // groups of (almost) one size
+  plan.chunk = std::min(plan.group, kHeadChunk);
+  return plan;
+}
+
 template <typename Kernel, typename... Args>
 int launch_pairs(Kernel* fn, int pairs, int threads, int smem, bool overlap, cudaStream_t stream, const Args&... kargs) {
   cudaLaunchConfig_t cfg = {};
@@ -750,8 +816,10 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
                  void* scratch, cudaStream_t stream) {
   const Problem& p = bp.fwd;
   const CUtensorMapDataType dt = kBf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  const int group = heads_per_group(p);
-  const int64_t rows = p.F, keys = plane_pitch(p.T);   // stores are clipped there, loads read zeros beyond
+  const int all_pairs = std::max(dev.sm_count / 2, 1);
+  const Plan plan = make_plan(p, all_pairs);
+  const int group = plan.group;
+  const int64_t rows = plan.rows, keys = plan.keys;
   uint16_t* plane_p = static_cast<uint16_t*>(scratch);
   uint16_t* plane_ds = plane_p + static_cast<int64_t>(group) * rows * keys;
 
@@ -820,6 +888,7 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
   sa.nk = (p.T + kKeyTile - 1) / kKeyTile;
   sa.slabs = (p.H + 63) / 64;
   sa.causal = p.causal ? 1 : 0;
+  sa.fold = plan.fold;
   sa.tiles_per_head = 0;
   for (int qb = 0; qb < sa.nq; ++qb) sa.tiles_per_head += p.causal ? std::min(sa.nk, 2 * qb + 2) : sa.nk;
   sa.idesc = ptx::umma_idesc(fmt, fmt, 0, 0, 2 * 128, kKeyTile);
@@ -842,7 +911,9 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
   ga.f_lim = (p.F + 63) / 64 * 64;
   ga.t_lim = (p.T + 63) / 64 * 64;
   ga.causal = sa.causal;
-  ga.num_slices = kGradSlices;
+  ga.fold = plan.fold;
+  ga.chunk = plan.chunk;
+  ga.num_slices = plan.slices;
   ga.idesc_t = ptx::umma_idesc(fmt, fmt, 1, 1, 2 * 128, 256);
   ga.idesc_n = ptx::umma_idesc(fmt, fmt, 0, 1, 2 * 128, 256);
   ga.head_scale = p.head_scale;
@@ -857,30 +928,30 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
     IXK_CUDA_OK(cudaFuncSetAttribute(grads, cudaFuncAttributeMaxDynamicSharedMemorySize, GradCfg::kSmemBytes));
     configured_device = dev.device;
   }
-  const int all_pairs = std::max(dev.sm_count / 2, 1);
-  const int slice_pairs = std::max(all_pairs / kGradSlices, 1);
+  const int slice_pairs = std::max(all_pairs / plan.slices, 1);
   bool first = true;
-  for (int b = 0; b < p.B; ++b) {
-    for (int n0 = 0; n0 < p.N; n0 += group) {
-      const int g = std::min(group, p.N - n0);
-      sa.bn0 = ga.bn0 = b * p.N + n0;
-      sa.heads = ga.heads = g;
-      const int64_t total = static_cast<int64_t>(sa.tiles_per_head) * g;
-      if (total > 0x7fffffff) return fail(IXK_UNIMPLEMENTED, "too many score tiles");
-      sa.total_tiles = static_cast<int>(total);
-      const int score_pairs = static_cast<int>(std::min<int64_t>(total, all_pairs));
-      if ((rc = launch_pairs(scores, score_pairs, ScoreCfg::kThreads, ScoreCfg::kSmemBytes, !first, stream, tq, tdo, tk, tv, tp, tds,
-                             sa)) != IXK_OK)
+  const int heads_all = p.B * p.N;
+  for (int bn0 = 0; bn0 < heads_all;) {
+    // a sliced group stays within one batch
+    const int g = std::min(group, plan.slices > 1 ? p.N - bn0 % p.N : heads_all - bn0);
+    sa.bn0 = ga.bn0 = bn0;
+    sa.heads = ga.heads = g;
+    bn0 += g;
+    const int64_t total = static_cast<int64_t>(sa.tiles_per_head) * g;
+    if (total > 0x7fffffff) return fail(IXK_UNIMPLEMENTED, "too many score tiles");
+    sa.total_tiles = static_cast<int>(total);
+    const int score_pairs = static_cast<int>(std::min<int64_t>(total, all_pairs));
+    if ((rc = launch_pairs(scores, score_pairs, ScoreCfg::kThreads, ScoreCfg::kSmemBytes, !first, stream, tq, tdo, tk, tv, tp, tds,
+                           sa)) != IXK_OK)
+      return rc;
+    first = false;
+    for (int slice = 0; slice < plan.slices; ++slice) {
+      ga.slice = slice;
+      ga.wait_first = slice == 0 ? 1 : 0;
+      const int tiles = (3 * g * ga.ranks - slice + plan.slices - 1) / plan.slices;
+      if ((rc = launch_pairs(grads, std::max(std::min(tiles, slice_pairs), 1), GradCfg::kThreads, GradCfg::kSmemBytes, true, stream, gm,
+                             ga)) != IXK_OK)
         return rc;
-      first = false;
-      for (int slice = 0; slice < kGradSlices; ++slice) {
-        ga.slice = slice;
-        ga.wait_first = slice == 0 ? 1 : 0;
-        const int tiles = (3 * g * ga.ranks - slice + kGradSlices - 1) / kGradSlices;
-        if ((rc = launch_pairs(grads, std::max(std::min(tiles, slice_pairs), 1), GradCfg::kThreads, GradCfg::kSmemBytes, true, stream, gm,
-                               ga)) != IXK_OK)
-          return rc;
-      }
     }
   }
   return IXK_OK;
@@ -889,8 +960,7 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
 }  // namespace
 
 size_t bwd_wide_scratch_bytes(const Problem& p) {
-  const size_t scores = static_cast<size_t>(heads_per_group(p)) * p.F * plane_pitch(p.T);
-  return (scores * 4 + 255) / 256 * 256 + (scores * 2 + 255) / 256 * 256;
+  return scratch_bytes(p);
 }
 
 // Per group of heads: one launch of the score kernel over all SM pairs, then the gradient tiles dealt

@@ -180,3 +180,16 @@ def test_full_size_against_fp32_autograd(pkg, cuda, causal):
             rel = ((got - want).norm() / want.norm()).item()
             assert rel < 1e-2, f"{name}[{b},{n}]: relative error {rel:.3e}"
             assert torch.allclose(got, want, rtol=2e-2, atol=2e-2), name
+
+
+@pytest.mark.parametrize("case", [
+    # more gradient tiles than SM pairs: two launches per group, groups of heads over batches
+    dict(B=2, N=8, F=900, T=900, H=256, causal=True, launches_expected=5),      # folded planes, even number of query blocks
+    dict(B=2, N=5, F=1200, T=1200, H=192, causal=True, launches_expected=5),    # odd number
+    dict(B=2, N=5, F=700, T=1100, H=256, causal=True, launches_expected=3),     # more keys than queries
+    dict(B=2, N=13, F=640, T=300, H=136, causal=True, launches_expected=5),     # fewer keys than queries: not folded
+    dict(B=2, N=9, F=300, T=700, H=192, launches_expected=5),                   # no mask, a group ends inside a batch
+    dict(B=2, N=7, F=1000, T=1000, H=160, causal=True, dtype=torch.float16, seq_major=True, launches_expected=3),
+], ids=lambda c: "B{B}N{N}F{F}T{T}H{H}".format(**c))
+def test_heads_wider_than_128_many_tiles(pkg, orc, cuda, case):
+    run_case(pkg, orc, cuda, seed=case["F"], **case)
