@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 from typing import Optional
 
 import torch
@@ -80,6 +81,10 @@ class _FmhaBwdDesc(ctypes.Structure):
     _fields_ = [("fwd", _FmhaDesc), ("do_strides", ctypes.c_int64 * 3), ("dq_strides", ctypes.c_int64 * 3),
                 ("dk_strides", ctypes.c_int64 * 3), ("dv_strides", ctypes.c_int64 * 3)]
 
+
+# the same layouts for struct, whose field order and padding they share
+_PACK_GEMM = struct.Struct("=2i4q2i4q2i4qq2f2i").pack
+_PACK_FMHA = struct.Struct("=7i2fi15q").pack
 
 _LIB: Optional[ctypes.CDLL] = None
 
@@ -187,14 +192,23 @@ def device_status() -> int:
     return word.value
 
 
+# A decode step is a dozen launches of a few microseconds, so what Python does for each call is part of
+# its time: descriptors are packed in one go, pointers and the stream travel as plain integers (the
+# current stream's handle is read without a Stream object around it).
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
+_current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
-def _stream_ptr(stream) -> ctypes.c_void_p:
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return ctypes.c_void_p(stream.cuda_stream)
+def _stream_ptr(stream) -> int:
+    if stream is not None:
+        return stream.cuda_stream
+    if _current_raw_stream is None or _current_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _current_raw_stream(_current_device())
 
 
 def _require_cuda(*tensors) -> None:
@@ -242,13 +256,15 @@ def run_gemm_custom_call(lhs: torch.Tensor, rhs: torch.Tensor, add: Optional[tor
     if epilogue not in EPILOGUES:
         raise IxkError(IXK_INVALID_ARGUMENT, "Unknown Epilogue.")  # onednn_matmul_utils.cc:52-54
     _require_cuda(lhs, rhs, add, output, bias, aux)
+    _launch_gemm(gemm_desc_from_attrs(attrs, epilogue), lhs, rhs, add, output, bias, stream, inv_scale_a, inv_scale_b, workspace, aux)
+
+
+def _launch_gemm(d: "_GemmDesc", lhs, rhs, add, output, bias, stream, inv_scale_a, inv_scale_b, workspace, aux) -> None:
     lib = load_library()
-    d = gemm_desc_from_attrs(attrs, epilogue)
     sp = _stream_ptr(stream)
-    ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
+    ws_bytes = 0 if workspace is None else workspace.nbytes
     if aux is not None:
-        order = int(attrs["output_order"])
-        aux_ld = aux.stride(-2) if order == ROW_MAJOR else aux.stride(-1)
+        aux_ld = aux.stride(-2) if d.output.order == ROW_MAJOR else aux.stride(-1)
         st = lib.ixk_gemm_aux(ctypes.byref(d), _ptr(lhs), _ptr(rhs), _ptr(add), _ptr(bias), _ptr(output), _ptr(aux),
                               int(aux_ld), sp)
     elif inv_scale_a is not None or inv_scale_b is not None:
@@ -272,23 +288,36 @@ def gemm_workspace_bytes(lhs: torch.Tensor, rhs: torch.Tensor, out_shape=None) -
     return int(load_library().ixk_gemm_workspace_bytes(ctypes.byref(d)))
 
 
-def _matrix_attrs(prefix: str, t: torch.Tensor) -> dict:
-    """Layout attributes of a 2-D or 3-D (batched) tensor view: whichever of the last two
-    dimensions has stride 1 decides the order."""
-    if t.dim() not in (2, 3):
+def _matrix_layout(prefix: str, t: torch.Tensor) -> tuple:
+    """(order, dtype, rows, cols, batch stride, leading dimension stride) of a 2-D or 3-D (batched)
+    tensor view: whichever of the last two dimensions has stride 1 decides the order."""
+    shape, strides = t.shape, t.stride()
+    if len(shape) not in (2, 3):
         raise IxkError(IXK_INVALID_ARGUMENT, f"{prefix}: expected a 2-D or 3-D tensor")
-    rows, cols = t.shape[-2], t.shape[-1]
-    sr, sc = t.stride(-2), t.stride(-1)
+    rows, cols = shape[-2], shape[-1]
+    sr, sc = strides[-2], strides[-1]
     if sc == 1 and (sr >= cols or rows == 1):
         order, ld = ROW_MAJOR, (sr if rows > 1 else max(sr, cols))
     elif sr == 1 and (sc >= rows or cols == 1):
         order, ld = COL_MAJOR, (sc if cols > 1 else max(sc, rows))
     else:
         raise IxkError(IXK_INVALID_ARGUMENT, f"{prefix}: neither of the last two dimensions is contiguous")
-    bs = t.stride(0) if t.dim() == 3 else rows * cols
+    return order, _TORCH_TO_IXK[t.dtype], rows, cols, (strides[0] if len(shape) == 3 else rows * cols), ld
+
+
+def _matrix_attrs(prefix: str, t: torch.Tensor) -> dict:
+    order, dtype, rows, cols, bs, ld = _matrix_layout(prefix, t)
     return {f"{prefix}_order": order, f"{prefix}_num_rows": rows, f"{prefix}_num_cols": cols,
-            f"{prefix}_batch_stride": bs, f"{prefix}_leading_dim_stride": ld,
-            f"{prefix}_layout_dtype": _TORCH_TO_IXK[t.dtype]}
+            f"{prefix}_batch_stride": bs, f"{prefix}_leading_dim_stride": ld, f"{prefix}_layout_dtype": dtype}
+
+
+def _gemm_desc(lhs: tuple, rhs: tuple, output: tuple, batch: int, alpha: float, beta: float, epilogue: str) -> "_GemmDesc":
+    """The descriptor of three _matrix_layout()s, as gemm_desc_from_attrs makes it of a dictionary."""
+    if epilogue not in EPILOGUES:
+        raise IxkError(IXK_INVALID_ARGUMENT, "Unknown Epilogue.")  # onednn_matmul_utils.cc:52-54
+    d = _GemmDesc.from_buffer_copy(_PACK_GEMM(*lhs, *rhs, *output, batch, 0.0, 0.0, EPILOGUES.index(epilogue), 0))
+    d.alpha, d.beta = alpha, beta      # (a value beyond fp32 becomes infinite here; struct would refuse it)
+    return d
 
 
 def gemm_attrs_for(lhs: torch.Tensor, rhs: torch.Tensor, output: torch.Tensor, beta: float = 0.0,
@@ -316,8 +345,10 @@ def gemm(lhs: torch.Tensor, rhs: torch.Tensor, *, bias: Optional[torch.Tensor] =
     if out is None:
         shape = (*lhs.shape[:-1], rhs.shape[-1])
         out = torch.empty(shape, device=lhs.device, dtype=out_dtype or lhs.dtype)
-    attrs = gemm_attrs_for(lhs, rhs, out, beta, alpha)
-    run_gemm_custom_call(lhs, rhs, c, out, bias, stream, attrs, epilogue, workspace=workspace, aux=aux)
+    d = _gemm_desc(_matrix_layout("lhs", lhs), _matrix_layout("rhs", rhs), _matrix_layout("output", out),
+                   out.shape[0] if out.dim() == 3 else 1, float(alpha), float(beta), epilogue)
+    _require_cuda(lhs, rhs, c, out, bias, aux)
+    _launch_gemm(d, lhs, rhs, c, out, bias, stream, None, None, workspace, aux)
     return out
 
 
@@ -329,13 +360,15 @@ def gemm_geglu(x: torch.Tensor, w_gate_up: torch.Tensor, *, out: Optional[torch.
     m, n2 = x.shape[-2], w_gate_up.shape[-1]
     if out is None:
         out = torch.empty((m, n2 // 2), device=x.device, dtype=x.dtype)
-    d = gemm_desc_from_attrs(gemm_attrs_for(x, w_gate_up, torch.empty((m, n2), device="meta", dtype=x.dtype)), "DEFAULT")
+    # (the product before the GeGLU: [m, n2] row-major, never stored)
+    d = _gemm_desc(_matrix_layout("lhs", x), _matrix_layout("rhs", w_gate_up), (ROW_MAJOR, _TORCH_TO_IXK[x.dtype], m, n2, m * n2, n2),
+                   1, 1.0, 0.0, "DEFAULT")
     lib = load_library()
     need = int(lib.ixk_gemm_geglu_workspace_bytes(ctypes.byref(d)))
     if workspace is None:
         workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
     _check(lib.ixk_gemm_geglu(ctypes.byref(d), _ptr(x), _ptr(w_gate_up), _ptr(out), out.stride(-2), _ptr(workspace),
-                              workspace.numel() * workspace.element_size(), _stream_ptr(stream)))
+                              workspace.nbytes, _stream_ptr(stream)))
     return out
 
 
@@ -477,37 +510,39 @@ def residual_add(x: torch.Tensor, partial: torch.Tensor, bias: Optional[torch.Te
 # ----------------------------------------------------------------------------- attention
 
 def _fmha_desc(query, key, value, bias, out, head_scale, causal, dropout_prob) -> _FmhaDesc:
-    if query.dim() != 4 or key.dim() != 4 or value.dim() != 4 or out.dim() != 4:
+    q_shape, k_shape = query.shape, key.shape
+    if len(q_shape) != 4 or len(k_shape) != 4 or value.dim() != 4 or out.dim() != 4:
         raise IxkError(IXK_INVALID_ARGUMENT, "q, k, v, out must be 4-D [B,N,S,H] views")
-    B, N, F, H = query.shape
-    T = key.shape[2]
+    B, N, F, H = q_shape
+    T = k_shape[2]
     # The descriptor carries one B, N and H for all four tensors: a K of [B,1,T,H] has to be
     # handed over as an expanded (stride-0) view, not as a smaller tensor that would be read
     # as if it had N heads.
-    if tuple(key.shape) != (B, N, T, H) or value.shape != key.shape or out.shape != query.shape:
+    if k_shape != (B, N, T, H) or value.shape != k_shape or out.shape != q_shape:
         raise IxkError(IXK_INVALID_ARGUMENT, "k and v must be [B,N,T,H] and out [B,N,F,H] with q's B, N and H "
                        "(share K/V between heads with .expand(), which gives stride 0)")
-    if not (key.dtype == value.dtype == out.dtype == query.dtype) or (bias is not None and bias.dtype != query.dtype):
+    dtype = query.dtype
+    if not (key.dtype == value.dtype == out.dtype == dtype) or (bias is not None and bias.dtype != dtype):
         raise IxkError(IXK_INVALID_ARGUMENT, "q, k, v, bias and out must have one element type")
-    d = _FmhaDesc()
-    d.dtype = _TORCH_TO_IXK[query.dtype]
-    d.causal = 1 if causal else 0
-    d.num_batches, d.num_heads, d.head_size, d.num_queries, d.num_keys = B, N, H, F, T
-    d.head_scale = float(head_scale)
-    d.dropout_prob = float(dropout_prob)
-    d.reserved = 0
-    for name, t in (("q", query), ("k", key), ("v", value), ("o", out)):
-        if t.stride(3) != 1 and t.shape[3] > 1:
+    dtype = _TORCH_TO_IXK[dtype]
+    strides = query.stride(), key.stride(), value.stride(), out.stride()
+    for name, st in zip("qkvo", strides):
+        if st[3] != 1 and H > 1:
             # xetla_gpu_fused_mha_runner.cc:114-116 CHECKs the same
             raise IxkError(IXK_INVALID_ARGUMENT, f"{name}: head_size must be the contiguous dimension")
-        getattr(d, f"{name}_strides")[:] = [t.stride(0), t.stride(1), t.stride(2)]
+    bias_strides = (0, 0, 0)
     if bias is not None:
         if bias.dim() != 4 or bias.shape[3] != T or bias.shape[2] != F:
             raise IxkError(IXK_INVALID_ARGUMENT, "bias must be [B|1, N|1, F, T]")
         if bias.stride(3) != 1:
             raise IxkError(IXK_INVALID_ARGUMENT, "bias: the key dimension must be contiguous")
-        d.bias_strides[:] = [bias.stride(0) if bias.shape[0] > 1 else 0,
-                             bias.stride(1) if bias.shape[1] > 1 else 0, bias.stride(2)]
+        bias_strides = (bias.stride(0) if bias.shape[0] > 1 else 0, bias.stride(1) if bias.shape[1] > 1 else 0, bias.stride(2))
+    qs, ks, vs, os_ = strides
+    d = _FmhaDesc.from_buffer_copy(_PACK_FMHA(dtype, 1 if causal else 0, B, N, H, F, T, 0.0, 0.0, 0, *qs[:3], *ks[:3], *vs[:3],
+                                              *os_[:3], *bias_strides))
+    d.head_scale = float(head_scale)
+    if dropout_prob:
+        d.dropout_prob = float(dropout_prob)
     return d
 
 
@@ -535,9 +570,9 @@ def fmha_forward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: t
     lib = load_library()
     d = _fmha_desc(query, key, value, bias, out, head_scale, causal, 0.0 if dropout_prob in (None, 1.0) else dropout_prob)
     need = int(lib.ixk_fmha_fwd_workspace_bytes(ctypes.byref(d)))
-    if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
+    if need and (workspace is None or workspace.nbytes < need):
         workspace = torch.empty(need, dtype=torch.uint8, device=query.device)
-    ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
+    ws_bytes = 0 if workspace is None else workspace.nbytes
     st = lib.ixk_fmha_fwd(ctypes.byref(d), _ptr(query), _ptr(key), _ptr(value), _ptr(bias), _ptr(out),
                           _ptr(activation if is_training else None), _ptr(workspace), ws_bytes, _stream_ptr(stream))
     _check(st)
@@ -580,9 +615,9 @@ def fmha_backward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: 
     lib = load_library()
     d = _fmha_bwd_desc(query, key, value, out, bias, grad_out, grad_query, grad_key, grad_value, head_scale, causal)
     need = int(lib.ixk_fmha_bwd_workspace_bytes(ctypes.byref(d)))
-    if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
+    if need and (workspace is None or workspace.nbytes < need):
         workspace = torch.empty(need, dtype=torch.uint8, device=query.device)
-    ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
+    ws_bytes = 0 if workspace is None else workspace.nbytes
     st = lib.ixk_fmha_bwd(ctypes.byref(d), _ptr(query), _ptr(key), _ptr(value), _ptr(out), _ptr(bias), _ptr(grad_out),
                           _ptr(activation), _ptr(grad_query), _ptr(grad_key), _ptr(grad_value), _ptr(workspace),
                           ws_bytes, _stream_ptr(stream))

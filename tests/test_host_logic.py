@@ -65,3 +65,18 @@ def test_quantize_fp8_matches_oracle(pkg, orc):
         codes, s2 = orc.quantize_fp8(x.numpy(), odt)
         assert s == pytest.approx(s2)
         assert np.array_equal(q.view(torch.uint8).numpy(), codes)
+
+
+@pytest.mark.parametrize("shape", [(5, 7, 3), (1, 64, 8), (16, 1, 1), (2, 6, 24, 40)], ids=str)
+@pytest.mark.parametrize("layout", ["rr", "rc", "cr"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float8_e4m3fn])
+def test_packed_gemm_descriptor(pkg, shape, layout, dtype):
+    """gemm() packs its descriptor in one go: field for field what the attribute dictionary gives."""
+    *batch, m, k, n = shape
+    lhs = torch.empty(*batch, m, k).to(dtype) if layout[0] == "r" else torch.empty(*batch, k, m).to(dtype).transpose(-1, -2)
+    rhs = torch.empty(*batch, k, n).to(dtype) if layout[1] == "r" else torch.empty(*batch, n, k).to(dtype).transpose(-1, -2)
+    out = torch.empty(*batch, m, n + 8, dtype=torch.float32)[..., :n]
+    want = pkg.gemm_desc_from_attrs(pkg.gemm_attrs_for(lhs, rhs, out, beta=0.5, alpha=2.0), "BIAS_GELU")
+    got = pkg._gemm_desc(*(pkg._matrix_layout(name, t) for name, t in (("lhs", lhs), ("rhs", rhs), ("output", out))),
+                         out.shape[0] if out.dim() == 3 else 1, 2.0, 0.5, "BIAS_GELU")
+    assert bytes(got) == bytes(want)
