@@ -193,11 +193,11 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
 }
 
 // One tile's epilogue for the calling warp (TMEM lanes [32 quarter, 32 quarter + 32) of the
-// accumulator at tmem_acc): scale, bias, residual, activation, one rounding, store.
+// accumulator at tmem_acc, `width` columns that start at column n_first of D): scale, bias, residual, activation, one rounding, store.
 template <int kBlockN>
 __device__ __forceinline__ void epilogue_tile(const KernelArgs& args, const CUtensorMap* tmap_d_ptr, uint32_t tmem_acc,
-                                              uint32_t stage_smem, int bz, int bm, int bn, int quarter, int lane,
-                                              uint32_t& n_store, int d_row_shift = 0) {
+                                              uint32_t stage_smem, int bz, int bm, int n_first, int quarter, int lane,
+                                              uint32_t& n_store, int width = kBlockN, int d_row_shift = 0) {
   const CUtensorMap& tmap_d = *tmap_d_ptr;
   if (bm * kBlockM >= args.M) return;  // a CTA pair's second half past the last row block
   const int row_in_tile = quarter * 32 + lane;
@@ -251,8 +251,8 @@ __device__ __forceinline__ void epilogue_tile(const KernelArgs& args, const CUte
       // 32 different lines each; those requests queue in front of the producer's and the
       // issuer's barrier traffic and cost 8-11 % of the kernel.
 #pragma unroll 1
-      for (int c0 = 0; c0 < kBlockN; c0 += 64) {
-        const int n = bn * kBlockN + c0;
+      for (int c0 = 0; c0 < width; c0 += 64) {
+        const int n = n_first + c0;
         if (n >= args.N) break;  // warp-uniform
         uint32_t wv[32];
 #pragma unroll
@@ -287,8 +287,8 @@ __device__ __forceinline__ void epilogue_tile(const KernelArgs& args, const CUte
       }
     } else {
 #pragma unroll 1
-      for (int c0 = 0; c0 < kBlockN; c0 += 32) {
-        const int n = bn * kBlockN + c0;
+      for (int c0 = 0; c0 < width; c0 += 32) {
+        const int n = n_first + c0;
         if (n >= args.N) break;  // warp-uniform
         const int count = min(32, args.N - n);
         float v[32];
@@ -465,7 +465,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       if (!ptx::mbar_wait(acc_full_bar(buf), acc_phase, ctl, kSiteEpilogue)) break;
       ptx::tc_fence_after_sync();
       epilogue_tile<kBlockN>(args, &tmap_d, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kBlockN, stage_smem,
-                             bz, bm, bn, quarter, lane, n_store);
+                             bz, bm, bn * kBlockN, quarter, lane, n_store);
       ptx::tc_fence_before_sync();
       ptx::mbar_arrive(acc_empty_bar(buf));
       buf ^= 1;
@@ -503,6 +503,7 @@ struct PairCfg {
   static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
   static_assert(kSmemBytes <= 232448, "shared memory budget");
 };
+constexpr int kMaxTailParts = 4;  // pieces of a tile of the last round
 enum : int { kSitePairFull = 111, kSitePairPeer = 112, kSitePairAcc = 113, kSitePairForward = 114 };
 
 // The tensor maps of D: one, or one per destination of a scattered output (rows of D dealt out
@@ -515,11 +516,11 @@ struct OutputMaps {
 template <int kKind, int kDests>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ OutputMaps<kDests> tmaps_d, const KernelArgs args) {
+                 const __grid_constant__ CUtensorMap tmap_b_tail, const __grid_constant__ OutputMaps<kDests> tmaps_d,
+                 const KernelArgs args) {
   using C = PairCfg;
   constexpr int kStages = C::kStages;
   constexpr int kBlockN = C::kBlockN;
-  constexpr int kHalfN = kBlockN / 2;
   constexpr int kElemBytes = kKind == ptx::kKindF16 ? 2 : (kKind == ptx::kKindTf32 ? 4 : 1);
   constexpr int kSlabElems = kSlabBytes / kElemBytes;
   constexpr int kUmmaK = 32 / kElemBytes;
@@ -578,21 +579,43 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   const int num_kb = (args.K + kSlabElems - 1) / kSlabElems;
   const int tiles_m2 = (args.tiles_m + 1) / 2;  // pair tiles along M
-  const int num_tiles = tiles_m2 * args.tiles_n * args.batch;
   const int pair_id = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
+  // Units of work: whole tiles, then the tiles of the last round cut into tail_parts narrower ones.
+  const int num_units = args.tail_from + (tiles_m2 * args.tiles_n * args.batch - args.tail_from) * args.tail_parts;
+  const int tail_width = kBlockN / args.tail_parts;
+  struct Unit {
+    int bz, bm2, n_first, width;
+  };
+  auto unit_at = [&](int u) {
+    Unit x;
+    int t = u, part = 0, bn;
+    x.width = kBlockN;
+    if (u >= args.tail_from) {
+      t = args.tail_from + (u - args.tail_from) / args.tail_parts;
+      part = (u - args.tail_from) % args.tail_parts;
+      x.width = tail_width;
+    }
+    tile_coords(t, tiles_m2, args.tiles_n, x.bz, x.bm2, bn);
+    x.n_first = bn * kBlockN + part * x.width;
+    return x;
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (each CTA: its A rows, its B columns)
     int stage = 0;
     uint32_t phase = 0;
     bool alive = true;
-    for (int t = pair_id; t < num_tiles && alive; t += num_pairs) {
-      int bz, bm2, bn;
-      tile_coords(t, tiles_m2, args.tiles_n, bz, bm2, bn);
-      const int m0 = (bm2 * 2 + static_cast<int>(rank)) * kBlockM;
-      const int n0 = bn * kBlockN + static_cast<int>(rank) * kHalfN;
+    for (int t = pair_id; t < num_units && alive; t += num_pairs) {
+      const Unit unit = unit_at(t);
+      const int bz = unit.bz;
+      const int m0 = (unit.bm2 * 2 + static_cast<int>(rank)) * kBlockM;
+      const int half_n = unit.width / 2;      // this CTA's columns
+      const int n0 = unit.n_first + static_cast<int>(rank) * half_n;
       const int az = args.a_broadcast ? 0 : bz;
+      const int b_boxes = (half_n + kSlabElems - 1) / kSlabElems;   // MN-major: boxes of one swizzle span of columns
+      const uint32_t stage_bytes = kATileBytes + (args.b_mn_major ? b_boxes * kSlabElems : half_n) * kSlabBytes;
+      const CUtensorMap* map_b = t < args.tail_from ? &tmap_b : &tmap_b_tail;
       for (int kb = 0; kb < num_kb; ++kb) {
         if (!ptx::mbar_wait(empty_bar(stage), phase ^ 1u, ctl, kSiteProducer)) {
           alive = false;
@@ -604,7 +627,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const uint32_t bar = ptx::map_to_cta(full_bar(stage), 0);
         const int k0 = kb * kSlabElems;
         if (ptx::elect_one()) {
-          if (rank == 0) ptx::mbar_expect_tx(full_bar(stage), 2 * C::kStageBytes);
+          if (rank == 0) ptx::mbar_expect_tx(full_bar(stage), 2 * stage_bytes);
           if (args.a_mn_major) {
 #pragma unroll
             for (int i = 0; i < kBlockM / kSlabElems; ++i)
@@ -613,11 +636,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             ptx::tma_load_3d_pair(a_dst, &tmap_a, bar, k0, m0, az);
           }
           if (args.b_mn_major) {
-#pragma unroll
-            for (int i = 0; i < kHalfN / kSlabElems; ++i)
-              ptx::tma_load_3d_pair(b_dst + i * (kSlabElems * kSlabBytes), &tmap_b, bar, n0 + i * kSlabElems, k0, bz);
+            for (int i = 0; i < b_boxes; ++i)
+              ptx::tma_load_3d_pair(b_dst + i * (kSlabElems * kSlabBytes), map_b, bar, n0 + i * kSlabElems, k0, bz);
           } else {
-            ptx::tma_load_3d_pair(b_dst, &tmap_b, bar, k0, n0, bz);
+            ptx::tma_load_3d_pair(b_dst, map_b, bar, k0, n0, bz);
           }
         }
         __syncwarp();
@@ -644,9 +666,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const bool a_sw32 = kKind == ptx::kKindTf32 && args.a_mn_major, b_sw32 = kKind == ptx::kKindTf32 && args.b_mn_major;
     const uint32_t a_sbo = a_sw32 ? 512 : 1024, b_sbo = b_sw32 ? 512 : 1024;
     const uint32_t a_type = a_sw32 ? 1 : 2, b_type = b_sw32 ? 1 : 2;
-    for (int t = pair_id; t < num_tiles && alive; t += num_pairs) {
+    for (int t = pair_id; t < num_units && alive; t += num_pairs) {
       if (!ptx::mbar_wait(acc_empty_bar(buf), acc_phase ^ 1u, ctl, kSitePairAcc)) break;
       ptx::tc_fence_after_sync();
+      const uint32_t idesc = t < args.tail_from ? args.idesc : args.idesc_tail;
       const uint32_t d_tmem = tmem_base + buf * kBlockN;
       for (int kb = 0; kb < num_kb; ++kb) {
         if (!ptx::mbar_wait(full_bar(stage), phase, ctl, kSitePairFull)) {
@@ -660,7 +683,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         for (int ks = 0; ks < kSlabElems / kUmmaK; ++ks) {
           const uint64_t da = ptx::umma_smem_desc(a_src + ks * a_kstep, a_lbo, a_sbo, a_type);
           const uint64_t db = ptx::umma_smem_desc(b_src + ks * b_kstep, b_lbo, b_sbo, b_type);
-          ptx::umma_ss_pair_elect<kKind>(d_tmem, da, db, args.idesc, (kb | ks) != 0 ? 1u : 0u);
+          ptx::umma_ss_pair_elect<kKind>(d_tmem, da, db, idesc, (kb | ks) != 0 ? 1u : 0u);
         }
         ptx::umma_commit_pair_elect(empty_bar(stage));  // both CTAs' producers may refill the slot
         if (++stage == kStages) {
@@ -679,16 +702,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     int buf = 0;
     uint32_t acc_phase = 0;
     uint32_t n_store = 0;
-    for (int t = pair_id; t < num_tiles; t += num_pairs) {
-      int bz, bm2, bn;
-      tile_coords(t, tiles_m2, args.tiles_n, bz, bm2, bn);
+    for (int t = pair_id; t < num_units; t += num_pairs) {
+      const Unit unit = unit_at(t);
       if (!ptx::mbar_wait(acc_full_bar(buf), acc_phase, ctl, kSiteEpilogue)) break;
       ptx::tc_fence_after_sync();
-      const int bm = bm2 * 2 + static_cast<int>(rank);
+      const int bm = unit.bm2 * 2 + static_cast<int>(rank);
       // scattered output: this row block's destination and the row that destination starts at
       const int dest = kDests > 1 ? (bm * kBlockM) / args.scatter_rows : 0;
       epilogue_tile<kBlockN>(args, &tmaps_d.m[dest], tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kBlockN,
-                             stage_smem, bz, bm, bn, quarter, lane, n_store, kDests > 1 ? dest * args.scatter_rows : 0);
+                             stage_smem, unit.bz, bm, unit.n_first, quarter, lane, n_store, unit.width,
+                             kDests > 1 ? dest * args.scatter_rows : 0);
       ptx::tc_fence_before_sync();
       if (rank == 0) {
         ptx::mbar_arrive(acc_empty_bar(buf));
@@ -739,8 +762,8 @@ int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& 
 }
 
 template <int kKind, int kDests>
-int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const OutputMaps<kDests>& td, const KernelArgs& args,
-                int pairs, cudaStream_t stream) {
+int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb_tail, const OutputMaps<kDests>& td,
+                const KernelArgs& args, int pairs, cudaStream_t stream) {
   auto* fn = &gemm_pair_kernel<kKind, kDests>;
   static thread_local int configured_device = -1;
   int dev = 0;
@@ -761,7 +784,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const OutputMaps<k
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  IXK_CUDA_OK(cudaLaunchKernelEx(&cfg, fn, ta, tb, td, args));
+  IXK_CUDA_OK(cudaLaunchKernelEx(&cfg, fn, ta, tb, tb_tail, td, args));
   count_launch();
   return IXK_OK;
 }
@@ -794,6 +817,11 @@ int launch(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
   bool pair = bn == 256 && tiles_m_all >= 2 && pair_tiles >= dev.sm_count / 2;
   if (const char* env = std::getenv("IXK_GEMM_PAIR")) pair = pair && std::atoi(env) != 0;
   const int b_box_rows = pair ? 128 : bn;
+  // The tiles beyond the last full round of pairs are cut into 2 or 4 narrower ones where the idle pairs
+  // can take the pieces: the round then takes about 1/2 or 1/3 of its time.
+  const int64_t pairs_all = dev.sm_count / 2;
+  const int64_t tail_tiles = pair && p.scatter_world == 0 ? pair_tiles % pairs_all : 0;
+  const int tail_parts = tail_tiles == 0 ? 1 : tail_tiles * kMaxTailParts <= pairs_all ? kMaxTailParts : tail_tiles * 2 <= pairs_all ? 2 : 1;
   if (p.scatter_world > 0) {
     // Only the kernel that large projections run on stores to several destinations, and only
     // whole row blocks of one CTA.
@@ -845,6 +873,12 @@ int launch(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
   rc = make_map(&tb, p.b, p.b_mn_major, p.N, p.ldb, p.b_batch_stride, b_box_rows, false);
   if (rc != IXK_OK) return rc;
 
+  CUtensorMap tb_tail = tb;
+  if (tail_parts > 1 && !p.b_mn_major) {
+    rc = make_map(&tb_tail, p.b, false, p.N, p.ldb, p.b_batch_stride, b_box_rows / tail_parts, false);
+    if (rc != IXK_OK) return rc;
+  }
+
   KernelArgs k{};
   k.M = static_cast<int>(p.M);
   k.N = static_cast<int>(p.N);
@@ -856,6 +890,10 @@ int launch(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
   k.b_mn_major = p.b_mn_major;
   k.idesc = ptx::umma_idesc(p.a_fmt, p.b_fmt, p.a_mn_major ? 1 : 0, p.b_mn_major ? 1 : 0, pair ? 2 * kBlockM : kBlockM, bn,
                             p.kind == ptx::kKindI8 ? 2u : 1u);
+  k.tail_from = static_cast<int>(pair_tiles - tail_tiles);
+  k.tail_parts = tail_parts;
+  k.idesc_tail = ptx::umma_idesc(p.a_fmt, p.b_fmt, p.a_mn_major ? 1 : 0, p.b_mn_major ? 1 : 0, 2 * kBlockM, PairCfg::kBlockN / tail_parts,
+                                 p.kind == ptx::kKindI8 ? 2u : 1u);
   k.bias = p.bias;
   k.c = (p.beta != 0.0f) ? p.c : nullptr;
   k.d = p.d;
@@ -925,11 +963,11 @@ int launch(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
     if (pair) {
       const int pairs = static_cast<int>(pair_tiles < dev.sm_count / 2 ? pair_tiles : dev.sm_count / 2);
       if (p.scatter_world > 0) {
-        if constexpr (kKind == ptx::kKindF16) return launch_pair<kKind, kMaxScatter>(ta, tb, td_scatter, k, pairs, stream);
+        if constexpr (kKind == ptx::kKindF16) return launch_pair<kKind, kMaxScatter>(ta, tb, tb_tail, td_scatter, k, pairs, stream);
       }
       OutputMaps<1> one;
       one.m[0] = td;
-      return launch_pair<kKind, 1>(ta, tb, one, k, pairs, stream);
+      return launch_pair<kKind, 1>(ta, tb, tb_tail, one, k, pairs, stream);
     }
     const int64_t tiles = static_cast<int64_t>(k.tiles_m) * k.tiles_n * k.batch;
     const int grid = static_cast<int>(tiles < dev.sm_count ? tiles : dev.sm_count);

@@ -52,6 +52,8 @@ struct KernelArgs {
   int tiles_m, tiles_n;
   int a_mn_major, b_mn_major;
   uint32_t idesc;
+  uint32_t idesc_tail;         // CTA-pair kernel: the narrower tiles of the last round
+  int tail_from, tail_parts;   // tiles from here on are cut into this many (1: none is)
   const void* bias;
   const void* c;
   void* d;

@@ -462,3 +462,38 @@ def test_geglu_projection_in_one_product(pkg, orc, cuda, shape):
     with pytest.raises(pkg.IxkError) as e:
         pkg.gemm_geglu(x, w, workspace=torch.empty(16, dtype=torch.uint8, device=cuda))
     assert e.value.status == pkg.IXK_WORKSPACE_TOO_SMALL
+
+
+@pytest.mark.parametrize("shape", [(3808, 208, 1200), (24016, 144, 208)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("kind", ["bf16", "e4m3", "s8", "f32"])
+@pytest.mark.parametrize("la", ["row", "col"])
+@pytest.mark.parametrize("lb", ["row", "col"])
+def test_cta_pair_last_round(pkg, cuda, monkeypatch, shape, kind, la, lb):
+    """75 and 94 tiles of 256 x 256 on 74 SM pairs: the tiles beyond the full round run as four and two
+    narrower ones, some of them past the last column.  Same products in the same order as the single-CTA
+    kernel: bit-identical."""
+    M, K, N = shape
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = torch.randn(M, K, generator=g, device=cuda)
+    w = torch.randn(K, N, generator=g, device=cuda)
+    if kind == "s8":
+        x, w = (t.mul(30).clamp(-127, 127).to(torch.int8) for t in (x, w))
+        run = lambda: pkg.gemm(as_layout(x, la), as_layout(w, lb), out_dtype=torch.int32)
+    elif kind == "e4m3":
+        x, w = (t.to(torch.float8_e4m3fn) for t in (x, w))
+        run = lambda: pkg.gemm_fp8(as_layout(x, la), as_layout(w, lb), 0.5, 2.0)
+    elif kind == "bf16":
+        x, w = x.bfloat16(), w.bfloat16()
+        b = torch.randn(N, generator=g, device=cuda).bfloat16()
+        run = lambda: pkg.gemm(as_layout(x, la), as_layout(w, lb), bias=b, epilogue="BIAS_RELU")
+    else:
+        run = lambda: pkg.gemm(as_layout(x, la), as_layout(w, lb))
+    out = run()
+    want = x.double() @ w.double()
+    if kind == "bf16":
+        want = (want + b.double()).relu()
+    # one rounding of the result (2^-9) or of tf32 operands (2 x 2^-11), measured against the rows' scale
+    tol = {"bf16": 2.0 ** -8, "e4m3": 2.0 ** -8, "s8": 0.0, "f32": 2.0 ** -9}[kind]
+    assert ((out.double() - want).abs().max() <= tol * want.abs().max()).item()
+    monkeypatch.setenv("IXK_GEMM_PAIR", "0")
+    assert torch.equal(out, run())
