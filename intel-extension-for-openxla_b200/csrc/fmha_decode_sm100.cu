@@ -67,7 +67,7 @@ __device__ __forceinline__ uint16_t from_f32(float x, bool bf16) {
 // 128-bit streaming load that does not pollute L1 (each K/V byte is used once).
 __device__ __forceinline__ uint4 ld_stream(const void* p) {
   uint4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                : "l"(p));
   return r;
@@ -85,6 +85,7 @@ fmha_decode_kernel(const DecodeArgs a) {
   __shared__ float sm_acc[kWarps][kQ][kHPad];
   __shared__ float sm_m[kWarps][kQ];
   __shared__ float sm_l[kWarps][kQ];
+  ptx::grid_dependency_sync();
 
   const bool bf16 = a.is_bf16 != 0;
   const int split = blockIdx.x % a.splits;
@@ -164,7 +165,7 @@ fmha_decode_kernel(const DecodeArgs a) {
 #pragma unroll
         for (int off = kLanesPerKey / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
         const bool seen = ok[u] && (kQ == 1 || !a.causal || t <= f0 + r);
-        if (seen && bias_row[r] != nullptr) s = fmaf(to_f32(__ldg(bias_row[r] + t), bf16), kLog2e, s);
+        if (seen && bias_row[r] != nullptr) s = fmaf(to_f32(bias_row[r][t], bf16), kLog2e, s);
         x[r][u] = seen ? s : -INFINITY;
       }
     }
@@ -260,6 +261,7 @@ fmha_decode_kernel(const DecodeArgs a) {
 
 // One CTA per (batch, head, query): merges the key splits.
 __global__ void fmha_decode_combine_kernel(const DecodeArgs a) {
+  ptx::grid_dependency_sync();
   const int64_t row = blockIdx.x;
   const int f = static_cast<int>(row % a.F);
   const int head = static_cast<int>((row / a.F) % a.N);
@@ -356,23 +358,18 @@ int launch_decode(const Problem& p, const DeviceInfo& dev, void* workspace, size
   }
   const int rows_per_cta = decode_rows_per_cta(p.F);
   dim3 grid(splits * ((p.F + rows_per_cta - 1) / rows_per_cta), p.N, p.B);
-  auto launch_lanes = [&](auto lanes_tag) {
+  auto launch_lanes = [&](auto lanes_tag) -> int {
     constexpr int kLanes = decltype(lanes_tag)::value;
-    if (rows_per_cta == 1) fmha_decode_kernel<kLanes, 1><<<grid, kThreads, 0, stream>>>(a);
-    else fmha_decode_kernel<kLanes, 2><<<grid, kThreads, 0, stream>>>(a);
+    return launch_overlapped(rows_per_cta == 1 ? fmha_decode_kernel<kLanes, 1> : fmha_decode_kernel<kLanes, 2>, grid, dim3(kThreads), 0,
+                             stream, a);
   };
-  if (p.H <= 64) launch_lanes(std::integral_constant<int, 8>{});
-  else if (p.H <= 128) launch_lanes(std::integral_constant<int, 16>{});
-  else launch_lanes(std::integral_constant<int, 32>{});
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
-  if (splits > 1) {
-    const int64_t rows = static_cast<int64_t>(p.B) * p.N * p.F;
-    fmha_decode_combine_kernel<<<static_cast<unsigned>(rows), 128, 0, stream>>>(a);
-    IXK_CUDA_OK(cudaGetLastError());
-    count_launch();
-  }
-  return IXK_OK;
+  int rc;
+  if (p.H <= 64) rc = launch_lanes(std::integral_constant<int, 8>{});
+  else if (p.H <= 128) rc = launch_lanes(std::integral_constant<int, 16>{});
+  else rc = launch_lanes(std::integral_constant<int, 32>{});
+  if (rc != IXK_OK || splits <= 1) return rc;
+  const int64_t rows = static_cast<int64_t>(p.B) * p.N * p.F;
+  return launch_overlapped(fmha_decode_combine_kernel, dim3(static_cast<unsigned>(rows)), dim3(128), 0, stream, a);
 }
 
 }  // namespace fmha

@@ -73,6 +73,7 @@ __device__ __forceinline__ float round_to(float v, int dtype) {
 // gate is activated and rounded, the up half rounded, then multiplied (the values a gate GEMM with
 // a GELU epilogue, an up GEMM and an elementwise product would have produced one after the other).
 __global__ void splitk_reduce_geglu_kernel(const ReduceArgs a) {
+  ptx::grid_dependency_sync();
   const int half = a.N / 2, h4 = half / 4;
   const int64_t plane4 = static_cast<int64_t>(a.M) * a.N / 4;
   const int64_t total = static_cast<int64_t>(a.M) * h4;
@@ -85,7 +86,7 @@ __global__ void splitk_reduce_geglu_kernel(const ReduceArgs a) {
     float4 g = make_float4(0.f, 0.f, 0.f, 0.f), u = g;
 #pragma unroll 4
     for (int s = 0; s < a.splits; ++s) {
-      const float4 gv = __ldg(gsrc + s * plane4), uv = __ldg(usrc + s * plane4);
+      const float4 gv = gsrc[s * plane4], uv = usrc[s * plane4];
       g.x += gv.x; g.y += gv.y; g.z += gv.z; g.w += gv.w;
       u.x += uv.x; u.y += uv.y; u.z += uv.z; u.w += uv.w;
     }
@@ -99,6 +100,7 @@ __global__ void splitk_reduce_geglu_kernel(const ReduceArgs a) {
 
 template <bool kVec>
 __global__ void splitk_reduce_kernel(const ReduceArgs a) {
+  ptx::grid_dependency_sync();
   const int64_t plane = static_cast<int64_t>(a.M) * a.N;
   if constexpr (kVec) {
     const int64_t total = plane / 4;
@@ -111,7 +113,7 @@ __global__ void splitk_reduce_kernel(const ReduceArgs a) {
       const float4* src = reinterpret_cast<const float4*>(a.partial) + i;
 #pragma unroll 4
       for (int s = 0; s < a.splits; ++s) {
-        const float4 v = __ldg(src + s * (plane / 4));
+        const float4 v = src[s * (plane / 4)];
         acc.x += v.x;
         acc.y += v.y;
         acc.z += v.z;
@@ -204,21 +206,15 @@ int launch_split_k(const Problem& p, int splits, void* workspace, const DeviceIn
     const int64_t total = p.M * (p.N / 8);
     int64_t blocks = (total + 255) / 256;
     if (blocks > 8 * dev.sm_count) blocks = 8 * dev.sm_count;
-    splitk_reduce_geglu_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(r);
-    IXK_CUDA_OK(cudaGetLastError());
-    count_launch();
-    return IXK_OK;
+    return launch_overlapped(splitk_reduce_geglu_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, r);
   }
   const bool vec = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0;
   const int64_t total = vec ? p.M * p.N / 4 : p.M * p.N;
   const int threads = 256;
   int64_t blocks = (total + threads - 1) / threads;
   if (blocks > 8 * dev.sm_count) blocks = 8 * dev.sm_count;
-  if (vec) splitk_reduce_kernel<true><<<static_cast<unsigned>(blocks), threads, 0, stream>>>(r);
-  else splitk_reduce_kernel<false><<<static_cast<unsigned>(blocks), threads, 0, stream>>>(r);
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
-  return IXK_OK;
+  return launch_overlapped(vec ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3(static_cast<unsigned>(blocks)),
+                           dim3(threads), 0, stream, r);
 }
 
 }  // namespace gemm

@@ -10,6 +10,7 @@
 #include <cuda_fp16.h>
 
 #include "host_common.h"
+#include "ptx.cuh"
 
 namespace ixk {
 namespace glue {
@@ -62,7 +63,8 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 template <bool kBf16, bool kRms>
 __global__ void __launch_bounds__(kNormThreads) row_norm_kernel(const uint4* x, uint4* y,  // may be one buffer: no __restrict__
                                                                 int cols, int64_t ldx_vec, int64_t ldy_vec, float eps,
-                                                                const uint4* __restrict__ gain, float gain_offset) {
+                                                                const uint4* gain, float gain_offset) {
+  ptx::grid_dependency_sync();
   __shared__ float scratch[kNormThreads / 32];
   const int nvec = cols / kVecElems;
   const uint4* xr = x + static_cast<int64_t>(blockIdx.x) * ldx_vec;
@@ -132,9 +134,10 @@ __global__ void __launch_bounds__(kNormThreads) row_norm_kernel(const uint4* x, 
 
 // One thread per 16-byte vector = four (even, odd) pairs of one head of one token.
 template <bool kBf16>
-__global__ void rotary_kernel(uint4* __restrict__ x, const float4* __restrict__ cos_t, const float4* __restrict__ sin_t,
+__global__ void rotary_kernel(uint4* x, const float4* cos_t, const float4* sin_t,
                               int64_t total_vecs, int vecs_per_head, int heads, int seq_len,
                               int64_t token_stride_vec, int64_t head_stride_vec) {
+  ptx::grid_dependency_sync();
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total_vecs;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int vec = static_cast<int>(i % vecs_per_head);
@@ -162,9 +165,10 @@ __global__ void rotary_kernel(uint4* __restrict__ x, const float4* __restrict__ 
 // pairs with element i + rotary_dim / 2.  One thread per 16-byte vector of the first half and its
 // partner vector in the second half.
 template <bool kBf16>
-__global__ void rotary_half_kernel(uint4* __restrict__ x, const float4* __restrict__ cos_t, const float4* __restrict__ sin_t,
+__global__ void rotary_half_kernel(uint4* x, const float4* cos_t, const float4* sin_t,
                                    int64_t total_vecs, int vecs_per_half, int heads, int seq_len,
                                    int64_t token_stride_vec, int64_t head_stride_vec) {
+  ptx::grid_dependency_sync();
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total_vecs;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int vec = static_cast<int>(i % vecs_per_half);
@@ -195,10 +199,10 @@ __global__ void rotary_half_kernel(uint4* __restrict__ x, const float4* __restri
 
 // This step's keys and values into the cache (the dynamic-update-slice of a decode step): one
 // thread per 16-byte vector of one (batch, head) row of K or V.
-__global__ void kv_append_kernel(const uint4* __restrict__ k_new, const uint4* __restrict__ v_new, uint4* __restrict__ k_cache,
-                                 uint4* __restrict__ v_cache, int64_t total_vecs, int vecs_per_head, int heads,
+__global__ void kv_append_kernel(const uint4* k_new, const uint4* v_new, uint4* k_cache, uint4* v_cache, int64_t total_vecs, int vecs_per_head, int heads,
                                  int64_t new_batch_vec, int64_t new_head_vec, int64_t cache_batch_vec, int64_t cache_head_vec,
                                  int64_t cache_offset_vec) {
+  ptx::grid_dependency_sync();
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < 2 * total_vecs;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const bool is_v = i >= total_vecs;
@@ -218,8 +222,8 @@ __global__ void kv_append_kernel(const uint4* __restrict__ k_new, const uint4* _
 // like a framework that materialises (partial + bias) before the residual add.
 template <bool kBf16>
 __global__ void residual_add_kernel(const uint4* x, const uint4* partial,  // out may alias either: no __restrict__
-                                    const uint4* __restrict__ bias, uint4* out, int64_t total_vecs,
-                                    int vecs_per_row) {
+                                    const uint4* bias, uint4* out, int64_t total_vecs, int vecs_per_row) {
+  ptx::grid_dependency_sync();
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total_vecs;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const uint4 a = x[i], p = partial[i];
@@ -282,15 +286,12 @@ static int row_norm_impl(int dtype, int kind, int64_t rows, int64_t cols, const 
   const int64_t lx = ldx / glue::kVecElems, ly = ldy / glue::kVecElems;
   const int c = static_cast<int>(cols);
   if (dtype == IXK_BF16) {
-    if (kind == IXK_NORM_RMS) glue::row_norm_kernel<true, true><<<grid, glue::kNormThreads, 0, s>>>(xv, yv, c, lx, ly, eps, gv, gain_offset);
-    else glue::row_norm_kernel<true, false><<<grid, glue::kNormThreads, 0, s>>>(xv, yv, c, lx, ly, eps, gv, gain_offset);
+    if (kind == IXK_NORM_RMS) return launch_overlapped(glue::row_norm_kernel<true, true>, grid, dim3(glue::kNormThreads), 0, s, xv, yv, c, lx, ly, eps, gv, gain_offset);
+    else return launch_overlapped(glue::row_norm_kernel<true, false>, grid, dim3(glue::kNormThreads), 0, s, xv, yv, c, lx, ly, eps, gv, gain_offset);
   } else {
-    if (kind == IXK_NORM_RMS) glue::row_norm_kernel<false, true><<<grid, glue::kNormThreads, 0, s>>>(xv, yv, c, lx, ly, eps, gv, gain_offset);
-    else glue::row_norm_kernel<false, false><<<grid, glue::kNormThreads, 0, s>>>(xv, yv, c, lx, ly, eps, gv, gain_offset);
+    if (kind == IXK_NORM_RMS) return launch_overlapped(glue::row_norm_kernel<false, true>, grid, dim3(glue::kNormThreads), 0, s, xv, yv, c, lx, ly, eps, gv, gain_offset);
+    else return launch_overlapped(glue::row_norm_kernel<false, false>, grid, dim3(glue::kNormThreads), 0, s, xv, yv, c, lx, ly, eps, gv, gain_offset);
   }
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
-  return IXK_OK;
 }
 
 int ixk_row_norm(int dtype, int kind, int64_t rows, int64_t cols, const void* x, int64_t ldx, void* y, int64_t ldy,
@@ -336,15 +337,12 @@ static int rotary_impl(bool half_split, int dtype, void* x, int64_t tokens, int6
   const int h = static_cast<int>(heads), sl = static_cast<int>(seq_len);
   const int64_t ts = token_stride / glue::kVecElems, hs = head_stride / glue::kVecElems;
   if (half_split) {
-    if (dtype == IXK_BF16) glue::rotary_half_kernel<true><<<grid, 256, 0, s>>>(xv, cv, sv, total, vph, h, sl, ts, hs);
-    else glue::rotary_half_kernel<false><<<grid, 256, 0, s>>>(xv, cv, sv, total, vph, h, sl, ts, hs);
+    if (dtype == IXK_BF16) return launch_overlapped(glue::rotary_half_kernel<true>, dim3(grid), dim3(256), 0, s, xv, cv, sv, total, vph, h, sl, ts, hs);
+    else return launch_overlapped(glue::rotary_half_kernel<false>, dim3(grid), dim3(256), 0, s, xv, cv, sv, total, vph, h, sl, ts, hs);
   } else {
-    if (dtype == IXK_BF16) glue::rotary_kernel<true><<<grid, 256, 0, s>>>(xv, cv, sv, total, vph, h, sl, ts, hs);
-    else glue::rotary_kernel<false><<<grid, 256, 0, s>>>(xv, cv, sv, total, vph, h, sl, ts, hs);
+    if (dtype == IXK_BF16) return launch_overlapped(glue::rotary_kernel<true>, dim3(grid), dim3(256), 0, s, xv, cv, sv, total, vph, h, sl, ts, hs);
+    else return launch_overlapped(glue::rotary_kernel<false>, dim3(grid), dim3(256), 0, s, xv, cv, sv, total, vph, h, sl, ts, hs);
   }
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
-  return IXK_OK;
 }
 
 int ixk_rotary_interleaved(int dtype, void* x, int64_t tokens, int64_t seq_len, int64_t heads, int64_t rotary_dim,
@@ -381,14 +379,11 @@ int ixk_kv_append(int dtype, int64_t batch, int64_t heads, int64_t head_dim, con
   const int64_t total = batch * heads * vph;
   if (total == 0) return IXK_OK;
   const int grid = glue::elementwise_grid(2 * total, 256, info.sm_count);
-  glue::kv_append_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(k_new), static_cast<const uint4*>(v_new), static_cast<uint4*>(k_cache),
+  return launch_overlapped(
+      glue::kv_append_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(k_new), static_cast<const uint4*>(v_new), static_cast<uint4*>(k_cache),
       static_cast<uint4*>(v_cache), total, vph, static_cast<int>(heads), new_batch_stride / glue::kVecElems,
       new_head_stride / glue::kVecElems, cache_batch_stride / glue::kVecElems, cache_head_stride / glue::kVecElems,
       position * (cache_token_stride / glue::kVecElems));
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
-  return IXK_OK;
 }
 
 int ixk_residual_add(int dtype, int64_t rows, int64_t cols, const void* x, const void* partial, const void* bias,
@@ -409,14 +404,11 @@ int ixk_residual_add(int dtype, int64_t rows, int64_t cols, const void* x, const
   auto s = static_cast<cudaStream_t>(stream);
   const int vpr = static_cast<int>(cols / glue::kVecElems);
   if (dtype == IXK_BF16)
-    glue::residual_add_kernel<true><<<grid, 256, 0, s>>>(static_cast<const uint4*>(x), static_cast<const uint4*>(partial),
+    return launch_overlapped(glue::residual_add_kernel<true>, dim3(grid), dim3(256), 0, s, static_cast<const uint4*>(x), static_cast<const uint4*>(partial),
                                                          static_cast<const uint4*>(bias), static_cast<uint4*>(out), total, vpr);
   else
-    glue::residual_add_kernel<false><<<grid, 256, 0, s>>>(static_cast<const uint4*>(x), static_cast<const uint4*>(partial),
+    return launch_overlapped(glue::residual_add_kernel<false>, dim3(grid), dim3(256), 0, s, static_cast<const uint4*>(x), static_cast<const uint4*>(partial),
                                                           static_cast<const uint4*>(bias), static_cast<uint4*>(out), total, vpr);
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
-  return IXK_OK;
 }
 
 }  // extern "C"

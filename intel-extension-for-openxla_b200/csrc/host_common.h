@@ -38,6 +38,29 @@ int get_device_info(DeviceInfo* info);
 
 void count_launch(uint64_t n = 1);
 
+// A launch that may start while the kernel before it in the stream still runs: its launch latency, block
+// set-up and first instructions overlap that kernel's tail.  The kernel has to execute
+// ptx::grid_dependency_wait() in every thread before it touches memory that another kernel may write or
+// read, and must not read such memory through the read-only path (__ldg, const __restrict__), whose loads
+// the compiler may move above the wait.  Between two such launches of 2 to 20 us each this hides about
+// 2 us.
+template <typename... KernelArgs, typename... Args>
+int launch_overlapped(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  IXK_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<KernelArgs>(args)...));
+  count_launch();
+  return IXK_OK;
+}
+
 // A named NVTX range around an entry point, for timelines of a host program that calls the library
 // (the reference marks its thunks through its profiler plug-in instead).  Off unless the
 // environment has IXK_NVTX=1 when the library is first used; costs one branch when off.

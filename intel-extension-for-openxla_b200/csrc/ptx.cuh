@@ -460,6 +460,11 @@ __device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void* tmap,
 // Programmatic dependent launch: wait for the kernel this one was launched behind (complete, its
 // writes visible) / let the kernel launched behind this one start.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// For a kernel started by launch_overlapped: wait for the kernel before it, then let the next one start.
+__device__ __forceinline__ void grid_dependency_sync() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Bounded wait on a barrier that a thread of the OTHER CTA of the cluster arrives on.
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, const AbortCtl& ctl, int code) {
