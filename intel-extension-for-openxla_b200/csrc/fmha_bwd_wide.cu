@@ -406,7 +406,7 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         ptx::tmem_ld_wait();
         // S and dP are in registers: the tile after next may overwrite them
         ptx::tc_fence_before_sync();
-        if (rank == 0) ptx::mbar_arrive(acc_empty(buf)); else ptx::mbar_arrive_cluster(acc_empty(buf), 0);
+        if (rank == 0) ptx::mbar_arrive(acc_empty(buf)); else ptx::mbar_arrive_cluster_tmem(acc_empty(buf), 0);
         buf ^= 1;
         if (buf == 0) acc_ph ^= 1u;
         uint32_t w[2][16];
@@ -715,7 +715,7 @@ wide_grads_kernel(const __grid_constant__ GradMaps maps, const __grid_constant__
       }
       if (g.slabs > 0) {
         ptx::tc_fence_before_sync();
-        if (rank == 0) ptx::mbar_arrive(acc_empty(buf)); else ptx::mbar_arrive_cluster(acc_empty(buf), 0);
+        if (rank == 0) ptx::mbar_arrive(acc_empty(buf)); else ptx::mbar_arrive_cluster_tmem(acc_empty(buf), 0);
         buf ^= 1;
         if (buf == 0) acc_ph ^= 1u;
       }

@@ -717,7 +717,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if (rank == 0) {
         ptx::mbar_arrive(acc_empty_bar(buf));
       } else {
-        ptx::mbar_arrive_cluster(acc_empty_bar(buf), 0);
+        ptx::mbar_arrive_cluster_tmem(acc_empty_bar(buf), 0);
       }
       buf ^= 1;
       if (buf == 0) acc_phase ^= 1u;
