@@ -96,11 +96,11 @@ __device__ __forceinline__ void stage_half_row(uint32_t box, int lane, int half,
 // Bytes through L2 per tile and CTA: 64 KB of K and V, 64 KB of P and dS, and Q and dO once per run,
 // about 75 bytes per cycle of the tile's 2048 MMA cycles.
 struct ScoreCfg {
-  static constexpr int kRing = 8;                                   // K / V slab halves in flight
+  static constexpr int kRing = 4;                                   // slots of two K / V slab halves in flight
   static constexpr int kOffQ = 0;
   static constexpr int kOffDo = kMaxSlabs * kBoxBytes;
   static constexpr int kOffRing = 2 * kMaxSlabs * kBoxBytes;
-  static constexpr int kOffStage = kOffRing + kRing * kHalfBox;     // one box per compute warp
+  static constexpr int kOffStage = kOffRing + kRing * 2 * kHalfBox;     // one box per compute warp
   static constexpr int kOffBars = kOffStage + 8 * 32 * 128;
   static constexpr int kSmemBytes = kOffBars + 512 + 1024;          // + alignment slack
   static_assert(kSmemBytes <= 232448, "shared memory budget");
@@ -159,7 +159,7 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
   const uint32_t bars = smem_base + C::kOffBars;
-  // slot s of the 8 resident slabs: Q slabs 0..3, dO slabs 4..7
+  // Barriers go by two slabs (128 head elements): resident pairs 0, 1 are Q, 2, 3 are dO.
   auto res_full = [&](int s) { return bars + 8u * s; };
   auto res_empty = [&](int s) { return bars + 8u * (8 + s); };
   auto kv_full = [&](int s) { return bars + 8u * (16 + s); };
@@ -227,17 +227,19 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       for (int kt = run.kt0; kt < run.kt1 && alive; ++kt) {
         const int key0 = kt * kKeyTile + static_cast<int>(rank) * 64;
         for (int operand = 0; operand < 2 && alive; ++operand) {   // Q.K^T, then dO.V^T
-          for (int s = 0; s < args.slabs; ++s) {
+          for (int s = 0; s < args.slabs; s += 2) {
+            const int n_slabs = min(2, args.slabs - s);
             if (kt == run.kt0) {
-              const int slot = operand * 4 + s;
-              if (!ptx::mbar_wait(res_empty(slot), res_ph ^ 1u, ctl, kSiteScoreQ)) {
+              const int res = operand * 2 + (s >> 1);
+              if (!ptx::mbar_wait(res_empty(res), res_ph ^ 1u, ctl, kSiteScoreQ)) {
                 alive = false;
                 break;
               }
               if (ptx::elect_one()) {
-                if (rank == 0) ptx::mbar_expect_tx(res_full(slot), 2 * kBoxBytes);
-                ptx::tma_load_4d_pair(smem_base + slot * kBoxBytes, operand == 0 ? &tmap_q : &tmap_do,
-                                      ptx::map_to_cta(res_full(slot), 0), s * 64, row0, n, b);
+                if (rank == 0) ptx::mbar_expect_tx(res_full(res), n_slabs * 2 * kBoxBytes);
+                for (int i = 0; i < n_slabs; ++i)
+                  ptx::tma_load_4d_pair(smem_base + (operand * 4 + s + i) * kBoxBytes, operand == 0 ? &tmap_q : &tmap_do,
+                                        ptx::map_to_cta(res_full(res), 0), (s + i) * 64, row0, n, b);
               }
               __syncwarp();
             }
@@ -246,9 +248,10 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
               break;
             }
             if (ptx::elect_one()) {
-              if (rank == 0) ptx::mbar_expect_tx(kv_full(st), 2 * kHalfBox);
-              ptx::tma_load_4d_pair(smem_base + C::kOffRing + st * kHalfBox, operand == 0 ? &tmap_k : &tmap_v,
-                                    ptx::map_to_cta(kv_full(st), 0), s * 64, key0, n, b);
+              if (rank == 0) ptx::mbar_expect_tx(kv_full(st), n_slabs * 2 * kHalfBox);
+              for (int i = 0; i < n_slabs; ++i)
+                ptx::tma_load_4d_pair(smem_base + C::kOffRing + (2 * st + i) * kHalfBox, operand == 0 ? &tmap_k : &tmap_v,
+                                      ptx::map_to_cta(kv_full(st), 0), (s + i) * 64, key0, n, b);
             }
             __syncwarp();
             if (++st == C::kRing) {
@@ -275,22 +278,25 @@ wide_scores_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         ptx::tc_fence_after_sync();
         for (int operand = 0; operand < 2 && alive; ++operand) {
           const uint32_t d_tmem = tmem_base + buf * 256 + operand * 128;
-          for (int s = 0; s < args.slabs; ++s) {
-            const int slot = operand * 4 + s;
-            if ((kt == run.kt0 && !ptx::mbar_wait(res_full(slot), res_ph, ctl, kSiteScoreFull)) ||
+          for (int s = 0; s < args.slabs; s += 2) {
+            const int n_slabs = min(2, args.slabs - s);
+            const int res = operand * 2 + (s >> 1);
+            if ((kt == run.kt0 && !ptx::mbar_wait(res_full(res), res_ph, ctl, kSiteScoreFull)) ||
                 !ptx::mbar_wait(kv_full(st), ph, ctl, kSiteScoreFull)) {
               alive = false;
               break;
             }
             ptx::tc_fence_after_sync();
+            for (int i = 0; i < n_slabs; ++i) {
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-              const uint64_t da = ptx::umma_smem_desc(smem_base + slot * kBoxBytes + ks * 32, 16, 1024);
-              const uint64_t db = ptx::umma_smem_desc(smem_base + C::kOffRing + st * kHalfBox + ks * 32, 16, 1024);
-              ptx::umma_ss_pair_elect<ptx::kKindF16>(d_tmem, da, db, args.idesc, (s | ks) != 0 ? 1u : 0u);
+              for (int ks = 0; ks < 4; ++ks) {
+                const uint64_t da = ptx::umma_smem_desc(smem_base + (operand * 4 + s + i) * kBoxBytes + ks * 32, 16, 1024);
+                const uint64_t db = ptx::umma_smem_desc(smem_base + C::kOffRing + (2 * st + i) * kHalfBox + ks * 32, 16, 1024);
+                ptx::umma_ss_pair_elect<ptx::kKindF16>(d_tmem, da, db, args.idesc, (s | i | ks) != 0 ? 1u : 0u);
+              }
             }
             ptx::umma_commit_pair_elect(kv_empty(st));
-            if (kt == run.kt1 - 1) ptx::umma_commit_pair_elect(res_empty(slot));
+            if (kt == run.kt1 - 1) ptx::umma_commit_pair_elect(res_empty(res));
             if (++st == C::kRing) {
               st = 0;
               ph ^= 1u;
