@@ -284,10 +284,10 @@ int ixk_fmha_fwd_static_scratch(const ixk_fmha_desc* desc, const void* q, const 
  * ixk_fmha_bwd_workspace_bytes(desc) bytes, 16-byte aligned.  q, k, v, out, grad_out: 16-byte
  * aligned with strides that are multiples of 8; dq, dk, dv likewise.  head_size <= 128 runs as one
  * fused tensor-core kernel between a prepare and a convert pass; 128 < head_size <= 256 (the
- * reference's 64x128x256 policy, fmha_policy.h:107-116) runs as a chain of batched tensor-core
- * GEMMs over a group of heads at a time, with the score-sized intermediates (12 bytes per
- * query-key pair of the group, at most about 192 MB unless one head alone needs more) in the
- * workspace: same formulas and roundings, more HBM traffic. */
+ * reference's 64x128x256 policy, fmha_policy.h:107-116) runs as two kernels over a group of heads at a
+ * time, P and dS first and the three products behind it, with P and dS as 16-bit planes in the
+ * workspace (6 bytes per query-key pair are asked for, at most about 192 MB unless one head alone needs
+ * more): same formulas and roundings. */
 typedef struct ixk_fmha_bwd_desc {
   ixk_fmha_desc fwd;
   int64_t do_strides[3]; /* B, N, F */

@@ -15,8 +15,9 @@
 // matmul operands, all sums are fp32, each gradient is rounded once.  D and -lse*log2(e) come from
 // the shared prepare kernel.
 //
-// What bounds it: operand delivery out of L2 beside the tensor pipe (see the kernels).  Measured at
-// B4 N16 F=T=2048 H256 causal: see the table at the launcher.
+// Measured, forward + backward at B4 N16 F=T=2048 H256 causal bf16: 2590 us as a chain of five GEMMs and
+// two elementwise passes, 745 with seven launches per group of eight heads, 641 as it is; of these 157
+// are the forward, 26 the prepare kernel and four times 53 + 50 the two kernels.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -87,7 +88,7 @@ __device__ __forceinline__ void stage_half_row(uint32_t box, int lane, int half,
 // ---------------------------------------------------------------------------------------------
 // Step 1: P and dS.  A CTA pair works on 256 queries x 128 keys: each CTA keeps its 128 rows of Q and
 // dO in shared memory (2 x 64 KB at head size 256) while the keys of a run go by, and loads half of
-// every K and V slab (64 keys x 64 head elements) into an 8-slot ring; the even CTA's issuer drives
+// every K and V slab (64 keys x 64 head elements) into a ring of 4 slots of two slabs; the even CTA's issuer drives
 // both tensor cores.  S and dP are double-buffered in tensor memory (4 x 128 columns), so that the
 // 256 compute threads of a CTA (one query row each, two warpgroups of 64 keys) work on one tile while
 // the next one is multiplied.  The score tiles of a group are numbered (head, query block, key tile)
@@ -95,6 +96,11 @@ __device__ __forceinline__ void stage_half_row(uint32_t box, int lane, int half,
 // the next run's slabs are requested one by one as the last tile of the current run releases them.
 // Bytes through L2 per tile and CTA: 64 KB of K and V, 64 KB of P and dS, and Q and dO once per run,
 // about 75 bytes per cycle of the tile's 2048 MMA cycles.
+// What bounds it is the issuing warp (clock64 trace, 16 heads of 2048, 16 tiles a pair): of 71k cycles 33k are
+// MMAs, 20k waits for loads (half of them at the start of a run) and the rest barrier round trips and
+// commits between them; that is why a ring slot holds two slabs.  The stores are 15 % (without them 53 us for
+// 62 then).  Twice the compute warps with 32 keys each, and two staging boxes per warp at the price of half the
+// ring, were measured and dropped (no change, 5 us a group slower).
 struct ScoreCfg {
   static constexpr int kRing = 4;                                   // slots of two K / V slab halves in flight
   static constexpr int kOffQ = 0;
@@ -969,10 +975,10 @@ size_t bwd_wide_scratch_bytes(const Problem& p) {
   return scratch_bytes(p);
 }
 
-// Per group of heads: one launch of the score kernel over all SM pairs, then the gradient tiles dealt
-// to kGradSlices launches that run side by side, each on its share of the SM pairs and with the same
+// Per group of heads: one launch of the score kernel over all SM pairs, then one of the gradient kernel
+// (make_plan), or its tiles dealt to kGradSlices launches that run side by side, each on its share of the SM pairs and with the same
 // mix of long and short tiles (programmatic dependent launch: every slice lets the next one start as
-// soon as it runs itself).  Seven launches a group is what a caller sees in ixk_launch_count.
+// soon as it runs itself; they start about 2.7 us apart).
 int launch_bwd_wide(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_lse2, const float* delta, int f_pad,
                     void* scratch, cudaStream_t stream) {
   return bp.fwd.dtype == IXK_BF16 ? launch_typed<true>(bp, dev, neg_lse2, delta, f_pad, scratch, stream)

@@ -26,8 +26,7 @@
 // S in place in TMEM as packed 16-bit pairs.  The running maximum is only raised when it moved by more than 2^8
 // (exact: the same stale maximum scales P, the row sum and O), which keeps the O rescale off
 // the common path.  exp is evaluated as exp2 with head_scale*log2(e) folded in.  bf16 P is cut
-// out of the fp32 bit pattern by a byte permute (a rounding conversion shares the quarter-rate
-// pipe with ex2); the mean truncation loss is compensated in the exponent and the row sum.
+// out of the fp32 bit pattern by a byte permute instead of a rounding conversion; the mean truncation loss is compensated in the exponent and the row sum.
 // O leaves through a swizzled staging box per tile and TMA stores: stores issued from registers
 // (16 bytes per lane, a different line each) queue thousands of requests at every item boundary
 // and hold up the barrier traffic of every other warp.  Q has a full/empty pair per tile, each
@@ -946,8 +945,8 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           const float m_use = (m_run == -INFINITY) ? 0.0f : m_run;
           const uint64_t mult2 = ptx::f32x2(mult, mult);
           // bf16 P is made by truncating the fp32 bit pattern (one byte-permute per pair) instead of
-          // a rounding conversion: conversions share the quarter-rate pipe with ex2, and at one per
-          // pair they cost half as much again as the exponentials.  Truncation loses 0.28 % on
+          // a rounding conversion.  (Conversions do not share the pipe of ex2: 109 lanes and more per cycle
+          // and SM against 16, measured apart and together.)  Truncation loses 0.28 % on
           // average (half an ulp over a log-uniform mantissa), so the exponent carries that much
           // extra (kTruncBias) and the row sum is deflated by the same factor in the epilogue.
           const bool trunc = bf16;

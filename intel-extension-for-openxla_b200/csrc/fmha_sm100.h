@@ -34,7 +34,7 @@ constexpr int kDecodeMaxQueries = 16;
 size_t prefill_workspace_bytes(const Problem& p, int sm_count);
 int launch_prefill(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 
-// ---- split-key decode kernel (fmha_decode_sm100.cu)
+// ---- split-key decode kernel (fmha_decode_sm100.cu): one query row, and what the one-pass kernel leaves
 // Number of key splits chosen for a problem, and the scratch it needs:
 // splits * B*N*F * (H + 2) floats (partial O, running max, running sum).
 int decode_splits(const Problem& p, int sm_count);
@@ -67,9 +67,9 @@ size_t bwd_workspace_bytes(const Problem& p);
 int launch_bwd(const BwdProblem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes,
                cudaStream_t stream);
 
-// ---- head sizes above 128 (fmha_bwd_wide.cu): the same gradients as a chain of batched GEMMs
-// over a group of heads at a time, with the score-sized intermediates in `scratch`
-// (bwd_wide_scratch_bytes); neg_lse2 / delta are the prepare kernel's per-row arrays [B*N, f_pad].
+// ---- head sizes above 128 (fmha_bwd_wide.cu): the same gradients in two kernels over a group of heads
+// at a time, with P and dS as 16-bit planes in `scratch` (bwd_wide_scratch_bytes); neg_lse2 / delta are
+// the prepare kernel's per-row arrays [B*N, f_pad].
 size_t bwd_wide_scratch_bytes(const Problem& p);
 int launch_bwd_wide(const BwdProblem& p, const DeviceInfo& dev, const float* neg_lse2, const float* delta, int f_pad,
                     void* scratch, cudaStream_t stream);
