@@ -35,8 +35,12 @@ namespace fmha {
 
 namespace {
 
-constexpr int kWarps = 8;                         // compute warps; one more for the loads
-constexpr int kThreads = (kWarps + 1) * 32;
+constexpr int kWarps = 8;                         // compute warps: two warpgroups
+constexpr int kThreads = (kWarps + 4) * 32;       // and one of which a single warp works, on the loads
+// Registers per thread.  At launch 168 (65536 / 384, a multiple of 8); the third warpgroup gives its share up:
+// 256 x 240 + 128 x 24 = 384 x 168.  (With 168 for all, the kernels for two blocks of rows spill up to 250 bytes.)
+constexpr int kComputeRegs = 240;
+constexpr int kLoadRegs = 24;
 constexpr int kMinKeysPerCta = 128;               // below that the merge costs more than the streaming saves
 constexpr size_t kMaxPartialBytes = IXK_STATIC_SCRATCH_BYTES;  // also the scratch of ixk_fmha_fwd_static_scratch
 constexpr float kLog2e = 1.4426950408889634f;
@@ -78,7 +82,6 @@ struct Cfg {
 
 struct Args {
   int B, N, H, F, T;
-  int causal;
   float scale_log2;
   int tiles_per_unit, total_tiles;
   const uint16_t* q;
@@ -192,9 +195,10 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   const int t_begin = range_begin(a.total_tiles, blockIdx.x, gridDim.x);
   const int t_end = range_begin(a.total_tiles, blockIdx.x + 1, gridDim.x);
 
-  if (warp == kWarps) {
+  if (warp >= kWarps) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    ptx::setmaxnreg_dec<kLoadRegs>();
+    if (warp == kWarps && lane == 0) {
       int unit = t_begin / a.tiles_per_unit;
       int in_unit = t_begin - unit * a.tiles_per_unit;
       for (int seq = 0; seq < t_end - t_begin; ++seq) {
@@ -221,6 +225,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       }
     }
   } else {
+    ptx::setmaxnreg_inc<kComputeRegs>();
     const int g = lane >> 2, c = lane & 3;        // fragment row / column-pair index
     const int group = warp / C::kWarpsPerTile;
     const int key_row = (warp % C::kWarpsPerTile) * 16;
@@ -337,7 +342,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
             for (int nt = 0; nt < kNT; ++nt) mma_16x8x16<kBf16>(acc[ks & 1][nt], af, qf[ks][nt][0], qf[ks][nt][1]);
           }
         }
-        const bool edge = a.causal || key0 + 16 > a.T;   // (warp-uniform)
+        const bool edge = key0 + 16 > a.T;   // (warp-uniform)
         uint32_t p_hi[kNT][2], p_lo[kNT][2];
 #pragma unroll
         for (int nt = 0; nt < kNT; ++nt) {
@@ -346,10 +351,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           for (int i = 0; i < 4; ++i) {
             x[i] = (acc[0][nt][i] + acc[1][nt][i]) * a.scale_log2;
             if (a.bias != nullptr) x[i] = fmaf(bias_v[nt][i], kLog2e, x[i]);
-            if (edge) {
-              const int key = key0 + g + (i >> 1) * 8;
-              if (key >= a.T || (a.causal && key > nt * 8 + 2 * c + (i & 1))) x[i] = -INFINITY;
-            }
+            if (edge && key0 + g + (i >> 1) * 8 >= a.T) x[i] = -INFINITY;
           }
           float mx[2] = {fmaxf(x[0], x[2]), fmaxf(x[1], x[3])};
 #pragma unroll
@@ -549,6 +551,11 @@ bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   const int keys = slabs_of(p.H) > 2 ? 32 : 64;
   const int64_t per_unit = (static_cast<int64_t>(p.T) + keys - 1) / keys;
   const int64_t total = per_unit * p.B * p.N;
+  // Under the mask row f sees keys 0..f: at most F keys of the cache count, and those behind them may not
+  // have been written yet (a product with P = 0 would turn their NaN into the result's).  The split-key
+  // kernel ends at the last row's key: B32 N16 H256, 3001 keys, F = 4: 38 us there, 271 as a pass over the
+  // whole cache; F = 16: 57 and 378.
+  if (p.causal) return false;
   // Two rows of a short cache stay with the split-key kernel: a unit's merge is paid for few keys
   // (B64 N16 H256, 33 keys: 31 us there, 36 us here; at 200 keys and B4 it is 22 and 19).
   if (p.F < 2 || p.F > kDecodeMaxQueries || (p.F == 2 && p.T <= kMinKeysPerCta) || total <= 0 || total > 0x7fffffff) return false;
@@ -638,7 +645,6 @@ int launch_decode_mma(const Problem& p, const DeviceInfo& dev, void* workspace, 
   if (make_map(&tk, p.k, p.k_strides) != IXK_OK || make_map(&tv, p.v, p.v_strides) != IXK_OK) return IXK_UNIMPLEMENTED;
   Args a{};
   a.B = p.B; a.N = p.N; a.H = p.H; a.F = p.F; a.T = p.T;
-  a.causal = p.causal ? 1 : 0;
   a.scale_log2 = p.head_scale * kLog2e;
   a.tiles_per_unit = plan.tiles_per_unit;
   a.total_tiles = plan.total_tiles;

@@ -280,7 +280,8 @@ MULTI_ROW_CASES = [
     (1, 1, 2, 1, 8, "bf16", False, False),          # one key, one 16-byte row
     (2, 3, 7, 17, 64, "fp16", False, False),        # one key past a slice, a row short of a block
     (3, 5, 8, 65, 72, "bf16", False, True),         # one key past a tile, a slab of 8 elements
-    (1, 2, 9, 63, 136, "fp16", True, False),        # second block of rows; causal: 9 of 63 keys seen
+    (1, 2, 9, 63, 136, "fp16", False, False),       # second block of rows
+    (1, 2, 9, 63, 136, "fp16", True, False),        # causal, 9 of 63 keys seen: the split-key kernel
     (37, 4, 3, 95, 192, "bf16", False, False),      # three slabs, units of three tiles
     (150, 1, 4, 33, 256, "bf16", False, False),     # more units than CTAs: ranges that cover whole units
     (1, 1, 16, 9000, 256, "bf16", False, False),    # one unit cut into many ranges, full blocks of rows
@@ -313,6 +314,25 @@ def test_decode_several_rows(pkg, orc, cuda, case):
     ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
     orc.check_close(f32(o), want, rtol=ulp, atol=1e-4, what=str(case))
     orc.check_close(f32(lse), want_lse, rtol=1e-5, atol=1e-4, what=f"lse {case}")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("F,H", [(2, 64), (3, 256), (4, 128), (8, 72), (9, 256), (16, 192)])
+def test_decode_several_rows_causal_unwritten_cache(pkg, orc, cuda, F, H, dtype):
+    """A prompt of a few tokens against a preallocated cache: rows 0..f of it are all that row f may see,
+    and what lies behind the prompt (NaN and infinities here) has no part in any result."""
+    B, N, T = 2, 3, 300
+    g = torch.Generator().manual_seed(F)
+    q = torch.randn(B, N, F, H, generator=g).to(dtype).to(cuda)
+    k, v = (torch.randn(B, T, N, H, generator=g).to(dtype).to(cuda).permute(0, 2, 1, 3) for _ in range(2))
+    k[:, :, F:], v[:, :, F:] = float("nan"), float("inf")
+    v[:, :, F + 1:: 2] = float("nan")
+    o, lse = run(pkg, q, k, v, causal=True, lse=True)
+    want, want_lse = orc.fmha_forward(f32(q), f32(k[:, :, :F]), f32(v[:, :, :F]), None, head_scale=H ** -0.5, causal=True,
+                                      dtype=orc.BF16 if dtype == torch.bfloat16 else orc.F16, round_p=False)
+    ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10     # one rounding of the result, as above
+    orc.check_close(f32(o), want, rtol=ulp, atol=1e-4, what="out")
+    orc.check_close(f32(lse), want_lse, rtol=1e-5, atol=1e-4, what="lse")
 
 
 def test_decode_several_rows_infinite_values(pkg, cuda):
