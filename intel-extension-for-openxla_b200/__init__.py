@@ -211,6 +211,25 @@ def _stream_ptr(stream) -> int:
     return _current_raw_stream(_current_device())
 
 
+def _on_stream(stream, device):
+    """Context in which torch allocates from the pool of the stream that a call was given."""
+    if not isinstance(stream, torch.cuda.Stream):
+        stream = torch.cuda.ExternalStream(stream.cuda_stream, device=device)
+    return torch.cuda.stream(stream)
+
+
+def _scratch(need: int, workspace: Optional[torch.Tensor], device, stream) -> Optional[torch.Tensor]:
+    """The caller's workspace where it holds `need` bytes, else one of the call's own.  That one is dropped when
+    the call returns, while its kernels may still run: it has to come from the pool of the stream they run on, whose
+    next tenant is ordered behind them.  (A block of another stream's pool could be in use there at once.)"""
+    if not need or (workspace is not None and workspace.nbytes >= need):
+        return workspace
+    if stream is None:
+        return torch.empty(need, dtype=torch.uint8, device=device)
+    with _on_stream(stream, device):
+        return torch.empty(need, dtype=torch.uint8, device=device)
+
+
 def _require_cuda(*tensors) -> None:
     for t in tensors:
         if t is not None and not t.is_cuda:
@@ -364,11 +383,10 @@ def gemm_geglu(x: torch.Tensor, w_gate_up: torch.Tensor, *, out: Optional[torch.
     d = _gemm_desc(_matrix_layout("lhs", x), _matrix_layout("rhs", w_gate_up), (ROW_MAJOR, _TORCH_TO_IXK[x.dtype], m, n2, m * n2, n2),
                    1, 1.0, 0.0, "DEFAULT")
     lib = load_library()
-    need = int(lib.ixk_gemm_geglu_workspace_bytes(ctypes.byref(d)))
     if workspace is None:
-        workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
+        workspace = _scratch(int(lib.ixk_gemm_geglu_workspace_bytes(ctypes.byref(d))), None, x.device, stream)
     _check(lib.ixk_gemm_geglu(ctypes.byref(d), _ptr(x), _ptr(w_gate_up), _ptr(out), out.stride(-2), _ptr(workspace),
-                              workspace.nbytes, _stream_ptr(stream)))
+                              0 if workspace is None else workspace.nbytes, _stream_ptr(stream)))
     return out
 
 
@@ -569,9 +587,7 @@ def fmha_forward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: t
         raise IxkError(IXK_INVALID_ARGUMENT, "is_training needs the activation (log-sum-exp) buffer")
     lib = load_library()
     d = _fmha_desc(query, key, value, bias, out, head_scale, causal, 0.0 if dropout_prob in (None, 1.0) else dropout_prob)
-    need = int(lib.ixk_fmha_fwd_workspace_bytes(ctypes.byref(d)))
-    if need and (workspace is None or workspace.nbytes < need):
-        workspace = torch.empty(need, dtype=torch.uint8, device=query.device)
+    workspace = _scratch(int(lib.ixk_fmha_fwd_workspace_bytes(ctypes.byref(d))), workspace, query.device, stream)
     ws_bytes = 0 if workspace is None else workspace.nbytes
     st = lib.ixk_fmha_fwd(ctypes.byref(d), _ptr(query), _ptr(key), _ptr(value), _ptr(bias), _ptr(out),
                           _ptr(activation if is_training else None), _ptr(workspace), ws_bytes, _stream_ptr(stream))
@@ -614,9 +630,7 @@ def fmha_backward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: 
         raise IxkError(IXK_INVALID_ARGUMENT, "activation must be the forward's dense fp32 [B,N,F] log-sum-exp")
     lib = load_library()
     d = _fmha_bwd_desc(query, key, value, out, bias, grad_out, grad_query, grad_key, grad_value, head_scale, causal)
-    need = int(lib.ixk_fmha_bwd_workspace_bytes(ctypes.byref(d)))
-    if need and (workspace is None or workspace.nbytes < need):
-        workspace = torch.empty(need, dtype=torch.uint8, device=query.device)
+    workspace = _scratch(int(lib.ixk_fmha_bwd_workspace_bytes(ctypes.byref(d))), workspace, query.device, stream)
     ws_bytes = 0 if workspace is None else workspace.nbytes
     st = lib.ixk_fmha_bwd(ctypes.byref(d), _ptr(query), _ptr(key), _ptr(value), _ptr(out), _ptr(bias), _ptr(grad_out),
                           _ptr(activation), _ptr(grad_query), _ptr(grad_key), _ptr(grad_value), _ptr(workspace),

@@ -395,3 +395,25 @@ def test_prefill_split_along_the_keys(pkg, orc, cuda, case):
     for got, got_lse in ((o, lse), (o1, lse1)):
         orc.check_close(f32(got)[keep], want[keep], rtol=2e-2, atol=2e-2 if dtype == torch.bfloat16 else 5e-3, what=str(case))
         orc.check_close(f32(got_lse)[keep], want_lse[keep], rtol=2e-3, atol=2e-3, what=f"lse {case}")
+
+
+def test_scratch_of_a_call_on_another_stream(pkg, cuda):
+    """A prefill on a stream of the caller's takes its scratch from that stream's pool, as a torch Stream and as any
+    object with a cuda_stream, and gives the current stream's bits."""
+    import types
+    g = torch.Generator().manual_seed(9)
+    q, k, v = (torch.randn(1, 2, S, 128, generator=g).bfloat16().to(cuda) for S in (300, 1100, 1100))
+    want, _ = run(pkg, q, k, v)
+    need = pkg.fmha_workspace_bytes(q, k, v, None, want, 128 ** -0.5)
+    assert need > 0                                                   # split along the keys
+    side = torch.cuda.Stream()
+    for stream in (side, types.SimpleNamespace(cuda_stream=side.cuda_stream)):
+        o = torch.zeros_like(want)
+        side.wait_stream(torch.cuda.current_stream())
+        pkg.fmha_forward_kernel(stream, q, k, v, None, None, 0.0, o, None, 128 ** -0.5, False)
+        side.synchronize()
+        assert torch.equal(o, want)
+        held = [s for s in torch.cuda.memory_snapshot() if s["stream"] == side.cuda_stream]
+        assert sum(s["total_size"] for s in held) >= need
+        del held
+        torch.cuda.empty_cache()                                      # (the second round has to take its own)

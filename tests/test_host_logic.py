@@ -1,5 +1,8 @@
 """CPU: the host-side mirror — layout attributes derived from tensor views, and the checks the
 reference's runners make before launching."""
+import contextlib
+import types
+
 import pytest
 import torch
 
@@ -80,3 +83,64 @@ def test_packed_gemm_descriptor(pkg, shape, layout, dtype):
     got = pkg._gemm_desc(*(pkg._matrix_layout(name, t) for name, t in (("lhs", lhs), ("rhs", rhs), ("output", out))),
                          out.shape[0] if out.dim() == 3 else 1, 2.0, 0.5, "BIAS_GELU")
     assert bytes(got) == bytes(want)
+
+
+class _FakeLibrary:
+    """Answers 4096 to every workspace query and records the arguments of the launches."""
+
+    def __init__(self, status=0):
+        self.calls, self.status = [], status
+
+    def __getattr__(self, name):
+        if name.endswith("_workspace_bytes"):
+            return lambda *args: 4096
+        return lambda *args: self.calls.append((name, args)) or self.status
+
+
+@pytest.fixture
+def fake_calls(pkg, monkeypatch):
+    """The package on a library that launches nothing.  allocated: for each torch.empty the stream whose pool it
+    was taken from (None: the current stream's)."""
+    lib, scope, allocated, empty = _FakeLibrary(), [None], [], torch.empty
+
+    @contextlib.contextmanager
+    def on(stream):
+        scope.append(stream)
+        yield
+        scope.pop()
+
+    def recorded(*args, **kwargs):
+        allocated.append(scope[-1])
+        return empty(*args, **kwargs)
+    monkeypatch.setattr(pkg, "load_library", lambda: lib)
+    monkeypatch.setattr(pkg, "_require_cuda", lambda *tensors: None)
+    monkeypatch.setattr(torch.cuda, "stream", on)
+    monkeypatch.setattr(torch.cuda, "ExternalStream", lambda ptr, device=None: ptr)
+    monkeypatch.setattr(torch, "empty", recorded)
+    return types.SimpleNamespace(lib=lib, allocated=allocated)
+
+
+@pytest.mark.parametrize("call", ["forward", "backward", "geglu"])
+def test_scratch_comes_from_the_pool_of_the_calls_stream(pkg, fake_calls, call):
+    """Scratch that a call takes for itself is free again when the call returns: only in the pool of the stream that
+    the call was given does its next tenant wait for the call's kernels."""
+    q = torch.zeros(1, 2, 64, 32, dtype=torch.bfloat16)
+    lse = torch.zeros(1, 2, 64)
+    stream = types.SimpleNamespace(cuda_stream=77)
+    own = torch.zeros(8192, dtype=torch.uint8)
+
+    def run(stream, workspace):
+        fake_calls.allocated.clear()
+        fake_calls.lib.calls.clear()
+        if call == "forward":
+            pkg.fmha_forward_kernel(stream, q, q, q, None, None, 0.0, q, None, 1.0, False, workspace=workspace)
+        elif call == "backward":
+            pkg.fmha_backward_kernel(stream, q, q, q, q, None, q, lse, q, q, q, 1.0, workspace=workspace)
+        else:
+            pkg.gemm_geglu(q[0, 0], torch.zeros(32, 16, dtype=torch.bfloat16), out=q[0, 0, :, :8], workspace=workspace, stream=stream)
+        (_, args), = fake_calls.lib.calls
+        assert args[-1] == 77 and args[-2] >= 4096 and (workspace is None or args[-3] == workspace.data_ptr())
+    run(stream, None)
+    assert fake_calls.allocated == [77]
+    run(stream, own)
+    assert fake_calls.allocated == []
