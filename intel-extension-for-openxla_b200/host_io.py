@@ -10,14 +10,23 @@ about as much as its largest leg (the input copy), and consecutive calls overlap
 input copies run under call i's last result copies).
 
 Host tensors should be pinned (`torch.Tensor.pin_memory()`): pageable memory makes the copies
-synchronous and the pipeline degenerates to the sequential form.  Results are bit-identical to
-the device-buffer call: the same kernel runs on the same values, one batch element at a time.
+synchronous and the pipeline degenerates to the sequential form.
+
+A prefill (more than 16 query rows) runs without scratch, so that no chunk is split along the keys: a
+sequence's result does not depend on the chunk or the batch it is in, and is bit for bit that of the
+device-buffer call without scratch (ixk_fmha_fwd with workspace NULL).  A device-buffer call with scratch
+may split its last round of work, whose partial sums are then rounded in another order; the copies, not
+the kernel, bound this pipeline.  (The key splits of a decode call depend on the batch size, on the device
+as here.)
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional
 
 import torch
+
+_DECODE_MAX_QUERIES = 16      # up to here ixk_fmha_fwd takes the decode path, which needs its scratch
 
 
 class HostAttention:
@@ -46,6 +55,16 @@ class HostAttention:
         self.computed = [torch.cuda.Event() for _ in range(n)]
         self.returned = [torch.cuda.Event() for _ in range(n)]
         self.used = False
+
+    def _attend(self, q, k, v, bias, out, scale: float) -> None:
+        """One chunk on the current stream."""
+        pkg = self.pkg
+        if self.shape[2] <= _DECODE_MAX_QUERIES:
+            pkg.fmha_forward_kernel(None, q, k, v, bias, None, 0.0, out, None, scale, False, causal=self.causal)
+            return
+        d = pkg._fmha_desc(q, k, v, bias, out, scale, self.causal, 0.0)
+        pkg._check(pkg.load_library().ixk_fmha_fwd(ctypes.byref(d), pkg._ptr(q), pkg._ptr(k), pkg._ptr(v), pkg._ptr(bias), pkg._ptr(out),
+                                                   None, None, 0, pkg._stream_ptr(None)))
 
     def __call__(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor,
                  bias: Optional[torch.Tensor] = None, scale: Optional[float] = None) -> torch.Tensor:
@@ -78,8 +97,7 @@ class HostAttention:
                 self.compute.wait_event(self.arrived[i])
                 if self.used:
                     self.compute.wait_event(self.returned[i])  # the previous call's result has left this chunk
-                pkg.fmha_forward_kernel(None, self.q[s], self.k[s], self.v[s], None if bias is None else self.bias[s],
-                                        None, 0.0, self.out[s], None, scale, False, causal=self.causal)
+                self._attend(self.q[s], self.k[s], self.v[s], None if bias is None else self.bias[s], self.out[s], scale)
                 self.computed[i].record(self.compute)
             with torch.cuda.stream(self.d2h):
                 self.d2h.wait_event(self.computed[i])
