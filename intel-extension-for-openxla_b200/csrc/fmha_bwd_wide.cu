@@ -3,8 +3,8 @@
 //
 // With 256-wide heads the dK and dV accumulators of a 128-key block alone fill the 512 columns of
 // tensor memory, so the single-kernel scheme of fmha_bwd_sm100.cu (S^T, dP^T, dK, dV resident
-// together) does not fit.  Here a group of heads of one batch is taken in two steps, and what passes
-// between them, P and dS as 16-bit [F, T] planes, is sized to stay in L2:
+// together) does not fit.  Here a group of heads is taken in two steps, with P and dS as 16-bit [F, T]
+// planes in scratch between them:
 //   1. wide_scores_kernel:  S = Q.K^T and dP = dO.V^T into tensor memory side by side, then
 //                           P = exp(head_scale*S + bias - lse) and dS = P * (dP - D), both stored once
 //                                                                       (fmha_backward.h:489-700)
@@ -40,9 +40,6 @@ constexpr int kMaxSlabs = 4;       // head size <= 256
 constexpr int kBoxBytes = 128 * kSlabBytes;   // 128 rows x 128 bytes
 constexpr int kHalfBox = 64 * kSlabBytes;     // 64 rows x 128 bytes
 constexpr size_t kGroupBudget = static_cast<size_t>(192) << 20;   // scratch per group of heads (see heads_per_group)
-// The gradient tiles of a group are dealt to this many launches of wide_grads_kernel that run side by
-// side (see launch_bwd_wide).
-constexpr int kGradSlices = 6;
 constexpr int kHeadChunk = 4;      // heads whose gradient tiles are sorted together
 
 // Where a block of 256 query rows lies in a plane.  Unfolded: at its own rows.  Under a causal mask block
@@ -484,8 +481,6 @@ struct GradArgs {
   int causal;
   Fold fold;
   int chunk;                   // heads whose tiles are sorted together
-  int slice, num_slices;       // this launch takes tiles slice, slice + num_slices, ...
-  int wait_first;              // the first slice of a group waits for the scores, the others follow it
   uint32_t idesc_t, idesc_n;   // A with its rows contiguous (dV, dK) / with K contiguous (dQ)
   float head_scale;
   int* status_word;
@@ -572,19 +567,14 @@ wide_grads_kernel(const __grid_constant__ GradMaps maps, const __grid_constant__
   ptx::cluster_sync_all();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  // The first slice waits for the score kernel before it lets the next slice start; the others start
-  // behind it and only make sure at their end that they do not complete before it.
-  if (args.wait_first) ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait();      // for the score kernel's planes
   ptx::grid_dependency_trigger();
 
   const int pair = blockIdx.x >> 1;
   const int pairs = gridDim.x >> 1;
   const int num_tiles = 3 * args.heads * args.ranks;
-  // tiles of this slice, dealt to its pairs in rounds of alternating direction
-  auto tile_index = [&](int round) {
-    const int i = round * pairs + ((round & 1) ? pairs - 1 - pair : pair);
-    return args.slice + i * args.num_slices;
-  };
+  // tiles are dealt to the pairs in rounds of alternating direction
+  auto tile_index = [&](int round) { return round * pairs + ((round & 1) ? pairs - 1 - pair : pair); };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -744,7 +734,6 @@ wide_grads_kernel(const __grid_constant__ GradMaps maps, const __grid_constant__
     ptx::tmem_dealloc_pair(tmem_base, 512);
   }
   ptx::cluster_sync_all();
-  if (!args.wait_first) ptx::grid_dependency_wait();
 }
 
 // ------------------------------------------------------------------------------------- host side
@@ -766,28 +755,20 @@ size_t scratch_bytes(const Problem& p) {
 
 struct Plan {
   int group;          // heads of a group
-  int slices;         // launches of the gradient kernel per group
-  int chunk;
+  int chunk;          // heads whose gradient tiles are sorted together
   Fold fold;
   int64_t rows, keys; // extents of a plane: stores are clipped there, loads read zeros beyond
 };
-Plan make_plan(const Problem& p, int pairs) {
+// Groups are as large as the scratch holds, over batches as well as heads, and their planes are folded where
+// that makes them smaller: every group costs about 18 us beside its work (ramp-up and the last round of both
+// kernels), more than planes that fit L2 would save (B4 N16 S2048 H256 causal, unfolded planes of 128 MB a
+// group: 691 us forward + backward, of 64 MB: 780, of 32 MB: 1116 and more).
+Plan make_plan(const Problem& p) {
   Plan plan{};
+  const int nq = (p.F + kRowBlock - 1) / kRowBlock;
+  plan.fold = Fold{0, nq};
   plan.rows = p.F;
   plan.keys = plane_pitch(p.T);
-  plan.group = heads_per_group(p);
-  plan.slices = kGradSlices;
-  plan.chunk = plan.group;
-  const int nq = (p.F + kRowBlock - 1) / kRowBlock, nk2 = (p.T + kRowBlock - 1) / kRowBlock;
-  plan.fold = Fold{0, nq};
-  const int64_t tiles = static_cast<int64_t>(3) * std::max(nq, nk2) * plan.group;
-  if (p.B == 1 || tiles <= pairs) return plan;
-  // Several batch elements, each with more gradient tiles than SM pairs: one launch of each kernel per
-  // group, the planes folded where that makes them smaller, and groups as large as the scratch holds, over
-  // batches as well as heads.  Every group costs about 18 us beside its work (ramp-up and the last round
-  // of both kernels).  (A single batch element keeps the groups and the seven launches of each that
-  // ixk_launch_count has always shown for it.)
-  plan.slices = 1;
   const int64_t folded_rows = static_cast<int64_t>(kRowBlock) * ((nq + 1) / 2), folded_keys = static_cast<int64_t>(kRowBlock) * (nq + 1);
   if (p.causal && folded_rows * folded_keys < plan.rows * plan.keys) {
     plan.fold.on = 1;
@@ -829,7 +810,7 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
   const Problem& p = bp.fwd;
   const CUtensorMapDataType dt = kBf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const int all_pairs = std::max(dev.sm_count / 2, 1);
-  const Plan plan = make_plan(p, all_pairs);
+  const Plan plan = make_plan(p);
   const int group = plan.group;
   const int64_t rows = plan.rows, keys = plan.keys;
   uint16_t* plane_p = static_cast<uint16_t*>(scratch);
@@ -925,7 +906,6 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
   ga.causal = sa.causal;
   ga.fold = plan.fold;
   ga.chunk = plan.chunk;
-  ga.num_slices = plan.slices;
   ga.idesc_t = ptx::umma_idesc(fmt, fmt, 1, 1, 2 * 128, 256);
   ga.idesc_n = ptx::umma_idesc(fmt, fmt, 0, 1, 2 * 128, 256);
   ga.head_scale = p.head_scale;
@@ -940,31 +920,24 @@ int launch_typed(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_l
     IXK_CUDA_OK(cudaFuncSetAttribute(grads, cudaFuncAttributeMaxDynamicSharedMemorySize, GradCfg::kSmemBytes));
     configured_device = dev.device;
   }
-  const int slice_pairs = std::max(all_pairs / plan.slices, 1);
   bool first = true;
   const int heads_all = p.B * p.N;
   for (int bn0 = 0; bn0 < heads_all;) {
-    // a sliced group stays within one batch
-    const int g = std::min(group, plan.slices > 1 ? p.N - bn0 % p.N : heads_all - bn0);
+    const int g = std::min(group, heads_all - bn0);
     sa.bn0 = ga.bn0 = bn0;
     sa.heads = ga.heads = g;
     bn0 += g;
     const int64_t total = static_cast<int64_t>(sa.tiles_per_head) * g;
-    if (total > 0x7fffffff) return fail(IXK_UNIMPLEMENTED, "too many score tiles");
+    const int64_t grad_tiles = static_cast<int64_t>(3) * g * ga.ranks;
+    if (total > 0x7fffffff || grad_tiles > 0x7fffffff) return fail(IXK_UNIMPLEMENTED, "too many score tiles");
     sa.total_tiles = static_cast<int>(total);
-    const int score_pairs = static_cast<int>(std::min<int64_t>(total, all_pairs));
-    if ((rc = launch_pairs(scores, score_pairs, ScoreCfg::kThreads, ScoreCfg::kSmemBytes, !first, stream, tq, tdo, tk, tv, tp, tds,
-                           sa)) != IXK_OK)
+    if ((rc = launch_pairs(scores, static_cast<int>(std::min<int64_t>(total, all_pairs)), ScoreCfg::kThreads, ScoreCfg::kSmemBytes, !first,
+                           stream, tq, tdo, tk, tv, tp, tds, sa)) != IXK_OK)
       return rc;
     first = false;
-    for (int slice = 0; slice < plan.slices; ++slice) {
-      ga.slice = slice;
-      ga.wait_first = slice == 0 ? 1 : 0;
-      const int tiles = (3 * g * ga.ranks - slice + plan.slices - 1) / plan.slices;
-      if ((rc = launch_pairs(grads, std::max(std::min(tiles, slice_pairs), 1), GradCfg::kThreads, GradCfg::kSmemBytes, true, stream, gm,
-                             ga)) != IXK_OK)
-        return rc;
-    }
+    if ((rc = launch_pairs(grads, static_cast<int>(std::min<int64_t>(grad_tiles, all_pairs)), GradCfg::kThreads, GradCfg::kSmemBytes, true,
+                           stream, gm, ga)) != IXK_OK)
+      return rc;
   }
   return IXK_OK;
 }
@@ -976,9 +949,8 @@ size_t bwd_wide_scratch_bytes(const Problem& p) {
 }
 
 // Per group of heads: one launch of the score kernel over all SM pairs, then one of the gradient kernel
-// (make_plan), or its tiles dealt to kGradSlices launches that run side by side, each on its share of the SM pairs and with the same
-// mix of long and short tiles (programmatic dependent launch: every slice lets the next one start as
-// soon as it runs itself; they start about 2.7 us apart).
+// (programmatic dependent launches: each sets itself up while its predecessor runs and waits for its end
+// before it touches the planes).
 int launch_bwd_wide(const BwdProblem& bp, const DeviceInfo& dev, const float* neg_lse2, const float* delta, int f_pad,
                     void* scratch, cudaStream_t stream) {
   return bp.fwd.dtype == IXK_BF16 ? launch_typed<true>(bp, dev, neg_lse2, delta, f_pad, scratch, stream)
