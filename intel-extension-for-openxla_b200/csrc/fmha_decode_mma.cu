@@ -6,10 +6,8 @@
 // tensor-core products whose M side is the cache:
 //   S^T [keys, rows] = K . Q^T         A = K as it lies in memory, B = Q (registers)
 //   O^T [head, rows] += V^T . P^T      A = V^T (transposing fragment loads), B = P
-// 8 rows cost one instruction per 16 x 16 block of K or V, 16 rows two: at head size 256 about a fifth
-// of the cycles that HBM takes to deliver the block.  (mma.sync and not tcgen05: with 8 rows the
-// product is 3 % of what the tensor core could do in the time; what counts is that nothing has to
-// travel through tensor memory between the two products.)
+// (mma.sync and not tcgen05: with 8 rows the product is 3 % of what the tensor core could do in the time;
+// what counts is that nothing has to travel through tensor memory between the two products.)
 //
 //   CTAs      persistent, one per SM; the (batch, head) units are cut into tiles of keys, the tiles
 //             numbered through, and every CTA takes an equal, contiguous range
@@ -20,8 +18,14 @@
 // A unit that a range boundary cuts leaves unnormalised partials (O, maximum, sum) in scratch, which
 // fmha_decode_mma_combine_kernel merges.
 //
-// P keeps its 32 bits: it is multiplied as the sum of two 16-bit numbers (hi + lo, 16 mantissa bits in
-// bf16, 21 in fp16), and all sums are fp32.
+// Precision is that of the fp32 arithmetic it replaces.  P goes into the second product as the sum of two
+// tf32 numbers (hi + lo, 22 bits of P at fp32's range of exponents; a pair of fp16 numbers would lose P
+// below 2^-25 of the row's largest), V as tf32, which holds both 16-bit types exactly.  The tensor core
+// truncates what it accumulates, so every product starts at zero and is added to S and O in fp32.
+// Measured against 64 bits, B2 N16 T2000, heads of 64 to 256, 4 and 16 rows: relative error of O equal to the
+// split-key kernel's to six digits (1.6617e-3 bf16, 2.0851e-4 fp16 at head size 256), of one key far above
+// 2000 others up to 2^36 times smaller 1.9e-4 (fp16); lse 3.4e-7 there, 3.3e-7 here.
+// B32 N16 T3001 H256 bf16: F = 2 411 -> 265 us, 4 767 -> 267, 8 1414 -> 270, 16 2772 -> 400 (6.0 TB/s at F = 4).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -107,23 +111,23 @@ __device__ __forceinline__ uint16_t from_f32(float x) {
   return kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(x)) : __half_as_ushort(__float2half_rn(x));
 }
 
-// Two probabilities as hi + lo pairs.  hi is the largest 16-bit number strictly below p (0 for p = 0),
-// so that lo > 0 wherever p > 0: with lo = 0 an infinite V would turn p * inf into inf + 0 * inf = NaN.
+// p >= 0 as the sum of two tf32 numbers.  hi is the largest of 11 bits strictly below p (0 for p = 0), so that
+// lo > 0 wherever p > 0: with lo = 0 an infinite V would turn p * inf into inf + 0 * inf = NaN.
+__device__ __forceinline__ void split_tf32(float p, uint32_t& hi, uint32_t& lo) {
+  const uint32_t bits = __float_as_uint(p);
+  hi = (p > 0.0f ? bits - 1u : bits) & 0xffffe000u;   // (NaN stays NaN)
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(p - __uint_as_float(hi)));
+}
+// The two 16-bit numbers of a register as tf32 (exact: tf32 has fp16's mantissa and bf16's exponents).
 template <bool kBf16>
-__device__ __forceinline__ void split_pair(float p0, float p1, uint32_t& hi, uint32_t& lo) {
-  const float b0 = p0 > 0.0f ? __uint_as_float(__float_as_uint(p0) - 1u) : p0;   // (NaN stays NaN)
-  const float b1 = p1 > 0.0f ? __uint_as_float(__float_as_uint(p1) - 1u) : p1;
+__device__ __forceinline__ void widen(uint32_t w, uint32_t& first, uint32_t& second) {
   if constexpr (kBf16) {
-    const float h0 = __uint_as_float(__float_as_uint(b0) & 0xffff0000u);
-    const float h1 = __uint_as_float(__float_as_uint(b1) & 0xffff0000u);
-    hi = __byte_perm(__float_as_uint(b0), __float_as_uint(b1), 0x7632);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(p0 - h0, p1 - h1);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
+    first = w << 16;
+    second = w & 0xffff0000u;
   } else {
-    const __half h0 = __float2half_rz(b0), h1 = __float2half_rz(b1);
-    hi = static_cast<uint32_t>(__half_as_ushort(h0)) | (static_cast<uint32_t>(__half_as_ushort(h1)) << 16);
-    const __half2 l = __floats2half2_rn(p0 - __half2float(h0), p1 - __half2float(h1));
-    lo = *reinterpret_cast<const uint32_t*>(&l);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+    first = __float_as_uint(f.x);
+    second = __float_as_uint(f.y);
   }
 }
 
@@ -144,16 +148,23 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
   return y;
 }
+// d = a . b
 template <bool kBf16>
 __device__ __forceinline__ void mma_16x8x16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   if constexpr (kBf16)
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
   else
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
+// d += a . b
+__device__ __forceinline__ void mma_16x8x8_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 template <int kSlabs, int kNT, bool kBf16>
@@ -319,7 +330,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         }
         const uint32_t k_tile = smem_base + slot * C::kStageBytes;
         const uint32_t v_tile = k_tile + C::kTileBytes;
-        // S^T: two accumulators per block of rows keep the chains short
+        // S^T: the products of 16 head elements each, summed in fp32 in two chains
         float acc[2][kNT][4];
 #pragma unroll
         for (int i = 0; i < 2; ++i)
@@ -331,19 +342,24 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         for (int ks = 0; ks < kSteps; ++ks) {
           uint32_t af[4];
           ldmatrix_x4(k_tile + (ks >> 2) * C::kBoxBytes + k_row * 128 + (((2 * (ks & 3) + k_col) ^ (k_row & 7)) << 4), af);
+          float part[kNT][4];
           if constexpr (C::kQShared) {
             uint32_t qb[4];     // b0, b1 of rows 0-7, b0, b1 of rows 8-15
             const int row = (lane & 7) + (lane >> 4) * 8;
             ldmatrix_x4(ptx::smem_u32(q_rows) + row * C::kHPad * 2 + (((2 * ks + ((lane >> 3) & 1)) ^ (row & 7)) << 4), qb);
-            mma_16x8x16<kBf16>(acc[ks & 1][0], af, qb[0], qb[1]);
-            mma_16x8x16<kBf16>(acc[ks & 1][kNT - 1], af, qb[2], qb[3]);
+            mma_16x8x16<kBf16>(part[0], af, qb[0], qb[1]);
+            mma_16x8x16<kBf16>(part[kNT - 1], af, qb[2], qb[3]);
           } else {
 #pragma unroll
-            for (int nt = 0; nt < kNT; ++nt) mma_16x8x16<kBf16>(acc[ks & 1][nt], af, qf[ks][nt][0], qf[ks][nt][1]);
+            for (int nt = 0; nt < kNT; ++nt) mma_16x8x16<kBf16>(part[nt], af, qf[ks][nt][0], qf[ks][nt][1]);
           }
+#pragma unroll
+          for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[ks & 1][nt][e] += part[nt][e];
         }
         const bool edge = key0 + 16 > a.T;   // (warp-uniform)
-        uint32_t p_hi[kNT][2], p_lo[kNT][2];
+        uint32_t p_hi[kNT][4], p_lo[kNT][4];   // row g (of a block): keys 2c, 2c + 1, 2c + 8, 2c + 9
 #pragma unroll
         for (int nt = 0; nt < kNT; ++nt) {
           float x[4];
@@ -382,21 +398,36 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
             l_run[nt][i & 1] += p[i];
           }
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {   // keys g (+ 8): [key][row] blocks turned into B fragments
-            uint32_t hi, lo;
-            split_pair<kBf16>(p[2 * i], p[2 * i + 1], hi, lo);
-            p_hi[nt][i] = transpose_8x8(hi);
-            p_lo[nt][i] = transpose_8x8(lo);
+          for (int i = 0; i < 2; ++i) {   // keys g (+ 8): [key][row] blocks turned over, the halves of P each
+            const uint32_t p0 = __float_as_uint(p[2 * i]), p1 = __float_as_uint(p[2 * i + 1]);
+            const uint32_t upper = transpose_8x8(__byte_perm(p0, p1, 0x7632));
+            const uint32_t lower = transpose_8x8(__byte_perm(p0, p1, 0x5410));
+            split_tf32(__uint_as_float(__byte_perm(lower, upper, 0x5410)), p_hi[nt][2 * i], p_lo[nt][2 * i]);
+            split_tf32(__uint_as_float(__byte_perm(lower, upper, 0x7632)), p_hi[nt][2 * i + 1], p_lo[nt][2 * i + 1]);
           }
         }
 #pragma unroll
         for (int mt = 0; mt < kSteps; ++mt) {
           uint32_t af[4];
           ldmatrix_x4_trans(v_tile + (mt >> 2) * C::kBoxBytes + v_row * 128 + (((2 * (mt & 3) + v_col) ^ (v_row & 7)) << 4), af);
+          // two products of 8 keys: 2c takes the place of key c, 2c + 1 that of c + 4, on both sides
+          uint32_t a8[2][4];
+          float part[kNT][4];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            widen<kBf16>(af[2 * i], a8[i][0], a8[i][2]);
+            widen<kBf16>(af[2 * i + 1], a8[i][1], a8[i][3]);
+          }
 #pragma unroll
           for (int nt = 0; nt < kNT; ++nt) {
-            mma_16x8x16<kBf16>(o[mt][nt], af, p_hi[nt][0], p_hi[nt][1]);
-            mma_16x8x16<kBf16>(o[mt][nt], af, p_lo[nt][0], p_lo[nt][1]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) part[nt][e] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) mma_16x8x8_tf32(part[nt], a8[i], p_lo[nt][2 * i], p_lo[nt][2 * i + 1]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) mma_16x8x8_tf32(part[nt], a8[i], p_hi[nt][2 * i], p_hi[nt][2 * i + 1]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[mt][nt][e] += part[nt][e];
           }
         }
         ptx::fence_proxy_async_smem();   // these reads come before the slot's next TMA write
@@ -495,7 +526,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         }
         if (threadIdx.x == 0) {
           if (whole) {
-            if (a.lse != nullptr) a.lse[static_cast<int64_t>(unit) * a.F + f] = (m_all + log2f(l_all)) * kLn2;
+            if (a.lse != nullptr) a.lse[static_cast<int64_t>(unit) * a.F + f] = fmaf(m_all, kLn2, logf(l_all));
           } else {
             part[f * (a.H + 2) + a.H] = m_all;
             part[f * (a.H + 2) + a.H + 1] = l_all;
@@ -538,7 +569,7 @@ fmha_decode_mma_combine_kernel(const __grid_constant__ Args a, int ctas) {
   }
   const int head = unit % a.N, batch = unit / a.N;
   if (d < a.H) a.out[batch * a.o_strides[0] + head * a.o_strides[1] + f * a.o_strides[2] + d] = from_f32<kBf16>(o / l_all);
-  if (d == 0 && a.lse != nullptr) a.lse[static_cast<int64_t>(unit) * a.F + f] = (m_all + log2f(l_all)) * kLn2;
+  if (d == 0 && a.lse != nullptr) a.lse[static_cast<int64_t>(unit) * a.F + f] = fmaf(m_all, kLn2, logf(l_all));
 }
 
 int slabs_of(int H) { return (H + 63) / 64; }
@@ -554,7 +585,7 @@ bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   // Under the mask row f sees keys 0..f: at most F keys of the cache count, and those behind them may not
   // have been written yet (a product with P = 0 would turn their NaN into the result's).  The split-key
   // kernel ends at the last row's key: B32 N16 H256, 3001 keys, F = 4: 38 us there, 271 as a pass over the
-  // whole cache; F = 16: 57 and 378.
+  // whole cache; F = 16: 57 and 400.
   if (p.causal) return false;
   // Two rows of a short cache stay with the split-key kernel: a unit's merge is paid for few keys
   // (B64 N16 H256, 33 keys: 31 us there, 36 us here; at 200 keys and B4 it is 22 and 19).

@@ -335,12 +335,38 @@ def test_decode_several_rows_causal_unwritten_cache(pkg, orc, cuda, F, H, dtype)
     orc.check_close(f32(lse), want_lse, rtol=1e-5, atol=1e-4, what="lse")
 
 
-def test_decode_several_rows_infinite_values(pkg, cuda):
-    """An infinite V element makes its output column infinite (never NaN) for every row that sees the key."""
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("F", [3, 12])
+@pytest.mark.parametrize("gap", [14, 25, 36])
+def test_decode_several_rows_one_dominant_key(pkg, cuda, dtype, F, gap):
+    """One key `gap` binades above 1999 others, with V = 0 there: the result is the sum of the small weights, which
+    count with the precision of fp32 whatever their size."""
+    import math
+    B, N, T, H = 1, 2, 2000, 64
+    g = torch.Generator().manual_seed(gap)
+    q = torch.ones(B, N, F, H, dtype=dtype)
+    k = torch.zeros(B, N, T, H, dtype=dtype)
+    k[:, :, 7, 0] = gap * math.sqrt(H) / math.log2(math.e)
+    v = torch.randn(B, N, T, H, generator=g).abs().mul(2.0 ** min(gap - 12, 14)).clamp(max=60000).to(dtype)
+    v[:, :, 7] = 0
+    want = torch.softmax((q.double() @ k.double().transpose(-1, -2)) * H ** -0.5, -1) @ v.double()
+    o, _ = run(pkg, q.to(cuda), k.to(cuda), v.to(cuda))
+    rel = ((o.cpu().double() - want).norm() / want.norm()).item()
+    assert rel <= (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -11)   # every element's one rounding at its worst
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("below", [0, 30, 110])
+def test_decode_several_rows_infinite_values(pkg, cuda, dtype, below):
+    """An infinite V element makes its output column infinite (never NaN) for every row that sees the key, also
+    where its weight is 2^-below of the weight of a key beside it."""
     B, N, F, T, H = 1, 2, 4, 300, 128
     g = torch.Generator().manual_seed(5)
-    q = torch.randn(B, N, F, H, generator=g).bfloat16().to(cuda)
-    k, v = (torch.randn(B, N, T, H, generator=g).bfloat16().to(cuda) for _ in range(2))
+    q = torch.randn(B, N, F, H, generator=g).to(dtype).to(cuda)
+    k, v = (torch.randn(B, N, T, H, generator=g).to(dtype).to(cuda) for _ in range(2))
+    if below:
+        q[..., 0], k[..., 0] = 1.0, 0.0
+        k[:, :, 35, 0] = below * H ** 0.5 * 0.6931
     v[:, :, 33, 7] = float("inf")
     o, _ = run(pkg, q, k, v)
     assert torch.all(torch.isposinf(o[..., 7]))
