@@ -587,10 +587,16 @@ def fmha_forward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: t
         raise IxkError(IXK_INVALID_ARGUMENT, "is_training needs the activation (log-sum-exp) buffer")
     lib = load_library()
     d = _fmha_desc(query, key, value, bias, out, head_scale, causal, 0.0 if dropout_prob in (None, 1.0) else dropout_prob)
-    workspace = _scratch(int(lib.ixk_fmha_fwd_workspace_bytes(ctypes.byref(d))), workspace, query.device, stream)
+    refused = None
+    try:
+        workspace = _scratch(int(lib.ixk_fmha_fwd_workspace_bytes(ctypes.byref(d))), workspace, query.device, stream)
+    except torch.OutOfMemoryError as e:
+        refused = e      # most calls only profit from scratch: those run without it
     ws_bytes = 0 if workspace is None else workspace.nbytes
     st = lib.ixk_fmha_fwd(ctypes.byref(d), _ptr(query), _ptr(key), _ptr(value), _ptr(bias), _ptr(out),
                           _ptr(activation if is_training else None), _ptr(workspace), ws_bytes, _stream_ptr(stream))
+    if refused is not None and st == IXK_WORKSPACE_TOO_SMALL:
+        raise refused
     _check(st)
 
 

@@ -144,3 +144,26 @@ def test_scratch_comes_from_the_pool_of_the_calls_stream(pkg, fake_calls, call):
     assert fake_calls.allocated == [77]
     run(stream, own)
     assert fake_calls.allocated == []
+
+
+@pytest.mark.parametrize("status", ["IXK_OK", "IXK_WORKSPACE_TOO_SMALL"])
+def test_forward_without_memory_for_scratch(pkg, fake_calls, monkeypatch, status):
+    """With no device memory left the forward goes in without scratch of its own: a prefill runs unsplit, as it
+    always could; only where the library cannot do without is the allocator's error the answer."""
+    q = torch.zeros(1, 2, 64, 32, dtype=torch.bfloat16)
+
+    def full(*args, **kwargs):
+        raise torch.OutOfMemoryError("no memory")
+    monkeypatch.setattr(torch, "empty", full)
+    fake_calls.lib.status = getattr(pkg, status)
+    for small in (None, torch.zeros(16, dtype=torch.uint8)):
+        fake_calls.lib.calls.clear()
+        run = lambda: pkg.fmha_forward_kernel(None, q, q, q, None, None, 0.0, q, None, 1.0, False, workspace=small)
+        monkeypatch.setattr(pkg, "_stream_ptr", lambda stream: 0)
+        if status == "IXK_OK":
+            run()
+        else:
+            with pytest.raises(torch.OutOfMemoryError):
+                run()
+        (_, args), = fake_calls.lib.calls
+        assert args[-3:-1] == ((None, 0) if small is None else (small.data_ptr(), 16))
