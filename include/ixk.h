@@ -250,10 +250,13 @@ size_t ixk_fmha_fwd_workspace_bytes(const ixk_fmha_desc* desc);
  * custom-call handler bound without a scratch allocator, or a process whose framework has already
  * reserved HBM for its own pool so that a library-side cudaMalloc would fail or stall the device.
  *
- * Same arguments and results as ixk_fmha_fwd, minus the workspace: the split-key decode path
- * keeps its partial results in an array of IXK_STATIC_SCRATCH_BYTES that is part of the library's
- * device image (each GPU that loads libixk.so holds that much memory until the process exits).
- * The call allocates nothing and frees nothing.
+ * Same arguments as ixk_fmha_fwd, minus the workspace: the decode path keeps its partial results in
+ * an array of IXK_STATIC_SCRATCH_BYTES that is part of the library's device image (each GPU that
+ * loads libixk.so holds that much memory until the process exits).  The call allocates nothing and
+ * frees nothing.  Where key splits need scratch, the result is that of ixk_fmha_fwd with that many
+ * bytes; where they need none, that of ixk_fmha_fwd without a workspace (a prefill is then never
+ * split along the keys, and decode calls of 2..16 rows for which one key split is enough run on the
+ * kernel that streams the cache once per two rows).
  *   - A problem whose key splits need more than IXK_STATIC_SCRATCH_BYTES is
  *     refused with IXK_WORKSPACE_TOO_SMALL and nothing is launched; use ixk_fmha_fwd then.
  *   - The first call on each device looks up the array's device address.  The call itself
@@ -261,7 +264,7 @@ size_t ixk_fmha_fwd_workspace_bytes(const ixk_fmha_desc* desc);
  *     runtime loads the part of the library image that holds the array, i.e. when the device
  *     memory behind it is actually reserved.  Make that first call at start-up, outside any stream
  *     capture; from the second call on, the free device memory does not change.
- *   - All calls on a device share the one array, which still holds the previous call's partials:
+ *   - All calls on a device whose key splits need scratch share the one array, which still holds the previous call's partials:
  *     the kernels overwrite every element they later read, so nothing needs clearing, but two
  *     calls that may overlap on the GPU (different streams, no ordering between them) race on it.
  *     Order them, or give the concurrent ones their own workspace through ixk_fmha_fwd. */

@@ -120,6 +120,8 @@ int ixk_fmha_fwd(const ixk_fmha_desc* desc, const void* q, const void* k, const 
   if ((rc = ixk::get_device_info(&dev)) != IXK_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   if (ixk::use_decode(p)) {
+    // (With less than the split-key kernel's scratch a call is refused, whichever kernel could do with it:
+    // callers size workspaces by the query, and what is refused does not depend on the kernel chosen.)
     const size_t split_key_need = ixk::fmha::decode_workspace_bytes(p, ixk::fmha::decode_splits(p, dev.sm_count));
     if (workspace_bytes >= split_key_need && ixk::fmha::decode_mma_applies(p, dev, workspace, workspace_bytes)) {
       rc = ixk::fmha::launch_decode_mma(p, dev, workspace, stream);

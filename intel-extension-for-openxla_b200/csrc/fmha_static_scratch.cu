@@ -10,9 +10,11 @@
 // The split-key decode path needs scratch for the per-split partial results.  Here that scratch
 // is a fixed array that lives in the library's device image: every GPU that loads libixk.so
 // carries IXK_STATIC_SCRATCH_BYTES of it until the process exits.  The entry point forwards to
-// the ordinary ixk_fmha_fwd with that array as the workspace, so results are identical to a
-// call that passes its own workspace of that size.  (Calls that only profit from scratch, such as
-// a prefill that is split along the keys, run without it: they share nothing with each other.)
+// the ordinary ixk_fmha_fwd with that array as the workspace where the problem's key splits need
+// scratch, and with none where they do not: results are those of a call with IXK_STATIC_SCRATCH_BYTES
+// of its own, or without any.  (A call that would only profit from scratch — a prefill split along the
+// keys, several decode rows where one key split is enough — keeps away from the array on purpose: such
+// calls share nothing, so they may overlap on the GPU.)
 #include <mutex>
 
 #include "host_common.h"

@@ -94,6 +94,26 @@ def test_python_wrapper_and_prefill_pass_through(pkg, orc, cuda):
     orc.check_close(f32(out), want, rtol=2e-2, atol=2e-2, what="static scratch prefill")
 
 
+@pytest.mark.parametrize("B,N,F,T,H,shares", [
+    (2, 4, 4, 4096, 256, True),       # key splits: the one-pass kernel on the library's array
+    (1, 2, 16, 1500, 128, True),
+    (19, 16, 16, 700, 64, False),     # one key split is enough: no scratch, the split-key kernel
+])
+def test_several_rows(pkg, cuda, B, N, F, T, H, shares):
+    """2..16 rows: the bits of the ordinary entry point with the array's size of workspace where key splits need
+    scratch, and without any where they do not."""
+    lib = pkg.load_library()
+    q, k, v = _inputs(cuda, B, N, F, T, H, seed=F)
+    got, want = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    got_lse, want_lse = (torch.full((B, N, F), float("nan"), device=cuda) for _ in range(2))
+    assert _call_static(pkg, q, k, v, got, got_lse) == pkg.IXK_OK
+    d = pkg._fmha_desc(q, k, v, None, want, H ** -0.5, False, 0.0)
+    ws = torch.empty(pkg.STATIC_SCRATCH_BYTES, dtype=torch.uint8, device=cuda) if shares else None
+    assert lib.ixk_fmha_fwd(ctypes.byref(d), q.data_ptr(), k.data_ptr(), v.data_ptr(), None, want.data_ptr(), want_lse.data_ptr(),
+                            pkg._ptr(ws), 0 if ws is None else ws.nbytes, torch.cuda.current_stream().cuda_stream) == pkg.IXK_OK
+    assert torch.equal(got, want) and torch.equal(got_lse, want_lse)
+
+
 def test_oversized_problem_is_refused_before_launch(pkg, cuda):
     # 2367 (batch, head) rows -> 2 key splits -> 2 x 2367 x 258 floats = 4.89 MB of partials > 4 MiB
     B, N, T, H = 263, 9, 512, 256
