@@ -298,6 +298,7 @@ MULTI_ROW_CASES = [
 @pytest.mark.parametrize("case", MULTI_ROW_CASES, ids=lambda c: "B{}N{}F{}T{}H{}{}c{}b{}".format(*c))
 def test_decode_several_rows(pkg, orc, cuda, case):
     B, N, F, T, H, dt, causal, use_bias = case
+    by_range = not causal and not (F == 2 and T <= 128)        # the kernel is the one-pass kernel
     dtype = torch.bfloat16 if dt == "bf16" else torch.float16
     g = torch.Generator().manual_seed(T + H)
     q = torch.randn(B, N, F, H, generator=g).to(dtype).to(cuda)
@@ -306,14 +307,62 @@ def test_decode_several_rows(pkg, orc, cuda, case):
     if use_bias:
         bias[..., 0] = torch.finfo(dtype).min       # a mask made of the type's lowest value
         bias[:, :, -1, : T // 2] = float("-inf")
+    launches = pkg.launch_count()
     o, lse = run(pkg, q, k, v, bias, causal, lse=True)
+    if by_range:      # a merge where a range boundary of equal shares of tiles cuts a unit, and only there
+        keys = 32 if H > 128 else 64
+        per_unit = -(-T // keys)
+        total = per_unit * B * N
+        ctas = max(min(148, -(-total * keys // 128), total, (4 << 20) // (8 * F * (H + 2))), 1)
+        assert pkg.launch_count() - launches == 1 + any(total * c // ctas % per_unit for c in range(1, ctas))
     want, want_lse = orc.fmha_forward(f32(q), f32(k), f32(v), None if bias is None else f32(bias), head_scale=H ** -0.5,
                                       causal=causal, dtype=orc.BF16 if dt == "bf16" else orc.F16, round_p=False)
-    # P is carried in 16 (bf16) or more bits and every sum in fp32: what is left is the one rounding of
-    # the result, which two correct sums may take to neighbouring values, one ulp = 2^-7 or 2^-10 apart
+    # P is carried in 22 bits and every sum in fp32: what is left is the one rounding of the result, which two correct sums may take to neighbouring values, one ulp = 2^-7 or 2^-10 apart
     ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
     orc.check_close(f32(o), want, rtol=ulp, atol=1e-4, what=str(case))
     orc.check_close(f32(lse), want_lse, rtol=1e-5, atol=1e-4, what=f"lse {case}")
+
+
+@pytest.mark.parametrize("F", [4, 12])
+@pytest.mark.parametrize("shared", ["heads", "batches", "both"])
+def test_decode_several_rows_shared_cache(pkg, orc, cuda, F, shared):
+    """K and V as expanded (stride 0) views: one cache for all heads or batches."""
+    B, N, T, H = 3, 5, 470, 136
+    g = torch.Generator().manual_seed(F)
+    q = torch.randn(B, N, F, H, generator=g).bfloat16().to(cuda)
+    size = (1 if shared != "heads" else B, 1 if shared != "batches" else N, T, H)
+    k, v = (torch.randn(*size, generator=g).bfloat16().to(cuda).expand(B, N, T, H) for _ in range(2))
+    o, lse = run(pkg, q, k, v, lse=True)
+    want, want_lse = orc.fmha_forward(f32(q), f32(k), f32(v), None, head_scale=H ** -0.5, dtype=orc.BF16, round_p=False)
+    orc.check_close(f32(o), want, rtol=2.0 ** -7, atol=1e-4, what=shared)
+    orc.check_close(f32(lse), want_lse, rtol=1e-5, atol=1e-4, what="lse")
+    dense, _ = run(pkg, q, k.contiguous(), v.contiguous())
+    assert torch.equal(o, dense)
+
+
+def test_decode_several_rows_little_scratch(pkg, cuda):
+    """Scratch for the split-key kernel but not for the one-pass kernel: the split-key kernel answers; less is refused."""
+    import ctypes
+    B, N, F, T, H = 40, 7, 16, 256, 64      # one key split; ranges cut units, so that the one-pass kernel wants scratch
+    g = torch.Generator().manual_seed(8)
+    q = torch.randn(B, N, F, H, generator=g).bfloat16().to(cuda)
+    k, v = (torch.randn(B, N, T, H, generator=g).bfloat16().to(cuda) for _ in range(2))
+    assert pkg.fmha_workspace_bytes(q, k, v, None, q, 1.0) > 0
+
+    def call(q, k, v, nbytes):
+        o = torch.full_like(q, float("nan"))
+        d = pkg._fmha_desc(q, k, v, None, o, H ** -0.5, False, 0.0)
+        ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=cuda)
+        return pkg.load_library().ixk_fmha_fwd(ctypes.byref(d), q.data_ptr(), k.data_ptr(), v.data_ptr(), None, o.data_ptr(), None,
+                                               ws.data_ptr() if nbytes else None, nbytes, torch.cuda.current_stream().cuda_stream), o
+    want, _ = run(pkg, q, k, v)
+    for nbytes in (0, 1024):
+        status, o = call(q, k, v, nbytes)
+        assert status == pkg.IXK_OK
+        # two kernels, each with one rounding of the result
+        assert torch.allclose(o.float(), want.float(), rtol=2.0 ** -7, atol=1e-4)
+    q, k, v = q[:2], k[:2, :, :200].repeat(1, 1, 5, 1), v[:2, :, :200].repeat(1, 1, 5, 1)      # four key splits
+    assert call(q, k, v, 1024)[0] == pkg.IXK_WORKSPACE_TOO_SMALL
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])

@@ -90,3 +90,56 @@ def test_gemma_decode_step_at_full_width(pkg, orc, cuda):
     assert pkg.launch_count() - n0 >= 5 * 2 + 2       # every projection split along K (+ reduce), attention + combine
     want = layers_oracle.gemma_decode_step(f32(x), {k: f32(v) for k, v in full.items()}, f32(kc), f32(vc), T - 1, heads, hd)
     orc.check_close(f32(y), want, rtol=2e-2, atol=6e-2, what="gemma decode, full width")
+
+
+@pytest.mark.parametrize("B", [1, 5])
+def test_decode_steps_overlap_without_changing_a_bit(pkg, cuda, monkeypatch, B):
+    """The kernels of a decode step start while their predecessors run and wait for them in front of their first
+    access.  Twelve steps over two layers' weights, each fed by the last, on the same buffers and scratch: the bits
+    of the same chain with the device idle before every launch, eagerly and as a graph replay."""
+    layers = importlib.import_module("ixk_b200.layers")
+    hidden, heads, hd, ffn, T, steps = 1024, 4, 256, 4096, 600, 6
+    g = torch.Generator(device=cuda).manual_seed(B)
+    r = lambda *s: (torch.randn(*s, generator=g, device=cuda) * 0.02).bfloat16()
+    weights = [layers.GemmaLayerWeights(wqkv=r(hidden, 3 * heads * hd), wo=r(heads * hd, hidden), wgateup=r(hidden, 2 * ffn),
+                                        wdown=r(ffn, hidden), heads_local=heads, head_dim=hd, norm_attn=r(hidden), norm_mlp=r(hidden))
+               for _ in range(2)]
+    x0 = torch.randn(B, 1, hidden, generator=g, device=cuda).bfloat16()
+    caches = [torch.randn(B, T, heads, hd, generator=g, device=cuda).bfloat16() for _ in range(4)]
+    ops = layers.KernelOps(pkg, gemm_workspace=torch.empty(32 << 20, dtype=torch.uint8, device=cuda))
+    workspace = torch.empty(8 << 20, dtype=torch.uint8, device=cuda)
+    ropes = [layers.rotary_tables(torch.tensor([T - steps + i], device=cuda), hd) for i in range(steps)]
+
+    def chain(c):
+        x = x0
+        for i in range(steps):
+            for n, w in enumerate(weights):
+                x = layers.gemma_decode_step(x, w, c[2 * n], c[2 * n + 1], T - steps + i, ops, workspace=workspace, rope=ropes[i])
+            x = pkg.residual_add(x, x)      # (no layer between: the next step's first norm reads what this one writes)
+        return x
+    stream_of = pkg._stream_ptr
+
+    def idle_first(stream):
+        torch.cuda.synchronize()
+        return stream_of(stream)
+    with monkeypatch.context() as m:
+        m.setattr(pkg, "_stream_ptr", idle_first)
+        apart = [c.clone() for c in caches]
+        want = chain(apart)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        together = [c.clone() for c in caches]
+        got = chain(together)
+        assert torch.equal(got, want) and all(torch.equal(a, b) for a, b in zip(together, apart))
+    together = [c.clone() for c in caches]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        got = chain(together)
+    for _ in range(3):
+        for t, c in zip(together, caches):
+            t.copy_(c)
+        graph.replay()
+        assert torch.equal(got, want) and all(torch.equal(a, b) for a, b in zip(together, apart))
+    del graph
