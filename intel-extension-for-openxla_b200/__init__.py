@@ -192,7 +192,7 @@ def device_status() -> int:
     return word.value
 
 
-# A decode step is a dozen launches of a few microseconds, so what Python does for each call is part of
+# A decode step is sixteen launches of a few microseconds, so what Python does for each call is part of
 # its time: descriptors are packed in one go, pointers and the stream travel as plain integers (the
 # current stream's handle is read without a Stream object around it).
 _current_device = getattr(torch._C, "_cuda_getDevice", None)
@@ -218,12 +218,10 @@ def _on_stream(stream, device):
     return torch.cuda.stream(stream)
 
 
-def _scratch(need: int, workspace: Optional[torch.Tensor], device, stream) -> Optional[torch.Tensor]:
-    """The caller's workspace where it holds `need` bytes, else one of the call's own.  That one is dropped when
-    the call returns, while its kernels may still run: it has to come from the pool of the stream they run on, whose
-    next tenant is ordered behind them.  (A block of another stream's pool could be in use there at once.)"""
-    if not need or (workspace is not None and workspace.nbytes >= need):
-        return workspace
+def _own_scratch(need: int, device, stream) -> torch.Tensor:
+    """Scratch that a call takes for itself.  It is dropped when the call returns, while its kernels may still run:
+    it has to come from the pool of the stream they run on, whose next tenant is ordered behind them.  (A block of
+    another stream's pool could be in use there at once.)"""
     if stream is None:
         return torch.empty(need, dtype=torch.uint8, device=device)
     with _on_stream(stream, device):
@@ -384,9 +382,9 @@ def gemm_geglu(x: torch.Tensor, w_gate_up: torch.Tensor, *, out: Optional[torch.
                    1, 1.0, 0.0, "DEFAULT")
     lib = load_library()
     if workspace is None:
-        workspace = _scratch(int(lib.ixk_gemm_geglu_workspace_bytes(ctypes.byref(d))), None, x.device, stream)
+        workspace = _own_scratch(lib.ixk_gemm_geglu_workspace_bytes(ctypes.byref(d)), x.device, stream)
     _check(lib.ixk_gemm_geglu(ctypes.byref(d), _ptr(x), _ptr(w_gate_up), _ptr(out), out.stride(-2), _ptr(workspace),
-                              0 if workspace is None else workspace.nbytes, _stream_ptr(stream)))
+                              workspace.nbytes, _stream_ptr(stream)))
     return out
 
 
@@ -588,10 +586,12 @@ def fmha_forward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: t
     lib = load_library()
     d = _fmha_desc(query, key, value, bias, out, head_scale, causal, 0.0 if dropout_prob in (None, 1.0) else dropout_prob)
     refused = None
-    try:
-        workspace = _scratch(int(lib.ixk_fmha_fwd_workspace_bytes(ctypes.byref(d))), workspace, query.device, stream)
-    except torch.OutOfMemoryError as e:
-        refused = e      # most calls only profit from scratch: those run without it
+    need = lib.ixk_fmha_fwd_workspace_bytes(ctypes.byref(d))
+    if need and (workspace is None or workspace.nbytes < need):
+        try:
+            workspace = _own_scratch(need, query.device, stream)
+        except torch.OutOfMemoryError as e:
+            refused = e      # most calls only profit from scratch: those run without it
     ws_bytes = 0 if workspace is None else workspace.nbytes
     st = lib.ixk_fmha_fwd(ctypes.byref(d), _ptr(query), _ptr(key), _ptr(value), _ptr(bias), _ptr(out),
                           _ptr(activation if is_training else None), _ptr(workspace), ws_bytes, _stream_ptr(stream))
@@ -636,7 +636,9 @@ def fmha_backward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: 
         raise IxkError(IXK_INVALID_ARGUMENT, "activation must be the forward's dense fp32 [B,N,F] log-sum-exp")
     lib = load_library()
     d = _fmha_bwd_desc(query, key, value, out, bias, grad_out, grad_query, grad_key, grad_value, head_scale, causal)
-    workspace = _scratch(int(lib.ixk_fmha_bwd_workspace_bytes(ctypes.byref(d))), workspace, query.device, stream)
+    need = lib.ixk_fmha_bwd_workspace_bytes(ctypes.byref(d))
+    if need and (workspace is None or workspace.nbytes < need):
+        workspace = _own_scratch(need, query.device, stream)
     ws_bytes = 0 if workspace is None else workspace.nbytes
     st = lib.ixk_fmha_bwd(ctypes.byref(d), _ptr(query), _ptr(key), _ptr(value), _ptr(out), _ptr(bias), _ptr(grad_out),
                           _ptr(activation), _ptr(grad_query), _ptr(grad_key), _ptr(grad_value), _ptr(workspace),
