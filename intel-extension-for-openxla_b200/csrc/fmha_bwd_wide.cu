@@ -15,9 +15,10 @@
 // matmul operands, all sums are fp32, each gradient is rounded once.  D and -lse*log2(e) come from
 // the shared prepare kernel.
 //
-// Measured, forward + backward at B4 N16 F=T=2048 H256 causal bf16: 2590 us as a chain of five GEMMs and
-// two elementwise passes, 745 with seven launches per group of eight heads, 641 as it is; of these 157
-// are the forward, 26 the prepare kernel and four times 53 + 50 the two kernels.
+// Measured at B4 N16 F=T=2048 H256 causal bf16, a call at a time with the L2 flushed: backward 2439 us as a
+// chain of five GEMMs and two elementwise passes, 492 as it is: 26 the prepare kernel and four groups of
+// 57 + 60 for the two kernels.  Forward and backward back to back, where the clock falls under the power cap:
+// 2596 and 713.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 

@@ -24,8 +24,8 @@
 // truncates what it accumulates, so every product starts at zero and is added to S and O in fp32.
 // Measured against 64 bits, B2 N16 T2000, heads of 64 to 256, 4 and 16 rows: relative error of O equal to the
 // split-key kernel's to six digits (1.6617e-3 bf16, 2.0851e-4 fp16 at head size 256), of one key far above
-// 2000 others up to 2^36 times smaller 1.9e-4 (fp16); lse 3.4e-7 there, 3.3e-7 here.
-// B32 N16 T3001 H256 bf16: F = 2 411 -> 265 us, 4 767 -> 267, 8 1414 -> 270, 16 2772 -> 400 (6.0 TB/s at F = 4).
+// 2000 others up to 2^36 times smaller 1.9e-4 (fp16); lse 3.6e-7 to 4.2e-7 there, 3.3e-7 to 3.7e-7 here.
+// B32 N16 T3001 H256 bf16: F = 2 411 -> 265 us, 4 765 -> 267 (5.9 TB/s), 8 1410 -> 269, 12 2106 -> 345, 16 2774 -> 398.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 

@@ -1083,7 +1083,8 @@ fmha_prefill_combine_kernel(const __grid_constant__ KernelArgs args, int first_i
 
 // Which items are split along the keys.  A CTA takes one item at a time, so a launch ends with a round in
 // which some CTAs have no item left, and a small problem is all such a round:
-//   non-causal   the items beyond the last full round, into as many parts as the idle CTAs can take
+//   non-causal   the items beyond the last full round, into as many parts as the idle CTAs can take (none
+//                where they fill more than half of a round: two parts each are two rounds of half the length)
 //   causal       only where there is not one item per CTA, all items, into parts of one length
 //                (with more items the work list balances them)
 // The merge costs a launch and a pass over the partials, about 4 us; a key block costs a CTA about 1.9 us:

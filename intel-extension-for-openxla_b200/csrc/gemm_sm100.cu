@@ -756,7 +756,7 @@ int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& 
     IXK_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
     configured_device = dev;
   }
-  // (bias, residual and auxiliary rows go through the read-only path: such a call starts in order)
+  // (bias and residual rows are read through the read-only path: such a call starts in order)
   if (args.bias == nullptr && args.c == nullptr) return launch_overlapped(fn, dim3(grid), dim3(kThreads), C::kSmemBytes, stream, ta, tb, td, args);
   fn<<<grid, kThreads, C::kSmemBytes, stream>>>(ta, tb, td, args);
   IXK_CUDA_OK(cudaGetLastError());

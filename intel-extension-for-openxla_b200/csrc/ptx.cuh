@@ -47,27 +47,16 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// The same after reads of tensor memory only (completed by tmem_ld_wait and ordered by
-// tc_fence_before_sync): no shared or global memory is handed over, so there is no release at cluster
-// scope, which waits for the thread's earlier stores and copies (about 2300 cycles per tile in
-// wide_scores_kernel's odd CTAs).
+// Arrive on the barrier at the same shared-memory offset in CTA `cta_rank` of the cluster, after reads of
+// tensor memory only (completed by tmem_ld_wait and ordered by tc_fence_before_sync): no shared or global
+// memory is handed over, so there is no release at cluster scope, which waits for the thread's earlier
+// stores and copies (about 2300 cycles per tile in wide_scores_kernel's odd CTAs).
 __device__ __forceinline__ void mbar_arrive_cluster_tmem(uint32_t bar, uint32_t cta_rank) {
   asm volatile(
       "{\n\t"
       ".reg .b32 remote;\n\t"
       "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
       "mbarrier.arrive.shared::cluster.b64 _, [remote];\n\t"
-      "}\n" ::"r"(bar),
-      "r"(cta_rank)
-      : "memory");
-}
-// Arrive on the barrier at the same shared-memory offset in CTA `cta_rank` of the cluster.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta_rank) {
-  asm volatile(
-      "{\n\t"
-      ".reg .b32 remote;\n\t"
-      "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n\t"
       "}\n" ::"r"(bar),
       "r"(cta_rank)
       : "memory");
