@@ -233,7 +233,8 @@ typedef struct ixk_fmha_desc {
  * probabilities handed to the P.V product are cut to bf16 by truncation, with the mean loss
  * (0.28 %) put back through the exponent and taken out of the row sum again, where the reference
  * rounds P to the storage type (fmha_forward.h:364-382); results agree within the 2e-2 the
- * parity tests allow, F16 and the decode path round to nearest.  lse (may be NULL) receives
+ * parity tests allow; F16 rounds to nearest.  The decode path (F <= 16) rounds no P: it is fp32, or for
+ * 2..16 rows in one pass over the cache the sum of two tf32 numbers (22 bits of it).  lse (may be NULL) receives
  * m + ln(l) per row — the reference's "activation" output when is_training
  * (fmha_forward.h:433-450).  workspace should hold ixk_fmha_fwd_workspace_bytes(desc) bytes.
  * The decode path (F <= 16) cannot do without the part of it that its key splits need and answers
@@ -255,8 +256,8 @@ size_t ixk_fmha_fwd_workspace_bytes(const ixk_fmha_desc* desc);
  * loads libixk.so holds that much memory until the process exits).  The call allocates nothing and
  * frees nothing.  Where key splits need scratch, the result is that of ixk_fmha_fwd with that many
  * bytes; where they need none, that of ixk_fmha_fwd without a workspace (a prefill is then never
- * split along the keys, and decode calls of 2..16 rows for which one key split is enough run on the
- * kernel that streams the cache once per two rows).
+ * split along the keys, and decode calls of 2..16 rows for which one key split is enough run in one
+ * pass over the cache only where that needs no scratch either).
  *   - A problem whose key splits need more than IXK_STATIC_SCRATCH_BYTES is
  *     refused with IXK_WORKSPACE_TOO_SMALL and nothing is launched; use ixk_fmha_fwd then.
  *   - The first call on each device looks up the array's device address.  The call itself

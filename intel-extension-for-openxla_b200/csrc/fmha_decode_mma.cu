@@ -9,8 +9,9 @@
 // (mma.sync and not tcgen05: with 8 rows the product is 3 % of what the tensor core could do in the time;
 // what counts is that nothing has to travel through tensor memory between the two products.)
 //
-//   CTAs      persistent, one per SM; the (batch, head) units are cut into tiles of keys, the tiles
-//             numbered through, and every CTA takes an equal, contiguous range
+//   CTAs      persistent, at most one per SM; the (batch, head) units are cut into tiles of keys, the tiles
+//             numbered through, and every CTA takes an equal, contiguous range of tiles or of whole units
+//             (make_plan)
 //   warp 8    TMA producer: K and V of a tile into one slot of a ring of up to 192 KB
 //   warps 0-7 16 keys of a tile each (so that a tile goes to 2 or 4 warps and the ring's slots are
 //             worked on side by side), every warp with its own running maximum, sum and O^T; merged
@@ -45,7 +46,6 @@ constexpr int kThreads = (kWarps + 4) * 32;       // and one of which a single w
 // 256 x 240 + 128 x 24 = 384 x 168.  (With 168 for all, the kernels for two blocks of rows spill up to 250 bytes.)
 constexpr int kComputeRegs = 240;
 constexpr int kLoadRegs = 24;
-constexpr int kMinKeysPerCta = 128;               // below that the merge costs more than the streaming saves
 constexpr size_t kMaxPartialBytes = IXK_STATIC_SCRATCH_BYTES;  // also the scratch of ixk_fmha_fwd_static_scratch
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -87,7 +87,7 @@ struct Cfg {
 struct Args {
   int B, N, H, F, T;
   float scale_log2;
-  int tiles_per_unit, total_tiles;
+  int tiles_per_unit, pieces, piece;
   const uint16_t* q;
   const uint16_t* bias;
   uint16_t* out;
@@ -98,8 +98,9 @@ struct Args {
   int* status_word;
 };
 
-__host__ __device__ __forceinline__ int range_begin(int total, int cta, int ctas) {
-  return static_cast<int>(static_cast<int64_t>(total) * cta / ctas);
+// First tile of a CTA's range: equal shares of `pieces` pieces of `piece` tiles (one tile, or a whole unit).
+__host__ __device__ __forceinline__ int range_begin(int pieces, int piece, int cta, int ctas) {
+  return static_cast<int>(static_cast<int64_t>(pieces) * cta / ctas) * piece;
 }
 
 template <bool kBf16>
@@ -203,8 +204,8 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   __syncthreads();
   ptx::grid_dependency_trigger();   // the combine kernel may be set up meanwhile; it waits for this grid's end
 
-  const int t_begin = range_begin(a.total_tiles, blockIdx.x, gridDim.x);
-  const int t_end = range_begin(a.total_tiles, blockIdx.x + 1, gridDim.x);
+  const int t_begin = range_begin(a.pieces, a.piece, blockIdx.x, gridDim.x);
+  const int t_end = range_begin(a.pieces, a.piece, blockIdx.x + 1, gridDim.x);
 
   if (warp >= kWarps) {
     // ------------------------------------------------------------ TMA producer
@@ -546,12 +547,12 @@ fmha_decode_mma_combine_kernel(const __grid_constant__ Args a, int ctas) {
   ptx::grid_dependency_wait();
   const int cta = blockIdx.x + 1;
   const int f = blockIdx.y;
-  const int cut = range_begin(a.total_tiles, cta, ctas);
+  const int cut = range_begin(a.pieces, a.piece, cta, ctas);
   const int unit = cut / a.tiles_per_unit;
   const int unit_t0 = unit * a.tiles_per_unit;
-  if (cut == unit_t0 || range_begin(a.total_tiles, cta - 1, ctas) > unit_t0) return;
+  if (cut == unit_t0 || range_begin(a.pieces, a.piece, cta - 1, ctas) > unit_t0) return;
   int last = cta;   // the CTA that finishes the unit
-  while (last + 1 < ctas && range_begin(a.total_tiles, last + 1, ctas) < unit_t0 + a.tiles_per_unit) ++last;
+  while (last + 1 < ctas && range_begin(a.pieces, a.piece, last + 1, ctas) < unit_t0 + a.tiles_per_unit) ++last;
   const int64_t pitch = static_cast<int64_t>(a.F) * (a.H + 2);
   const float* row = a.partial + f * (a.H + 2);
   auto part = [&](int c) { return row + (2 * c + (c == cta - 1 ? 1 : 0)) * pitch; };
@@ -575,30 +576,75 @@ fmha_decode_mma_combine_kernel(const __grid_constant__ Args a, int ctas) {
 int slabs_of(int H) { return (H + 63) / 64; }
 
 struct Plan {
-  int tiles_per_unit = 0, total_tiles = 0, ctas = 0;
+  int tiles_per_unit = 0, pieces = 0, piece = 1, ctas = 0;
   bool cut = false;   // some unit is shared by several CTAs
 };
+
+// What the two kernels take, in ns (L2-warm launches in a CUDA graph, bf16, 4 to 1024 units, 17 to 4096 keys, fitted
+// with 5 to 7 % mean error).  The split-key kernel runs two rows a CTA and two CTAs an SM in waves; here a unit costs
+// its merge, which grows with the rows and the head, beside its keys, and a cut unit the merge kernel.
+struct Cost {
+  int split_per_key, split_merge;                  // [slabs - 1]
+  int unit[2], row[2], per_key[2];                 // up to 8 rows, more
+};
+constexpr Cost kCosts[4] = {{14, 2800, {800, 1000}, {200, 260}, {6, 9}},
+                            {30, 3200, {1050, 1600}, {230, 320}, {8, 13}},
+                            {59, 3900, {1250, 2600}, {240, 330}, {15, 19}},
+                            {59, 4300, {1850, 3400}, {290, 370}, {18, 28}}};
+constexpr int kCutCost[2] = {4200, 4900}, kCutPerCta[2] = {170, 280};
+// Keys that a CTA streams in the time a cut costs, about: a unit is cut into ranges of at least half as many, and
+// whole units are dealt out unless the CTAs that go without in the last round could take more than that each.
+// (Whole units against equal shares of the tiles, 160 to 512 units, heads above 128: 0.73 of the time where that is
+// 64 to 128 keys, 0.95 at 400 to 512, 1.01 at 512 to 640, 1.13 at 1000 to 1400; smaller heads 0.68, 0.84, 0.90, 0.99.)
+constexpr int kKeysPerCut = 512;
+
 bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   const int keys = slabs_of(p.H) > 2 ? 32 : 64;
   const int64_t per_unit = (static_cast<int64_t>(p.T) + keys - 1) / keys;
-  const int64_t total = per_unit * p.B * p.N;
+  const int64_t units = static_cast<int64_t>(p.B) * p.N, total = per_unit * units;
+  if (p.F < 2 || p.F > kDecodeMaxQueries || total <= 0 || total > 0x7fffffff) return false;
   // Under the mask row f sees keys 0..f: at most F keys of the cache count, and those behind them may not
   // have been written yet (a product with P = 0 would turn their NaN into the result's).  The split-key
   // kernel ends at the last row's key: B32 N16 H256, 3001 keys, F = 4: 38 us there, 271 as a pass over the
   // whole cache; F = 16: 57 and 400.
   if (p.causal) return false;
-  // Two rows of a short cache stay with the split-key kernel: a unit's merge is paid for few keys
-  // (B64 N16 H256, 33 keys: 31 us there, 36 us here; at 200 keys and B4 it is 22 and 19).
-  if (p.F < 2 || p.F > kDecodeMaxQueries || (p.F == 2 && p.T <= kMinKeysPerCta) || total <= 0 || total > 0x7fffffff) return false;
+  const Cost& cost = kCosts[slabs_of(p.H) - 1];
+  const int wide = p.F > 8 ? 1 : 0;
   const int64_t cta_partials = 2 * static_cast<int64_t>(p.F) * (p.H + 2) * static_cast<int64_t>(sizeof(float));
   const int64_t fit = static_cast<int64_t>(kMaxPartialBytes) / cta_partials;
-  const int64_t useful = (total * keys + kMinKeysPerCta - 1) / kMinKeysPerCta;
+  const int64_t unit_ns = cost.unit[wide] + static_cast<int64_t>(cost.row[wide]) * p.F;
+  const int64_t keys_ns = static_cast<int64_t>(cost.per_key[wide]) * p.T;
+  // No more units than SMs: each unit is cut into as many ranges as there are SMs for it (72 units of 130 keys H256
+  // F16: 16 us, 30 as equal ranges of 128 keys and more that end anywhere).  More: whole units (B20 N16 H256 F16,
+  // 130 keys: 43 us, 59 cut), or equal shares of the tiles.
+  int64_t ctas, ns;
+  bool whole = true;
+  if (units <= sm_count) {
+    const int64_t ranges = std::max<int64_t>(std::min({sm_count / units, static_cast<int64_t>(2 * p.T / kKeysPerCut), fit / units}), 1);
+    whole = ranges == 1;
+    ctas = units * ranges;
+    ns = unit_ns + keys_ns / ranges + (whole ? 0 : kCutCost[wide] + kCutPerCta[wide] * ranges);
+  } else {
+    const int64_t per_cta = (units + sm_count - 1) / sm_count;
+    whole = (per_cta * sm_count - units) * p.T <= static_cast<int64_t>(kKeysPerCut) * sm_count;
+    ctas = whole ? sm_count : std::min<int64_t>(sm_count, fit);
+    ns = whole ? per_cta * (unit_ns + keys_ns) : unit_ns + units * (unit_ns + keys_ns) / sm_count + kCutCost[wide];
+  }
+  // The split-key kernel stays where the estimates do not put this one 10 % ahead: short caches, and few units with
+  // many rows (one-pass against split-key: 8 units of 480 keys H256 F16 23 and 20 us, F8 14 and 20; 1024 units of 17
+  // keys H256 F2 22 and 15).  Of 5600 sizes 20 are then more than 2 % slower than there, by half a microsecond.
+  const int splits = decode_splits(p, sm_count);
+  const int64_t split_ctas = units * ((p.F + 1) / 2) * splits, waves = (split_ctas + 2 * sm_count - 1) / (2 * sm_count);
+  const int64_t split_ns = 550 + waves * (2750 + static_cast<int64_t>(cost.split_per_key) * ((p.T + splits - 1) / splits)) +
+                           (splits > 1 ? cost.split_merge : 0);
+  if ((2500 + ns) * 11 > split_ns * 10) return false;
   plan->tiles_per_unit = static_cast<int>(per_unit);
-  plan->total_tiles = static_cast<int>(total);
-  plan->ctas = static_cast<int>(std::max<int64_t>(std::min({static_cast<int64_t>(sm_count), useful, total, fit}), 1));
+  plan->piece = whole ? static_cast<int>(per_unit) : 1;
+  plan->pieces = static_cast<int>(whole ? units : total);
+  plan->ctas = static_cast<int>(std::max<int64_t>(std::min<int64_t>(ctas, plan->pieces), 1));
   plan->cut = false;
   for (int c = 1; c < plan->ctas; ++c)
-    if (range_begin(plan->total_tiles, c, plan->ctas) % plan->tiles_per_unit != 0) plan->cut = true;
+    if (range_begin(plan->pieces, plan->piece, c, plan->ctas) % plan->tiles_per_unit != 0) plan->cut = true;
   return true;
 }
 size_t partial_bytes(const Problem& p, const Plan& plan) {
@@ -678,7 +724,8 @@ int launch_decode_mma(const Problem& p, const DeviceInfo& dev, void* workspace, 
   a.B = p.B; a.N = p.N; a.H = p.H; a.F = p.F; a.T = p.T;
   a.scale_log2 = p.head_scale * kLog2e;
   a.tiles_per_unit = plan.tiles_per_unit;
-  a.total_tiles = plan.total_tiles;
+  a.pieces = plan.pieces;
+  a.piece = plan.piece;
   a.q = static_cast<const uint16_t*>(p.q);
   a.bias = static_cast<const uint16_t*>(p.bias);
   a.out = static_cast<uint16_t*>(p.out);

@@ -294,7 +294,7 @@ __global__ void fmha_decode_combine_kernel(const DecodeArgs a) {
 // Query rows one CTA serves.  Two rows share every K and V load; with four the kernel is bound by
 // instruction issue (the per-row dot products and their shuffle reductions) and by the registers
 // of four accumulators (one CTA per SM), and ran slower than two passes of two rows.  More than one row
-// comes here under the causal mask, with a short cache or without scratch (fmha_decode_mma.cu takes the others).
+// comes here under the causal mask, and where fmha_decode_mma.cu's plan leaves it (short caches, little scratch).
 int decode_rows_per_cta(int F) { return F >= 2 ? 2 : 1; }
 
 int decode_splits(const Problem& p, int /*sm_count*/) {

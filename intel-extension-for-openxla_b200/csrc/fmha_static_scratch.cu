@@ -13,8 +13,8 @@
 // the ordinary ixk_fmha_fwd with that array as the workspace where the problem's key splits need
 // scratch, and with none where they do not: results are those of a call with IXK_STATIC_SCRATCH_BYTES
 // of its own, or without any.  (A call that would only profit from scratch — a prefill split along the
-// keys, several decode rows where one key split is enough — keeps away from the array on purpose: such
-// calls share nothing, so they may overlap on the GPU.)
+// keys, several decode rows for which one key split is enough but one pass would cut units — keeps away
+// from the array on purpose: such calls share nothing, so they may overlap on the GPU.)
 #include <mutex>
 
 #include "host_common.h"

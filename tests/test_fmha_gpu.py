@@ -273,8 +273,9 @@ def test_rejections(pkg, cuda):
     assert e.value.status == pkg.IXK_UNIMPLEMENTED          # head_size % 8
 
 
-# Several query rows in one pass over the cache (fmha_decode_mma.cu): tiles of 64 keys (32 above head
-# size 128) in slices of 16, blocks of 8 rows, head slabs of 64, ranges of tiles cut anywhere in a unit.
+# Several query rows: on the one-pass kernel (fmha_decode_mma.cu: tiles of 64 keys, 32 above head size 128, in
+# slices of 16, blocks of 8 rows, head slabs of 64, whole units or ranges of tiles cut anywhere in a unit) or, with a
+# short cache and few units, on the split-key kernel.
 MULTI_ROW_CASES = [
     # B, N, F, T, H, dtype, causal, bias
     (1, 1, 2, 1, 8, "bf16", False, False),          # one key, one 16-byte row
@@ -295,10 +296,45 @@ MULTI_ROW_CASES = [
 ]
 
 
+# ... and the last field: launches of the one-pass kernel's route (2 with the merge of cut units)
+ONE_PASS_CASES = [
+    (75, 8, 16, 1, 64, "bf16", False, False, 1),       # one key, full blocks of rows
+    (75, 8, 8, 17, 8, "bf16", False, True, 1),         # one key past a slice, one 16-byte row
+    (75, 4, 7, 17, 64, "fp16", False, False, 1),       # a row short of a block
+    (60, 5, 8, 65, 72, "bf16", False, True, 1),        # one key past a tile, a slab of 8 elements
+    (50, 6, 9, 63, 136, "fp16", False, False, 1),      # second block of rows, a tile of 32 keys and one of 31
+    (40, 8, 15, 33, 200, "bf16", False, True, 1),      # one key past a tile of 32
+    (150, 1, 4, 97, 256, "bf16", False, False, 1),     # two more units than CTAs
+    (1, 3, 7, 3100, 256, "fp16", False, False, 2),     # every unit cut into twelve ranges
+    (1, 1, 5, 5000, 256, "bf16", False, True, 2),      # one unit, 19 ranges
+    (2, 2, 16, 6000, 256, "bf16", False, False, 2),    # as many ranges as partials fit the scratch
+    (53, 3, 2, 1300, 64, "bf16", False, False, 2),     # equal shares of the tiles of 159 units
+    (53, 3, 12, 900, 192, "fp16", False, False, 2),
+]
+
+
+def kernel_names(fn):
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    return [e.key for e in prof.key_averages()]
+
+
+@pytest.mark.parametrize("case", ONE_PASS_CASES, ids=lambda c: "B{}N{}F{}T{}H{}{}c{}b{}".format(*c))
+def test_decode_several_rows_one_pass(pkg, orc, cuda, case):
+    *case, launches = case
+    B, N, F, T, H = case[:5]
+    dtype = torch.bfloat16 if case[5] == "bf16" else torch.float16
+    q, k = torch.zeros(B, N, F, H, dtype=dtype, device=cuda), torch.zeros(1, 1, T, H, dtype=dtype, device=cuda).expand(B, N, T, H)
+    n = pkg.launch_count()
+    names = kernel_names(lambda: run(pkg, q, k, k))
+    assert pkg.launch_count() - n == launches and any("fmha_decode_mma_kernel" in name for name in names), names
+    test_decode_several_rows(pkg, orc, cuda, case)
+
+
 @pytest.mark.parametrize("case", MULTI_ROW_CASES, ids=lambda c: "B{}N{}F{}T{}H{}{}c{}b{}".format(*c))
 def test_decode_several_rows(pkg, orc, cuda, case):
     B, N, F, T, H, dt, causal, use_bias = case
-    by_range = not causal and not (F == 2 and T <= 128)        # the kernel is the one-pass kernel
     dtype = torch.bfloat16 if dt == "bf16" else torch.float16
     g = torch.Generator().manual_seed(T + H)
     q = torch.randn(B, N, F, H, generator=g).to(dtype).to(cuda)
@@ -307,14 +343,7 @@ def test_decode_several_rows(pkg, orc, cuda, case):
     if use_bias:
         bias[..., 0] = torch.finfo(dtype).min       # a mask made of the type's lowest value
         bias[:, :, -1, : T // 2] = float("-inf")
-    launches = pkg.launch_count()
     o, lse = run(pkg, q, k, v, bias, causal, lse=True)
-    if by_range:      # a merge where a range boundary of equal shares of tiles cuts a unit, and only there
-        keys = 32 if H > 128 else 64
-        per_unit = -(-T // keys)
-        total = per_unit * B * N
-        ctas = max(min(148, -(-total * keys // 128), total, (4 << 20) // (8 * F * (H + 2))), 1)
-        assert pkg.launch_count() - launches == 1 + any(total * c // ctas % per_unit for c in range(1, ctas))
     want, want_lse = orc.fmha_forward(f32(q), f32(k), f32(v), None if bias is None else f32(bias), head_scale=H ** -0.5,
                                       causal=causal, dtype=orc.BF16 if dt == "bf16" else orc.F16, round_p=False)
     # P is carried in 22 bits and every sum in fp32: what is left is the one rounding of the result, which two correct sums may take to neighbouring values, one ulp = 2^-7 or 2^-10 apart
@@ -323,11 +352,11 @@ def test_decode_several_rows(pkg, orc, cuda, case):
     orc.check_close(f32(lse), want_lse, rtol=1e-5, atol=1e-4, what=f"lse {case}")
 
 
-@pytest.mark.parametrize("F", [4, 12])
+@pytest.mark.parametrize("F,T", [(4, 470), (12, 470), (4, 1100), (12, 1100)])
 @pytest.mark.parametrize("shared", ["heads", "batches", "both"])
-def test_decode_several_rows_shared_cache(pkg, orc, cuda, F, shared):
-    """K and V as expanded (stride 0) views: one cache for all heads or batches."""
-    B, N, T, H = 3, 5, 470, 136
+def test_decode_several_rows_shared_cache(pkg, orc, cuda, F, T, shared):
+    """K and V as expanded (stride 0) views: one cache for all heads or batches, whole units and cut ones."""
+    B, N, H = 3, 5, 136
     g = torch.Generator().manual_seed(F)
     q = torch.randn(B, N, F, H, generator=g).bfloat16().to(cuda)
     size = (1 if shared != "heads" else B, 1 if shared != "batches" else N, T, H)
@@ -343,7 +372,7 @@ def test_decode_several_rows_shared_cache(pkg, orc, cuda, F, shared):
 def test_decode_several_rows_little_scratch(pkg, cuda):
     """Scratch for the split-key kernel but not for the one-pass kernel: the split-key kernel answers; less is refused."""
     import ctypes
-    B, N, F, T, H = 40, 7, 16, 256, 64      # one key split; ranges cut units, so that the one-pass kernel wants scratch
+    B, N, F, T, H = 20, 16, 16, 700, 64     # one key split; ranges cut units, so that the one-pass kernel wants scratch
     g = torch.Generator().manual_seed(8)
     q = torch.randn(B, N, F, H, generator=g).bfloat16().to(cuda)
     k, v = (torch.randn(B, N, T, H, generator=g).bfloat16().to(cuda) for _ in range(2))
@@ -361,8 +390,7 @@ def test_decode_several_rows_little_scratch(pkg, cuda):
         assert status == pkg.IXK_OK
         # two kernels, each with one rounding of the result
         assert torch.allclose(o.float(), want.float(), rtol=2.0 ** -7, atol=1e-4)
-    q, k, v = q[:2], k[:2, :, :200].repeat(1, 1, 5, 1), v[:2, :, :200].repeat(1, 1, 5, 1)      # four key splits
-    assert call(q, k, v, 1024)[0] == pkg.IXK_WORKSPACE_TOO_SMALL
+    assert call(q[:2], k[:2], v[:2], 1024)[0] == pkg.IXK_WORKSPACE_TOO_SMALL
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
@@ -391,7 +419,7 @@ def test_decode_several_rows_one_dominant_key(pkg, cuda, dtype, F, gap):
     """One key `gap` binades above 1999 others, with V = 0 there: the result is the sum of the small weights, which
     count with the precision of fp32 whatever their size."""
     import math
-    B, N, T, H = 1, 2, 2000, 64
+    B, N, T, H = 8, 10, 2000, 64
     g = torch.Generator().manual_seed(gap)
     q = torch.ones(B, N, F, H, dtype=dtype)
     k = torch.zeros(B, N, T, H, dtype=dtype)
@@ -409,7 +437,7 @@ def test_decode_several_rows_one_dominant_key(pkg, cuda, dtype, F, gap):
 def test_decode_several_rows_infinite_values(pkg, cuda, dtype, below):
     """An infinite V element makes its output column infinite (never NaN) for every row that sees the key, also
     where its weight is 2^-below of the weight of a key beside it."""
-    B, N, F, T, H = 1, 2, 4, 300, 128
+    B, N, F, T, H = 2, 3, 4, 300, 128
     g = torch.Generator().manual_seed(5)
     q = torch.randn(B, N, F, H, generator=g).to(dtype).to(cuda)
     k, v = (torch.randn(B, N, T, H, generator=g).to(dtype).to(cuda) for _ in range(2))

@@ -96,8 +96,9 @@ def test_python_wrapper_and_prefill_pass_through(pkg, orc, cuda):
 
 @pytest.mark.parametrize("B,N,F,T,H,shares", [
     (2, 4, 4, 4096, 256, True),       # key splits: the one-pass kernel on the library's array
-    (1, 2, 16, 1500, 128, True),
-    (19, 16, 16, 700, 64, False),     # one key split is enough: no scratch, the split-key kernel
+    (2, 4, 3, 1031, 128, True),
+    (19, 16, 16, 700, 64, False),     # one key split is enough, cut units want scratch: the split-key kernel
+    (75, 4, 16, 120, 64, False),      # no kernel wants any: the one-pass kernel on whole units
 ])
 def test_several_rows(pkg, cuda, B, N, F, T, H, shares):
     """2..16 rows: the bits of the ordinary entry point with the array's size of workspace where key splits need
