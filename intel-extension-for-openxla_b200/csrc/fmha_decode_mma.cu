@@ -10,8 +10,8 @@
 // what counts is that nothing has to travel through tensor memory between the two products.)
 //
 //   CTAs      persistent, at most one per SM; the (batch, head) units are cut into tiles of keys, the tiles
-//             numbered through, and every CTA takes an equal, contiguous range of tiles or of whole units
-//             (make_plan)
+//             numbered through, and every CTA takes whole units, a range of one unit, or an equal share of
+//             all tiles (make_plan)
 //   warp 8    TMA producer: K and V of a tile into one slot of a ring of up to 192 KB
 //   warps 0-7 16 keys of a tile each (so that a tile goes to 2 or 4 warps and the ring's slots are
 //             worked on side by side), every warp with its own running maximum, sum and O^T; merged
@@ -87,12 +87,12 @@ struct Cfg {
 struct Args {
   int B, N, H, F, T;
   float scale_log2;
-  int tiles_per_unit, pieces, piece;
+  int tiles_per_unit, pieces, piece, slots;
   const uint16_t* q;
   const uint16_t* bias;
   uint16_t* out;
   float* lse;
-  float* partial;   // [2 * grid][F][H + 2]: the unit a CTA's range starts inside of, and the one it starts
+  float* partial;   // [grid][slots][F][H + 2]: with two, the unit a CTA's range starts inside of and the one it starts
   int k_head_mul, k_batch_mul, v_head_mul, v_batch_mul;   // 0: one K / V for all heads / batches
   int64_t q_strides[3], o_strides[3], bias_strides[3];
   int* status_word;
@@ -503,7 +503,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       }
       ptx::named_barrier_sync(1, kWarps * 32);
       const bool whole = t == unit_t0 && seg_end == unit_t0 + a.tiles_per_unit;
-      float* part = a.partial + (static_cast<int64_t>(blockIdx.x) * 2 + (t == unit_t0 ? 1 : 0)) * a.F * (a.H + 2);
+      float* part = a.partial + (static_cast<int64_t>(blockIdx.x) * a.slots + (a.slots == 2 && t == unit_t0 ? 1 : 0)) * a.F * (a.H + 2);
       for (int f = 0; f < a.F; ++f) {
         float m_all = -INFINITY;
 #pragma unroll
@@ -555,7 +555,7 @@ fmha_decode_mma_combine_kernel(const __grid_constant__ Args a, int ctas) {
   while (last + 1 < ctas && range_begin(a.pieces, a.piece, last + 1, ctas) < unit_t0 + a.tiles_per_unit) ++last;
   const int64_t pitch = static_cast<int64_t>(a.F) * (a.H + 2);
   const float* row = a.partial + f * (a.H + 2);
-  auto part = [&](int c) { return row + (2 * c + (c == cta - 1 ? 1 : 0)) * pitch; };
+  auto part = [&](int c) { return row + (a.slots * c + (a.slots == 2 && c == cta - 1 ? 1 : 0)) * pitch; };
   float m_all = -INFINITY;
   for (int c = cta - 1; c <= last; ++c) m_all = fmaxf(m_all, part(c)[a.H]);
   float l_all = 0.0f, o = 0.0f;
@@ -577,7 +577,7 @@ int slabs_of(int H) { return (H + 63) / 64; }
 
 struct Plan {
   int tiles_per_unit = 0, pieces = 0, piece = 1, ctas = 0;
-  bool cut = false;   // some unit is shared by several CTAs
+  int slots = 0;      // partials that a CTA may leave: 0 whole units, 1 a range inside a unit, 2 a range over several
 };
 
 // What the two kernels take, in ns (L2-warm launches in a CUDA graph, bf16, 4 to 1024 units, 17 to 4096 keys, fitted
@@ -591,12 +591,7 @@ constexpr Cost kCosts[4] = {{14, 2800, {800, 1000}, {200, 260}, {6, 9}},
                             {30, 3200, {1050, 1600}, {230, 320}, {8, 13}},
                             {59, 3900, {1250, 2600}, {240, 330}, {15, 19}},
                             {59, 4300, {1850, 3400}, {290, 370}, {18, 28}}};
-constexpr int kCutCost[2] = {4200, 4900}, kCutPerCta[2] = {170, 280};
-// Keys that a CTA streams in the time a cut costs, about: a unit is cut into ranges of at least half as many, and
-// whole units are dealt out unless the CTAs that go without in the last round could take more than that each.
-// (Whole units against equal shares of the tiles, 160 to 512 units, heads above 128: 0.73 of the time where that is
-// 64 to 128 keys, 0.95 at 400 to 512, 1.01 at 512 to 640, 1.13 at 1000 to 1400; smaller heads 0.68, 0.84, 0.90, 0.99.)
-constexpr int kKeysPerCut = 512;
+constexpr int kCutCost[2] = {4200, 4900}, kCutPerRange[2] = {170, 280};
 
 bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   const int keys = slabs_of(p.H) > 2 ? 32 : 64;
@@ -610,45 +605,47 @@ bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   if (p.causal) return false;
   const Cost& cost = kCosts[slabs_of(p.H) - 1];
   const int wide = p.F > 8 ? 1 : 0;
-  const int64_t cta_partials = 2 * static_cast<int64_t>(p.F) * (p.H + 2) * static_cast<int64_t>(sizeof(float));
-  const int64_t fit = static_cast<int64_t>(kMaxPartialBytes) / cta_partials;
+  const int64_t fit = static_cast<int64_t>(kMaxPartialBytes / (static_cast<size_t>(p.F) * (p.H + 2) * sizeof(float)));
   const int64_t unit_ns = cost.unit[wide] + static_cast<int64_t>(cost.row[wide]) * p.F;
   const int64_t keys_ns = static_cast<int64_t>(cost.per_key[wide]) * p.T;
-  // No more units than SMs: each unit is cut into as many ranges as there are SMs for it (72 units of 130 keys H256
-  // F16: 16 us, 30 as equal ranges of 128 keys and more that end anywhere).  More: whole units (B20 N16 H256 F16,
-  // 130 keys: 43 us, 59 cut), or equal shares of the tiles.
-  int64_t ctas, ns;
-  bool whole = true;
-  if (units <= sm_count) {
-    const int64_t ranges = std::max<int64_t>(std::min({sm_count / units, static_cast<int64_t>(2 * p.T / kKeysPerCut), fit / units}), 1);
-    whole = ranges == 1;
-    ctas = units * ranges;
-    ns = unit_ns + keys_ns / ranges + (whole ? 0 : kCutCost[wide] + kCutPerCta[wide] * ranges);
-  } else {
-    const int64_t per_cta = (units + sm_count - 1) / sm_count;
-    whole = (per_cta * sm_count - units) * p.T <= static_cast<int64_t>(kKeysPerCut) * sm_count;
-    ctas = whole ? sm_count : std::min<int64_t>(sm_count, fit);
-    ns = whole ? per_cta * (unit_ns + keys_ns) : unit_ns + units * (unit_ns + keys_ns) / sm_count + kCutCost[wide];
+  // Whole units; or, with no more units than SMs, each cut into equal ranges (equal shares of the tiles, which end
+  // anywhere, were slower there: 16 units of 480 keys H256 F4 17 us, 11 whole); or, with more, equal shares (B20 N16
+  // H256 F16, 130 keys: 59 us, 43 whole; 160 to 512 units H256, where the CTAs that go without in the last round could
+  // take 64 to 128 keys each, 1 : 0.73, at 1000 to 1400 keys 1 : 1.13).
+  int64_t ns = (units + sm_count - 1) / sm_count * (unit_ns + keys_ns), ranges = 1;
+  plan->slots = 0;
+  for (int64_t r = 2; r <= std::min({sm_count / units, static_cast<int64_t>(p.T / 128), fit / units}); ++r) {
+    const int64_t t = unit_ns + keys_ns / r + kCutCost[wide] + kCutPerRange[wide] * r;
+    if (t < ns) {
+      ns = t;
+      ranges = r;
+      plan->slots = 1;
+    }
   }
-  // The split-key kernel stays where the estimates do not put this one 10 % ahead: short caches, and few units with
+  const int64_t shares = std::min<int64_t>(sm_count, fit / 2);
+  if (units > sm_count && shares > 1) {
+    const int64_t t = unit_ns + units * (unit_ns + keys_ns) / shares + kCutCost[wide];
+    if (t < ns) {
+      ns = t;
+      plan->slots = 2;
+    }
+  }
+  // The split-key kernel stays where the estimates do not put this one 5 % ahead: short caches, and few units with
   // many rows (one-pass against split-key: 8 units of 480 keys H256 F16 23 and 20 us, F8 14 and 20; 1024 units of 17
-  // keys H256 F2 22 and 15).  Of 5600 sizes 20 are then more than 2 % slower than there, by half a microsecond.
+  // keys H256 F2 22 and 15).
   const int splits = decode_splits(p, sm_count);
   const int64_t split_ctas = units * ((p.F + 1) / 2) * splits, waves = (split_ctas + 2 * sm_count - 1) / (2 * sm_count);
   const int64_t split_ns = 550 + waves * (2750 + static_cast<int64_t>(cost.split_per_key) * ((p.T + splits - 1) / splits)) +
                            (splits > 1 ? cost.split_merge : 0);
-  if ((2500 + ns) * 11 > split_ns * 10) return false;
+  if ((2500 + ns) * 21 > split_ns * 20) return false;
   plan->tiles_per_unit = static_cast<int>(per_unit);
-  plan->piece = whole ? static_cast<int>(per_unit) : 1;
-  plan->pieces = static_cast<int>(whole ? units : total);
-  plan->ctas = static_cast<int>(std::max<int64_t>(std::min<int64_t>(ctas, plan->pieces), 1));
-  plan->cut = false;
-  for (int c = 1; c < plan->ctas; ++c)
-    if (range_begin(plan->pieces, plan->piece, c, plan->ctas) % plan->tiles_per_unit != 0) plan->cut = true;
+  plan->piece = plan->slots == 0 ? static_cast<int>(per_unit) : 1;
+  plan->pieces = static_cast<int>(plan->slots == 0 ? units : total);
+  plan->ctas = static_cast<int>(plan->slots == 0 ? std::min<int64_t>(units, sm_count) : plan->slots == 1 ? units * ranges : shares);
   return true;
 }
 size_t partial_bytes(const Problem& p, const Plan& plan) {
-  return plan.cut ? static_cast<size_t>(plan.ctas) * 2 * p.F * (p.H + 2) * sizeof(float) : 0;
+  return static_cast<size_t>(plan.ctas) * plan.slots * p.F * (p.H + 2) * sizeof(float);
 }
 
 template <int kSlabs, int kNT, bool kBf16>
@@ -664,7 +661,7 @@ int launch_typed(const CUtensorMap& tk, const CUtensorMap& tv, const Args& a, co
   fn<<<plan.ctas, kThreads, C::kSmemBytes, stream>>>(tk, tv, a);
   IXK_CUDA_OK(cudaGetLastError());
   count_launch();
-  if (plan.cut) {
+  if (plan.slots > 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(plan.ctas - 1, a.F, 1);
     cfg.blockDim = dim3(256, 1, 1);
@@ -726,6 +723,7 @@ int launch_decode_mma(const Problem& p, const DeviceInfo& dev, void* workspace, 
   a.tiles_per_unit = plan.tiles_per_unit;
   a.pieces = plan.pieces;
   a.piece = plan.piece;
+  a.slots = plan.slots;
   a.q = static_cast<const uint16_t*>(p.q);
   a.bias = static_cast<const uint16_t*>(p.bias);
   a.out = static_cast<uint16_t*>(p.out);

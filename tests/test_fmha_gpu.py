@@ -372,7 +372,7 @@ def test_decode_several_rows_shared_cache(pkg, orc, cuda, F, T, shared):
 def test_decode_several_rows_little_scratch(pkg, cuda):
     """Scratch for the split-key kernel but not for the one-pass kernel: the split-key kernel answers; less is refused."""
     import ctypes
-    B, N, F, T, H = 20, 16, 16, 700, 64     # one key split; ranges cut units, so that the one-pass kernel wants scratch
+    B, N, F, T, H = 19, 16, 16, 700, 64     # one key split; shares of the tiles, so that the one-pass kernel wants scratch
     g = torch.Generator().manual_seed(8)
     q = torch.randn(B, N, F, H, generator=g).bfloat16().to(cuda)
     k, v = (torch.randn(B, N, T, H, generator=g).bfloat16().to(cuda) for _ in range(2))
@@ -461,9 +461,21 @@ SPLIT_CASES = [
     (19, 8, 200, 1500, 64, "bf16", False, False, "bsnh"),      # whole items in a full round, four split ones behind it
     (1, 2, 1300, 1300, 128, "bf16", True, False, "bsnh"),     # causal: parts with work for the second tile only
     (1, 1, 2049, 2049, 40, "fp16", True, False, "bnsh"),
-    (1, 2, 700, 1900, 256, "bf16", True, True, "bnsh"),       # more keys than queries; bias and mask
+    (1, 2, 1100, 1900, 256, "bf16", True, True, "bnsh"),      # more keys than queries; bias and mask
     (1, 1, 1500, 900, 96, "bf16", True, False, "bnsh"),       # fewer keys than queries
 ]
+
+
+@pytest.mark.parametrize("shape", [(1, 16, 700, 700, 128, False), (3, 8, 700, 700, 128, True), (1, 16, 1500, 1500, 128, True),
+                                   (10, 10, 640, 640, 64, False)], ids=lambda s: "x".join(map(str, s)))
+def test_prefill_not_split_where_the_merge_costs_more(pkg, cuda, shape):
+    """Sizes that took 20 to 50 % longer split than whole."""
+    B, N, F, T, H, causal = shape
+    q, k = (torch.zeros(B, N, S, H, dtype=torch.bfloat16, device=cuda) for S in (F, T))
+    assert pkg.fmha_workspace_bytes(q, k, k, None, q, 1.0, causal) == 0
+    n = pkg.launch_count()
+    run(pkg, q, k, k, causal=causal)
+    assert pkg.launch_count() - n == 1
 
 
 @pytest.mark.parametrize("case", SPLIT_CASES, ids=lambda c: "B{}N{}F{}T{}H{}{}c{}b{}{}".format(*c))
