@@ -1110,19 +1110,21 @@ SplitPlan split_plan(const KernelArgs& a, int64_t items, int sms) {
   const int tail = a.causal ? 0 : static_cast<int>(items % sms);
   if (a.causal ? items >= sms : tail == 0) return plan;
   const int longest = item_blocks<kQTiles>(a, a.num_qblocks - 1);
-  const int64_t rounds = (items + sms - 1) / sms;
+  const int64_t pairs = static_cast<int64_t>(a.N) * a.B, rounds = (items + sms - 1) / sms;
+  int64_t blocks = static_cast<int64_t>(tail) * longest;   // to be cut, at most sms parts
+  if (a.causal)
+    for (int qb = 0; qb < a.num_qblocks; ++qb) blocks += pairs * item_blocks<kQTiles>(a, qb);
   int64_t best = (8000 + rounds * longest * cost.block) * 6 / 100;
-  for (int len = 2; len < longest; ++len) {
-    int64_t parts = 0;
+  for (int len = static_cast<int>(std::max<int64_t>(2, (blocks + sms - 1) / sms)); len < longest; ++len) {
+    const int64_t saved = static_cast<int64_t>(longest - len) * cost.block - cost.merge[a.causal];
+    if (saved <= best) break;
+    int64_t parts = static_cast<int64_t>(tail) * ((longest + len - 1) / len);
     if (a.causal) {
       for (int qb = 0; qb < a.num_qblocks; ++qb) parts += (item_blocks<kQTiles>(a, qb) + len - 1) / len;
-      parts *= static_cast<int64_t>(a.N) * a.B;
-    } else {
-      parts = static_cast<int64_t>(tail) * ((longest + len - 1) / len);
+      parts *= pairs;
     }
-    if (parts > sms) continue;
-    const int64_t gain = static_cast<int64_t>(longest - len) * cost.block - cost.merge[a.causal] - parts * kQTiles * cost.tile[a.causal];
-    if (gain > best) {
+    const int64_t gain = saved - parts * kQTiles * cost.tile[a.causal];
+    if (parts <= sms && gain > best) {
       best = gain;
       plan.num_direct = a.causal ? 0 : static_cast<int>(items - tail);
       plan.split_len = len;

@@ -167,3 +167,50 @@ def test_forward_without_memory_for_scratch(pkg, fake_calls, monkeypatch, status
                 run()
         (_, args), = fake_calls.lib.calls
         assert args[-3:-1] == ((None, 0) if small is None else (small.data_ptr(), 16))
+
+
+def _workspace(pkg, B, N, F, T, H, causal):
+    import ctypes
+    d = pkg._FmhaDesc()
+    d.dtype, d.causal = pkg.IXK_BF16, int(causal)
+    d.num_batches, d.num_heads, d.head_size, d.num_queries, d.num_keys, d.head_scale = B, N, H, F, T, 1.0
+    return pkg.load_library().ixk_fmha_fwd_workspace_bytes(ctypes.byref(d))
+
+
+def test_scratch_of_a_split_prefill(pkg):
+    """The query (made without a GPU for 148 SMs): partials of at most one part per SM, 128 rows of the padded head
+    and two statistics each; none with a row of items per SM under the mask, or where the merge costs more."""
+    import random
+    rng = random.Random(4)
+    split = 0
+    for _ in range(2000):
+        B, N, H = rng.randint(1, 16), rng.randint(1, 16), rng.choice([40, 64, 96, 128, 160, 256])
+        F, T, causal = rng.randint(17, 5000), rng.randint(1, 6000), rng.random() < 0.5
+        need = _workspace(pkg, B, N, F, T, H, causal)
+        padded = 64 if H <= 64 else 128 if H <= 128 else 256
+        tiles, rest = divmod(need, 128 * (padded + 2) * 4)
+        per_item = 2 if F > 128 and H <= 128 else 1
+        assert rest == 0 and tiles % per_item == 0 and tiles // per_item <= 148
+        items = -(-F // (128 * per_item)) * B * N
+        assert need == 0 or (items < 148 if causal else items % 148 != 0)
+        split += need > 0
+    assert split > 300
+    assert _workspace(pkg, 2, 10, 4096, 4096, 64, False) == 144 * 2 * 128 * 66 * 4          # 24 items in parts of six blocks
+    assert _workspace(pkg, 3, 8, 700, 700, 128, True) == 0                                  # slower split than whole
+    assert _workspace(pkg, 1, 1, 100000, 100000, 128, True) == 0                            # an item per SM and more
+
+
+@pytest.mark.parametrize("F", range(1, 17))
+def test_scratch_of_a_decode_call(pkg, F):
+    """What the key splits need, which a call cannot do without, or the one-pass kernel's partials (at most 4 MiB) where
+    those are more; under the mask the key splits alone."""
+    import random
+    rng = random.Random(F)
+    for _ in range(300):
+        B, N, T, H = rng.randint(1, 64), rng.randint(1, 32), rng.randint(1, 9000), 8 * rng.randint(1, 32)
+        groups = B * N * -(-F // (2 if F > 1 else 1))
+        splits = max(min(-(-16 * 148 // groups), -(-T // 256)), 1)
+        key_splits = splits * B * N * F * (H + 2) * 4 if splits > 1 else 0
+        need = _workspace(pkg, B, N, F, T, H, False)
+        assert need == key_splits or key_splits < need <= pkg.STATIC_SCRATCH_BYTES
+        assert _workspace(pkg, B, N, F, T, H, True) == key_splits
