@@ -26,7 +26,7 @@
 // Measured against 64 bits, B2 N16 T2000, heads of 64 to 256, 4 and 16 rows: relative error of O equal to the
 // split-key kernel's to six digits (1.6617e-3 bf16, 2.0851e-4 fp16 at head size 256), of one key far above
 // 2000 others up to 2^36 times smaller 1.9e-4 (fp16); lse 3.6e-7 to 4.2e-7 there, 3.3e-7 to 3.7e-7 here.
-// B32 N16 T3001 H256 bf16: F = 2 411 -> 265 us, 4 765 -> 267 (5.9 TB/s), 8 1410 -> 269, 12 2106 -> 345, 16 2774 -> 398.
+// B32 N16 T3001 H256 bf16: F = 2 411 -> 265 us, 4 765 -> 267 (5.9 TB/s), 8 1410 -> 269, 12 2106 -> 345, 16 2771 -> 377.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -601,7 +601,7 @@ bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   // Under the mask row f sees keys 0..f: at most F keys of the cache count, and those behind them may not
   // have been written yet (a product with P = 0 would turn their NaN into the result's).  The split-key
   // kernel ends at the last row's key: B32 N16 H256, 3001 keys, F = 4: 38 us there, 271 as a pass over the
-  // whole cache; F = 16: 57 and 400.
+  // whole cache; F = 16: 57 and 377.
   if (p.causal) return false;
   const Cost& cost = kCosts[slabs_of(p.H) - 1];
   const int wide = p.F > 8 ? 1 : 0;
@@ -632,7 +632,8 @@ bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   }
   // The split-key kernel stays where the estimates do not put this one 5 % ahead: short caches, and few units with
   // many rows (one-pass against split-key: 8 units of 480 keys H256 F16 23 and 20 us, F8 14 and 20; 1024 units of 17
-  // keys H256 F2 22 and 15).
+  // keys H256 F2 22 and 15).  95 of the 5600 sizes are more than 2 % slower by this choice, 15 % at most; on average
+  // they take 0.53 of the split-key kernel's time.
   const int splits = decode_splits(p, sm_count);
   const int64_t split_ctas = units * ((p.F + 1) / 2) * splits, waves = (split_ctas + 2 * sm_count - 1) / (2 * sm_count);
   const int64_t split_ns = 550 + waves * (2750 + static_cast<int64_t>(cost.split_per_key) * ((p.T + splits - 1) / splits)) +
