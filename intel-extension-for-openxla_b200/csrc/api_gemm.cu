@@ -1,6 +1,7 @@
 // GEMM entry points: the host logic of RunGemm (xla/service/gpu/onednn_matmul_utils.cc:533-621)
 // — attribute dictionary → matrix descriptors → column-major-output rewrite → typed dispatch —
 // restated over the C ABI, in front of the tcgen05 kernel.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <utility>
@@ -238,15 +239,20 @@ int run(const ixk_gemm_desc* desc, const void* a, const void* b, const void* c, 
     if (workspace == nullptr || !aligned16(workspace) || workspace_bytes < need)
       return fail(IXK_WORKSPACE_TOO_SMALL, "GeGLU projection: need " + std::to_string(need) + " bytes of 16-byte aligned scratch");
     p.ldd = geglu_ld;   // of the [M, N'] result; the product itself goes to the scratch
-    return gemm::launch_split_k(p, splits, workspace, dev, static_cast<cudaStream_t>(stream), true);
+    return gemm::launch_split_k(p, gemm::stream_applies(p) ? gemm::stream_splits(p.M, p.N, p.K, es, workspace_bytes) : splits, workspace, dev, static_cast<cudaStream_t>(stream), true);
   }
 
   if (const char* env = std::getenv("IXK_GEMM_BLOCK_N")) p.force_block_n = std::atoi(env);
 
   DeviceInfo dev;
   if ((rc = get_device_info(&dev)) != IXK_OK) return rc;
-  // Skinny problems are cut along K when the caller handed over enough scratch for the partials;
+  // Skinny problems are cut along K as far as the caller handed over scratch for the partials;
   // without it they run un-split (same result, fewer SMs busy).
+  if (gemm::stream_applies(p)) {
+    const int splits = gemm::stream_splits(p.M, p.N, p.K, es, workspace != nullptr && aligned16(workspace) ? workspace_bytes : 0);
+    return splits > 1 ? gemm::launch_split_k(p, splits, workspace, dev, static_cast<cudaStream_t>(stream))
+                      : gemm::launch_stream(p, 1, nullptr, dev, static_cast<cudaStream_t>(stream));
+  }
   const int splits = (p.force_block_n > 0 || p.aux != nullptr) ? 1 : gemm::split_k_factor(p.M, p.N, p.K, p.batch, p.fp8);
   if (splits > 1 && workspace != nullptr && aligned16(workspace) &&
       workspace_bytes >= gemm::split_k_workspace_bytes(p.M, p.N, splits))
@@ -328,7 +334,9 @@ size_t workspace_query(const ixk_gemm_desc* desc) {
   const int64_t K = desc->lhs.num_cols;
   const bool fp8 = is_fp8(desc->lhs.dtype);
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  return gemm::split_k_workspace_bytes(M, N, gemm::split_k_factor(M, N, K, desc->batch_size, fp8));
+  const size_t tiled = gemm::split_k_workspace_bytes(M, N, gemm::split_k_factor(M, N, K, desc->batch_size, fp8));
+  if (!gemm::stream_takes(M, N) || desc->batch_size != 1) return tiled;
+  return std::max(tiled, gemm::split_k_workspace_bytes(M, N, gemm::stream_splits(M, N, K, elem_bytes(desc->lhs.dtype), SIZE_MAX / 4)));
 }
 
 }  // namespace

@@ -26,6 +26,7 @@ constexpr int kThreads = kWarps * 32;
 constexpr int kUnroll = 4;      // keys in flight per lane group
 constexpr int kMinKeysPerSplit = 256;
 constexpr int kTargetCtas = 16 * 148;
+constexpr int kCarveoutPercent = 30;   // of an SM's L1 as shared memory (see launch_decode)
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
@@ -361,8 +362,17 @@ int launch_decode(const Problem& p, const DeviceInfo& dev, void* workspace, size
   dim3 grid(splits * ((p.F + rows_per_cta - 1) / rows_per_cta), p.N, p.B);
   auto launch_lanes = [&](auto lanes_tag) -> int {
     constexpr int kLanes = decltype(lanes_tag)::value;
-    return launch_overlapped(rows_per_cta == 1 ? fmha_decode_kernel<kLanes, 1> : fmha_decode_kernel<kLanes, 2>, grid, dim3(kThreads), 0,
-                             stream, a);
+    auto* fn = rows_per_cta == 1 ? fmha_decode_kernel<kLanes, 1> : fmha_decode_kernel<kLanes, 2>;
+    // What a load has in flight lives in L1.  Behind kernels that leave an SM no idle moment the split between L1 and
+    // shared memory stays what the last large kernel wanted, so this one states its own: B64 N16 T4096 H256 inside a
+    // decoder layer 700 us with a GEMM of two CTAs per SM before it, 640 with 30 % (the same as launched in order;
+    // 15 % 655, 0 % 1312: too little shared memory for the CTAs).
+    static thread_local int configured_device[2] = {-1, -1};
+    if (configured_device[rows_per_cta - 1] != dev.device) {
+      IXK_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveoutPercent));
+      configured_device[rows_per_cta - 1] = dev.device;
+    }
+    return launch_overlapped(fn, grid, dim3(kThreads), 0, stream, a);
   };
   int rc;
   if (p.H <= 64) rc = launch_lanes(std::integral_constant<int, 8>{});

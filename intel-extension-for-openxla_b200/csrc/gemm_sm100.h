@@ -84,5 +84,11 @@ size_t split_k_workspace_bytes(int64_t M, int64_t N, int splits);
 int launch_split_k(const Problem& p, int splits, void* workspace, const DeviceInfo& dev, cudaStream_t stream,
                    bool geglu = false);
 
+// Few rows: the problem as a stream of the weights (gemm_stream.cu).
+bool stream_takes(int64_t M, int64_t N);
+bool stream_applies(const Problem& p);
+int stream_splits(int64_t M, int64_t N, int64_t K, int elem_bytes, size_t workspace_bytes);
+int launch_stream(const Problem& p, int splits, float* partial, const DeviceInfo& dev, cudaStream_t stream);
+
 }  // namespace gemm
 }  // namespace ixk

@@ -1,12 +1,15 @@
-// Split-K for skinny GEMMs (M <= 128: decode-time projections, where the whole problem is one
+// Split-K for skinny GEMMs (decode-time projections, where the whole problem is one
 // stream of the weight matrix through the chip).  With a single row of output tiles there are too
-// few tiles to occupy 148 SMs, so the K range is cut into `splits` chunks that run as the batch
-// dimension of the tensor-core kernel (each chunk writes an fp32 partial [M, N] into the caller's
-// workspace), and this file's second kernel sums the partials and applies the epilogue once.
+// few tiles to occupy 148 SMs, so the K range is cut into `splits` chunks, each of which leaves an fp32
+// partial [M, N] in the caller's workspace (gemm_stream_kernel; for an A with its rows contiguous, which that kernel
+// does not take, the batch dimension of gemm_kernel), and this file's kernel sums the partials and applies the
+// epilogue once.
 // The reference reaches the same end with shared-local-memory k-slicing inside a work-group
 // (SLM_KS in xla/service/gpu/xetla/gemm/gemm_dispatch.h:183-214); here the slices are CTAs.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <algorithm>
 
 #include "gemm_sm100.h"
 #include "ptx.cuh"
@@ -64,9 +67,25 @@ __device__ __forceinline__ void reduce_epilogue_store(const ReduceArgs& a, int m
   store_from_f32(a.d, static_cast<int64_t>(m) * a.ldd + n, a.out_dtype, v);
 }
 
-// A thread sums four consecutive columns of one row over the chunks, in chunk order, with the
-// loads of all chunks in flight together (kVec: N is a multiple of 4, so the partial planes can be
-// read 16 bytes at a time); otherwise one element per thread.
+// Four consecutive columns of one row summed over the chunks, in chunk order, with the loads of eight chunks in flight
+// together: a decode step's reduce is a few dozen threads whose time is the number of trips to L2.
+__device__ __forceinline__ float4 sum_chunks(const float4* src, int64_t plane4, int splits) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < splits; s0 += 8) {
+    float4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = s0 + i < splits ? src[(s0 + i) * plane4] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      acc.x += v[i].x;
+      acc.y += v[i].y;
+      acc.z += v[i].z;
+      acc.w += v[i].w;
+    }
+  }
+  return acc;
+}
+// (kVec: N is a multiple of 4, so the partial planes can be read 16 bytes at a time; otherwise one element per thread.)
 __device__ __forceinline__ float round_to(float v, int dtype) {
   if (dtype == IXK_BF16) return __bfloat162float(__float2bfloat16_rn(v));
   if (dtype == IXK_F16) return __half2float(__float2half_rn(v));
@@ -87,13 +106,7 @@ __global__ void splitk_reduce_geglu_kernel(const ReduceArgs a) {
     const int n = static_cast<int>(i - static_cast<int64_t>(m) * h4) * 4;
     const float4* gsrc = reinterpret_cast<const float4*>(a.partial) + (static_cast<int64_t>(m) * a.N + n) / 4;
     const float4* usrc = gsrc + h4;
-    float4 g = make_float4(0.f, 0.f, 0.f, 0.f), u = g;
-#pragma unroll 4
-    for (int s = 0; s < a.splits; ++s) {
-      const float4 gv = gsrc[s * plane4], uv = usrc[s * plane4];
-      g.x += gv.x; g.y += gv.y; g.z += gv.z; g.w += gv.w;
-      u.x += uv.x; u.y += uv.y; u.z += uv.z; u.w += uv.w;
-    }
+    const float4 g = sum_chunks(gsrc, plane4, a.splits), u = sum_chunks(usrc, plane4, a.splits);
     const float gs[4] = {g.x, g.y, g.z, g.w}, us[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e)
@@ -113,16 +126,7 @@ __global__ void splitk_reduce_kernel(const ReduceArgs a) {
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
       const int m = static_cast<int>(i / n4);
       const int n = static_cast<int>(i - static_cast<int64_t>(m) * n4) * 4;
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4* src = reinterpret_cast<const float4*>(a.partial) + i;
-#pragma unroll 4
-      for (int s = 0; s < a.splits; ++s) {
-        const float4 v = src[s * (plane / 4)];
-        acc.x += v.x;
-        acc.y += v.y;
-        acc.z += v.z;
-        acc.w += v.w;
-      }
+      const float4 acc = sum_chunks(reinterpret_cast<const float4*>(a.partial) + i, plane / 4, a.splits);
       reduce_epilogue_store(a, m, n, acc.x);
       reduce_epilogue_store(a, m, n + 1, acc.y);
       reduce_epilogue_store(a, m, n + 2, acc.z);
@@ -141,6 +145,16 @@ __global__ void splitk_reduce_kernel(const ReduceArgs a) {
 }
 
 }  // namespace
+
+// Threads and CTAs for `total` items: small CTAs where that spreads few items over more SMs.
+struct ReduceGrid {
+  unsigned blocks, threads;
+};
+static ReduceGrid reduce_grid(int64_t total, int sm_count) {
+  const unsigned threads = total <= 256 * static_cast<int64_t>(sm_count) ? 64 : 256;
+  const int64_t blocks = std::min<int64_t>((total + threads - 1) / threads, static_cast<int64_t>(kReduceCtasPerSm) * sm_count);
+  return ReduceGrid{static_cast<unsigned>(blocks), threads};
+}
 
 int split_k_factor(int64_t M, int64_t N, int64_t K, int64_t batch, bool fp8) {
   if (batch != 1 || M > 128 || fp8) return 1;
@@ -188,7 +202,7 @@ int launch_split_k(const Problem& p, int splits, void* workspace, const DeviceIn
   part.ldd = p.N;
   part.d_batch_stride = p.M * p.N;
   part.force_block_n = 128;
-  int rc = launch(part, dev, stream);
+  int rc = stream_applies(p) ? launch_stream(p, splits, static_cast<float*>(workspace), dev, stream) : launch(part, dev, stream);
   if (rc != IXK_OK) return rc;
 
   ReduceArgs r{};
@@ -208,17 +222,13 @@ int launch_split_k(const Problem& p, int splits, void* workspace, const DeviceIn
   r.geglu = geglu ? 1 : 0;
   if (geglu) {
     const int64_t total = p.M * (p.N / 8);
-    int64_t blocks = (total + 255) / 256;
-    if (blocks > kReduceCtasPerSm * dev.sm_count) blocks = kReduceCtasPerSm * dev.sm_count;
-    return launch_overlapped(splitk_reduce_geglu_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, r);
+    const ReduceGrid g = reduce_grid(total, dev.sm_count);
+    return launch_overlapped(splitk_reduce_geglu_kernel, dim3(g.blocks), dim3(g.threads), 0, stream, r);
   }
   const bool vec = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0;
   const int64_t total = vec ? p.M * p.N / 4 : p.M * p.N;
-  const int threads = 256;
-  int64_t blocks = (total + threads - 1) / threads;
-  if (blocks > kReduceCtasPerSm * dev.sm_count) blocks = kReduceCtasPerSm * dev.sm_count;
-  return launch_overlapped(vec ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3(static_cast<unsigned>(blocks)),
-                           dim3(threads), 0, stream, r);
+  const ReduceGrid g = reduce_grid(total, dev.sm_count);
+  return launch_overlapped(vec ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3(g.blocks), dim3(g.threads), 0, stream, r);
 }
 
 }  // namespace gemm

@@ -497,3 +497,42 @@ def test_cta_pair_last_round(pkg, cuda, monkeypatch, shape, kind, la, lb):
     assert ((out.double() - want).abs().max() <= tol * want.abs().max()).item()
     monkeypatch.setenv("IXK_GEMM_PAIR", "0")
     assert torch.equal(out, run())
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 8), (1, 5000, 1000), (3, 16384, 600), (16, 72, 136), (17, 520, 4096), (33, 1032, 248), (100, 2000, 304),
+                                   (128, 648, 20000), (128, 64, 128), (129, 2064, 1160), (256, 1000, 18936)],
+                         ids=lambda s: "M{}K{}N{}".format(*s))
+@pytest.mark.parametrize("kind", ["bf16", "fp16", "e4m3"])
+@pytest.mark.parametrize("lb", ["row", "col"])
+@pytest.mark.parametrize("scratch", [True, False])
+def test_few_rows(pkg, cuda, shape, kind, lb, scratch):
+    """Few rows: rows, columns and K that end inside a tile or a slab, one chunk of K and many, with the epilogue in the
+    GEMM and in the pass behind it."""
+    M, K, N = shape
+    es = 1 if kind == "e4m3" else 2
+    if any(d * es % 16 for d in (K, N if lb == "row" else K)):
+        K, N = (K + 15) // 16 * 16, (N + 15) // 16 * 16
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x, w = torch.randn(M, K, generator=g, device=cuda), torch.randn(K, N, generator=g, device=cuda) * 0.05
+    dtype = {"bf16": torch.bfloat16, "fp16": torch.float16, "e4m3": torch.float8_e4m3fn}[kind]
+    x, w = x.to(dtype), w.to(dtype)
+    wd = as_layout(w, lb)
+    out_dtype = torch.bfloat16 if kind == "e4m3" else dtype
+    bias = torch.randn(N, generator=g, device=cuda).to(out_dtype)
+    want = x.double() @ w.double() + bias.double()
+    half = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -11    # one rounding of the result: 8 and 11 bits
+    sums = (K + 16) * 2.0 ** -23 * (x.double().abs() @ w.double().abs() + 1).max()   # fp32 sums, each addition cut off at 24 bits
+    if kind == "e4m3":
+        out = pkg.gemm_fp8(x, wd, 0.5, 2.0, bias=bias, epilogue="BIAS_RELU")
+    else:
+        need = pkg.gemm_workspace_bytes(x, wd)
+        ws = torch.full((need,), 255, dtype=torch.uint8, device=cuda) if scratch and need else None
+        n0 = pkg.launch_count()
+        out = pkg.gemm(x, wd, bias=bias, epilogue="BIAS_RELU", workspace=ws)
+        assert pkg.launch_count() - n0 == (2 if ws is not None else 1)
+    assert ((out.double() - want.relu()).abs().max() <= 1.01 * half * want.abs().max() + sums).item()
+    if kind != "e4m3":
+        c = torch.randn(M, N, generator=g, device=cuda)
+        out32 = pkg.gemm(x, wd, c=c, beta=-0.5, out=torch.empty_like(c), workspace=ws)
+        want = x.double() @ w.double() - 0.5 * c.double()
+        assert ((out32.double() - want).abs().max() <= sums + 2.0 ** -22 * c.abs().max()).item()
