@@ -130,6 +130,7 @@ int ixk_fmha_fwd(const ixk_fmha_desc* desc, const void* q, const void* k, const 
     }
     return ixk::fmha::launch_decode(p, dev, workspace, workspace_bytes, stream);
   }
+  if (ixk::fmha::short_applies(p)) return ixk::fmha::launch_short(p, dev, stream);
   return ixk::fmha::launch_prefill(p, dev, workspace, workspace_bytes, stream);
 }
 

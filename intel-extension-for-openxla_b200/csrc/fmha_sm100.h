@@ -34,6 +34,10 @@ constexpr int kDecodeMaxQueries = 16;
 size_t prefill_workspace_bytes(const Problem& p, int sm_count);
 int launch_prefill(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 
+// ---- the same for at most 128 keys without a bias, head sizes up to 128 (fmha_short_sm100.cu); no scratch
+bool short_applies(const Problem& p);
+int launch_short(const Problem& p, const DeviceInfo& dev, cudaStream_t stream);
+
 // ---- split-key decode kernel (fmha_decode_sm100.cu): one query row, and what the one-pass kernel leaves
 // Number of key splits chosen for a problem, and the scratch it needs:
 // splits * B*N*F * (H + 2) floats (partial O, running max, running sum).

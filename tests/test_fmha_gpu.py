@@ -532,3 +532,37 @@ def test_scratch_of_a_call_on_another_stream(pkg, cuda):
         assert sum(s["total_size"] for s in held) >= need
         del held
         torch.cuda.empty_cache()                                      # (the second round has to take its own)
+
+
+@pytest.mark.parametrize("case", [
+    # B, N, F, T, H, dtype, causal, layout
+    (1, 1, 17, 1, 8, "bf16", False, "bnsh"),              # one key, one row past the decode kernels
+    (2, 3, 128, 128, 64, "fp16", True, "bsnh"),           # full tiles, diagonal
+    (2, 20, 300, 77, 64, "fp16", False, "bsnh"),          # ragged rows and keys, many CTAs per SM
+    (1, 2, 129, 16, 40, "bf16", False, "bsnh"),           # one row in the last tile
+    (1, 2, 400, 33, 72, "bf16", True, "bnsh"),            # more rows than keys under the mask; two boxes, the second short
+    (2, 2, 100, 100, 128, "bf16", True, "bsnh"),
+    (1, 5, 257, 113, 128, "fp16", False, "bnsh"),
+    (1, 2, 60, 90, 96, "bf16", False, "odd"),             # O rows that TMA cannot store
+    (2, 4, 140, 50, 64, "bf16", False, "mqa"),            # one K and V for all heads
+], ids=lambda c: "B{}N{}F{}T{}H{}{}c{}{}".format(*c))
+def test_at_most_128_keys(pkg, orc, cuda, case):
+    """One block of keys: the kernel without a running maximum, at the edges of its tiles."""
+    B, N, F, T, H, dt, causal, lay = case
+    dtype = {"bf16": torch.bfloat16, "fp16": torch.float16}[dt]
+    g = torch.Generator().manual_seed(F * 3 + T)
+    def mk(s, n=N):
+        if lay in ("bsnh", "mqa"):
+            return torch.randn(B, s, n, H, generator=g).to(dtype).to(cuda).permute(0, 2, 1, 3)
+        return torch.randn(B, n, s, H, generator=g).to(dtype).to(cuda)
+    q, k, v = mk(F), mk(T, 1 if lay == "mqa" else N), mk(T, 1 if lay == "mqa" else N)
+    k, v = k.expand(B, N, T, H), v.expand(B, N, T, H)
+    o = torch.full((B, N, F, H + 3), float("nan"), dtype=dtype, device=cuda)[..., :H] if lay == "odd" else torch.full_like(q, float("nan"))
+    lse = torch.full((B, N, F), float("nan"), dtype=torch.float32, device=cuda)
+    pkg.fmha_forward_kernel(None, q, k, v, None, None, 0.0, o, lse, H ** -0.5, True, causal=causal)
+    want, want_lse = orc.fmha_forward(f32(q), f32(k), f32(v), None, head_scale=H ** -0.5, causal=causal,
+                                      dtype=orc.BF16 if dt == "bf16" else orc.F16)
+    # P and O rounded once each to 8 (11) bits, against outputs of at most a few units
+    tol = 2e-2 if dt == "bf16" else 3e-3
+    orc.check_close(f32(o), want, rtol=tol, atol=tol, what=str(case))
+    orc.check_close(f32(lse), want_lse, rtol=1e-4, atol=1e-4, what=f"lse {case}")
