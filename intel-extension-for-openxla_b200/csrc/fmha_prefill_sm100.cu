@@ -70,18 +70,23 @@ enum : int { kSiteLoad = 201, kSiteMmaQ = 202, kSiteMmaKV = 203, kSiteMmaP = 204
               kSiteLoadQ = 207, kSiteMmaO = 208, kSiteLoadBias = 209, kSiteSoftmaxBias = 210 };
 
 constexpr int kBiasTileBytes = 2 * kChunkBytes;  // 128 query rows x 128 keys, 16-bit, as two swizzled boxes
+// How an additive bias reaches shared memory: not at all, by TMA, or, where its address or strides do not suit
+// TMA (a pitch of an odd number of elements, a row broadcast over the queries), as aligned 4-byte words that the
+// control warpgroup's two spare warps copy.
+enum : int { kNoBias = 0, kBiasTma = 1, kBiasWords = 2 };
+constexpr int kBiasWarp = 10;     // kBiasWords: warp kBiasWarp + t copies query tile t's bias
 constexpr int kBiasPrefetch = 8;  // 16-byte groups of a bias row (the first box) read before the scores arrive
 
-template <int kHeadDim, int kQTiles, bool kBias>
+template <int kHeadDim, int kQTiles, int kBias>
 struct Cfg {
   static constexpr int kChunks = kHeadDim / kChunkElems;          // 128-byte column blocks per row
   static constexpr int kTileBytes = kChunks * kChunkBytes;        // a 128-row Q, K or V tile
-  // with a TMA-fed bias tile per query tile the K/V ring gives up one slot to make room
+  // with a bias tile per query tile the K/V ring gives up one slot to make room
   static constexpr int kKvSlots = (kHeadDim == 256) ? 2 : (kBias ? 3 : 4);
   static constexpr int kQBytes = kQTiles * kTileBytes;
   static constexpr int kBiasBytes = kBias ? kQTiles * kBiasTileBytes : 0;
   // O leaves through shared memory and TMA stores, one 64-column box per query tile at a time
-  // (no room is left for it beside the TMA-fed bias tiles: that variant stores from registers)
+  // (no room is left for it beside the bias tiles: those variants store from registers)
   static constexpr int kStageBytes = kBias ? 0 : kQTiles * kChunkBytes;
   static constexpr int kSmemBytes = kQBytes + kKvSlots * kTileBytes + kBiasBytes + kStageBytes + 320 + 2 * kBlockQ * 4 + 1024;
   static_assert(kSmemBytes <= 232448, "shared memory budget");
@@ -98,7 +103,6 @@ struct KernelArgs {
   float head_scale;
   const uint16_t* bias;
   int64_t bias_strides[3];
-  int bias_vec_ok;
   uint16_t* out;
   int64_t o_strides[3];
   int out_vec_ok;
@@ -308,7 +312,7 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_
       : "memory");
 }
 
-template <int kHeadDim, int kQTiles, int kPolyOf4, bool kBias, bool kSplit>
+template <int kHeadDim, int kQTiles, int kBias, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 1)
 fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_bias,
@@ -367,7 +371,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       for (int quarter = 0; quarter < 4; ++quarter) ptx::mbar_init(p_part(t, quarter), 128);
       ptx::mbar_init(o_final(t), 1);
       ptx::mbar_init(o_free(t), 128);
-      ptx::mbar_init(bias_full(t), 1);
+      ptx::mbar_init(bias_full(t), kBias == kBiasWords ? 32 : 1);
       ptx::mbar_init(bias_empty(t), 128);
       ptx::mbar_init(stage_sync(t), 128);
       ptx::mbar_init(stats_full(t), 128);
@@ -377,7 +381,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     ptx::prefetch_tmap(&tmap_q);
     ptx::prefetch_tmap(&tmap_k);
     ptx::prefetch_tmap(&tmap_v);
-    if (kBias) ptx::prefetch_tmap(&tmap_bias);
+    if (kBias == kBiasTma) ptx::prefetch_tmap(&tmap_bias);
     if (C::kStageBytes > 0) ptx::prefetch_tmap(&tmap_o);
   }
   if (warp == kMmaWarp) {
@@ -441,7 +445,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           for (int c = 0; c < C::kChunks; ++c)
             ptx::tma_load_4d(kv_smem + slot * C::kTileBytes + c * kChunkBytes, map, kv_full(slot), c * kChunkElems,
                              item.key_block(i >> 1) * kBlockKV, kv_head, kv_batch);
-          if (kBias && (i & 1) == 0) {
+          if (kBias == kBiasTma && (i & 1) == 0) {
             // right behind K_j: the bias tile of key block j for each query tile (one buffer per
             // tile, handed back by the softmax warpgroup as soon as it has read it)
             const int j = i >> 1;
@@ -754,7 +758,77 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     // the staging boxes must outlive the TMA stores that read them
     if (C::kStageBytes > 0 && elected) ptx::bulk_wait_group<0>();
   } else if (warp > kMmaWarp) {
-    ptx::setmaxnreg_dec<kControlRegs>();  // idle warps of the control warpgroup
+    ptx::setmaxnreg_dec<kControlRegs>();
+    if constexpr (kBias == kBiasWords) {
+      // ---------------------------------------------------------------- bias tiles that TMA cannot fetch
+      // One warp per query tile, 32 lanes x 4 bytes = one 128-byte row of a box per copy, into the layout that
+      // TMA would have made: coalesced, 256 copies of a tile in flight and no register between memory and shared memory.
+      // A row whose address is odd in units of two bytes starts one element early (the aligned word holds an element of
+      // the row, so it is part of the same allocation); its reader shifts it.  Read element by element by the softmax
+      // threads, each its own row, the same bias took 32 L1 lines per load: see launch_bias for both.
+      const int t = warp - kBiasWarp;
+      if (t < kQTiles) {
+        uint32_t dst[8];   // rows r, r + 8, ... of the first box: the swizzle depends on the row modulo 8
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          dst[r] = bias_smem + t * kBiasTileBytes + r * 128 + (((lane >> 2) ^ r) << 4) + (lane & 3) * 4;
+        const int64_t pitch = args.bias_strides[2] * 2;
+        uint32_t n_bias = 0;
+        bool alive = true;
+        uint32_t it = 0;
+        for (int w = item_of(args, sched, 0); w < args.num_items && alive; w = item_of(args, sched, ++it)) {
+          const Item item = get_item<kQTiles, kSplit>(args, w);
+          const int my_blocks = item.nblk(t);
+          const int row0 = item.q0 + t * kBlockQ;
+          const int rows = min(kBlockQ, args.F - row0);   // (what stands in the rows behind the last query matters to nobody)
+          const char* first_row = reinterpret_cast<const char*>(args.bias + item.batch * args.bias_strides[0] + item.head * args.bias_strides[1] +
+                                                                row0 * args.bias_strides[2]);
+          for (int j = 0; j < my_blocks; ++j, ++n_bias) {
+            const int kv0 = item.key_block(item.first(t) + j) * kBlockKV;
+            if (!ptx::mbar_wait(bias_empty(t), (n_bias & 1u) ^ 1u, ctl, kSiteLoadBias)) {
+              alive = false;
+              break;
+            }
+            uintptr_t row = reinterpret_cast<uintptr_t>(first_row) + kv0 * 2;
+            if (rows == kBlockQ && kv0 + kBlockKV <= args.T) {
+#pragma unroll 1
+              for (uint32_t off = 0; off < static_cast<uint32_t>(kChunkBytes); off += 1024) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r, row += pitch) {
+                  const uintptr_t src = (row & ~static_cast<uintptr_t>(3)) + lane * 4;
+                  ptx::cp_async_4(dst[r] + off, src, 4u);
+                  ptx::cp_async_4(dst[r] + off + kChunkBytes, src + 128, 4u);
+                }
+              }
+            } else {
+              // Bytes of this lane's words that belong to the row, for rows that start on an even / odd element.  Nothing is
+              // read where that is 0: the address is the row's start then.
+              uint32_t bytes[2][2];
+#pragma unroll
+              for (int odd = 0; odd < 2; ++odd)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                  const int left = args.T - (kv0 + c * kChunkElems + 2 * lane - odd);
+                  bytes[odd][c] = left <= 0 ? 0u : left == 1 ? 2u : 4u;
+                }
+#pragma unroll 1
+              for (int r0 = 0; r0 < rows; r0 += 8) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r, row += pitch) {
+                  if (r0 + r >= rows) break;
+                  const bool odd = (row & 2u) != 0;
+                  const uintptr_t start = row & ~static_cast<uintptr_t>(3);
+                  const uint32_t b0 = odd ? bytes[1][0] : bytes[0][0], b1 = odd ? bytes[1][1] : bytes[0][1];
+                  ptx::cp_async_4(dst[r] + r0 * 128, b0 != 0 ? start + lane * 4 : start, b0);
+                  ptx::cp_async_4(dst[r] + r0 * 128 + kChunkBytes, b1 != 0 ? start + lane * 4 + 128 : start, b1);
+                }
+              }
+            }
+            ptx::cp_async_arrive_noinc(bias_full(t));
+          }
+        }
+      }
+    }
   } else {
     // ------------------------------------------------------------------ softmax
     ptx::setmaxnreg_inc<kSoftmaxRegs>();
@@ -778,10 +852,13 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         const int q0 = item.q0, head = item.head, batch = item.batch;
         const int f = q0 + t * kBlockQ + row_in_tile;
         const bool row_ok = f < args.F;
-        const uint16_t* bias_row = nullptr;
-        if (args.bias != nullptr && row_ok)
+        [[maybe_unused]] const uint16_t* bias_row = nullptr;
+        [[maybe_unused]] bool bias_shift = false;
+        if constexpr (kBias == kBiasWords) {
           bias_row = args.bias + batch * args.bias_strides[0] + head * args.bias_strides[1] +
-                     static_cast<int64_t>(f) * args.bias_strides[2];
+                     static_cast<int64_t>(min(f, args.F - 1)) * args.bias_strides[2];
+          bias_shift = (reinterpret_cast<uintptr_t>(bias_row) & 2u) != 0;
+        }
         float m_run = -INFINITY;
         float l_run = 0.0f;
         const int kv_step = item.reversed ? -kBlockKV : kBlockKV;
@@ -792,7 +869,11 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           [[maybe_unused]] uint4 bw[kBiasPrefetch];
           [[maybe_unused]] const uint8_t* bias_tile =
               smem_gen + (bias_smem - smem_base) + t * kBiasTileBytes + row_in_tile * 128;
-          if constexpr (kBias) {
+          [[maybe_unused]] uint32_t bias_last = 0u;   // kBiasWords, a row shifted by an element: its last one
+          if constexpr (kBias == kBiasWords) {
+            if (bias_shift && row_ok && kv0 + kBlockKV <= args.T) bias_last = bias_row[kv0 + kBlockKV - 1];
+          }
+          if constexpr (kBias != kNoBias) {
             if (!ptx::mbar_wait(bias_full(t), n_bias & 1u, ctl, kSiteSoftmaxBias)) {
               alive = false;
               break;
@@ -816,7 +897,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           // mult = head_scale * log2(e) (> 0, so the row maximum can be taken on r).  With a
           // non-positive scale, r is first rewritten as the full log2-domain score and mult = 1.
           float mult = args.scale_log2;
-          if (args.bias == nullptr && !(args.scale_log2 > 0.0f)) {
+          if (kBias == kNoBias && !(args.scale_log2 > 0.0f)) {
             mult = 1.0f;
   #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -824,75 +905,40 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
               for (int i = 0; i < 32; ++i) r[c][i] = __float_as_uint(__uint_as_float(r[c][i]) * args.scale_log2);
             }
           }
-          if (args.bias != nullptr) {
+          if constexpr (kBias != kNoBias) {
             // With a bias, r becomes the natural-log score head_scale * r + bias in one fused
             // multiply-add per element and mult = log2(e) (> 0 whatever the sign of the scale).
+            // The bias tile is two 128-byte-swizzled boxes of 64 keys; this thread reads its own row, 16 bytes at
+            // a time (8 consecutive rows touch 8 different 16-byte columns, so the reads are bank-conflict free).
             mult = kLog2e;
             const float hs = args.head_scale;
-            if (kBias) {
-              // The bias tile was brought in by TMA as two 128-byte-swizzled boxes of 64 keys; this
-              // thread reads its own row, 16 bytes at a time (8 consecutive rows touch 8 different
-              // 16-byte columns, so the reads are bank-conflict free).
-              const uint8_t* tile = bias_tile;
+            [[maybe_unused]] const uint32_t shift = bias_shift ? 0x5432u : 0x3210u;   // kBiasWords: which halves of two words make a pair
+            auto group = [&](int grp) {   // 16-byte group of 8 keys
+              return grp < kBiasPrefetch ? bw[grp < kBiasPrefetch ? grp : 0]
+                                         : *reinterpret_cast<const uint4*>(bias_tile + (grp >> 3) * kChunkBytes +
+                                                                           (((grp & 7) ^ (row_in_tile & 7)) << 4));
+            };
 #pragma unroll
-              for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < 4; ++c) {
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                  const int grp = c * 4 + g;  // 16-byte group of 8 keys
-                  const uint4 w = grp < kBiasPrefetch
-                                      ? bw[grp < kBiasPrefetch ? grp : 0]
-                                      : *reinterpret_cast<const uint4*>(tile + (grp >> 3) * kChunkBytes +
-                                                                        (((grp & 7) ^ (row_in_tile & 7)) << 4));
-                  const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+              for (int g = 0; g < 4; ++g) {
+                const int grp = c * 4 + g;
+                const uint4 w = group(grp);
+                const uint32_t raw[5] = {w.x, w.y, w.z, w.w, kBias != kBiasWords ? 0u : grp < 15 ? group(grp + 1).x : bias_last};
 #pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const int i = g * 8 + e * 2;
-                    r[c][i] = __float_as_uint(fmaf(__uint_as_float(r[c][i]), hs, unpack_lo(ww[e], bf16)));
-                    r[c][i + 1] = __float_as_uint(fmaf(__uint_as_float(r[c][i + 1]), hs, unpack_hi(ww[e], bf16)));
-                  }
+                for (int e = 0; e < 4; ++e) {
+                  const uint32_t ww = kBias == kBiasWords ? __byte_perm(raw[e], raw[e + 1], shift) : raw[e];
+                  const int i = g * 8 + e * 2;
+                  r[c][i] = __float_as_uint(fmaf(__uint_as_float(r[c][i]), hs, unpack_lo(ww, bf16)));
+                  r[c][i + 1] = __float_as_uint(fmaf(__uint_as_float(r[c][i + 1]), hs, unpack_hi(ww, bf16)));
                 }
-              }
-              // The next tile is written by TMA, i.e. through the async proxy: this thread's reads
-              // (generic proxy) have to be fenced against it, the barrier alone does not order them
-              // (seen with an earlier hand-back: single rows picked up the next tile's values).
-              ptx::fence_proxy_async_smem();
-              ptx::mbar_arrive(bias_empty(t));
-            } else if (bias_row != nullptr) {
-              const uint16_t* bp = bias_row + kv0;
-              const int count = min(kBlockKV, args.T - kv0);
-              if (args.bias_vec_ok && count == kBlockKV) {
-  #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-  #pragma unroll
-                  for (int g = 0; g < 4; ++g) {
-                    const uint4 w = __ldg(reinterpret_cast<const uint4*>(bp + c * 32) + g);
-                    const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-  #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                      const int i = g * 8 + e * 2;
-                      r[c][i] = __float_as_uint(fmaf(unpack_lo(ww[e], bf16), kLog2e, __uint_as_float(r[c][i])));
-                      r[c][i + 1] = __float_as_uint(fmaf(unpack_hi(ww[e], bf16), kLog2e, __uint_as_float(r[c][i + 1])));
-                    }
-                  }
-                }
-              } else {
-  #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-  #pragma unroll
-                  for (int i = 0; i < 32; ++i) {
-                    const int col = c * 32 + i;
-                    const float bias_v = col < count ? unpack_lo(__ldg(bp + col), bf16) : 0.0f;
-                    r[c][i] = __float_as_uint(fmaf(__uint_as_float(r[c][i]), hs, bias_v));
-                  }
-                }
-              }
-            } else {
-  #pragma unroll
-              for (int c = 0; c < 4; ++c) {
-  #pragma unroll
-                for (int i = 0; i < 32; ++i) r[c][i] = __float_as_uint(__uint_as_float(r[c][i]) * hs);
               }
             }
+            // The next tile is written by TMA, i.e. through the async proxy: this thread's reads
+            // (generic proxy) have to be fenced against it, the barrier alone does not order them
+            // (seen with an earlier hand-back: single rows picked up the next tile's values).
+            if (kBias == kBiasTma) ptx::fence_proxy_async_smem();
+            ptx::mbar_arrive(bias_empty(t));
           }
           // masks: keys past T (tile padding) and, under causal, keys after the query
           const bool tail_block = kv0 + kBlockKV > args.T;
@@ -952,11 +998,9 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           const bool trunc = bf16;
           const float bias_log2 = trunc ? kTruncBiasLog2 : 0.0f;
           const uint64_t negm2 = ptx::f32x2(bias_log2 - m_use, bias_log2 - m_use);
-          uint64_t sum_a = ptx::f32x2(0.0f, 0.0f), sum_b = ptx::f32x2(0.0f, 0.0f);
+          uint64_t sum = ptx::f32x2(0.0f, 0.0f);
           // P (16-bit pairs) overwrites the first 64 columns of this tile's S: the 32 scores of
           // chunk c become 16 packed columns at [16 c, 16 c + 16), already read by this thread.
-          // Of every four pairs, kPolyOf4 take their 2^x from the FMA pipe, the rest from the
-          // special-function unit, so that neither pipe alone bounds the softmax.
           auto exp_block = [&](auto trunc_tag) {
           constexpr bool kTrunc = decltype(trunc_tag)::value;
 #pragma unroll
@@ -968,14 +1012,9 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                   ptx::fma2(ptx::f32x2(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])), mult2, negm2);
               float x0, x1, p0, p1;
               ptx::f32x2_split(x2, x0, x1);
-              if (((i >> 1) & 3) < kPolyOf4) {
-                ptx::ex2_poly2(fmaxf(x0, -126.0f), fmaxf(x1, -126.0f), p0, p1);
-                sum_b = ptx::add2(sum_b, ptx::f32x2(p0, p1));
-              } else {
-                p0 = ptx::ex2_approx(x0);
-                p1 = ptx::ex2_approx(x1);
-                sum_a = ptx::add2(sum_a, ptx::f32x2(p0, p1));
-              }
+              p0 = ptx::ex2_approx(x0);
+              p1 = ptx::ex2_approx(x1);
+              sum = ptx::add2(sum, ptx::f32x2(p0, p1));
               pk[i >> 1] = kTrunc ? __byte_perm(__float_as_uint(p0), __float_as_uint(p1), 0x7632) : pack2(p0, p1, false);
             }
             ptx::tmem_st_32x16(s_addr + c * 16, pk);
@@ -993,7 +1032,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             exp_block(std::false_type{});
           }
           float s0, s1;
-          ptx::f32x2_split(ptx::add2(sum_a, sum_b), s0, s1);
+          ptx::f32x2_split(sum, s0, s1);
           l_run = l_run * alpha + (s0 + s1);
         }
         if (!alive) break;
@@ -1184,7 +1223,7 @@ bool build_schedule(const KernelArgs& a, int grid, Schedule* out) {
   return ok;
 }
 
-template <int kHeadDim, int kQTiles, int kPolyOf4, bool kBias>
+template <int kHeadDim, int kQTiles, int kBias>
 int launch_cfg(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   using C = Cfg<kHeadDim, kQTiles, kBias>;
   const CUtensorMapDataType dt = p.dtype == IXK_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -1224,8 +1263,8 @@ int launch_cfg(const Problem& p, const DeviceInfo& dev, void* workspace, size_t 
   for (int i = 0; i < 3; ++i) out_tma = out_tma && p.o_strides[i] % 8 == 0;
   out_tma = out_tma && p.o_strides[2] >= p.H;
   if (out_tma && (rc = make_map(&to, p.out, p.o_strides, p.F)) != IXK_OK) return rc;
-  tbias = tq;  // placeholder, never dereferenced unless kBias
-  if (kBias) {
+  tbias = tq;  // placeholder, never dereferenced unless kBiasTma
+  if (kBias == kBiasTma) {
     // bias [B|1, N|1, F, T]: a broadcast dimension becomes extent 1 (coordinate always 0)
     TmapSpec s{};
     s.dtype = dt;
@@ -1264,20 +1303,17 @@ int launch_cfg(const Problem& p, const DeviceInfo& dev, void* workspace, size_t 
   a.k_batch_mul = p.k_strides[0] == 0 ? 0 : 1;
   a.v_head_mul = p.v_strides[1] == 0 ? 0 : 1;
   a.v_batch_mul = p.v_strides[0] == 0 ? 0 : 1;
-  bool bias_vec = p.bias != nullptr && (reinterpret_cast<uintptr_t>(p.bias) & 15u) == 0;
   bool out_vec = (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
   for (int i = 0; i < 3; ++i) {
     a.bias_strides[i] = p.bias_strides[i];
     a.o_strides[i] = p.o_strides[i];
-    bias_vec = bias_vec && (p.bias_strides[i] % 8 == 0);
     out_vec = out_vec && (p.o_strides[i] % 8 == 0);
   }
-  a.bias_vec_ok = bias_vec ? 1 : 0;
   a.out_vec_ok = out_vec ? 1 : 0;
   a.out_tma = out_tma ? 1 : 0;
 
-  auto* whole_kernel = &fmha_prefill_kernel<kHeadDim, kQTiles, kPolyOf4, kBias, false>;
-  auto* split_kernel = &fmha_prefill_kernel<kHeadDim, kQTiles, kPolyOf4, kBias, kPolyOf4 == 0>;   // (the tuning variants never split)
+  auto* whole_kernel = &fmha_prefill_kernel<kHeadDim, kQTiles, kBias, false>;
+  auto* split_kernel = &fmha_prefill_kernel<kHeadDim, kQTiles, kBias, true>;
   static thread_local int configured_device = -1;
   if (configured_device != dev.device) {
     IXK_CUDA_OK(cudaFuncSetAttribute(whole_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
@@ -1290,7 +1326,7 @@ int launch_cfg(const Problem& p, const DeviceInfo& dev, void* workspace, size_t 
   if (items > 0x7fffffff) return fail(IXK_UNIMPLEMENTED, "too many (batch, head, query block) work items");
   const int base_items = static_cast<int>(items);
   SplitPlan split = split_plan<kHeadDim, kQTiles>(a, items, dev.sm_count);
-  if (kPolyOf4 != 0 || workspace == nullptr || workspace_bytes < split_bytes<kHeadDim, kQTiles>(split) ||
+  if (workspace == nullptr || workspace_bytes < split_bytes<kHeadDim, kQTiles>(split) ||
       (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0)
     split.parts = 0;
   a.num_direct = split.parts > 0 ? split.num_direct : base_items;
@@ -1345,8 +1381,7 @@ size_t split_bytes_for(const Problem& p, int sms) {
 
 }  // namespace
 
-// A bias whose rows start on 16-byte boundaries can be fetched by TMA; any other goes through
-// per-thread global loads in the softmax warps.
+// A bias whose rows start on 16-byte boundaries can be fetched by TMA.
 bool bias_fits_tma(const Problem& p) {
   if (p.bias == nullptr) return false;
   if ((reinterpret_cast<uintptr_t>(p.bias) & 15u) != 0) return false;
@@ -1354,10 +1389,15 @@ bool bias_fits_tma(const Problem& p) {
   return p.bias_strides[1] % 8 == 0 && p.bias_strides[0] % 8 == 0;
 }
 
-template <int kHeadDim, int kQTiles, int kPolyOf4>
+// Every bias goes through shared memory, by TMA or as words; read by the softmax threads each from its own row, a bias
+// that TMA does not take cost 32 lines a load.  Loads per thread -> words (bf16, us; the next size that TMA takes): B8 N16
+// S2047 H128 per batch 4569 -> 634 (2048: 296), B4 N8 S1031 H128 per batch 379 -> 68, B2 N8 S1501 per head H64 489 -> 77
+// (1504: 39), H256 779 -> 116 (61).
+template <int kHeadDim, int kQTiles>
 int launch_bias(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-  if (bias_fits_tma(p)) return launch_cfg<kHeadDim, kQTiles, kPolyOf4, true>(p, dev, workspace, workspace_bytes, stream);
-  return launch_cfg<kHeadDim, kQTiles, kPolyOf4, false>(p, dev, workspace, workspace_bytes, stream);
+  if (p.bias == nullptr) return launch_cfg<kHeadDim, kQTiles, kNoBias>(p, dev, workspace, workspace_bytes, stream);
+  if (bias_fits_tma(p)) return launch_cfg<kHeadDim, kQTiles, kBiasTma>(p, dev, workspace, workspace_bytes, stream);
+  return launch_cfg<kHeadDim, kQTiles, kBiasWords>(p, dev, workspace, workspace_bytes, stream);
 }
 
 // Scratch a launch can make use of (none is needed: without it no item is split).
@@ -1369,23 +1409,14 @@ size_t prefill_workspace_bytes(const Problem& p, int sms) {
 
 int launch_prefill(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   // Head-size buckets follow the reference's policy pick (fmha_forward.h:621-646): <=64, <=128, <=256.
-  constexpr int kPoly = 0;  // pairs of every four whose 2^x runs on the FMA pipe instead of the special-function unit
   if (p.H <= 64)
-    return p.F > kBlockQ ? launch_bias<64, 2, kPoly>(p, dev, workspace, workspace_bytes, stream)
-                         : launch_bias<64, 1, kPoly>(p, dev, workspace, workspace_bytes, stream);
+    return p.F > kBlockQ ? launch_bias<64, 2>(p, dev, workspace, workspace_bytes, stream)
+                         : launch_bias<64, 1>(p, dev, workspace, workspace_bytes, stream);
   if (p.H <= 128) {
-    if (p.F <= kBlockQ) return launch_bias<128, 1, kPoly>(p, dev, workspace, workspace_bytes, stream);
-    // Tuning override for the main configuration: IXK_FMHA_POLY = 0..2.
-    if (const char* env = std::getenv("IXK_FMHA_POLY")) {
-      switch (std::atoi(env)) {
-        case 1: return launch_cfg<128, 2, 1, false>(p, dev, workspace, workspace_bytes, stream);
-        case 2: return launch_cfg<128, 2, 2, false>(p, dev, workspace, workspace_bytes, stream);
-        default: break;
-      }
-    }
-    return launch_bias<128, 2, kPoly>(p, dev, workspace, workspace_bytes, stream);
+    if (p.F <= kBlockQ) return launch_bias<128, 1>(p, dev, workspace, workspace_bytes, stream);
+    return launch_bias<128, 2>(p, dev, workspace, workspace_bytes, stream);
   }
-  return launch_bias<256, 1, kPoly>(p, dev, workspace, workspace_bytes, stream);
+  return launch_bias<256, 1>(p, dev, workspace, workspace_bytes, stream);
 }
 
 }  // namespace fmha

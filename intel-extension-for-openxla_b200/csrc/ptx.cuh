@@ -160,6 +160,14 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint
       "l"(tmap), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+// Copy of one 4-byte word global -> shared, both 4-byte aligned: `bytes` (0..4) of it, zeros behind them.
+__device__ __forceinline__ void cp_async_4(uint32_t dst, uintptr_t src, uint32_t bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// One arrival on `bar`, counted once all of this thread's cp.async copies so far have landed.
+__device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
 // Hint: bring a tile into L2.  Reads nothing, so it needs no ordering with whoever writes the tensor.
 __device__ __forceinline__ void tma_prefetch_l2_2d(const void* tmap, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
@@ -629,25 +637,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
-}
-
-// 2^x for a pair, on the FMA pipe instead of the special-function unit: x = n + f with
-// n = round(x), |f| <= 1/2; 2^f by a degree-3 minimax polynomial (relative error 7.5e-5, well
-// inside the 2^-9 of a 16-bit P); 2^n by adding n to the exponent field.  Inputs must be
-// >= -126 (callers clamp) and below 127.
-__device__ __forceinline__ void ex2_poly2(float x0, float x1, float& y0, float& y1) {
-  const uint64_t magic = f32x2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: the add rounds to an integer
-  const uint64_t x = f32x2(x0, x1);
-  const uint64_t xr = add2(x, magic);
-  const uint64_t f = sub2(x, sub2(xr, magic));
-  uint64_t p = fma2(f, f32x2(0.0551716685f, 0.0551716685f), f32x2(0.242611125f, 0.242611125f));
-  p = fma2(p, f, f32x2(0.693260968f, 0.693260968f));
-  p = fma2(p, f, f32x2(0.999928057f, 0.999928057f));
-  float p0, p1, r0, r1;
-  f32x2_split(p, p0, p1);
-  f32x2_split(xr, r0, r1);
-  y0 = __uint_as_float(__float_as_uint(p0) + (__float_as_uint(r0) << 23));
-  y1 = __uint_as_float(__float_as_uint(p1) + (__float_as_uint(r1) << 23));
 }
 
 // ---------------------------------------------------------------- misc math

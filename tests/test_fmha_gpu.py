@@ -566,3 +566,32 @@ def test_at_most_128_keys(pkg, orc, cuda, case):
     tol = 2e-2 if dt == "bf16" else 3e-3
     orc.check_close(f32(o), want, rtol=tol, atol=tol, what=str(case))
     orc.check_close(f32(lse), want_lse, rtol=1e-4, atol=1e-4, what=f"lse {case}")
+
+
+@pytest.mark.parametrize("case", [
+    # B, N, F, T, H, dtype, causal, heads of the bias, kind
+    (2, 2, 131, 131, 128, "bf16", False, 1, "odd"),          # rows start on either half of a word; last word of a row half used
+    (1, 3, 300, 257, 64, "fp16", False, 3, "odd"),           # a key block of one key
+    (1, 2, 129, 258, 256, "bf16", True, 2, "even"),          # pitch a multiple of 4 bytes, not of 16; one tile per item
+    (2, 2, 100, 384, 128, "bf16", False, 1, "offset"),       # pitch fits TMA, the first row's address does not
+    (1, 2, 390, 255, 40, "fp16", False, 1, "offset"),
+    (2, 2, 260, 392, 128, "fp16", False, 1, "row"),          # one row for all queries (a padding mask)
+    (1, 2, 140, 391, 128, "bf16", True, 2, "row"),
+], ids=lambda c: "B{}N{}F{}T{}H{}{}c{}b{}{}".format(*c))
+def test_bias_that_tma_does_not_take(pkg, orc, cuda, case):
+    """An additive bias at any address and pitch, and one row broadcast over the queries: word copies instead of TMA."""
+    B, N, F, T, H, dt, causal, heads, kind = case
+    dtype = {"bf16": torch.bfloat16, "fp16": torch.float16}[dt]
+    g = torch.Generator().manual_seed(F * 5 + T)
+    q, k, v = (torch.randn(B, N, s, H, generator=g).to(dtype) for s in (F, T, T))
+    rows = 1 if kind == "row" else F
+    n = B * heads * rows * T
+    first = 1 if kind in ("offset", "row") else 0
+    store = torch.randn(n + 2, generator=g).to(dtype)
+    store[:first] = float("nan")                             # what stands before and behind the bias is not taken for it
+    store[first + n:] = float("nan")
+    bias = store.to(cuda)[first:first + n].view(B, heads, rows, T).expand(B, heads, F, T)
+    o, lse = run(pkg, q.to(cuda), k.to(cuda), v.to(cuda), bias, causal, lse=True)
+    want, want_lse = orc.fmha_forward(f32(q), f32(k), f32(v), f32(bias), head_scale=H ** -0.5, causal=causal)
+    orc.check_close(f32(o), want, rtol=2e-2, atol=2e-2, what=str(case))
+    orc.check_close(f32(lse), want_lse, rtol=2e-3, atol=2e-3, what=f"lse {case}")
