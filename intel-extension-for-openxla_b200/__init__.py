@@ -14,6 +14,8 @@ raises IxkError otherwise.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import struct
 from typing import Optional
@@ -165,8 +167,32 @@ def load_library() -> ctypes.CDLL:
         fn = getattr(lib, name)  # AttributeError if the library does not export it
         fn.restype = restype
         fn.argtypes = argtypes
+    _bind_native(lib)
     _LIB = lib
     return lib
+
+
+# The calls' native twins (csrc/py_calls.cc), from the first load_library() on.  Each answers None for what it leaves to
+# the Python code behind it, else a status or the result tensor.
+_NATIVE = None
+
+
+def _bind_native(lib) -> None:
+    global _NATIVE
+    path = os.path.join(os.path.dirname(library_path()), "ixk_calls.so")
+    if not os.path.exists(path):
+        raise IxkError(IXK_NO_DEVICE, f"{path} is missing: it is built with {library_path()}")
+    loader = importlib.machinery.ExtensionFileLoader("ixk_calls", path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("ixk_calls", path, loader=loader))
+    module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in ABI_SYMBOLS})
+    _NATIVE = module
+
+
+def _native_result(r):
+    """A native call's answer that is not None: the result tensor, or a status."""
+    if type(r) is int:
+        _check(r)
+    return r
 
 
 def _check(status: int) -> None:
@@ -359,6 +385,10 @@ def gemm(lhs: torch.Tensor, rhs: torch.Tensor, *, bias: Optional[torch.Tensor] =
     """out = act(alpha * lhs @ rhs + bias + beta*c) through "__cublas$lt$matmul"'s path.  Any mix of
     row-/column-major 2-D (or batched 3-D) views is passed through as-is, never copied.  With a
     *_AUX epilogue `aux` receives the values the activation is applied to."""
+    if _NATIVE is not None and aux is None and epilogue in EPILOGUES:
+        r = _NATIVE.gemm(lhs, rhs, bias, c, out, out_dtype, alpha, beta, EPILOGUES.index(epilogue), workspace, stream, None, None)
+        if r is not None:
+            return _native_result(r)
     if out is None:
         shape = (*lhs.shape[:-1], rhs.shape[-1])
         out = torch.empty(shape, device=lhs.device, dtype=out_dtype or lhs.dtype)
@@ -374,6 +404,10 @@ def gemm_geglu(x: torch.Tensor, w_gate_up: torch.Tensor, *, out: Optional[torch.
     """gelu_tanh(x @ w[:, :N']) * (x @ w[:, N':]) for x [M <= 128, K] and w [K, 2 N'] in one GEMM and one
     combining pass (decode-time GeGLU).  `workspace`: uint8 scratch of gemm_geglu_workspace_bytes()
     bytes (allocated here when absent)."""
+    if _NATIVE is not None:
+        r = _NATIVE.geglu(x, w_gate_up, out, workspace, stream)
+        if r is not None:
+            return _native_result(r)
     m, n2 = x.shape[-2], w_gate_up.shape[-1]
     if out is None:
         out = torch.empty((m, n2 // 2), device=x.device, dtype=x.dtype)
@@ -404,6 +438,11 @@ def gemm_fp8(lhs_q: torch.Tensor, rhs_q: torch.Tensor, inv_scale_a: float, inv_s
              out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16,
              stream=None) -> torch.Tensor:
     """out = cast((lhs_q @ rhs_q in fp32) * inv_scale_a * inv_scale_b [+ bias, act])."""
+    if _NATIVE is not None and epilogue in EPILOGUES:
+        r = _NATIVE.gemm(lhs_q, rhs_q, bias, None, out, out_dtype, 1.0, 0.0, EPILOGUES.index(epilogue), None, stream, inv_scale_a,
+                         inv_scale_b)
+        if r is not None:
+            return _native_result(r)
     if out is None:
         out = torch.empty((*lhs_q.shape[:-1], rhs_q.shape[-1]), device=lhs_q.device, dtype=out_dtype)
     attrs = gemm_attrs_for(lhs_q, rhs_q, out, 0.0)
@@ -448,6 +487,10 @@ def row_norm(x: torch.Tensor, *, kind: int = NORM_LAYER, eps: float = 1e-5, out:
              stream=None, gain: Optional[torch.Tensor] = None, gain_offset: float = 0.0) -> torch.Tensor:
     """LayerNorm (zero shift) or RMSNorm over the last dimension of a dense tensor; with `gain` [cols]
     the normalised row is multiplied by (gain_offset + gain) before the one rounding."""
+    if _NATIVE is not None:
+        r = _NATIVE.row_norm(x, kind, eps, out, gain, gain_offset, stream)
+        if r is not None:
+            return _native_result(r)
     if not x.is_contiguous():
         raise IxkError(IXK_INVALID_ARGUMENT, "row_norm wants a contiguous tensor")
     out = torch.empty_like(x) if out is None else out
@@ -471,6 +514,11 @@ def rotary_interleaved_(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, s
     """In place on x [tokens, heads, head_dim] (any token pitch, unit element stride): pairs (2i, 2i+1)
     of the first rotary_dim elements of every head (half_split: pairs (i, i + rotary_dim/2)), token
     t at position t % seq_len; cos/sin fp32 [seq_len, rotary_dim/2]."""
+    if _NATIVE is not None:
+        r = _NATIVE.rotary(x, cos, sin, seq_len, rotary_dim, half_split, stream)
+        if r is not None:
+            _check(r)
+            return x
     if x.dim() != 3 or x.stride(2) != 1:
         raise IxkError(IXK_INVALID_ARGUMENT, "x must be [tokens, heads, head_dim] with unit element stride")
     if cos.dtype != torch.float32 or sin.dtype != torch.float32 or not cos.is_contiguous() or not sin.is_contiguous() \
@@ -494,6 +542,11 @@ def kv_append_(k_cache: torch.Tensor, v_cache: torch.Tensor, k_new: torch.Tensor
     """k_cache / v_cache [B, T, heads, head_dim] (any strides with unit element stride, the same for
     both): cache[:, position] = new, new [B, heads, head_dim] views (e.g. slices of a fused QKV
     projection), both tensors in one launch."""
+    if _NATIVE is not None:
+        r = _NATIVE.kv_append(k_cache, v_cache, k_new, v_new, position, stream)
+        if r is not None:
+            _check(r)
+            return
     B, T, N, H = k_cache.shape
     if v_cache.shape != k_cache.shape or v_cache.stride() != k_cache.stride() or k_new.shape != (B, N, H) or \
             v_new.shape != (B, N, H) or k_new.stride() != v_new.stride() or k_cache.stride(3) != 1 or k_new.stride(2) != 1:
@@ -508,6 +561,10 @@ def kv_append_(k_cache: torch.Tensor, v_cache: torch.Tensor, k_new: torch.Tensor
 def residual_add(x: torch.Tensor, partial: torch.Tensor, bias: Optional[torch.Tensor] = None,
                  out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
     """x + partial, or x + round(partial + bias) with bias along the last dimension."""
+    if _NATIVE is not None:
+        r = _NATIVE.residual_add(x, partial, bias, out, stream)
+        if r is not None:
+            return _native_result(r)
     if not x.is_contiguous() or not partial.is_contiguous() or partial.numel() != x.numel() or partial.dtype != x.dtype:
         raise IxkError(IXK_INVALID_ARGUMENT, "x and partial must be dense tensors of one size and type")
     cols = x.shape[-1]
@@ -578,6 +635,11 @@ def fmha_forward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: t
     `dropout` must be None: the runner rejects dropout (xetla_gpu_fused_mha_runner.cc:56-62).
     `causal` is a real flag here; the reference compiles it out (sdp_forward.cc:41) and expects
     callers to fold the mask into `bias`."""
+    if _NATIVE is not None and dropout is None and dropout_prob in (None, 0.0, 1.0) and (activation is not None) == bool(is_training):
+        r = _NATIVE.fmha_forward(query, key, value, bias, out, activation, head_scale, causal, workspace, stream)
+        if r is not None:
+            _check(r)
+            return
     _require_cuda(query, key, value, bias, out, activation)
     if dropout is not None:
         raise IxkError(IXK_UNIMPLEMENTED, "Unimplemented dropout")
@@ -630,6 +692,12 @@ def fmha_backward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: 
     gradients [B,N,T,H] views (any strides with H contiguous); `activation` is the forward's
     log-sum-exp [B,N,F] fp32.  The reference's dp_sum and grad_query_accum scratch buffers are one
     `workspace` here (allocated if not given)."""
+    if _NATIVE is not None:
+        r = _NATIVE.fmha_backward(query, key, value, out, bias, grad_out, activation, grad_query, grad_key, grad_value, head_scale,
+                                  causal, workspace, stream)
+        if r is not None:
+            _check(r)
+            return
     _require_cuda(query, key, value, out, bias, grad_out, activation, grad_query, grad_key, grad_value)
     if activation is None or activation.dtype != torch.float32 or not activation.is_contiguous() \
             or activation.shape != query.shape[:3]:

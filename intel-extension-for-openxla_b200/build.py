@@ -1,4 +1,5 @@
-"""Builds lib/libixk.so from csrc/*.cu with nvcc for sm_100a (cross-compiles without a GPU).
+"""Builds lib/libixk.so from csrc/*.cu with nvcc for sm_100a (cross-compiles without a GPU), and lib/ixk_calls.so, the
+Python package's native calls, from csrc/py_calls.cc with the host compiler against the installed torch.
 
 Run as a script (python build.py [--force] [--verbose]) or call build().
 Objects go to build/ next to this file; both folders are git-ignored build products.
@@ -10,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -17,6 +19,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libixk.so")
+CALLS_PATH = os.path.join(LIB_DIR, "ixk_calls.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -75,7 +78,26 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_calls(force)
     return LIB_PATH
+
+
+def build_calls(force: bool = False) -> str:
+    import torch
+    source = os.path.join(CSRC, "py_calls.cc")
+    inputs = [source, os.path.join(INCLUDE, "ixk.h"), os.path.abspath(__file__), torch.__file__]
+    if not force and os.path.exists(CALLS_PATH) and os.path.getmtime(CALLS_PATH) > _newest(inputs):
+        return CALLS_PATH
+    home = os.path.dirname(torch.__file__)
+    cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", INCLUDE, "-I", os.path.join(home, "include"), "-I", os.path.join(home, "include", "torch", "csrc", "api", "include"),
+           "-I", sysconfig.get_paths()["include"], "-I", cuda_include, source, "-o", CALLS_PATH,
+           "-L", os.path.join(home, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on py_calls.cc:\n{r.stdout}\n{r.stderr}")
+    return CALLS_PATH
 
 
 if __name__ == "__main__":
