@@ -13,6 +13,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "fmha_sm100.h"
 #include "ptx.cuh"
 
@@ -21,11 +23,13 @@ namespace fmha {
 
 namespace {
 
-constexpr int kWarps = 8;
-constexpr int kThreads = kWarps * 32;
-constexpr int kUnroll = 4;      // keys in flight per lane group
+constexpr int kWarpsMany = 8;
+constexpr int kUnrollMany = 4;  // keys in flight per lane group
 constexpr int kMinKeysPerSplit = 256;
 constexpr int kTargetCtas = 16 * 148;
+// With no more CTAs than SMs the time is a chain of loads, not bandwidth: such a launch has twice the warps per CTA
+// and twice the keys in flight per warp (one CTA of them fills an SM's registers).
+constexpr int kWarpsFew = 16, kUnrollFew = 8;
 constexpr int kCarveoutPercent = 30;   // of an SM's L1 as shared memory (see launch_decode)
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -78,8 +82,8 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {
 // consecutive query rows: every K and V vector is loaded once and used for all of them, so a
 // step with a few query rows per sequence (2 <= F <= 16) streams the cache ceil(F / kQ) times,
 // not F times.
-template <int kLanesPerKey, int kQ>
-__global__ void __launch_bounds__(kThreads, 2)
+template <int kLanesPerKey, int kQ, int kWarps, int kUnroll>
+__global__ void __launch_bounds__(kWarps * 32, 16 / kWarps)
 fmha_decode_kernel(const DecodeArgs a) {
   constexpr int kGroups = 32 / kLanesPerKey;  // keys handled side by side in one warp
   constexpr int kHPad = kLanesPerKey * 8;
@@ -170,9 +174,11 @@ fmha_decode_kernel(const DecodeArgs a) {
         x[r][u] = seen ? s : -INFINITY;
       }
     }
-    float vf[kUnroll][8];
+    float vf[kUnroll > kUnrollMany ? 1 : kUnroll][8];
+    if constexpr (kUnroll <= kUnrollMany) {
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) unpack8(vw[u], bf16, vf[u]);
+      for (int u = 0; u < kUnroll; ++u) unpack8(vw[u], bf16, vf[u]);
+    }
 #pragma unroll
     for (int r = 0; r < kQ; ++r) {
       float mx = x[r][0];
@@ -190,8 +196,9 @@ fmha_decode_kernel(const DecodeArgs a) {
         for (int u = 0; u < kUnroll; ++u) {
           const float p = ptx::ex2_approx(x[r][u] - m_run[r]);  // 0 for masked / absent keys
           l_run[r] += p;
+          if constexpr (kUnroll > kUnrollMany) unpack8(vw[u], bf16, vf[0]);   // (64 more registers otherwise)
 #pragma unroll
-          for (int i = 0; i < 8; ++i) acc[r][i] = fmaf(p, vf[u][i], acc[r][i]);
+          for (int i = 0; i < 8; ++i) acc[r][i] = fmaf(p, vf[kUnroll > kUnrollMany ? 0 : u][i], acc[r][i]);
         }
       }
     }
@@ -260,33 +267,46 @@ fmha_decode_kernel(const DecodeArgs a) {
   }
 }
 
-// One CTA per (batch, head, query): merges the key splits.
-__global__ void fmha_decode_combine_kernel(const DecodeArgs a) {
+// One CTA per (batch, head, query): merges the key splits.  A warp holds the splits' weights one to a lane and hands
+// them round, so that a thread's loads of the partial results wait for nothing but each other.
+__global__ void __launch_bounds__(128) fmha_decode_combine_kernel(const DecodeArgs a) {
   ptx::grid_dependency_sync();
   const int64_t row = blockIdx.x;
   const int f = static_cast<int>(row % a.F);
   const int head = static_cast<int>((row / a.F) % a.N);
   const int batch = static_cast<int>(row / (static_cast<int64_t>(a.F) * a.N));
   const bool bf16 = a.is_bf16 != 0;
-  const float* part = a.partial + row * a.splits * (a.H + 2);
+  const int lane = threadIdx.x & 31;
+  const int pitch = a.H + 2;
+  const float* part = a.partial + row * a.splits * pitch;
   float m_all = -INFINITY;
-  for (int s = 0; s < a.splits; ++s) m_all = fmaxf(m_all, part[s * (a.H + 2) + a.H]);
-  float l_all = 0.0f;
-  for (int s = 0; s < a.splits; ++s) {
-    const float m_s = part[s * (a.H + 2) + a.H];
-    const float c = (m_s == -INFINITY) ? 0.0f : ptx::ex2_approx(m_s - m_all);
-    l_all += part[s * (a.H + 2) + a.H + 1] * c;
-  }
-  for (int d = threadIdx.x; d < a.H; d += blockDim.x) {
-    float o = 0.0f;
-    for (int s = 0; s < a.splits; ++s) {
-      const float m_s = part[s * (a.H + 2) + a.H];
-      const float c = (m_s == -INFINITY) ? 0.0f : ptx::ex2_approx(m_s - m_all);
-      o += part[s * (a.H + 2) + d] * c;
+  for (int s = lane; s < a.splits; s += 32) m_all = fmaxf(m_all, part[static_cast<int64_t>(s) * pitch + a.H]);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m_all = fmaxf(m_all, __shfl_xor_sync(0xffffffffu, m_all, off));
+  float l_all = 0.0f, o[2] = {0.0f, 0.0f};
+  const int d0 = threadIdx.x, d1 = threadIdx.x + 128;
+  const bool d0_ok = d0 < a.H, d1_ok = d1 < a.H;
+  for (int s0 = 0; s0 < a.splits; s0 += 32) {
+    const int count = min(32, a.splits - s0);
+    const float* block = part + static_cast<int64_t>(s0) * pitch;
+    float c = 0.0f, l = 0.0f;
+    if (lane < count) {
+      const float2 st = *reinterpret_cast<const float2*>(block + lane * pitch + a.H);   // (H and the pitch are even)
+      c = (st.x == -INFINITY) ? 0.0f : ptx::ex2_approx(st.x - m_all);
+      l = st.y * c;
     }
-    a.out[batch * a.o_strides[0] + head * a.o_strides[1] + static_cast<int64_t>(f) * a.o_strides[2] + d] =
-        from_f32(o / l_all, bf16);
+#pragma unroll 8
+    for (int j = 0; j < count; ++j) {
+      const float cj = __shfl_sync(0xffffffffu, c, j);
+      l_all += __shfl_sync(0xffffffffu, l, j);
+      const float* src = block + j * pitch;
+      if (d0_ok) o[0] = fmaf(src[d0], cj, o[0]);
+      if (d1_ok) o[1] = fmaf(src[d1], cj, o[1]);
+    }
   }
+  uint16_t* out = a.out + batch * a.o_strides[0] + head * a.o_strides[1] + static_cast<int64_t>(f) * a.o_strides[2];
+  if (d0_ok) out[d0] = from_f32(o[0] / l_all, bf16);
+  if (d1_ok) out[d1] = from_f32(o[1] / l_all, bf16);
   if (threadIdx.x == 0 && a.lse != nullptr) a.lse[row] = (m_all + log2f(l_all)) * kLn2;
 }
 
@@ -362,17 +382,21 @@ int launch_decode(const Problem& p, const DeviceInfo& dev, void* workspace, size
   dim3 grid(splits * ((p.F + rows_per_cta - 1) / rows_per_cta), p.N, p.B);
   auto launch_lanes = [&](auto lanes_tag) -> int {
     constexpr int kLanes = decltype(lanes_tag)::value;
-    auto* fn = rows_per_cta == 1 ? fmha_decode_kernel<kLanes, 1> : fmha_decode_kernel<kLanes, 2>;
+    const bool few = rows_per_cta == 1 && static_cast<int64_t>(grid.x) * grid.y * grid.z <= dev.sm_count;
+    auto* fn = few                 ? fmha_decode_kernel<kLanes, 1, kWarpsFew, kUnrollFew>
+               : rows_per_cta == 1 ? fmha_decode_kernel<kLanes, 1, kWarpsMany, kUnrollMany>
+                                   : fmha_decode_kernel<kLanes, 2, kWarpsMany, kUnrollMany>;
+    const int which = few ? 2 : rows_per_cta - 1;
     // What a load has in flight lives in L1.  Behind kernels that leave an SM no idle moment the split between L1 and
     // shared memory stays what the last large kernel wanted, so this one states its own: B64 N16 T4096 H256 inside a
     // decoder layer 700 us with a GEMM of two CTAs per SM before it, 640 with 30 % (the same as launched in order;
     // 15 % 655, 0 % 1312: too little shared memory for the CTAs).
-    static thread_local int configured_device[2] = {-1, -1};
-    if (configured_device[rows_per_cta - 1] != dev.device) {
+    static thread_local int configured_device[3] = {-1, -1, -1};
+    if (configured_device[which] != dev.device) {
       IXK_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveoutPercent));
-      configured_device[rows_per_cta - 1] = dev.device;
+      configured_device[which] = dev.device;
     }
-    return launch_overlapped(fn, grid, dim3(kThreads), 0, stream, a);
+    return launch_overlapped(fn, grid, dim3((few ? kWarpsFew : kWarpsMany) * 32), 0, stream, a);
   };
   int rc;
   if (p.H <= 64) rc = launch_lanes(std::integral_constant<int, 8>{});

@@ -595,3 +595,22 @@ def test_bias_that_tma_does_not_take(pkg, orc, cuda, case):
     want, want_lse = orc.fmha_forward(f32(q), f32(k), f32(v), f32(bias), head_scale=H ** -0.5, causal=causal)
     orc.check_close(f32(o), want, rtol=2e-2, atol=2e-2, what=str(case))
     orc.check_close(f32(lse), want_lse, rtol=2e-3, atol=2e-3, what=f"lse {case}")
+
+
+@pytest.mark.parametrize("B,N,T,H,dt", [
+    (1, 1, 1, 64, "bf16"), (1, 2, 127, 256, "bf16"), (2, 3, 129, 128, "fp16"), (1, 16, 1001, 256, "bf16"),
+    (1, 2, 8450, 64, "fp16"),     # 34 key splits: more than a warp of the merge has lanes
+    (1, 148, 200, 40, "bf16"),    # one CTA per SM
+    (1, 149, 200, 40, "bf16"),    # one more
+])
+def test_decode_one_row_few_ctas(pkg, orc, cuda, B, N, T, H, dt):
+    """One query row, up to one CTA per SM and beyond: twice the warps and keys in flight, and the merge of the splits."""
+    dtype, odt = {"bf16": (torch.bfloat16, orc.BF16), "fp16": (torch.float16, orc.F16)}[dt]
+    g = torch.Generator().manual_seed(T + H)
+    q = torch.randn(B, N, 1, H, generator=g).to(dtype)
+    k, v = (torch.randn(B, T, N, H, generator=g).to(dtype).permute(0, 2, 1, 3) for _ in range(2))
+    o, lse = run(pkg, q.to(cuda), k.to(cuda), v.to(cuda), lse=True)
+    want, want_lse = orc.fmha_forward(f32(q), f32(k), f32(v), None, head_scale=H ** -0.5, dtype=odt)
+    # (the oracle rounds P, the kernel does not: 2^-9 or 2^-12 of the values summed, and one rounding of O)
+    orc.check_close(f32(o), want, rtol=2e-2, atol=1e-2, what="O")
+    orc.check_close(f32(lse), want_lse, rtol=1e-5, atol=1e-5, what="lse")
