@@ -152,6 +152,7 @@ __device__ __forceinline__ float2 unpack16(uint32_t w, int is_bf16) {
 // head, query) arithmetic is done once per group: with one 64-bit division chain per ROW the
 // kernel was bound by instruction issue (about 400 instructions per row) at 2.5 TB/s.
 __global__ void bwd_prepare_kernel(const PrepArgs a) {
+  ptx::grid_dependency_sync();
   constexpr int kRows = 4;
   const int lane = threadIdx.x & 31;
   const int64_t groups = static_cast<int64_t>(a.B) * a.N * (a.f_pad / kRows);
@@ -212,6 +213,7 @@ struct ConvertArgs {
 
 // One thread per 8 head elements: two float4 in, 16 bytes out.
 __global__ void bwd_convert_kernel(const ConvertArgs a) {
+  ptx::grid_dependency_sync();
   const int groups = a.H / 8;
   const int64_t total = static_cast<int64_t>(a.B) * a.N * a.F * groups;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -350,6 +352,7 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  ptx::grid_dependency_sync();
 
   if (warp == kBwdProducerWarp) {
     // ------------------------------------------------------------------ TMA producer
@@ -693,6 +696,12 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   }
 }
 
+// The three kernels start under one another where each is a few microseconds; of long ones the next one's early CTAs
+// only stand in the way (B8 N16 S2048 H128 causal, 14 rounds: forward and backward 708 us in order, 723).
+bool bwd_overlaps(const Problem& p, const DeviceInfo& dev) {
+  return static_cast<int64_t>((p.T + kBlk - 1) / kBlk) * p.N * p.B <= 2 * dev.sm_count;
+}
+
 template <int kHeadDim, bool kBias, bool kBf16>
 int launch_bwd_cfg(const BwdProblem& bp, const DeviceInfo& dev, float* neg_lse2, float* delta, float* dq_acc,
                    int f_pad, cudaStream_t stream) {
@@ -758,10 +767,7 @@ int launch_bwd_cfg(const BwdProblem& bp, const DeviceInfo& dev, float* neg_lse2,
   }
   const int64_t ctas = static_cast<int64_t>(a.num_kblocks) * p.N * p.B;
   if (ctas > 0x7fffffff) return fail(IXK_UNIMPLEMENTED, "too many (batch, head, key block) work items");
-  fn<<<static_cast<unsigned>(ctas), kBwdThreads, C::kSmemBytes, stream>>>(tq, tk, tv, tdo, a);
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
-  return IXK_OK;
+  return launch_kernel(bwd_overlaps(p, dev), fn, dim3(static_cast<unsigned>(ctas)), dim3(kBwdThreads), C::kSmemBytes, stream, tq, tk, tv, tdo, a);
 }
 
 template <int kHeadDim>
@@ -816,15 +822,13 @@ int launch_bwd(const BwdProblem& bp, const DeviceInfo& dev, void* workspace, siz
   pa.delta = delta;
   pa.dq_acc = dq_acc;
   const int prep_grid = static_cast<int>(std::min<int64_t>((rows / 4 + 7) / 8, static_cast<int64_t>(dev.sm_count) * 8));
-  bwd_prepare_kernel<<<prep_grid, 256, 0, stream>>>(pa);
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
+  int rc = launch_kernel(bwd_overlaps(p, dev), &bwd_prepare_kernel, dim3(prep_grid), dim3(256), 0, stream, pa);
+  if (rc != IXK_OK) return rc;
 
   if (wide) {
     unsigned char* scratch = static_cast<unsigned char*>(workspace) + (static_cast<size_t>(rows) * 2 * sizeof(float) + 255) / 256 * 256;
     return launch_bwd_wide(bp, dev, neg_lse2, delta, f_pad, scratch, stream);
   }
-  int rc;
   const bool bias = p.bias != nullptr;
   if (head_pad == 64) {
     rc = launch_bwd_dtype<64>(bp, dev, neg_lse2, delta, dq_acc, f_pad, stream, bias);
@@ -842,10 +846,7 @@ int launch_bwd(const BwdProblem& bp, const DeviceInfo& dev, void* workspace, siz
   for (int i = 0; i < 3; ++i) ca.dq_strides[i] = bp.dq_strides[i];
   const int64_t pairs = static_cast<int64_t>(p.B) * p.N * p.F * (p.H / 8);
   const int conv_grid = static_cast<int>(std::min<int64_t>((pairs + 255) / 256, static_cast<int64_t>(dev.sm_count) * 8));
-  bwd_convert_kernel<<<conv_grid, 256, 0, stream>>>(ca);
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
-  return IXK_OK;
+  return launch_kernel(bwd_overlaps(p, dev), &bwd_convert_kernel, dim3(conv_grid), dim3(256), 0, stream, ca);
 }
 }  // namespace fmha
 }  // namespace ixk

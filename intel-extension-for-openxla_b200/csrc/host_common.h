@@ -44,8 +44,9 @@ void count_launch(uint64_t n = 1);
 // read, and must not read such memory through the read-only path (__ldg, const __restrict__), whose loads
 // the compiler may move above the wait.  Between two such launches of 2 to 20 us each this hides about
 // 2 us.
+// (overlap = false: in order.)
 template <typename... KernelArgs, typename... Args>
-int launch_overlapped(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const Args&... args) {
+int launch_kernel(bool overlap, void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const Args&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -55,10 +56,14 @@ int launch_overlapped(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   IXK_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<KernelArgs>(args)...));
   count_launch();
   return IXK_OK;
+}
+template <typename... KernelArgs, typename... Args>
+int launch_overlapped(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const Args&... args) {
+  return launch_kernel(true, kernel, grid, block, smem, stream, args...);
 }
 
 // A named NVTX range around an entry point, for timelines of a host program that calls the library
