@@ -250,8 +250,9 @@ int run(const ixk_gemm_desc* desc, const void* a, const void* b, const void* c, 
   // without it they run un-split (same result, fewer SMs busy).
   if (gemm::stream_applies(p)) {
     const int splits = gemm::stream_splits(p.M, p.N, p.K, es, workspace != nullptr && aligned16(workspace) ? workspace_bytes : 0);
-    return splits > 1 ? gemm::launch_split_k(p, splits, workspace, dev, static_cast<cudaStream_t>(stream))
-                      : gemm::launch_stream(p, 1, nullptr, dev, static_cast<cudaStream_t>(stream));
+    if (splits > 1) return gemm::launch_split_k(p, splits, workspace, dev, static_cast<cudaStream_t>(stream));
+    return gemm::stream_alone(p) ? gemm::launch_stream(p, 1, nullptr, dev, static_cast<cudaStream_t>(stream))
+                                 : gemm::launch(p, dev, static_cast<cudaStream_t>(stream));
   }
   const int splits = (p.force_block_n > 0 || p.aux != nullptr) ? 1 : gemm::split_k_factor(p.M, p.N, p.K, p.batch, p.fp8);
   if (splits > 1 && workspace != nullptr && aligned16(workspace) &&
@@ -335,7 +336,7 @@ size_t workspace_query(const ixk_gemm_desc* desc) {
   const bool fp8 = is_fp8(desc->lhs.dtype);
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const size_t tiled = gemm::split_k_workspace_bytes(M, N, gemm::split_k_factor(M, N, K, desc->batch_size, fp8));
-  if (!gemm::stream_takes(M, N) || desc->batch_size != 1) return tiled;
+  if (!gemm::stream_takes(M) || desc->batch_size != 1) return tiled;
   return std::max(tiled, gemm::split_k_workspace_bytes(M, N, gemm::stream_splits(M, N, K, elem_bytes(desc->lhs.dtype), SIZE_MAX / 4)));
 }
 

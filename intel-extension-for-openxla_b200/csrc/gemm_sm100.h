@@ -85,8 +85,9 @@ int launch_split_k(const Problem& p, int splits, void* workspace, const DeviceIn
                    bool geglu = false);
 
 // Few rows: the problem as a stream of the weights (gemm_stream.cu).
-bool stream_takes(int64_t M, int64_t N);
+bool stream_takes(int64_t M);
 bool stream_applies(const Problem& p);
+bool stream_alone(const Problem& p);   // also without scratch for chunks of K
 int stream_splits(int64_t M, int64_t N, int64_t K, int elem_bytes, size_t workspace_bytes);
 int launch_stream(const Problem& p, int splits, float* partial, const DeviceInfo& dev, cudaStream_t stream);
 

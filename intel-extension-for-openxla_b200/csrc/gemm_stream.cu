@@ -1,10 +1,10 @@
-// GEMM for few rows (M <= 128, and up to 256 where the CTA-pair kernel has no full round: decode-time projections):
-// the time is one stream of the weight matrix through the chip, so everything here serves the stream.
+// GEMM for few rows (M <= 128: decode-time projections): the time is one stream of the weight matrix through the
+// chip, so everything here serves the stream.
 //
 //   D^T[n, m] = sum_k B[k, n] A[m, k]
 //
 // The weights are the M side of the MMA (128 columns of B = 128 lanes of tensor memory) and the rows of A
-// its N side (16 to 256 wide, M rounded up to 16), so a pipeline stage is 16 KB of weights and 2 KB of A at
+// its N side (16 to 128 wide, M rounded up to 16), so a pipeline stage is 16 KB of weights and 2 KB of A at
 // M <= 16 where gemm_kernel moves and zero-fills 16 KB of A whatever M is.  One CTA works on 128 columns and
 // one chunk of K; chunk count and shared memory are chosen so that all CTAs are on the chip at once, two or
 // three per SM, and HBM sees one even wave instead of rounds of whole tiles.  While the kernel before it in
@@ -16,8 +16,9 @@
 // Bound by HBM.  Calls back to back in a graph, gemm_kernel -> this (M x N x K, us; at 6.46 TB/s): 1 x 12288 x 3072
 // 21.2 -> 15.1 (11.7), 1 x 3072 x 4096 10.6 -> 9.0 (3.9), 1 x 49152 x 3072 with GeGLU 75.4 -> 48.6 (46.7),
 // 1 x 3072 x 24576 32.6 -> 26.4 (23.4); the same with 64 rows 20.5 -> 18.7, 11.4 -> 10.7, 59.5 -> 56.8, 31.4 -> 30.9;
-// 16 x 1000 x 5000, whose K gemm_kernel did not cut, 21.2 -> 7.8.  Without the L2 hint 0.2 to 1 us more; one CTA per
-// SM with the whole ring, or three, up to 1 us more.
+// 16 x 1000 x 5000, whose K gemm_kernel did not cut, 21.2 -> 7.8.  Without the L2 hint 0.2 to 1 us more; chunks for one
+// CTA per SM with the whole ring, or for three, up to 1 us more.  Every 32 rows cost the epilogue 1 us, which a CTA that
+// finishes D itself has nothing to hide behind: see stream_alone.
 //
 // 192 threads: warp 0 TMA producer, warp 1 tensor memory + MMA issue, warps 2-5 epilogue (thread = one
 // column of D, so a warp's accesses to a row of D are 32 consecutive elements).
@@ -60,6 +61,7 @@ struct StreamArgs {
   void* d;
   int64_t ldc, ldd;
   int out_dtype, bias_dtype, act;
+  int d_pairs;                       // 16-bit D whose columns come in 4-byte pairs
   int* status_word;
 };
 
@@ -73,10 +75,17 @@ __device__ __forceinline__ float load_f32(const void* p, int64_t i, int dtype) {
   const uint16_t h = static_cast<const uint16_t*>(p)[i];
   return dtype == IXK_BF16 ? __uint_as_float(static_cast<uint32_t>(h) << 16) : __half2float(__ushort_as_half(h));
 }
-__device__ __forceinline__ void store_f32(void* p, int64_t i, int dtype, float v) {
-  if (dtype == IXK_F32) static_cast<float*>(p)[i] = v;
-  else if (dtype == IXK_BF16) static_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
-  else static_cast<__half*>(p)[i] = __float2half_rn(v);
+// 32 rows of one column, a pitch apart (the lanes of a warp are 32 consecutive columns).
+__device__ __forceinline__ void store_rows_f32(float* dst, int64_t pitch, const float (&v)[32], int rows, bool ok) {
+  if (!ok) return;
+  if (rows == 32) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i, dst += pitch) *dst = v[i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i, dst += pitch)
+      if (i < rows) *dst = v[i];
+  }
 }
 
 template <int kKind>
@@ -209,25 +218,56 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         ptx::tmem_ld_32x32(acc + m0, r);
         ptx::tmem_ld_wait();
         const int rows = min(32, args.M - m0);
-        if (n_ok) {   // (the loads above are warp-collective)
-          if (args.partial != nullptr) {
-            float* dst = args.partial + (static_cast<int64_t>(split) * args.M + m0) * args.N + n;
+        float v[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < rows) dst[static_cast<int64_t>(i) * args.N] = __uint_as_float(r[i]) * args.acc_scale;
-          } else {
+        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * args.acc_scale;
+        if (args.partial != nullptr) {
+          store_rows_f32(args.partial + (static_cast<int64_t>(split) * args.M + m0) * args.N + n, args.N, v, rows, n_ok);
+          continue;
+        }
+        if (args.bias != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              if (i >= rows) continue;
-              float v = __uint_as_float(r[i]) * args.acc_scale + bias;
-              if (args.c != nullptr) v = fmaf(args.beta, load_f32(args.c, (m0 + i) * args.ldc + n, args.out_dtype), v);
-              if (args.act == kActRelu) v = fmaxf(v, 0.0f);
-              if (args.act == kActGelu) v = gelu_tanh(v);
-              store_f32(args.d, (m0 + i) * args.ldd + n, args.out_dtype, v);
+          for (int i = 0; i < 32; ++i) v[i] += bias;
+        }
+        if (args.c != nullptr && n_ok) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (i < rows) v[i] = fmaf(args.beta, load_f32(args.c, (m0 + i) * args.ldc + n, args.out_dtype), v[i]);
+        }
+        if (args.act == kActRelu) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i], 0.0f);
+        } else if (args.act == kActGelu) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
+        }
+        if (args.out_dtype == IXK_F32) {
+          store_rows_f32(static_cast<float*>(args.d) + m0 * args.ldd + n, args.ldd, v, rows, n_ok);
+        } else {
+          // Rows 2k and 2k + 1 as 16-bit pairs; neighbouring lanes swap halves, so that even lanes hold two columns of
+          // the first row, odd lanes two of the second: 4-byte stores, 64 bytes of two rows per instruction.
+          __syncwarp();
+          uint16_t* d = static_cast<uint16_t*>(args.d) + m0 * args.ldd + n;
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            uint32_t w;
+            if (args.out_dtype == IXK_BF16) {
+              const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+              w = *reinterpret_cast<const uint32_t*>(&h);
+            } else {
+              const __half2 h = __floats2half2_rn(v[2 * k], v[2 * k + 1]);
+              w = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            if (args.d_pairs != 0) {
+              const uint32_t other = __shfl_xor_sync(0xffffffffu, w, 1);
+              const uint32_t both = (lane & 1) == 0 ? __byte_perm(w, other, 0x5410) : __byte_perm(other, w, 0x7632);
+              if (n_ok && 2 * k + (lane & 1) < rows) *reinterpret_cast<uint32_t*>(d + (2 * k + (lane & 1)) * args.ldd - (lane & 1)) = both;
+            } else if (n_ok) {
+              if (2 * k < rows) d[2 * k * args.ldd] = static_cast<uint16_t>(w & 0xffffu);
+              if (2 * k + 1 < rows) d[(2 * k + 1) * args.ldd] = static_cast<uint16_t>(w >> 16);
             }
           }
         }
-        __syncwarp();
       }
     }
   }
@@ -243,20 +283,31 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 
 }  // namespace
 
-// More than 128 rows: as long as the CTA-pair kernel would not have a tile for every pair of SMs.
-bool stream_takes(int64_t M, int64_t N) { return M <= 128 || (M <= 256 && (N + 255) / 256 < kAssumedSms / 2); }
+bool stream_takes(int64_t M) { return M <= 128; }
 
 bool stream_applies(const Problem& p) {
-  return stream_takes(p.M, p.N) && p.batch == 1 && (p.kind == kKindF16 || p.kind == kKindF8) && !p.a_mn_major && p.aux == nullptr &&
+  return stream_takes(p.M) && p.batch == 1 && (p.kind == kKindF16 || p.kind == kKindF8) && !p.a_mn_major && p.aux == nullptr &&
          p.scatter_world == 0 && p.force_block_n == 0;
 }
 
-// Chunks of K: as many as give every SM its two CTAs in one wave, each of kMinChunk slabs at least, and no more than
-// the scratch holds partials of.
+// One chunk of K, D finished by the CTAs: up to 32 rows, or where the columns alone make a CTA for two SMs of three; else
+// gemm_kernel's narrower tiles are level or ahead (us, gemm_kernel and this, bf16: 16 x 512 x 1024 6.3 and 6.1, 64 rows
+// 6.4 and 7.2; 16 x 4096 x 4096 17.8 and 16.7, 128 rows 18.2 and 20.3; 16 x 16384 x 4096 32.4 and 22.6, 128 rows 32.8
+// and 26.6; 64 x 8192 x 8192 32.5 and 32.3).  fp8 with more rows only on K-major weights (128 x 16384 x 4096: 18.5 and
+// 16.8, N-major 13.7 and 16.3).
+bool stream_alone(const Problem& p) {
+  if (p.M <= 32) return true;
+  if (p.N < kTileN * 96) return false;
+  return p.kind == kKindF16 || !p.b_mn_major;
+}
+
+// Chunks of K: as many as give every SM its two CTAs in one wave, each of kMinChunk slabs at least, no more than
+// the scratch holds partials of, and none that would make writing and reading the partials (8 bytes an element) more
+// than half of the weights' bytes.
 int stream_splits(int64_t M, int64_t N, int64_t K, int elem_bytes, size_t workspace_bytes) {
   const int64_t tiles = (N + kTileN - 1) / kTileN, slabs = (K * elem_bytes + kSlabBytes - 1) / kSlabBytes;
   const int64_t fit = static_cast<int64_t>(workspace_bytes / (static_cast<size_t>(M) * N * sizeof(float)));
-  int64_t chunks = std::min<int64_t>({kCtasPerSm * kAssumedSms / tiles, slabs / kMinChunk, kMaxChunks, fit});
+  int64_t chunks = std::min<int64_t>({kCtasPerSm * kAssumedSms / tiles, slabs / kMinChunk, kMaxChunks, fit, K * elem_bytes / (16 * M)});
   chunks = std::max<int64_t>(chunks, 1);
   const int64_t chunk = (slabs + chunks - 1) / chunks;
   return static_cast<int>((slabs + chunk - 1) / chunk);
@@ -311,12 +362,13 @@ int launch_stream(const Problem& p, int splits, float* partial, const DeviceInfo
   a.out_dtype = p.out_dtype;
   a.bias_dtype = p.bias_dtype;
   a.act = p.act;
+  a.d_pairs = p.N % 2 == 0 && p.ldd % 2 == 0 && (reinterpret_cast<uintptr_t>(p.d) & 3u) == 0 ? 1 : 0;
   a.status_word = dev.status_word;
   const int64_t ctas = static_cast<int64_t>(a.tiles) * splits;
   if (ctas > 0x7fffffff) return fail(IXK_UNIMPLEMENTED, "too many tiles");
-  // Three CTAs per SM where two are not enough for one wave.  Shared memory is cut so that no more fit than tensor
-  // memory has columns for: a CTA must not wait for another one's columns while the kernel behind it waits for both.
-  const int per_sm = ctas > kCtasPerSm * dev.sm_count && a.tmem_cols <= 128 ? 3 : kCtasPerSm;
+  // Shared memory for as many CTAs per SM as one wave takes (the ring of a lone CTA is as deep as there is room), three
+  // at most, and no more than tensor memory has columns for.
+  const int per_sm = ctas <= dev.sm_count ? 1 : ctas > kCtasPerSm * dev.sm_count && a.tmem_cols <= 128 ? 3 : kCtasPerSm;
   const int stage_bytes = kWeightBytes + a.x_bytes;
   a.stages = std::min<int>(kMaxStages, ((228 * 1024) / per_sm - 2 * 1024 - kTailBytes) / stage_bytes);
   const size_t smem = static_cast<size_t>(a.stages) * stage_bytes + kTailBytes + 1024;

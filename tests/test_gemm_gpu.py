@@ -500,7 +500,8 @@ def test_cta_pair_last_round(pkg, cuda, monkeypatch, shape, kind, la, lb):
 
 
 @pytest.mark.parametrize("shape", [(1, 8, 8), (1, 5000, 1000), (3, 16384, 600), (16, 72, 136), (17, 520, 4096), (33, 1032, 248), (100, 2000, 304),
-                                   (128, 648, 20000), (128, 64, 128), (129, 2064, 1160), (256, 1000, 18936)],
+                                   (128, 648, 20000), (128, 64, 128), (129, 2064, 1160), (256, 1000, 18936),
+                                   (40, 1000, 12296), (96, 72, 12304)],
                          ids=lambda s: "M{}K{}N{}".format(*s))
 @pytest.mark.parametrize("kind", ["bf16", "fp16", "e4m3"])
 @pytest.mark.parametrize("lb", ["row", "col"])
