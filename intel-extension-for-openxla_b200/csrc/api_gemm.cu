@@ -254,7 +254,9 @@ int run(const ixk_gemm_desc* desc, const void* a, const void* b, const void* c, 
     return gemm::stream_alone(p) ? gemm::launch_stream(p, 1, nullptr, dev, static_cast<cudaStream_t>(stream))
                                  : gemm::launch(p, dev, static_cast<cudaStream_t>(stream));
   }
-  const int splits = (p.force_block_n > 0 || p.aux != nullptr) ? 1 : gemm::split_k_factor(p.M, p.N, p.K, p.batch, p.fp8);
+  int splits = (p.force_block_n > 0 || p.aux != nullptr) ? 1 : gemm::split_k_factor(p.M, p.N, p.K, p.batch, p.fp8);
+  if (splits <= 1 && p.force_block_n == 0 && p.aux == nullptr && (p.kind == gemm::kKindF16 || p.kind == gemm::kKindF8))
+    splits = gemm::tiled_splits(p.M, p.N, p.K, p.batch, es, workspace != nullptr && aligned16(workspace) ? workspace_bytes : 0);
   if (splits > 1 && workspace != nullptr && aligned16(workspace) &&
       workspace_bytes >= gemm::split_k_workspace_bytes(p.M, p.N, splits))
     return gemm::launch_split_k(p, splits, workspace, dev, static_cast<cudaStream_t>(stream));
@@ -336,7 +338,9 @@ size_t workspace_query(const ixk_gemm_desc* desc) {
   const bool fp8 = is_fp8(desc->lhs.dtype);
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const size_t tiled = gemm::split_k_workspace_bytes(M, N, gemm::split_k_factor(M, N, K, desc->batch_size, fp8));
-  if (!gemm::stream_takes(M) || desc->batch_size != 1) return tiled;
+  if (!fp8 && elem_bytes(desc->lhs.dtype) != 2) return tiled;   // (16-bit and fp8 operands only)
+  if (!gemm::stream_takes(M) || desc->batch_size != 1)
+    return std::max(tiled, gemm::split_k_workspace_bytes(M, N, gemm::tiled_splits(M, N, K, desc->batch_size, elem_bytes(desc->lhs.dtype), SIZE_MAX / 4)));
   return std::max(tiled, gemm::split_k_workspace_bytes(M, N, gemm::stream_splits(M, N, K, elem_bytes(desc->lhs.dtype), SIZE_MAX / 4)));
 }
 

@@ -367,8 +367,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         tile_coords(t, args.tiles_m, args.tiles_n, bz, bm, bn);
         const int m0 = bm * kBlockM;
         const int n0 = bn * kBlockN;
-        const int az = args.a_broadcast ? 0 : bz;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const int az = args.a_broadcast || args.k_chunk > 0 ? 0 : bz;
+        const int zb = args.k_chunk > 0 ? 0 : bz;
+        const int kb0 = args.k_chunk * bz;                                                  // (0 without chunks)
+        const int kb1 = args.k_chunk > 0 ? min(num_kb, kb0 + args.k_chunk) : num_kb;
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!ptx::mbar_wait(empty_bar(stage), phase ^ 1u, ctl, kSiteProducer)) {
             alive = false;
             break;
@@ -392,9 +395,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 #pragma unroll
             for (int i = 0; i < kBlockN / kSlabElems; ++i)
               ptx::tma_load_3d(b_dst + i * (kSlabElems * kSlabBytes), &tmap_b, bar,
-                               n0 + i * kSlabElems, k0, bz);
+                               n0 + i * kSlabElems, k0, zb);
           } else {
-            ptx::tma_load_3d(b_dst, &tmap_b, bar, k0, n0, bz);
+            ptx::tma_load_3d(b_dst, &tmap_b, bar, k0, n0, zb);
           }
           }
           __syncwarp();
@@ -429,7 +432,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         if (!ptx::mbar_wait(acc_empty_bar(buf), acc_phase ^ 1u, ctl, kSiteMmaAcc)) break;
         ptx::tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + buf * kBlockN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const int chunk0 = args.k_chunk * (t / (args.tiles_m * args.tiles_n));
+        const int count = args.k_chunk > 0 ? min(num_kb - chunk0, args.k_chunk) : num_kb;
+        for (int kb = 0; kb < count; ++kb) {
           if (!ptx::mbar_wait(full_bar(stage), phase, ctl, kSiteMmaFull)) {
             alive = false;
             break;
@@ -816,7 +821,7 @@ int launch(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
   // Large problems run on CTA pairs (256 x 256 tiles): worth it once every pair of SMs has a tile.
   const int64_t tiles_m_all = (p.M + kBlockM - 1) / kBlockM;
   const int64_t pair_tiles = ((tiles_m_all + 1) / 2) * ((p.N + 255) / 256) * p.batch;
-  bool pair = bn == 256 && tiles_m_all >= 2 && pair_tiles >= dev.sm_count / 2;
+  bool pair = bn == 256 && tiles_m_all >= 2 && p.k_chunk == 0 && pair_tiles >= dev.sm_count / 2;
   if (const char* env = std::getenv("IXK_GEMM_PAIR")) pair = pair && std::atoi(env) != 0;
   const int b_box_rows = pair ? 128 : bn;
   // The tiles beyond the last full round of pairs are cut into 2 or 4 narrower ones where the idle pairs
@@ -861,6 +866,7 @@ int launch(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
       s.box[0] = slab_elems;
       s.box[1] = block_mn;
     }
+    broadcast = broadcast || p.k_chunk > 0;
     s.dims[2] = broadcast ? 1 : p.batch;
     s.box[2] = 1;
     s.strides_bytes[0] = static_cast<uint64_t>(ld) * es;
@@ -915,6 +921,7 @@ int launch(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
   k.d_vec_ok = aligned16(p.d) && (p.ldd * out_es) % 16 == 0 && (p.d_batch_stride * out_es) % 16 == 0;
   k.c_vec_ok = k.c && aligned16(p.c) && (p.ldc * out_es) % 16 == 0 && (p.c_batch_stride * out_es) % 16 == 0;
   k.bias_vec_ok = p.bias && aligned16(p.bias) && (p.bias_batch_stride * bias_es) % 16 == 0;
+  k.k_chunk = p.k_chunk;
   k.a_broadcast = p.a_broadcast ? 1 : 0;
   k.bias_batch_stride = p.bias_batch_stride;
   k.aux = p.aux;

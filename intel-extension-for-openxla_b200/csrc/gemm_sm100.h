@@ -39,6 +39,7 @@ struct Problem {
   float acc_scale = 1.0f;
   float beta = 0.0f;
   int force_block_n = 0;  // tuning override; 0 = heuristic
+  int k_chunk = 0;        // > 0: the batches are chunks of K, this many slabs each (the last one what is left), of one A and B
   // Scattered output (row-parallel projection feeding an all-reduce): row block o of D, rows
   // [o * M / scatter_world, (o + 1) * M / scatter_world), is stored dense ([M / world, N], pitch N)
   // at scatter_dest[o], which may be another GPU's memory.  0 = D goes to `d` as usual.
@@ -51,6 +52,7 @@ struct KernelArgs {
   int M, N, K, batch;
   int tiles_m, tiles_n;
   int a_mn_major, b_mn_major;
+  int k_chunk;                 // slabs of K per batch, 0: all of them (single-CTA kernel)
   uint32_t idesc;
   uint32_t idesc_tail;         // CTA-pair kernel: the narrower tiles of the last round
   int tail_from, tail_parts;   // tiles from here on are cut into this many (1: none is)
@@ -78,6 +80,8 @@ int launch(const Problem& p, const DeviceInfo& dev, cudaStream_t stream);
 // split; depends on the shape only, so the workspace query needs no device), the fp32 scratch it
 // takes, and the two-kernel launch (partial GEMMs as a batch, then reduce + epilogue).
 int split_k_factor(int64_t M, int64_t N, int64_t K, int64_t batch, bool fp8);
+// The same for problems of more rows whose tiles leave most SMs idle, as far as the scratch goes.
+int tiled_splits(int64_t M, int64_t N, int64_t K, int64_t batch, int elem_bytes, size_t workspace_bytes);
 size_t split_k_workspace_bytes(int64_t M, int64_t N, int splits);
 // (geglu: the N columns are [gate | up]; the reduce writes gelu(gate) * up, N / 2 columns, to p.d / p.ldd;
 // splits may be 1 then: one GEMM into the scratch + the GeGLU pass)

@@ -20,8 +20,10 @@ namespace gemm {
 namespace {
 
 constexpr int kAssumedSms = 148;
-constexpr int kSlabElems16 = 64;   // K elements per pipeline stage, 16-bit operands
+constexpr int kSlabBytes = 128;    // bytes of K per pipeline stage
+constexpr int kSlabElems16 = kSlabBytes / 2;
 constexpr int kMinChunk = 512;     // smallest K chunk worth a CTA
+constexpr int64_t kSlabNarrowNs = 160, kSlabWideNs = 210, kReduceNs = 3500, kReduceBytesPerNs = 2500;   // see tiled_splits
 // CTAs of a reduce launch at most, per SM.  It is set up while the GEMM still runs, whose CTA leaves an SM room for seven
 // of the eight CTAs of 256 threads it otherwise holds: a grid of just eight would end with a round of stragglers (128 x
 // 12288 x 3072 in a graph: 24.3 us with 8, 24.1 with 6, 22.8 with 16; 23.3 launched in order with 8).
@@ -182,17 +184,29 @@ int split_k_factor(int64_t M, int64_t N, int64_t K, int64_t batch, bool fp8) {
   return best;
 }
 
+int tiled_splits(int64_t M, int64_t N, int64_t K, int64_t batch, int elem_bytes, size_t workspace_bytes) {
+  const int64_t tiles = (M + 127) / 128 * ((N + 127) / 128), slabs = (K * elem_bytes + kSlabBytes - 1) / kSlabBytes;
+  const int64_t plane = M * N * static_cast<int64_t>(sizeof(float));
+  const int64_t splits = std::min<int64_t>({kAssumedSms / tiles, slabs / 8, 16, static_cast<int64_t>(workspace_bytes) / plane});
+  if (batch != 1 || elem_bytes > 2 || splits < 2) return 1;
+  // ns: a slab of a 128 x 64 tile (what the problem runs on unsplit) and of a 128 x 128 tile, the pass over the
+  // partials and its launch
+  const int64_t whole = slabs * kSlabNarrowNs, cut = (slabs + splits - 1) / splits * kSlabWideNs + kReduceNs + splits * plane / kReduceBytesPerNs;
+  if (cut * 10 > whole * 9) return 1;
+  const int64_t chunk = (slabs + splits - 1) / splits;
+  return static_cast<int>((slabs + chunk - 1) / chunk);
+}
+
 size_t split_k_workspace_bytes(int64_t M, int64_t N, int splits) {
   return splits <= 1 ? 0 : static_cast<size_t>(splits) * M * N * sizeof(float);
 }
 
 int launch_split_k(const Problem& p, int splits, void* workspace, const DeviceInfo& dev, cudaStream_t stream, bool geglu) {
-  const int64_t chunk = p.K / splits;
+  const int slab = kSlabBytes / (p.kind == kKindF16 ? 2 : 1);
+  const int slabs = static_cast<int>((p.K + slab - 1) / slab);
   Problem part = p;
-  part.K = chunk;
   part.batch = splits;
-  part.a_batch_stride = p.a_mn_major ? chunk * p.lda : chunk;
-  part.b_batch_stride = p.b_mn_major ? chunk * p.ldb : chunk;
+  part.k_chunk = (slabs + splits - 1) / splits;
   part.c = nullptr;
   part.bias = nullptr;
   part.beta = 0.0f;

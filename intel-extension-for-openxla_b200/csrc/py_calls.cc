@@ -22,6 +22,7 @@ namespace {
 
 decltype(&ixk_gemm) g_gemm;
 decltype(&ixk_gemm_fp8) g_gemm_fp8;
+decltype(&ixk_gemm_workspace_bytes) g_gemm_bytes;
 decltype(&ixk_gemm_geglu) g_geglu;
 decltype(&ixk_fmha_fwd) g_fwd;
 decltype(&ixk_fmha_fwd_workspace_bytes) g_fwd_bytes;
@@ -172,6 +173,18 @@ IXK_PY_FUNCTION(py_gemm, 13)
   d.alpha = static_cast<float>(alpha);
   d.beta = static_cast<float>(beta);
   d.epilogue = static_cast<int32_t>(epilogue);
+  // An fp8 call has no scratch argument: for cutting K, where that pays, it takes its own (with a result of the caller's it
+  // allocates nothing, as a caller that captures it may count on).
+  at::Tensor own;
+  if (fp8 && ws == nullptr && a[4] == Py_None && a[10] == Py_None) {
+    if (const size_t need = g_gemm_bytes(&d)) {
+      try {
+        own = at::empty({static_cast<int64_t>(need)}, at::TensorOptions().device(lhs->device()).dtype(at::kByte));
+        ws = &own;
+      } catch (const c10::OutOfMemoryError&) {   // it runs without
+      }
+    }
+  }
   const size_t bytes = size_of(ws);
   void *pa = ptr(lhs), *pb = ptr(rhs), *pc = ptr(c), *pbias = ptr(bias), *pd = ptr(out), *pw = ptr(ws);
   const int st = unlocked([&] {
@@ -384,6 +397,7 @@ PyObject* py_bind(PyObject*, PyObject* table) {
   const Entry entries[] = {
       {"ixk_gemm", reinterpret_cast<void**>(&g_gemm)},
       {"ixk_gemm_fp8", reinterpret_cast<void**>(&g_gemm_fp8)},
+      {"ixk_gemm_workspace_bytes", reinterpret_cast<void**>(&g_gemm_bytes)},
       {"ixk_gemm_geglu", reinterpret_cast<void**>(&g_geglu)},
       {"ixk_fmha_fwd", reinterpret_cast<void**>(&g_fwd)},
       {"ixk_fmha_fwd_workspace_bytes", reinterpret_cast<void**>(&g_fwd_bytes)},

@@ -537,3 +537,34 @@ def test_few_rows(pkg, cuda, shape, kind, lb, scratch):
         out32 = pkg.gemm(x, wd, c=c, beta=-0.5, out=torch.empty_like(c), workspace=ws)
         want = x.double() @ w.double() - 0.5 * c.double()
         assert ((out32.double() - want).abs().max() <= sums + 2.0 ** -22 * c.abs().max()).item()
+
+
+@pytest.mark.parametrize("shape", [(300, 8200, 520), (257, 5000, 128), (1500, 8256, 136), (900, 16000, 304)], ids=lambda s: "M{}K{}N{}".format(*s))
+@pytest.mark.parametrize("kind", ["bf16", "fp16", "e4m3"])
+@pytest.mark.parametrize("la", ["row", "col"])
+@pytest.mark.parametrize("lb", ["row", "col"])
+def test_few_tiles_long_k(pkg, cuda, shape, kind, la, lb):
+    """More rows than the weight stream takes, few tiles, long K: cut along K, the last chunk shorter and K ending inside a
+    slab, both operands in both orders."""
+    M, K, N = shape
+    if kind == "e4m3" or (la == "col" and M % 8):
+        M, K, N = ((d + 15) // 16 * 16 for d in (M, K, N))
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    dtype = {"bf16": torch.bfloat16, "fp16": torch.float16, "e4m3": torch.float8_e4m3fn}[kind]
+    x, w = torch.randn(M, K, generator=g, device=cuda).to(dtype), (torch.randn(K, N, generator=g, device=cuda) * 0.05).to(dtype)
+    xd, wd = as_layout(x, la), as_layout(w, lb)
+    plain = x.double() @ w.double()
+    half = 2.0 ** -11 if kind == "fp16" else 2.0 ** -8
+    sums = (K + 16) * 2.0 ** -23 * (x.double().abs() @ w.double().abs()).max()
+    n0 = pkg.launch_count()
+    if kind == "e4m3":
+        out, c = pkg.gemm_fp8(xd, wd, 0.5, 2.0), 0.0
+    else:
+        need = pkg.gemm_workspace_bytes(xd, wd)
+        assert need > 0
+        c = torch.randn(M, N, generator=g, device=cuda).to(dtype)
+        out = pkg.gemm(xd, wd, c=c, beta=1.0, workspace=torch.full((need,), 255, dtype=torch.uint8, device=cuda))
+        c = c.double()
+    assert pkg.launch_count() - n0 == 2
+    want = plain + c
+    assert ((out.double() - want).abs().max() <= 1.01 * half * want.abs().max() + sums + 2.0 ** -22).item()
