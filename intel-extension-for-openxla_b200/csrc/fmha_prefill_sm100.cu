@@ -72,9 +72,9 @@ enum : int { kSiteLoad = 201, kSiteMmaQ = 202, kSiteMmaKV = 203, kSiteMmaP = 204
 constexpr int kBiasTileBytes = 2 * kChunkBytes;  // 128 query rows x 128 keys, 16-bit, as two swizzled boxes
 // How an additive bias reaches shared memory: not at all, by TMA, or, where its address or strides do not suit
 // TMA (a pitch of an odd number of elements, a row broadcast over the queries), as aligned 4-byte words that the
-// control warpgroup's two spare warps copy.
+// control warpgroup's two spare warps and the epilogue's four copy (see bias_copier).
 enum : int { kNoBias = 0, kBiasTma = 1, kBiasWords = 2 };
-constexpr int kBiasWarp = 10;     // kBiasWords: warp kBiasWarp + t copies query tile t's bias
+constexpr int kBiasWarp = 10;     // the first of these six warps
 constexpr int kBiasPrefetch = 8;  // 16-byte groups of a bias row (the first box) read before the scores arrive
 
 template <int kHeadDim, int kQTiles, int kBias>
@@ -320,6 +320,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     const __grid_constant__ Schedule sched) {
   using C = Cfg<kHeadDim, kQTiles, kBias>;
   constexpr int kSlots = C::kKvSlots;
+  [[maybe_unused]] constexpr int kBiasShares = kQTiles == 1 ? 6 : 3;   // warps that copy a tile's bias (kBiasWords)
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -371,7 +372,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       for (int quarter = 0; quarter < 4; ++quarter) ptx::mbar_init(p_part(t, quarter), 128);
       ptx::mbar_init(o_final(t), 1);
       ptx::mbar_init(o_free(t), 128);
-      ptx::mbar_init(bias_full(t), kBias == kBiasWords ? 32 : 1);
+      ptx::mbar_init(bias_full(t), kBias == kBiasWords ? 32 * kBiasShares : 1);
       ptx::mbar_init(bias_empty(t), 128);
       ptx::mbar_init(stage_sync(t), 128);
       ptx::mbar_init(stats_full(t), 128);
@@ -393,6 +394,69 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   ptx::grid_dependency_sync();   // (the combine kernel and the next call's wait for this grid's end)
+
+  // Bias tiles that TMA cannot fetch: this warp's share of an item's (groups of eight rows dealt among the tile's warps),
+  // 32 lanes x 4 bytes = one 128-byte row of a box per copy, into the layout that TMA would have made: coalesced, and no
+  // register between memory and shared memory.  A row whose address is odd in units of two bytes starts one element early
+  // (the aligned word holds an element of the row, so it is part of the same allocation); its reader shifts it.
+  // A warp gets a copy out every 40 cycles, 10000 for a tile alone: hence three warps per tile, where there are two tiles.
+  // The epilogue's warps copy an item's bias before they turn to its results.
+  [[maybe_unused]] auto bias_copier = [&](const Item& item, uint32_t& n_bias) {
+    const int who = warp - kBiasWarp;                                     // 0, 1: spare warps; 2..5: epilogue
+    const int t = kQTiles == 1 ? 0 : who < 2 ? who : (who - 2) >> 1;
+    const int share = kQTiles == 1 ? who : who < 2 ? 0 : 1 + (who & 1);
+    uint32_t dst[8];   // rows r, r + 8, ... of the first box: the swizzle depends on the row modulo 8
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      dst[r] = bias_smem + t * kBiasTileBytes + r * 128 + (((lane >> 2) ^ r) << 4) + (lane & 3) * 4;
+    const int64_t pitch = args.bias_strides[2] * 2;
+    const int my_blocks = item.nblk(t);
+    const int row0 = item.q0 + t * kBlockQ;
+    const int rows = min(kBlockQ, args.F - row0);   // (what stands in the rows behind the last query matters to nobody)
+    const char* first_row = reinterpret_cast<const char*>(args.bias + item.batch * args.bias_strides[0] + item.head * args.bias_strides[1] +
+                                                          (row0 + share * 8) * args.bias_strides[2]);
+    for (int j = 0; j < my_blocks; ++j, ++n_bias) {
+      const int kv0 = item.key_block(item.first(t) + j) * kBlockKV;
+      if (!ptx::mbar_wait(bias_empty(t), (n_bias & 1u) ^ 1u, ctl, kSiteLoadBias)) return false;
+      uintptr_t row = reinterpret_cast<uintptr_t>(first_row) + kv0 * 2;
+      if (rows == kBlockQ && kv0 + kBlockKV <= args.T) {
+#pragma unroll 1
+        for (uint32_t r0 = share * 8; r0 < kBlockQ; r0 += 8 * kBiasShares, row += pitch * (8 * (kBiasShares - 1))) {
+#pragma unroll
+          for (int r = 0; r < 8; ++r, row += pitch) {
+            const uintptr_t src = (row & ~static_cast<uintptr_t>(3)) + lane * 4;
+            ptx::cp_async_4(dst[r] + r0 * 128, src, 4u);
+            ptx::cp_async_4(dst[r] + r0 * 128 + kChunkBytes, src + 128, 4u);
+          }
+        }
+      } else {
+        // Bytes of this lane's words that belong to the row, for rows that start on an even / odd element.  Nothing is
+        // read where that is 0: the address is the row's start then.
+        uint32_t bytes[2][2];
+#pragma unroll
+        for (int odd = 0; odd < 2; ++odd)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int left = args.T - (kv0 + c * kChunkElems + 2 * lane - odd);
+            bytes[odd][c] = left <= 0 ? 0u : left == 1 ? 2u : 4u;
+          }
+#pragma unroll 1
+        for (int r0 = share * 8; r0 < rows; r0 += 8 * kBiasShares, row += pitch * (8 * (kBiasShares - 1))) {
+#pragma unroll
+          for (int r = 0; r < 8; ++r, row += pitch) {
+            if (r0 + r >= rows) break;
+            const bool odd = (row & 2u) != 0;
+            const uintptr_t start = row & ~static_cast<uintptr_t>(3);
+            const uint32_t b0 = odd ? bytes[1][0] : bytes[0][0], b1 = odd ? bytes[1][1] : bytes[0][1];
+            ptx::cp_async_4(dst[r] + r0 * 128, b0 != 0 ? start + lane * 4 : start, b0);
+            ptx::cp_async_4(dst[r] + r0 * 128 + kChunkBytes, b1 != 0 ? start + lane * 4 + 128 : start, b1);
+          }
+        }
+      }
+      ptx::cp_async_arrive_noinc(bias_full(t));
+    }
+    return true;
+  };
 
   if (warp == kProducerWarp) {
     // ------------------------------------------------------------------ TMA producer
@@ -641,10 +705,15 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const bool elected = warp == kEpilogueWarp && lane == 0;  // issues every TMA store
     uint32_t n_fin0 = 0, n_fin1 = 0;    // items finished per tile
     uint32_t n_sync0 = 0, n_sync1 = 0;  // rendezvous of the four warps around a tile's staging box
+    [[maybe_unused]] uint32_t n_bias = 0;
     bool alive = true;
     uint32_t it = 0;
     for (int w = item_of(args, sched, 0); w < args.num_items && alive; w = item_of(args, sched, ++it)) {
       const Item item = get_item<kQTiles, kSplit>(args, w);
+      if constexpr (kBias == kBiasWords) {
+        if (!bias_copier(item, n_bias)) break;
+        __syncwarp();
+      }
       for (int tt = 0; tt < kQTiles && alive; ++tt) {
         const int t = item.reversed ? kQTiles - 1 - tt : tt;  // the tile that started first is served first
         if (item.nblk(t) == 0) continue;
@@ -760,74 +829,11 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   } else if (warp > kMmaWarp) {
     ptx::setmaxnreg_dec<kControlRegs>();
     if constexpr (kBias == kBiasWords) {
-      // ---------------------------------------------------------------- bias tiles that TMA cannot fetch
-      // One warp per query tile, 32 lanes x 4 bytes = one 128-byte row of a box per copy, into the layout that
-      // TMA would have made: coalesced, 256 copies of a tile in flight and no register between memory and shared memory.
-      // A row whose address is odd in units of two bytes starts one element early (the aligned word holds an element of
-      // the row, so it is part of the same allocation); its reader shifts it.  Read element by element by the softmax
-      // threads, each its own row, the same bias took 32 L1 lines per load: see launch_bias for both.
-      const int t = warp - kBiasWarp;
-      if (t < kQTiles) {
-        uint32_t dst[8];   // rows r, r + 8, ... of the first box: the swizzle depends on the row modulo 8
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-          dst[r] = bias_smem + t * kBiasTileBytes + r * 128 + (((lane >> 2) ^ r) << 4) + (lane & 3) * 4;
-        const int64_t pitch = args.bias_strides[2] * 2;
-        uint32_t n_bias = 0;
-        bool alive = true;
-        uint32_t it = 0;
-        for (int w = item_of(args, sched, 0); w < args.num_items && alive; w = item_of(args, sched, ++it)) {
-          const Item item = get_item<kQTiles, kSplit>(args, w);
-          const int my_blocks = item.nblk(t);
-          const int row0 = item.q0 + t * kBlockQ;
-          const int rows = min(kBlockQ, args.F - row0);   // (what stands in the rows behind the last query matters to nobody)
-          const char* first_row = reinterpret_cast<const char*>(args.bias + item.batch * args.bias_strides[0] + item.head * args.bias_strides[1] +
-                                                                row0 * args.bias_strides[2]);
-          for (int j = 0; j < my_blocks; ++j, ++n_bias) {
-            const int kv0 = item.key_block(item.first(t) + j) * kBlockKV;
-            if (!ptx::mbar_wait(bias_empty(t), (n_bias & 1u) ^ 1u, ctl, kSiteLoadBias)) {
-              alive = false;
-              break;
-            }
-            uintptr_t row = reinterpret_cast<uintptr_t>(first_row) + kv0 * 2;
-            if (rows == kBlockQ && kv0 + kBlockKV <= args.T) {
-#pragma unroll 1
-              for (uint32_t off = 0; off < static_cast<uint32_t>(kChunkBytes); off += 1024) {
-#pragma unroll
-                for (int r = 0; r < 8; ++r, row += pitch) {
-                  const uintptr_t src = (row & ~static_cast<uintptr_t>(3)) + lane * 4;
-                  ptx::cp_async_4(dst[r] + off, src, 4u);
-                  ptx::cp_async_4(dst[r] + off + kChunkBytes, src + 128, 4u);
-                }
-              }
-            } else {
-              // Bytes of this lane's words that belong to the row, for rows that start on an even / odd element.  Nothing is
-              // read where that is 0: the address is the row's start then.
-              uint32_t bytes[2][2];
-#pragma unroll
-              for (int odd = 0; odd < 2; ++odd)
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                  const int left = args.T - (kv0 + c * kChunkElems + 2 * lane - odd);
-                  bytes[odd][c] = left <= 0 ? 0u : left == 1 ? 2u : 4u;
-                }
-#pragma unroll 1
-              for (int r0 = 0; r0 < rows; r0 += 8) {
-#pragma unroll
-                for (int r = 0; r < 8; ++r, row += pitch) {
-                  if (r0 + r >= rows) break;
-                  const bool odd = (row & 2u) != 0;
-                  const uintptr_t start = row & ~static_cast<uintptr_t>(3);
-                  const uint32_t b0 = odd ? bytes[1][0] : bytes[0][0], b1 = odd ? bytes[1][1] : bytes[0][1];
-                  ptx::cp_async_4(dst[r] + r0 * 128, b0 != 0 ? start + lane * 4 : start, b0);
-                  ptx::cp_async_4(dst[r] + r0 * 128 + kChunkBytes, b1 != 0 ? start + lane * 4 + 128 : start, b1);
-                }
-              }
-            }
-            ptx::cp_async_arrive_noinc(bias_full(t));
-          }
-        }
-      }
+      uint32_t n_bias = 0;
+      bool alive = true;
+      uint32_t it = 0;
+      for (int w = item_of(args, sched, 0); w < args.num_items && alive; w = item_of(args, sched, ++it))
+        alive = bias_copier(get_item<kQTiles, kSplit>(args, w), n_bias);
     }
   } else {
     // ------------------------------------------------------------------ softmax
@@ -1384,8 +1390,8 @@ bool bias_fits_tma(const Problem& p) {
 
 // Every bias goes through shared memory, by TMA or as words; read by the softmax threads each from its own row, a bias
 // that TMA does not take cost 32 lines a load.  Loads per thread -> words (bf16, us; the next size that TMA takes): B8 N16
-// S2047 H128 per batch 4569 -> 634 (2048: 296), B4 N8 S1031 H128 per batch 379 -> 68, B2 N8 S1501 per head H64 489 -> 77
-// (1504: 39), H256 779 -> 116 (61).
+// S2047 H128 per batch 4569 -> 595 (2048: 296), B4 N8 S1031 H128 per batch 379 -> 67, B2 N8 S1501 per head H64 489 -> 61
+// (1504: 39), H256 779 -> 74 (61); copied by two warps in place of six 634, 68, 77, 116.
 template <int kHeadDim, int kQTiles>
 int launch_bias(const Problem& p, const DeviceInfo& dev, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   if (p.bias == nullptr) return launch_cfg<kHeadDim, kQTiles, kNoBias>(p, dev, workspace, workspace_bytes, stream);
