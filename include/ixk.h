@@ -128,10 +128,11 @@ typedef struct ixk_gemm_desc {
  * type for 16-bit operands and the output's type otherwise.
  * workspace is optional scratch (the reference hands its scratch allocator down
  * this path, sycl_onednn.h:37).  ixk_gemm_workspace_bytes returns what a problem
- * can use: non-zero only for skinny problems (M <= 128, one batch, a long K),
- * which then run split along K with fp32 partials in the workspace and a reduce
- * pass that applies the epilogue.  With workspace == NULL or fewer bytes the
- * single-pass kernel runs; results agree within fp32 summation order. */
+ * can use: non-zero only for problems of one batch with 16-bit or fp8 operands that
+ * alone leave much of the GPU idle (M <= 128, or few tiles and a long K), which then
+ * run split along K with fp32 partials in the workspace and a reduce pass that
+ * applies the epilogue.  With fewer bytes K is cut into fewer chunks, or, as with
+ * workspace == NULL, one pass runs; results agree within fp32 summation order. */
 int ixk_gemm(const ixk_gemm_desc* desc, const void* a, const void* b,
              const void* c, const void* bias, void* d, void* workspace,
              size_t workspace_bytes, void* cuda_stream);

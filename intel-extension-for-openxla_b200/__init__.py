@@ -292,8 +292,8 @@ def run_gemm_custom_call(lhs: torch.Tensor, rhs: torch.Tensor, add: Optional[tor
     {lhs,rhs,output}_{order,num_rows,num_cols,batch_stride,leading_dim_stride,layout_dtype},
     batch_size, alpha, beta.  `add` is the C operand read when beta != 0 (it may be `output`).
     With inv_scale_a/b given the operands are fp8 and the scaled-GEMM entry point is used.
-    `workspace` is the scratch the reference's handler passes down (sycl_onednn.h:37): skinny
-    problems (M <= 128) use it to split K over more SMs; see gemm_workspace_bytes().  `aux` is the
+    `workspace` is the scratch the reference's handler passes down (sycl_onednn.h:37): problems
+    of few rows (M <= 128) or few tiles use it to split K over more SMs; see gemm_workspace_bytes().  `aux` is the
     second result of the GELU_AUX / BIAS_GELU_AUX epilogues (the pre-activation values, the
     output's type, shape and order)."""
     if epilogue not in EPILOGUES:
