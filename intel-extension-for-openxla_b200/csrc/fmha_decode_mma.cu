@@ -27,6 +27,11 @@
 // split-key kernel's to six digits (1.6617e-3 bf16, 2.0851e-4 fp16 at head size 256), of one key far above
 // 2000 others up to 2^36 times smaller 1.9e-4 (fp16); lse 3.6e-7 to 4.2e-7 there, 3.3e-7 to 3.7e-7 here.
 // B32 N16 T3001 H256 bf16: F = 2 411 -> 265 us, 4 765 -> 267 (5.9 TB/s), 8 1410 -> 269, 12 2106 -> 345, 16 2771 -> 377.
+// Short caches are bound by what surrounds the stream.  Started under the kernel before it, barriers set by a thread each,
+// the warps' O merged without bank conflicts (read row by row they met 8 or 16 to a bank) and by all threads, the merge
+// kernel a CTA per cut unit with its loads together, in place of one per range that read part after part (calls back to
+// back, bf16, us): B1 N16 F16 T2127 H64 21.0 -> 10.6, B2 N16 F8 T1126 H128 14.7 -> 9.4, B1 N8 F2 T4000 H128 14.4 -> 9.6,
+// B11 N16 F8 T64 H256 14.4 -> 11.3, B20 N16 F16 T130 H256 47 -> 39, B64 N8 F2 T700 H128 39 -> 35, and F = 4 above 251 -> 246.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -191,18 +196,19 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   ptx::AbortCtl ctl{abort_flag, a.status_word};
-  if (threadIdx.x == 0) {
-    *abort_flag = 0;
-    for (int i = 0; i < C::kBars; ++i) {
-      ptx::mbar_init(full(i), 1);
-      ptx::mbar_init(empty(i), C::kWarpsPerTile);
-    }
+  static_assert(C::kBars < kThreads, "a thread per pair of barriers");
+  if (threadIdx.x < C::kBars) {
+    ptx::mbar_init(full(threadIdx.x), 1);
+    ptx::mbar_init(empty(threadIdx.x), C::kWarpsPerTile);
     ptx::fence_mbar_init();
+  }
+  if (threadIdx.x == kThreads - 1) {
+    *abort_flag = 0;
     ptx::prefetch_tmap(&tmap_k);
     ptx::prefetch_tmap(&tmap_v);
   }
   __syncthreads();
-  ptx::grid_dependency_trigger();   // the combine kernel may be set up meanwhile; it waits for this grid's end
+  ptx::grid_dependency_sync();   // (the combine kernel is set up meanwhile; it waits for this grid's end)
 
   const int t_begin = range_begin(a.pieces, a.piece, blockIdx.x, gridDim.x);
   const int t_end = range_begin(a.pieces, a.piece, blockIdx.x + 1, gridDim.x);
@@ -262,7 +268,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         for (int i = threadIdx.x; i < C::kRows * kSlabs * 8; i += kWarps * 32) {
           const int f = i / (kSlabs * 8), piece = i % (kSlabs * 8);
           uint4 w = make_uint4(0u, 0u, 0u, 0u);
-          if (f < a.F && piece * 8 < a.H) w = __ldg(reinterpret_cast<const uint4*>(q_base + f * a.q_strides[2] + piece * 8));
+          if (f < a.F && piece * 8 < a.H) w = *reinterpret_cast<const uint4*>(q_base + f * a.q_strides[2] + piece * 8);
           *reinterpret_cast<uint4*>(q_rows + f * C::kHPad * 2 + ((piece ^ (f & 7)) << 4)) = w;
         }
         ptx::named_barrier_sync(1, kWarps * 32);
@@ -276,7 +282,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
               const int d = ks * 16 + i * 8 + 2 * c;
-              qf[ks][nt][i] = (f < a.F && d < a.H) ? __ldg(reinterpret_cast<const uint32_t*>(qrow + d)) : 0u;   // H is a multiple of 8
+              qf[ks][nt][i] = (f < a.F && d < a.H) ? *reinterpret_cast<const uint32_t*>(qrow + d) : 0u;   // H is a multiple of 8
             }
           }
         }
@@ -321,7 +327,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const int key = key0 + g + (i >> 1) * 8;
-              if (bias_row[nt][i & 1] != nullptr && key < a.T) bias_v[nt][i] = to_f32<kBf16>(__ldg(bias_row[nt][i & 1] + key));
+              if (bias_row[nt][i & 1] != nullptr && key < a.T) bias_v[nt][i] = to_f32<kBf16>(bias_row[nt][i & 1][key]);
             }
         }
         const int bar = seq % C::kBars;
@@ -437,6 +443,11 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       }
 
       // ---- merge the eight warps: the upper four into the lower four, then all threads over the rest
+      // Element (d, row) of a warp's O in the merge buffer: rows in pairs, the pairs of a d exchanged by d, so that a warp
+      // that reads one pair of 32 consecutive d meets no bank twice in 128 bytes.
+      auto merge_at = [&](int w4, int d, int pair) {
+        return merge + (w4 * C::kHPad + d) * C::kRows + 2 * (pair ^ (kNT == 1 ? (d >> 2) & 3 : (d >> 1) & 7));
+      };
       auto put = [&](int w4) {
 #pragma unroll
         for (int nt = 0; nt < kNT; ++nt) {
@@ -444,8 +455,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           for (int mt = 0; mt < kSteps; ++mt) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-              float* dst = merge + ((w4 * C::kHPad + mt * 16 + g + i * 8) * kNT + nt) * 8 + 2 * c;
-              *reinterpret_cast<float2*>(dst) = make_float2(o[mt][nt][2 * i], o[mt][nt][2 * i + 1]);
+              *reinterpret_cast<float2*>(merge_at(w4, mt * 16 + g + i * 8, nt * 4 + c)) = make_float2(o[mt][nt][2 * i], o[mt][nt][2 * i + 1]);
             }
           }
         }
@@ -491,8 +501,7 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           for (int mt = 0; mt < kSteps; ++mt) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-              const float2 v =
-                  *reinterpret_cast<const float2*>(merge + ((warp * C::kHPad + mt * 16 + g + i * 8) * kNT + nt) * 8 + 2 * c);
+              const float2 v = *reinterpret_cast<const float2*>(merge_at(warp, mt * 16 + g + i * 8, nt * 4 + c));
               o[mt][nt][2 * i] = o[mt][nt][2 * i] * cs[0] + v.x * co[0];
               o[mt][nt][2 * i + 1] = o[mt][nt][2 * i + 1] * cs[1] + v.y * co[1];
             }
@@ -504,33 +513,40 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       ptx::named_barrier_sync(1, kWarps * 32);
       const bool whole = t == unit_t0 && seg_end == unit_t0 + a.tiles_per_unit;
       float* part = a.partial + (static_cast<int64_t>(blockIdx.x) * a.slots + (a.slots == 2 && t == unit_t0 ? 1 : 0)) * a.F * (a.H + 2);
-      for (int f = 0; f < a.F; ++f) {
-        float m_all = -INFINITY;
+      // A thread takes one d of two rows at a time, neighbours the next d.
+      for (int item = threadIdx.x; item < (a.F + 1) / 2 * C::kHPad; item += kWarps * 32) {
+        const int pair = item / C::kHPad, d = item % C::kHPad;
+        float2 v[4];
 #pragma unroll
-        for (int w = 0; w < 4; ++w) m_all = fmaxf(m_all, sm_m[w * C::kRows + f]);
-        float l_all = 0.0f, cw[4];
+        for (int w = 0; w < 4; ++w) v[w] = *reinterpret_cast<const float2*>(merge_at(w, d, pair));
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const float m_w = sm_m[w * C::kRows + f];
-          cw[w] = m_w == -INFINITY ? 0.0f : ptx::ex2_approx(m_w - m_all);
-          l_all += sm_l[w * C::kRows + f] * cw[w];
-        }
-        const int d = threadIdx.x;
-        if (d < a.H) {
-          float v = 0.0f;
+        for (int i = 0; i < 2; ++i) {
+          const int f = 2 * pair + i;
+          if (f >= a.F) break;
+          float m_all = -INFINITY;
 #pragma unroll
-          for (int w = 0; w < 4; ++w) v += merge[(w * C::kHPad + d) * C::kRows + f] * cw[w];
-          if (whole)
-            a.out[batch * a.o_strides[0] + head * a.o_strides[1] + f * a.o_strides[2] + d] = from_f32<kBf16>(v / l_all);
-          else
-            part[f * (a.H + 2) + d] = v;
-        }
-        if (threadIdx.x == 0) {
-          if (whole) {
-            if (a.lse != nullptr) a.lse[static_cast<int64_t>(unit) * a.F + f] = fmaf(m_all, kLn2, logf(l_all));
-          } else {
-            part[f * (a.H + 2) + a.H] = m_all;
-            part[f * (a.H + 2) + a.H + 1] = l_all;
+          for (int w = 0; w < 4; ++w) m_all = fmaxf(m_all, sm_m[w * C::kRows + f]);
+          float l_all = 0.0f, o_all = 0.0f;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            const float m_w = sm_m[w * C::kRows + f];
+            const float cw = m_w == -INFINITY ? 0.0f : ptx::ex2_approx(m_w - m_all);
+            l_all += sm_l[w * C::kRows + f] * cw;
+            o_all += (i == 0 ? v[w].x : v[w].y) * cw;
+          }
+          if (d < a.H) {
+            if (whole)
+              a.out[batch * a.o_strides[0] + head * a.o_strides[1] + f * a.o_strides[2] + d] = from_f32<kBf16>(o_all / l_all);
+            else
+              part[f * (a.H + 2) + d] = o_all;
+          }
+          if (d == 0) {
+            if (whole) {
+              if (a.lse != nullptr) a.lse[static_cast<int64_t>(unit) * a.F + f] = fmaf(m_all, kLn2, logf(l_all));
+            } else {
+              part[f * (a.H + 2) + a.H] = m_all;
+              part[f * (a.H + 2) + a.H + 1] = l_all;
+            }
           }
         }
       }
@@ -540,33 +556,60 @@ fmha_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   if (*abort_flag != 0) __nanosleep(2000000);
 }
 
-// One CTA per (range boundary, row): the first boundary inside a unit merges the unit's partials.
+// One CTA per (cut unit, row), thread = head element.  Units cut into `ranges` equal ranges: a CTA for each.  Ranges that
+// end anywhere (ranges 0): a CTA for each boundary, of which the first one inside a unit merges it.
 template <bool kBf16>
 __global__ void __launch_bounds__(256)
-fmha_decode_mma_combine_kernel(const __grid_constant__ Args a, int ctas) {
+fmha_decode_mma_combine_kernel(const __grid_constant__ Args a, int ctas, int ranges) {
   ptx::grid_dependency_wait();
-  const int cta = blockIdx.x + 1;
   const int f = blockIdx.y;
-  const int cut = range_begin(a.pieces, a.piece, cta, ctas);
-  const int unit = cut / a.tiles_per_unit;
-  const int unit_t0 = unit * a.tiles_per_unit;
-  if (cut == unit_t0 || range_begin(a.pieces, a.piece, cta - 1, ctas) > unit_t0) return;
-  int last = cta;   // the CTA that finishes the unit
-  while (last + 1 < ctas && range_begin(a.pieces, a.piece, last + 1, ctas) < unit_t0 + a.tiles_per_unit) ++last;
+  int unit, cta, last;   // CTA cta - 1 starts the unit or has its first tiles, CTA last finishes it
+  if (ranges > 0) {
+    unit = blockIdx.x;
+    cta = unit * ranges + 1;
+    last = cta + ranges - 2;
+  } else {
+    cta = blockIdx.x + 1;
+    const int cut = range_begin(a.pieces, a.piece, cta, ctas);
+    unit = cut / a.tiles_per_unit;
+    const int unit_t0 = unit * a.tiles_per_unit;
+    if (cut == unit_t0 || range_begin(a.pieces, a.piece, cta - 1, ctas) > unit_t0) return;
+    last = cta;
+    while (last + 1 < ctas && range_begin(a.pieces, a.piece, last + 1, ctas) < unit_t0 + a.tiles_per_unit) ++last;
+  }
   const int64_t pitch = static_cast<int64_t>(a.F) * (a.H + 2);
   const float* row = a.partial + f * (a.H + 2);
   auto part = [&](int c) { return row + (a.slots * c + (a.slots == 2 && c == cta - 1 ? 1 : 0)) * pitch; };
-  float m_all = -INFINITY;
-  for (int c = cta - 1; c <= last; ++c) m_all = fmaxf(m_all, part(c)[a.H]);
-  float l_all = 0.0f, o = 0.0f;
+  // Maxima, sums and values of many parts are asked for together: one trip to memory in place of one for each.
+  constexpr int kHeld = 16;
   const int d = threadIdx.x;
-#pragma unroll 4
-  for (int c = cta - 1; c <= last; ++c) {
-    const float* pc = part(c);
-    const float m = pc[a.H];
-    const float coef = m == -INFINITY ? 0.0f : ptx::ex2_approx(m - m_all);
-    l_all += pc[a.H + 1] * coef;
-    if (d < a.H) o += pc[d] * coef;
+  float m_all = -INFINITY, l_all = 0.0f, o = 0.0f;
+  for (int c0 = cta - 1; c0 <= last; c0 += kHeld) {
+    float m[kHeld], l[kHeld], v[kHeld];
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      m[i] = -INFINITY;
+      l[i] = v[i] = 0.0f;
+      if (c0 + i <= last) {
+        const float* pc = part(c0 + i);
+        m[i] = pc[a.H];
+        l[i] = pc[a.H + 1];
+        if (d < a.H) v[i] = pc[d];
+      }
+    }
+    float m_new = m_all;
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) m_new = fmaxf(m_new, m[i]);
+    const float old = m_all == -INFINITY ? 0.0f : ptx::ex2_approx(m_all - m_new);
+    l_all *= old;
+    o *= old;
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const float coef = m[i] == -INFINITY ? 0.0f : ptx::ex2_approx(m[i] - m_new);
+      l_all += l[i] * coef;
+      o += v[i] * coef;
+    }
+    m_all = m_new;
   }
   const int head = unit % a.N, batch = unit / a.N;
   if (d < a.H) a.out[batch * a.o_strides[0] + head * a.o_strides[1] + f * a.o_strides[2] + d] = from_f32<kBf16>(o / l_all);
@@ -582,7 +625,8 @@ struct Plan {
 
 // What the two kernels take, in ns (L2-warm launches in a CUDA graph, bf16, 4 to 1024 units, 17 to 4096 keys, fitted
 // with 5 to 7 % mean error).  The split-key kernel runs two rows a CTA and two CTAs an SM in waves; here a unit costs
-// its merge, which grows with the rows and the head, beside its keys, and a cut unit the merge kernel.
+// its merge, which grows with the rows and the head, beside its keys, and a cut unit the merge kernel.  (Launches of
+// whole units have become 2 to 3 us shorter since, cut ones 4 to 10: the lines lie on the other ways' side.)
 struct Cost {
   int split_per_key, split_merge;                  // [slabs - 1]
   int unit[2], row[2], per_key[2];                 // up to 8 rows, more
@@ -659,23 +703,12 @@ int launch_typed(const CUtensorMap& tk, const CUtensorMap& tv, const Args& a, co
     IXK_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
     configured_device = dev.device;
   }
-  fn<<<plan.ctas, kThreads, C::kSmemBytes, stream>>>(tk, tv, a);
-  IXK_CUDA_OK(cudaGetLastError());
-  count_launch();
-  if (plan.slots > 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(plan.ctas - 1, a.F, 1);
-    cfg.blockDim = dim3(256, 1, 1);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    IXK_CUDA_OK(cudaLaunchKernelEx(&cfg, &fmha_decode_mma_combine_kernel<kBf16>, a, plan.ctas));
-    count_launch();
-  }
-  return IXK_OK;
+  const int rc = launch_overlapped(fn, dim3(plan.ctas), dim3(kThreads), C::kSmemBytes, stream, tk, tv, a);
+  if (rc != IXK_OK || plan.slots == 0) return rc;
+  // (slots 1: equal ranges inside units, ctas = units * ranges)
+  const int units = plan.pieces / plan.tiles_per_unit, ranges = plan.slots == 1 ? plan.ctas / units : 0;
+  return launch_overlapped(&fmha_decode_mma_combine_kernel<kBf16>, dim3(ranges > 0 ? units : plan.ctas - 1, a.F), dim3(kSlabs * 64), 0, stream, a,
+                           plan.ctas, ranges);
 }
 
 }  // namespace

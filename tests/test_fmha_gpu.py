@@ -393,6 +393,27 @@ def test_decode_several_rows_little_scratch(pkg, cuda):
     assert call(q[:2], k[:2], v[:2], 1024)[0] == pkg.IXK_WORKSPACE_TOO_SMALL
 
 
+@pytest.mark.parametrize("case", [(150, 1, 5, 97, 256), (1, 3, 7, 3100, 256), (1, 1, 16, 5000, 64), (53, 3, 12, 900, 192)],
+                         ids=["whole", "ranges", "one-unit", "shares"])
+def test_decode_several_rows_in_a_chain(pkg, cuda, case):
+    """Every call's queries are the result of the call before it, which may still run when it starts, and all use the same
+    scratch: the bits of the chain with the device idle before every call."""
+    B, N, F, T, H = case
+    g = torch.Generator().manual_seed(T)
+    q = torch.randn(B, N, F, H, generator=g).bfloat16().to(cuda)
+    k, v = (torch.randn(B, N, T, H, generator=g).bfloat16().to(cuda) for _ in range(2))
+    ws = torch.empty(max(16, pkg.fmha_workspace_bytes(q, k, v, None, q, H ** -0.5)), dtype=torch.uint8, device=cuda)
+
+    def chain(idle):
+        x = [q.clone(), torch.empty_like(q)]
+        for i in range(12):
+            pkg.fmha_forward_kernel(None, x[i % 2], k, v, None, None, 0.0, x[1 - i % 2], None, H ** -0.5, workspace=ws)
+            if idle:
+                torch.cuda.synchronize()
+        return x
+    assert all(torch.equal(a, b) for a, b in zip(chain(False), chain(True)))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
 @pytest.mark.parametrize("F,H", [(2, 64), (3, 256), (4, 128), (8, 72), (9, 256), (16, 192)])
 def test_decode_several_rows_causal_unwritten_cache(pkg, orc, cuda, F, H, dtype):
