@@ -623,19 +623,22 @@ struct Plan {
   int slots = 0;      // partials that a CTA may leave: 0 whole units, 1 a range inside a unit, 2 a range over several
 };
 
-// What the two kernels take, in ns (L2-warm launches in a CUDA graph, bf16, 4 to 1024 units, 17 to 4096 keys, fitted
-// with 5 to 7 % mean error).  The split-key kernel runs two rows a CTA and two CTAs an SM in waves; here a unit costs
-// its merge, which grows with the rows and the head, beside its keys, and a cut unit the merge kernel.  (Launches of
-// whole units have become 2 to 3 us shorter since, cut ones 4 to 10: the lines lie on the other ways' side.)
+// What the two kernels take, in ns (L2-warm launches in a CUDA graph, bf16, heads of 64, 128 and 256, 4 to 512 units, 40 to
+// 4000 keys, 2 to 16 rows; fitted with 4 to 7 % mean error, heads of up to 192 in between).  The split-key kernel runs two
+// rows a CTA and two CTAs an SM in waves; here a unit costs its merge, which grows with the rows and the head, beside its
+// keys, and a cut unit the merge kernel.
 struct Cost {
-  int split_per_key, split_merge;                  // [slabs - 1]
-  int unit[2], row[2], per_key[2];                 // up to 8 rows, more
+  int split_per_key, split_merge, split_percent;   // [slabs - 1]
+  int unit[2], row[2], per_key_tenths[2], cut_per_range[2];   // up to 8 rows, more
 };
-constexpr Cost kCosts[4] = {{14, 2800, {800, 1000}, {200, 260}, {6, 9}},
-                            {30, 3200, {1050, 1600}, {230, 320}, {8, 13}},
-                            {59, 3900, {1250, 2600}, {240, 330}, {15, 19}},
-                            {59, 4300, {1850, 3400}, {290, 370}, {18, 28}}};
-constexpr int kCutCost[2] = {4200, 4900}, kCutPerRange[2] = {170, 280};
+constexpr Cost kCosts[4] = {{14, 2800, 100, {760, 1110}, {29, 70}, {56, 86}, {30, 20}},
+                            {30, 3200, 93, {850, 1970}, {129, 170}, {70, 126}, {30, 36}},
+                            {59, 3900, 90, {960, 3000}, {172, 190}, {137, 180}, {50, 70}},
+                            {59, 4300, 88, {1350, 3660}, {255, 224}, {169, 240}, {80, 100}}};
+constexpr int kCutCost[2] = {2300, 2600}, kShareCost[2] = {4200, 4900};   // (400 above the fit of a cut: near it whole units win)
+// With no SM left free, the merge and the kernel behind it start only as these CTAs, which fill an SM's registers, end
+// (8 units of 4000 keys H64, 16 and 18 ranges: F4 6.6 and 8.4 us, F16 9.3 and 12.5; 16 of 2000 keys, 8 and 9: F4 6.4 and 8.3).
+constexpr int64_t kFullCost = 2000;
 
 bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   const int keys = slabs_of(p.H) > 2 ? 32 : 64;
@@ -651,7 +654,7 @@ bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   const int wide = p.F > 8 ? 1 : 0;
   const int64_t fit = static_cast<int64_t>(kMaxPartialBytes / (static_cast<size_t>(p.F) * (p.H + 2) * sizeof(float)));
   const int64_t unit_ns = cost.unit[wide] + static_cast<int64_t>(cost.row[wide]) * p.F;
-  const int64_t keys_ns = static_cast<int64_t>(cost.per_key[wide]) * p.T;
+  const int64_t keys_ns = static_cast<int64_t>(cost.per_key_tenths[wide]) * p.T / 10;
   // Whole units; or, with no more units than SMs, each cut into equal ranges (equal shares of the tiles, which end
   // anywhere, were slower there: 16 units of 480 keys H256 F4 17 us, 11 whole); or, with more, equal shares (B20 N16
   // H256 F16, 130 keys: 59 us, 43 whole; 160 to 512 units H256, where the CTAs that go without in the last round could
@@ -659,7 +662,7 @@ bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   int64_t ns = (units + sm_count - 1) / sm_count * (unit_ns + keys_ns), ranges = 1;
   plan->slots = 0;
   for (int64_t r = 2; r <= std::min({sm_count / units, static_cast<int64_t>(p.T / 128), fit / units}); ++r) {
-    const int64_t t = unit_ns + keys_ns / r + kCutCost[wide] + kCutPerRange[wide] * r;
+    const int64_t t = unit_ns + keys_ns / r + kCutCost[wide] + cost.cut_per_range[wide] * r + (units * r * 8 > sm_count * 7 ? kFullCost : 0);
     if (t < ns) {
       ns = t;
       ranges = r;
@@ -668,21 +671,21 @@ bool make_plan(const Problem& p, int sm_count, Plan* plan) {
   }
   const int64_t shares = std::min<int64_t>(sm_count, fit / 2);
   if (units > sm_count && shares > 1) {
-    const int64_t t = unit_ns + units * (unit_ns + keys_ns) / shares + kCutCost[wide];
+    const int64_t t = unit_ns + units * (unit_ns + keys_ns) / shares + kShareCost[wide];
     if (t < ns) {
       ns = t;
       plan->slots = 2;
     }
   }
-  // The split-key kernel stays where the estimates do not put this one 5 % ahead: short caches, and few units with
-  // many rows (one-pass against split-key: 8 units of 480 keys H256 F16 23 and 20 us, F8 14 and 20; 1024 units of 17
-  // keys H256 F2 22 and 15).  95 of the 5600 sizes are more than 2 % slower by this choice, 15 % at most; on average
-  // they take 0.53 of the split-key kernel's time.
+  // The split-key kernel stays where the estimates do not put this one 5 % ahead: short caches with many units and few
+  // rows, and few units of 256-wide heads with many rows (one-pass against split-key, us: 4 units of 300 keys H256 F16 14
+  // and 12; 16 units of 40 keys H128 F8 4.0 and 3.5; the other way 4 units of 4000 keys H64 F16 9.1 and 19, H128 F4 7.4 and
+  // 15, 16 of 1000 keys H64 F16 7.8 and 15, 64 of 40 keys H64 F16 4.4 and 7.8).
   const int splits = decode_splits(p, sm_count);
   const int64_t split_ctas = units * ((p.F + 1) / 2) * splits, waves = (split_ctas + 2 * sm_count - 1) / (2 * sm_count);
   const int64_t split_ns = 550 + waves * (2750 + static_cast<int64_t>(cost.split_per_key) * ((p.T + splits - 1) / splits)) +
                            (splits > 1 ? cost.split_merge : 0);
-  if ((2500 + ns) * 21 > split_ns * 20) return false;
+  if ((2000 + ns) * 105 > split_ns * cost.split_percent) return false;
   plan->tiles_per_unit = static_cast<int>(per_unit);
   plan->piece = plan->slots == 0 ? static_cast<int>(per_unit) : 1;
   plan->pieces = static_cast<int>(plan->slots == 0 ? units : total);
