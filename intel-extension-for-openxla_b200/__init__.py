@@ -436,18 +436,27 @@ def quantize_fp8(x: torch.Tensor, dtype: torch.dtype):
 def gemm_fp8(lhs_q: torch.Tensor, rhs_q: torch.Tensor, inv_scale_a: float, inv_scale_b: float, *,
              bias: Optional[torch.Tensor] = None, epilogue: str = "DEFAULT",
              out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16,
-             stream=None) -> torch.Tensor:
-    """out = cast((lhs_q @ rhs_q in fp32) * inv_scale_a * inv_scale_b [+ bias, act])."""
+             stream=None, workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """out = cast((lhs_q @ rhs_q in fp32) * inv_scale_a * inv_scale_b [+ bias, act]).  `workspace`: as in gemm().  A call
+    that makes its own result also takes the scratch it can use; one into `out` allocates nothing (it may be in a
+    capture that torch knows nothing of) and cuts K only with `workspace`."""
     if _NATIVE is not None and epilogue in EPILOGUES:
-        r = _NATIVE.gemm(lhs_q, rhs_q, bias, None, out, out_dtype, 1.0, 0.0, EPILOGUES.index(epilogue), None, stream, inv_scale_a,
+        r = _NATIVE.gemm(lhs_q, rhs_q, bias, None, out, out_dtype, 1.0, 0.0, EPILOGUES.index(epilogue), workspace, stream, inv_scale_a,
                          inv_scale_b)
         if r is not None:
             return _native_result(r)
+    takes_scratch = out is None and workspace is None
     if out is None:
         out = torch.empty((*lhs_q.shape[:-1], rhs_q.shape[-1]), device=lhs_q.device, dtype=out_dtype)
-    attrs = gemm_attrs_for(lhs_q, rhs_q, out, 0.0)
-    run_gemm_custom_call(lhs_q, rhs_q, None, out, bias, stream, attrs, epilogue,
-                         inv_scale_a=inv_scale_a, inv_scale_b=inv_scale_b)
+    d = gemm_desc_from_attrs(gemm_attrs_for(lhs_q, rhs_q, out, 0.0), epilogue)
+    _require_cuda(lhs_q, rhs_q, out, bias)
+    need = load_library().ixk_gemm_workspace_bytes(ctypes.byref(d)) if takes_scratch else 0
+    if need:
+        try:
+            workspace = _own_scratch(need, lhs_q.device, stream)
+        except torch.OutOfMemoryError:      # it runs without
+            pass
+    _launch_gemm(d, lhs_q, rhs_q, None, out, bias, stream, inv_scale_a, inv_scale_b, workspace, None)
     return out
 
 

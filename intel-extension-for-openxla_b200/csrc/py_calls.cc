@@ -153,7 +153,7 @@ IXK_PY_FUNCTION(py_gemm, 13)
     Py_RETURN_NONE;
   double sa = 1.0, sb = 1.0;
   const bool fp8 = a[11] != Py_None || a[12] != Py_None;
-  if (fp8 && (!number(a[11], &sa) || !number(a[12], &sb))) Py_RETURN_NONE;
+  if (fp8 && (!number(a[11], &sa) || !number(a[12], &sb) || (out == nullptr && a[5] == Py_None))) Py_RETURN_NONE;
   ixk_gemm_desc d{};
   if (!layout(*lhs, &d.lhs) || !layout(*rhs, &d.rhs)) Py_RETURN_NONE;
   at::Tensor made;
@@ -173,11 +173,12 @@ IXK_PY_FUNCTION(py_gemm, 13)
   d.alpha = static_cast<float>(alpha);
   d.beta = static_cast<float>(beta);
   d.epilogue = static_cast<int32_t>(epilogue);
-  // An fp8 call has no scratch argument: for cutting K, where that pays, it takes its own (with a result of the caller's it
-  // allocates nothing, as a caller that captures it may count on).
+  // An fp8 call that makes its own result takes the scratch it can use as well, from the pool of the stream it was given
+  // (where that is not the current one the twin does).
   at::Tensor own;
-  if (fp8 && ws == nullptr && a[4] == Py_None && a[10] == Py_None) {
+  if (fp8 && ws == nullptr && a[4] == Py_None) {
     if (const size_t need = g_gemm_bytes(&d)) {
+      if (a[10] != Py_None) Py_RETURN_NONE;
       try {
         own = at::empty({static_cast<int64_t>(need)}, at::TensorOptions().device(lhs->device()).dtype(at::kByte));
         ws = &own;

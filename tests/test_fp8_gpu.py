@@ -2,6 +2,8 @@
 operands.  Tolerance: the bf16 output tolerance (rtol 2e-2, atol 2e-2 x output RMS) — the
 kernel's only error sources are fp32 accumulation order and the final rounding."""
 import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -111,3 +113,35 @@ def test_bf16_operands_rejected_by_fp8_entry(pkg, cuda):
     with pytest.raises(pkg.IxkError) as e:
         pkg.gemm_fp8(x, x, 1.0, 1.0)
     assert e.value.status == pkg.IXK_INVALID_ARGUMENT
+
+
+FIRST_CALLS = """
+import sys
+sys.path.insert(0, sys.argv[1])
+import torch
+import __graft_entry__ as entry
+pkg = entry.load_package()
+g = torch.Generator(device="cuda").manual_seed(3)
+x = torch.randn(256, 4096, generator=g, device="cuda").to(torch.float8_e4m3fn)
+w = torch.randn(4096, 4096, generator=g, device="cuda").to(torch.float8_e4m3fn)
+counts, outs = [0], []
+side = torch.cuda.Stream()
+torch.cuda.synchronize()
+for stream in (None, None, side):       # the first call of the process, the same again, and one on a stream that it is given
+    outs.append(pkg.gemm_fp8(x, w, 0.01, 0.02, stream=stream))
+    counts.append(pkg.launch_count())
+need = pkg.gemm_workspace_bytes(x, w)
+outs.append(pkg.gemm_fp8(x, w, 0.01, 0.02, out=torch.empty_like(outs[0]), workspace=torch.empty(need, dtype=torch.uint8, device="cuda")))
+counts.append(pkg.launch_count())
+torch.cuda.synchronize()
+assert [b - a for a, b in zip(counts, counts[1:])] == [2] * 4, counts
+assert all(torch.equal(o, outs[0]) for o in outs)
+"""
+
+
+def test_first_call_of_a_process_is_like_the_next(cuda):
+    """A product that is cut along K is cut in the first call too, on a stream that the call is given, and into the
+    caller's result with the caller's scratch: the same launches, the same bits."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_CALLS, root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr

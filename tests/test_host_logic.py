@@ -169,6 +169,31 @@ def test_forward_without_memory_for_scratch(pkg, fake_calls, monkeypatch, status
         assert args[-3:-1] == ((None, 0) if small is None else (small.data_ptr(), 16))
 
 
+def test_scratch_of_an_fp8_call(pkg, fake_calls, monkeypatch):
+    """A call that makes its own result takes scratch for cutting K too, from the pool of its stream; one into the
+    caller's result allocates nothing and hands on the scratch that it was given; with no memory left it runs without."""
+    x, w = torch.zeros(16, 32).to(torch.float8_e4m3fn), torch.zeros(32, 48).to(torch.float8_e4m3fn)
+    stream = types.SimpleNamespace(cuda_stream=77)
+    out, own = torch.zeros(16, 48, dtype=torch.bfloat16), torch.zeros(64, dtype=torch.uint8)
+
+    def run(**kw):
+        fake_calls.allocated.clear()
+        fake_calls.lib.calls.clear()
+        pkg.gemm_fp8(x, w, 0.5, 2.0, stream=stream, **kw)
+        (name, args), = fake_calls.lib.calls
+        assert name == "ixk_gemm_fp8" and args[-1] == 77
+        return args[-3:-1]
+    assert run()[1] == 4096 and fake_calls.allocated == [None, 77]      # the result, the scratch
+    assert run(out=out) == (None, 0) and fake_calls.allocated == []
+    assert run(out=out, workspace=own) == (own.data_ptr(), 64) and fake_calls.allocated == []
+    assert run(workspace=own) == (own.data_ptr(), 64) and fake_calls.allocated == [None]
+
+    def full(need, device, stream):
+        raise torch.OutOfMemoryError("no memory")
+    monkeypatch.setattr(pkg, "_own_scratch", full)
+    assert run() == (None, 0)
+
+
 def _workspace(pkg, B, N, F, T, H, causal):
     import ctypes
     d = pkg._FmhaDesc()
