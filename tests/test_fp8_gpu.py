@@ -122,8 +122,8 @@ import torch
 import __graft_entry__ as entry
 pkg = entry.load_package()
 g = torch.Generator(device="cuda").manual_seed(3)
-x = torch.randn(256, 4096, generator=g, device="cuda").to(torch.float8_e4m3fn)
-w = torch.randn(4096, 4096, generator=g, device="cuda").to(torch.float8_e4m3fn)
+x = torch.randn(256, 16384, generator=g, device="cuda").to(torch.float8_e4m3fn)
+w = torch.randn(16384, 512, generator=g, device="cuda").to(torch.float8_e4m3fn)
 counts, outs = [0], []
 side = torch.cuda.Stream()
 torch.cuda.synchronize()
