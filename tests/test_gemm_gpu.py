@@ -539,6 +539,25 @@ def test_few_rows(pkg, cuda, shape, kind, lb, scratch):
         assert ((out32.double() - want).abs().max() <= sums + 2.0 ** -22 * c.abs().max()).item()
 
 
+@pytest.mark.parametrize("shape", [(1, 64, 16), (31, 72, 136), (33, 1032, 1000), (100, 80, 12304), (128, 72, 12296)],
+                         ids=lambda s: "M{}K{}N{}".format(*s))
+@pytest.mark.parametrize("dtype,out_dtype", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("in_place", [True, False])
+def test_few_rows_residual(pkg, cuda, shape, dtype, out_dtype, in_place):
+    """A residual read by the GEMM itself (one chunk of K): blocks of 32 rows, whole and not, C a buffer of its own or D."""
+    M, K, N = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w = torch.randn(M, K, generator=g, device=cuda).to(dtype), (torch.randn(K, N, generator=g, device=cuda) * 0.1).to(dtype)
+    c = torch.randn(M, N, generator=g, device=cuda).to(out_dtype)
+    want = x.double() @ w.double() - 0.5 * c.double()
+    n0 = pkg.launch_count()
+    out = pkg.gemm(x, w, c=c, beta=-0.5, out=c if in_place else torch.empty_like(c))
+    assert pkg.launch_count() - n0 == 1
+    half = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -22}[out_dtype]
+    sums = (K + 16) * 2.0 ** -23 * (x.double().abs() @ w.double().abs() + 1).max()
+    assert ((out.double() - want).abs().max() <= 1.01 * half * want.abs().max() + sums).item()
+
+
 @pytest.mark.parametrize("shape", [(300, 8200, 520), (257, 5000, 128), (1500, 8256, 136), (900, 16000, 304)], ids=lambda s: "M{}K{}N{}".format(*s))
 @pytest.mark.parametrize("kind", ["bf16", "fp16", "e4m3"])
 @pytest.mark.parametrize("la", ["row", "col"])
