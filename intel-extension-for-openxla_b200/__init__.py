@@ -377,14 +377,24 @@ def gemm_attrs_for(lhs: torch.Tensor, rhs: torch.Tensor, output: torch.Tensor, b
     return attrs
 
 
+def _require_c(c: torch.Tensor, out: torch.Tensor) -> None:
+    """C is read with the result's type, order and pitch: it has to lie in memory as the result does (dimensions of one
+    entry aside), or be dense rows of the same length where the result is."""
+    same = [(n, s) for n, s in zip(c.shape, c.stride()) if n != 1] == [(n, s) for n, s in zip(out.shape, out.stride()) if n != 1]
+    dense = c.is_contiguous() and out.is_contiguous() and c.numel() == out.numel() and (c.dim() < 2 or c.shape[-1] == out.shape[-1])
+    if c.dtype != out.dtype or not (same or dense):
+        raise IxkError(IXK_INVALID_ARGUMENT, "c must have the result's type, shape and strides")
+
+
 def gemm(lhs: torch.Tensor, rhs: torch.Tensor, *, bias: Optional[torch.Tensor] = None,
          c: Optional[torch.Tensor] = None, beta: float = 0.0, epilogue: str = "DEFAULT",
          out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
          stream=None, workspace: Optional[torch.Tensor] = None, alpha: float = 1.0,
          aux: Optional[torch.Tensor] = None) -> torch.Tensor:
     """out = act(alpha * lhs @ rhs + bias + beta*c) through "__cublas$lt$matmul"'s path.  Any mix of
-    row-/column-major 2-D (or batched 3-D) views is passed through as-is, never copied.  With a
-    *_AUX epilogue `aux` receives the values the activation is applied to."""
+    row-/column-major 2-D (or batched 3-D) views is passed through as-is, never copied; c has the
+    result's type, shape and strides.  With a *_AUX epilogue `aux` receives the values the
+    activation is applied to."""
     if _NATIVE is not None and aux is None and epilogue in EPILOGUES:
         r = _NATIVE.gemm(lhs, rhs, bias, c, out, out_dtype, alpha, beta, EPILOGUES.index(epilogue), workspace, stream, None, None)
         if r is not None:
@@ -394,6 +404,8 @@ def gemm(lhs: torch.Tensor, rhs: torch.Tensor, *, bias: Optional[torch.Tensor] =
         out = torch.empty(shape, device=lhs.device, dtype=out_dtype or lhs.dtype)
     d = _gemm_desc(_matrix_layout("lhs", lhs), _matrix_layout("rhs", rhs), _matrix_layout("output", out),
                    out.shape[0] if out.dim() == 3 else 1, float(alpha), float(beta), epilogue)
+    if c is not None and d.beta != 0.0:
+        _require_c(c, out)
     _require_cuda(lhs, rhs, c, out, bias, aux)
     _launch_gemm(d, lhs, rhs, c, out, bias, stream, None, None, workspace, aux)
     return out

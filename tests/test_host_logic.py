@@ -169,6 +169,35 @@ def test_forward_without_memory_for_scratch(pkg, fake_calls, monkeypatch, status
         assert args[-3:-1] == ((None, 0) if small is None else (small.data_ptr(), 16))
 
 
+def test_gemm_refuses_a_residual_that_does_not_lie_like_the_result(pkg, fake_calls):
+    """C is read with the result's pitch, order and type: a pitched, transposed, smaller or wider-typed one is an error,
+    not a read of other memory; what lies as the result does is taken, whatever it is called."""
+    bf16 = torch.bfloat16
+    x, w = torch.zeros(6, 16, dtype=bf16), torch.zeros(16, 8, dtype=bf16)
+    out = torch.zeros(6, 8, dtype=bf16)
+    pitched = torch.zeros(6, 24, dtype=bf16)[:, :8]
+    refused = [(out, pitched), (out, torch.zeros(8, 6, dtype=bf16).t()), (out, torch.zeros(8, 6, dtype=bf16)), (out, out.float()),
+               (out, torch.zeros(5, 8, dtype=bf16)), (out, torch.zeros(8, dtype=bf16)), (out, torch.zeros(1, 8, dtype=bf16).expand(6, 8)),
+               (pitched, out), (torch.zeros(8, 6, dtype=bf16).t(), out), (None, pitched)]
+    for o, c in refused:
+        with pytest.raises(pkg.IxkError, match="c must have") as e:
+            pkg.gemm(x, w, c=c, beta=1.0, out=o, stream=types.SimpleNamespace(cuda_stream=1))
+        assert e.value.status == pkg.IXK_INVALID_ARGUMENT
+    assert fake_calls.lib.calls == []
+    taken = [(out, out), (out, torch.zeros(1, 6, 8, dtype=bf16)), (out, torch.zeros(48, dtype=bf16)), (out, torch.zeros(2, 3, 8, dtype=bf16)),
+             (pitched, torch.zeros(6, 24, dtype=bf16)[:, 8:16]), (None, out)]
+    for o, c in taken:
+        pkg.gemm(x, w, c=c, beta=1.0, out=o, stream=types.SimpleNamespace(cuda_stream=1))
+    pkg.gemm(x, w, c=pitched, out=out, stream=types.SimpleNamespace(cuda_stream=1))      # (beta 0: not read)
+    one = torch.zeros(1, 24, dtype=bf16)[:, :8]
+    pkg.gemm(x[:1], w, c=one, beta=1.0, out=out[:1], stream=types.SimpleNamespace(cuda_stream=1))   # (one row: no pitch)
+    b = torch.zeros(2, 6, 8, dtype=bf16)
+    pkg.gemm(x.expand(2, 6, 16), w.expand(2, 16, 8), c=b, beta=1.0, out=torch.zeros_like(b), stream=types.SimpleNamespace(cuda_stream=1))
+    with pytest.raises(pkg.IxkError, match="c must have"):
+        pkg.gemm(x.expand(2, 6, 16), w.expand(2, 16, 8), c=out, beta=1.0, out=b, stream=types.SimpleNamespace(cuda_stream=1))
+    assert len(fake_calls.lib.calls) == len(taken) + 3
+
+
 def test_scratch_of_an_fp8_call(pkg, fake_calls, monkeypatch):
     """A call that makes its own result takes scratch for cutting K too, from the pool of its stream; one into the
     caller's result allocates nothing and hands on the scratch that it was given; with no memory left it runs without."""
