@@ -1,4 +1,4 @@
-"""Builds lib/libixk.so from csrc/*.cu with nvcc for sm_100a (cross-compiles without a GPU), and lib/ixk_calls.so, the
+"""Builds lib/libixk.so from csrc/*.cu with nvcc for sm_100a (cross-compiles without a GPU), and lib/ixk_calls-*.so, the
 Python package's native calls, from csrc/py_calls.cc with the host compiler against the installed torch.
 
 Run as a script (python build.py [--force] [--verbose]) or call build().
@@ -19,7 +19,6 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libixk.so")
-CALLS_PATH = os.path.join(LIB_DIR, "ixk_calls.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -78,26 +77,38 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    build_calls(force)
+    try:
+        build_calls(force)
+    except (ImportError, OSError, RuntimeError) as e:      # (the library and the Python package work without)
+        print(f"native calls not built, the package's calls go through Python: {e}", file=sys.stderr)
     return LIB_PATH
+
+
+def calls_path(lib_dir: str = LIB_DIR) -> str:
+    """Where the native calls for this interpreter and torch are.  They use torch's C++ classes, whose layout is each
+    version's own: one built against another is another file, which nobody loads."""
+    import torch
+    made_for = f"torch{torch.__version__}-cxx{int(torch._C._GLIBCXX_USE_CXX11_ABI)}"
+    return os.path.join(lib_dir, f"ixk_calls-{made_for}{sysconfig.get_config_var('EXT_SUFFIX')}")
 
 
 def build_calls(force: bool = False) -> str:
     import torch
+    path = calls_path()
     source = os.path.join(CSRC, "py_calls.cc")
-    inputs = [source, os.path.join(INCLUDE, "ixk.h"), os.path.abspath(__file__), torch.__file__]
-    if not force and os.path.exists(CALLS_PATH) and os.path.getmtime(CALLS_PATH) > _newest(inputs):
-        return CALLS_PATH
+    inputs = [source, os.path.join(INCLUDE, "ixk.h"), os.path.abspath(__file__)]
+    if not force and os.path.exists(path) and os.path.getmtime(path) > _newest(inputs):
+        return path
     home = os.path.dirname(torch.__file__)
     cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-I", INCLUDE, "-I", os.path.join(home, "include"), "-I", os.path.join(home, "include", "torch", "csrc", "api", "include"),
-           "-I", sysconfig.get_paths()["include"], "-I", cuda_include, source, "-o", CALLS_PATH,
+           "-I", sysconfig.get_paths()["include"], "-I", cuda_include, source, "-o", path,
            "-L", os.path.join(home, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on py_calls.cc:\n{r.stdout}\n{r.stderr}")
-    return CALLS_PATH
+    return path
 
 
 if __name__ == "__main__":

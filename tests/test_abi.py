@@ -270,6 +270,24 @@ def test_missing_library_fails_loudly(pkg, monkeypatch):
         pkg.load_library()
 
 
+def test_native_calls_belong_to_this_interpreter_and_torch(pkg, monkeypatch, tmp_path):
+    """The extension's name says what it was built for; without one for this interpreter and torch the library loads all
+    the same and the package's calls go through Python."""
+    import sysconfig
+
+    import torch
+    name = os.path.basename(pkg.calls_path())
+    assert torch.__version__ in name and name.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+    assert pkg._NATIVE is not None and pkg._NATIVE.__file__ == pkg.calls_path()
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    assert os.path.basename(pkg.calls_path()) != name and not os.path.exists(pkg.calls_path())
+    monkeypatch.setattr(pkg, "_LIB", None)
+    monkeypatch.setattr(pkg, "_NATIVE", None)
+    assert pkg.load_library().ixk_version() and pkg._NATIVE is None
+    with pytest.raises(pkg.IxkError, match="no CPU path"):
+        pkg.gemm(torch.zeros(8, 8), torch.zeros(8, 8))
+
+
 def test_cpu_tensors_are_rejected(pkg):
     import torch
     x = torch.zeros(8, 8, dtype=torch.bfloat16)
