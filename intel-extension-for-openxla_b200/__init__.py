@@ -301,7 +301,7 @@ def run_gemm_custom_call(lhs: torch.Tensor, rhs: torch.Tensor, add: Optional[tor
     output's type, shape and order)."""
     if epilogue not in EPILOGUES:
         raise IxkError(IXK_INVALID_ARGUMENT, "Unknown Epilogue.")  # onednn_matmul_utils.cc:52-54
-    _require_cuda(lhs, rhs, add, output, bias, aux)
+    _require_cuda(lhs, rhs, add, output, bias, aux, workspace)
     _launch_gemm(gemm_desc_from_attrs(attrs, epilogue), lhs, rhs, add, output, bias, stream, inv_scale_a, inv_scale_b, workspace, aux)
 
 
@@ -409,7 +409,7 @@ def gemm(lhs: torch.Tensor, rhs: torch.Tensor, *, bias: Optional[torch.Tensor] =
                    out.shape[0] if out.dim() == 3 else 1, float(alpha), float(beta), epilogue)
     if c is not None and d.beta != 0.0:
         _require_c(c, out)
-    _require_cuda(lhs, rhs, c, out, bias, aux)
+    _require_cuda(lhs, rhs, c, out, bias, aux, workspace)
     _launch_gemm(d, lhs, rhs, c, out, bias, stream, None, None, workspace, aux)
     return out
 
@@ -429,6 +429,7 @@ def gemm_geglu(x: torch.Tensor, w_gate_up: torch.Tensor, *, out: Optional[torch.
     # (the product before the GeGLU: [m, n2] row-major, never stored)
     d = _gemm_desc(_matrix_layout("lhs", x), _matrix_layout("rhs", w_gate_up), (ROW_MAJOR, _TORCH_TO_IXK[x.dtype], m, n2, m * n2, n2),
                    1, 1.0, 0.0, "DEFAULT")
+    _require_cuda(x, w_gate_up, out, workspace)
     lib = load_library()
     if workspace is None:
         workspace = _own_scratch(lib.ixk_gemm_geglu_workspace_bytes(ctypes.byref(d)), x.device, stream)
@@ -464,7 +465,7 @@ def gemm_fp8(lhs_q: torch.Tensor, rhs_q: torch.Tensor, inv_scale_a: float, inv_s
     if out is None:
         out = torch.empty((*lhs_q.shape[:-1], rhs_q.shape[-1]), device=lhs_q.device, dtype=out_dtype)
     d = gemm_desc_from_attrs(gemm_attrs_for(lhs_q, rhs_q, out, 0.0), epilogue)
-    _require_cuda(lhs_q, rhs_q, out, bias)
+    _require_cuda(lhs_q, rhs_q, out, bias, workspace)
     need = load_library().ixk_gemm_workspace_bytes(ctypes.byref(d)) if takes_scratch else 0
     if need:
         try:
@@ -495,6 +496,7 @@ def gemm_qkv(x: torch.Tensor, w_qkv: torch.Tensor, *, bias: Optional[torch.Tenso
             raise IxkError(IXK_INVALID_ARGUMENT, "outputs must be row-major [m,n] of the input type with one pitch")
     if bias is not None and (bias.shape != (3, n) or not bias.is_contiguous() or bias.dtype != x.dtype):
         raise IxkError(IXK_INVALID_ARGUMENT, "bias must be a contiguous [3,n] tensor of the input type")
+    _require_cuda(x, w_qkv, bias, *outs)
     lib = load_library()
     _check(lib.ixk_gemm_qkv(_TORCH_TO_IXK[x.dtype], m, n, k, x.data_ptr(), x.stride(0), w_qkv.data_ptr(), n,
                             bias.data_ptr() if bias is not None else None, outs[0].data_ptr(), outs[1].data_ptr(),
@@ -517,6 +519,7 @@ def row_norm(x: torch.Tensor, *, kind: int = NORM_LAYER, eps: float = 1e-5, out:
             return _native_result(r)
     if not x.is_contiguous():
         raise IxkError(IXK_INVALID_ARGUMENT, "row_norm wants a contiguous tensor")
+    _require_cuda(x, out, gain)
     out = torch.empty_like(x) if out is None else out
     if out.shape != x.shape or out.dtype != x.dtype or not out.is_contiguous():
         raise IxkError(IXK_INVALID_ARGUMENT, "out must match x")
@@ -550,6 +553,7 @@ def rotary_interleaved_(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, s
         raise IxkError(IXK_INVALID_ARGUMENT, "cos/sin must be contiguous fp32 [seq_len, rotary_dim/2]")
     if rotary_dim > x.shape[2]:
         raise IxkError(IXK_INVALID_ARGUMENT, "rotary_dim exceeds head_dim")
+    _require_cuda(x, cos, sin)
     fn = load_library().ixk_rotary_half if half_split else load_library().ixk_rotary_interleaved
     _check(fn(_TORCH_TO_IXK[x.dtype], x.data_ptr(), x.shape[0], seq_len, x.shape[1], rotary_dim, x.stride(0), x.stride(1),
               cos.data_ptr(), sin.data_ptr(), _stream_ptr(stream)))
@@ -577,6 +581,7 @@ def kv_append_(k_cache: torch.Tensor, v_cache: torch.Tensor, k_new: torch.Tensor
         raise IxkError(IXK_INVALID_ARGUMENT, "caches [B,T,N,H] and new rows [B,N,H] of matching shapes and strides are expected")
     if not 0 <= position < T:
         raise IxkError(IXK_INVALID_ARGUMENT, "position outside the cache")
+    _require_cuda(k_cache, v_cache, k_new, v_new)
     _check(load_library().ixk_kv_append(_TORCH_TO_IXK[k_cache.dtype], B, N, H, k_new.data_ptr(), v_new.data_ptr(),
                                         k_new.stride(0), k_new.stride(1), k_cache.data_ptr(), v_cache.data_ptr(),
                                         k_cache.stride(0), k_cache.stride(1), k_cache.stride(2), position, _stream_ptr(stream)))
@@ -594,6 +599,7 @@ def residual_add(x: torch.Tensor, partial: torch.Tensor, bias: Optional[torch.Te
     cols = x.shape[-1]
     if bias is not None and (bias.shape != (cols,) or bias.dtype != x.dtype or not bias.is_contiguous()):
         raise IxkError(IXK_INVALID_ARGUMENT, "bias must be a dense [cols] vector of the input type")
+    _require_cuda(x, partial, bias, out)
     out = torch.empty_like(x) if out is None else out
     if out.numel() != x.numel() or out.dtype != x.dtype or not out.is_contiguous():
         raise IxkError(IXK_INVALID_ARGUMENT, "out must match x")
@@ -664,7 +670,7 @@ def fmha_forward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: t
         if r is not None:
             _check(r)
             return
-    _require_cuda(query, key, value, bias, out, activation)
+    _require_cuda(query, key, value, bias, out, activation, workspace)
     if dropout is not None:
         raise IxkError(IXK_UNIMPLEMENTED, "Unimplemented dropout")
     if is_training and activation is None:
@@ -722,7 +728,7 @@ def fmha_backward_kernel(stream, query: torch.Tensor, key: torch.Tensor, value: 
         if r is not None:
             _check(r)
             return
-    _require_cuda(query, key, value, out, bias, grad_out, activation, grad_query, grad_key, grad_value)
+    _require_cuda(query, key, value, out, bias, grad_out, activation, grad_query, grad_key, grad_value, workspace)
     if activation is None or activation.dtype != torch.float32 or not activation.is_contiguous() \
             or activation.shape != query.shape[:3]:
         raise IxkError(IXK_INVALID_ARGUMENT, "activation must be the forward's dense fp32 [B,N,F] log-sum-exp")

@@ -298,6 +298,19 @@ def test_cpu_tensors_are_rejected(pkg):
         pkg.fmha_forward_kernel(None, q, q, q, None, None, 0.0, q.clone(), None, 1.0, False)
 
 
+@pytest.mark.parametrize("call", ["norm", "rotary", "append", "residual", "geglu", "qkv"])
+def test_cpu_tensors_are_rejected_between_the_calls_too(pkg, call):
+    import torch
+    x, w = torch.zeros(8, 16, dtype=torch.bfloat16), torch.zeros(16, 32, dtype=torch.bfloat16)
+    rows, cache, table = x.view(8, 1, 16), torch.zeros(8, 4, 1, 16, dtype=torch.bfloat16), torch.zeros(8, 4)
+    calls = {"norm": lambda: pkg.row_norm(x), "rotary": lambda: pkg.rotary_interleaved_(rows, table, table, 8, 8),
+             "append": lambda: pkg.kv_append_(cache, cache.clone(), rows, rows, 0), "residual": lambda: pkg.residual_add(x, x),
+             "geglu": lambda: pkg.gemm_geglu(x, w, workspace=torch.zeros(1 << 16, dtype=torch.uint8)),
+             "qkv": lambda: pkg.gemm_qkv(x, torch.zeros(3, 16, 8, dtype=torch.bfloat16))}
+    with pytest.raises(pkg.IxkError, match="no CPU path"):
+        calls[call]()
+
+
 def test_oracle_is_not_imported_by_the_product(pkg):
     """The package must not reach into oracle/ (the oracle is test infrastructure)."""
     pkg_dir = os.path.dirname(pkg.__file__)
