@@ -382,10 +382,18 @@ int launch_decode(const Problem& p, const DeviceInfo& dev, void* workspace, size
   dim3 grid(splits * ((p.F + rows_per_cta - 1) / rows_per_cta), p.N, p.B);
   auto launch_lanes = [&](auto lanes_tag) -> int {
     constexpr int kLanes = decltype(lanes_tag)::value;
-    const bool few = rows_per_cta == 1 && static_cast<int64_t>(grid.x) * grid.y * grid.z <= dev.sm_count;
-    auto* fn = few                 ? fmha_decode_kernel<kLanes, 1, kWarpsFew, kUnrollFew>
-               : rows_per_cta == 1 ? fmha_decode_kernel<kLanes, 1, kWarpsMany, kUnrollMany>
-                                   : fmha_decode_kernel<kLanes, 2, kWarpsMany, kUnrollMany>;
+    // Keys that the usual CTA has in flight at once; up to two rounds of them take less time than setting up and merging
+    // twice the warps (B9 N1 H256, 17 keys 2.6 and 4.1 us; a head of 256 with 33 to 64 keys 3.9 and 4.3, 65 to 128 5.3 and
+    // 4.5, more 10.9 to 16 and 8.4 to 12; a head of 128 with 65 to 128 4.3 and 4.5, more 7 to 10 and 5.4 to 8).  Heads of up
+    // to 64 never have more, a CTA having at most kMinKeysPerSplit where there are few.
+    constexpr int kKeysAtOnce = kWarpsMany * (32 / kLanes) * kUnrollMany;
+    constexpr bool kFewPays = 2 * kKeysAtOnce < kMinKeysPerSplit;
+    const bool few = kFewPays && rows_per_cta == 1 && a.keys_per_split > 2 * kKeysAtOnce &&
+                     static_cast<int64_t>(grid.x) * grid.y * grid.z <= dev.sm_count;
+    auto* fn = rows_per_cta == 1 ? fmha_decode_kernel<kLanes, 1, kWarpsMany, kUnrollMany> : fmha_decode_kernel<kLanes, 2, kWarpsMany, kUnrollMany>;
+    if constexpr (kFewPays) {
+      if (few) fn = fmha_decode_kernel<kLanes, 1, kWarpsFew, kUnrollFew>;
+    }
     const int which = few ? 2 : rows_per_cta - 1;
     // What a load has in flight lives in L1.  Behind kernels that leave an SM no idle moment the split between L1 and
     // shared memory stays what the last large kernel wanted, so this one states its own: B64 N16 T4096 H256 inside a
