@@ -28,6 +28,7 @@ namespace {
 
 constexpr int kTileQ = 128;
 constexpr int kMaxKeys = 128;
+constexpr int kAssumedSms = 148;
 constexpr int kThreads = 160;
 constexpr int kBoxElems = 64;                 // 16-bit elements per 128-byte swizzle row
 constexpr int kQBoxBytes = kTileQ * 128;
@@ -250,9 +251,14 @@ fmha_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
 }  // namespace
 
+// Heads of up to 64 always (four CTAs per SM: 0.41 to 0.96 of the general kernel's time over 186 sizes).  Wider ones, two
+// CTAs per SM, up to four tiles an SM, or sixteen with up to 64 keys, beyond which the general kernel's ring hides more
+// than this one's neighbours (H 96 to 128, us, general and this: 4 tiles an SM 0.7 to 1.0 of its time; T 71, 5 tiles an SM,
+// 21.1 and 23.0; T 95, 21 tiles 54 and 73; T 125, 80 tiles 176 and 290; T 28, 20 tiles 50.7 and 53.1).
 bool short_applies(const Problem& p) {
   const int64_t ctas = static_cast<int64_t>(p.B) * p.N * ((p.F + kTileQ - 1) / kTileQ);
-  return p.T <= kMaxKeys && p.H <= 128 && p.bias == nullptr && ctas <= 0x7fffffff;
+  if (p.T > kMaxKeys || p.H > 128 || p.bias != nullptr || ctas > 0x7fffffff) return false;
+  return p.H <= kBoxElems || ctas <= (p.T <= 64 ? 16 : 4) * kAssumedSms;
 }
 
 int launch_short(const Problem& p, const DeviceInfo& dev, cudaStream_t stream) {
