@@ -36,7 +36,7 @@ class KernelOps:
 
     def gemm_residual(self, x, w, residual):
         """residual + x @ w, one rounding: the residual add in the GEMM's epilogue (or its reduce pass)."""
-        return self.pkg.gemm(x, w, c=residual, beta=1.0, workspace=self.gemm_workspace)
+        return self.gemm(x, w, c=residual, beta=1.0)
 
     def gemm_geglu(self, x, w_gate_up):
         """gelu(x @ gate) * (x @ up) with [gate | up] as one weight: one GEMM + one combining pass (decode
@@ -307,7 +307,9 @@ def gemma_decode_step(x: torch.Tensor, w: GemmaLayerWeights, k_cache: torch.Tens
     With `comm` (a comm.Communicator) each row-parallel projection writes its partial into the
     NVLink exchange buffer and one libixk kernel does the exchange and the residual add that
     follows it (the two partials use different offsets, so the second exchange never waits for
-    readers of the first).  Numerics are the Gemma block's: RMSNorm with the (1 + w) scale,
+    readers of the first).  Without an exchange (one rank, no `reduce`) the two projections add the
+    residual in their epilogue: x + projection is rounded once there, twice (projection, sum) with
+    an exchange or an `ops` that has no gemm_residual.  Numerics are the Gemma block's: RMSNorm with the (1 + w) scale,
     rotary embedding on half-split pairs over the whole head, GeGLU with the tanh GELU."""
     B, _, hidden = x.shape
     hl, hd = w.heads_local, w.head_dim

@@ -268,3 +268,16 @@ def test_scratch_of_a_decode_call(pkg, F):
         need = _workspace(pkg, B, N, F, T, H, False)
         assert need == key_splits or key_splits < need <= pkg.STATIC_SCRATCH_BYTES
         assert _workspace(pkg, B, N, F, T, H, True) == key_splits
+
+
+def test_residual_projection_goes_through_the_gemm_of_the_ops(pkg):
+    """A decode step's projections that add the residual are GEMMs like the others: an ops class with a gemm of its own
+    (another scratch, a record of the calls) sees them."""
+    import importlib
+    layers = importlib.import_module("ixk_b200.layers")
+
+    class Ops(layers.KernelOps):
+        def gemm(self, x, w, **kw):
+            return kw
+    r = torch.zeros(2, 8)
+    assert Ops(pkg).gemm_residual(torch.zeros(2, 4), torch.zeros(4, 8), r) == {"c": r, "beta": 1.0}
