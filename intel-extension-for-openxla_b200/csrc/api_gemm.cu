@@ -239,7 +239,8 @@ int run(const ixk_gemm_desc* desc, const void* a, const void* b, const void* c, 
     if (workspace == nullptr || !aligned16(workspace) || workspace_bytes < need)
       return fail(IXK_WORKSPACE_TOO_SMALL, "GeGLU projection: need " + std::to_string(need) + " bytes of 16-byte aligned scratch");
     p.ldd = geglu_ld;   // of the [M, N'] result; the product itself goes to the scratch
-    return gemm::launch_split_k(p, gemm::stream_applies(p) ? gemm::stream_splits(p.M, p.N, p.K, es, workspace_bytes) : splits, workspace, dev, static_cast<cudaStream_t>(stream), true);
+    const int chunks = gemm::stream_applies(p) ? gemm::stream_splits(p.M, p.N, p.K, es, workspace_bytes, /*summed=*/true) : splits;
+    return gemm::launch_split_k(p, chunks, workspace, dev, static_cast<cudaStream_t>(stream), true);
   }
 
   if (const char* env = std::getenv("IXK_GEMM_BLOCK_N")) p.force_block_n = std::atoi(env);

@@ -16,7 +16,7 @@ constexpr int kMaxScatter = 8;  // destinations of a scattered output (= the mos
 // either dimension contiguous.
 struct Problem {
   int64_t M = 0, N = 0, K = 0, batch = 1;
-  bool fp8 = false;          // any operand type other than the 16-bit floats (no split-K path)
+  bool fp8 = false;          // any operand type other than the 16-bit floats
   int kind = 0;              // tcgen05.mma kind: kKindF16 / kKindF8 / kKindTf32 / kKindI8
   int ab_dtype = IXK_BF16;   // 16-bit operand type when kind == kKindF16
   uint32_t a_fmt = 0, b_fmt = 0;  // tcgen05 operand format codes
@@ -92,7 +92,7 @@ int launch_split_k(const Problem& p, int splits, void* workspace, const DeviceIn
 bool stream_takes(int64_t M);
 bool stream_applies(const Problem& p);
 bool stream_alone(const Problem& p);   // also without scratch for chunks of K
-int stream_splits(int64_t M, int64_t N, int64_t K, int elem_bytes, size_t workspace_bytes);
+int stream_splits(int64_t M, int64_t N, int64_t K, int elem_bytes, size_t workspace_bytes, bool summed = false);
 int launch_stream(const Problem& p, int splits, float* partial, const DeviceInfo& dev, cudaStream_t stream);
 
 }  // namespace gemm

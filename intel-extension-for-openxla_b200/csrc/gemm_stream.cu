@@ -6,8 +6,9 @@
 // The weights are the M side of the MMA (128 columns of B = 128 lanes of tensor memory) and the rows of A
 // its N side (16 to 128 wide, M rounded up to 16), so a pipeline stage is 16 KB of weights and 2 KB of A at
 // M <= 16 where gemm_kernel moves and zero-fills 16 KB of A whatever M is.  One CTA works on 128 columns and
-// one chunk of K; chunk count and shared memory are chosen so that all CTAs are on the chip at once, two or
-// three per SM, and HBM sees one even wave instead of rounds of whole tiles.  While the kernel before it in
+// one chunk of K; chunk count and shared memory are chosen so that all CTAs are on the chip at once, up to
+// three per SM, and HBM sees one even wave instead of rounds of whole tiles (up to 56832 columns on 148 SMs;
+// wider products run in rounds: see stream_alone).  While the kernel before it in
 // the stream still runs, a CTA asks for its first stages of weights to be brought into L2 (a hint that reads
 // nothing, so it needs no ordering with that kernel), which uses the HBM time that a decode step's small
 // kernels leave idle.  With several chunks each CTA leaves an fp32 partial [M, 128] in scratch for
@@ -44,6 +45,9 @@ constexpr int kMaxStages = 12;
 constexpr int kTailBytes = 256;      // barriers, tensor-memory address, abort flag
 constexpr int kAssumedSms = 148;
 constexpr int kCtasPerSm = 2;        // CTAs of an SM that a problem is cut for
+constexpr int kMaxCtasPerSm = 3;     // ... and that there are at once where the columns alone are more
+constexpr int kAloneTiles = 96;      // tiles of columns that one chunk of K is enough for
+constexpr int kShortK = 2048;        // bytes of K
 constexpr int kMinChunk = 8;         // slabs of K worth a CTA
 constexpr int kMaxChunks = 32;
 
@@ -77,7 +81,7 @@ __device__ __forceinline__ float load_f32(const void* p, int64_t i, int dtype) {
 }
 // 32 rows of one column, a pitch apart (the lanes of a warp are 32 consecutive columns).  All loads go out together, the
 // type decided once for them: with a decision for each element each load waited for the one before (100 x 16208 x 80 with C
-// in fp32: 34 us, 10 like this).
+// in fp32: 34 us, 6.7 like this; 100 x 182192 x 320, bf16: 222, 62).
 __device__ __forceinline__ void load_rows_f32(const void* src, int64_t at, int64_t pitch, int dtype, int rows, bool ok, float (&v)[32]) {
   if (dtype == IXK_F32) {
     const float* p = static_cast<const float*>(src) + at;
@@ -313,18 +317,29 @@ bool stream_applies(const Problem& p) {
 // gemm_kernel's narrower tiles are level or ahead (us, gemm_kernel and this, bf16: 16 x 512 x 1024 6.3 and 6.1, 64 rows
 // 6.4 and 7.2; 16 x 4096 x 4096 17.8 and 16.7, 128 rows 18.2 and 20.3; 16 x 16384 x 4096 32.4 and 22.6, 128 rows 32.8
 // and 26.6; 64 x 8192 x 8192 32.5 and 32.3).  fp8 with more rows only on K-major weights (128 x 16384 x 4096: 18.5 and
-// 16.8, N-major 13.7 and 16.3).
+// 16.8, N-major 13.7 and 16.3).  More tiles than three CTAs per SM are rounds, each with a set-up and an epilogue that
+// nothing hides, which more than 64 rows do not bear (128 x 59824 x 224 13.1 and 19.7, 80 x 58128 x 6576 128 and 168; 64
+// rows 0.83 of gemm_kernel's time on average and 1.09 at most, 32 rows 0.67), nor more than 16 where a long K is streamed
+// once more for a second round of a third of the CTAs or fewer (64 x 60000 x 6600 132 and 153, 32 x 60000 x 3088 62 and
+// 69); and nor does the epilogue of more than 96 rows behind a short K pay (128 x 35984 x 464 11.4 and 13.9).
 bool stream_alone(const Problem& p) {
+  const int64_t tiles = (p.N + kTileN - 1) / kTileN, k_bytes = p.K * (p.kind == kKindF16 ? 2 : 1);
+  const bool rounds = tiles > kMaxCtasPerSm * kAssumedSms;
+  if (rounds && tiles <= (kMaxCtasPerSm + 1) * kAssumedSms && k_bytes >= 2 * kShortK) return p.M <= 16;
   if (p.M <= 32) return true;
-  if (p.N < kTileN * 96) return false;
-  return p.kind == kKindF16 || !p.b_mn_major;
+  if (tiles < kAloneTiles || (p.kind == kKindF8 && p.b_mn_major)) return false;
+  if (rounds) return p.M <= 64;
+  return p.M <= 96 || tiles > kCtasPerSm * kAssumedSms || k_bytes >= kShortK;
 }
 
 // Chunks of K: as many as give every SM its two CTAs in one wave, each of kMinChunk slabs at least, no more than
 // the scratch holds partials of, and none that would make writing and reading the partials (8 bytes an element) more
-// than half of the weights' bytes.
-int stream_splits(int64_t M, int64_t N, int64_t K, int elem_bytes, size_t workspace_bytes) {
+// than half of the weights' bytes.  Where the columns alone make a CTA for two SMs of three, a second chunk gains less than
+// the pass over the partials costs (one chunk and two, us: 16 x 12832 x 1312 9.8 and 10.9, 64 x 15888 x 2944 19.0 and 23.8,
+// 80 x 13248 x 22368 92.7 and 94.0), unless there is a pass over them anyway (`summed`: GeGLU).
+int stream_splits(int64_t M, int64_t N, int64_t K, int elem_bytes, size_t workspace_bytes, bool summed) {
   const int64_t tiles = (N + kTileN - 1) / kTileN, slabs = (K * elem_bytes + kSlabBytes - 1) / kSlabBytes;
+  if (tiles > kAloneTiles && !summed) return 1;
   const int64_t fit = static_cast<int64_t>(workspace_bytes / (static_cast<size_t>(M) * N * sizeof(float)));
   int64_t chunks = std::min<int64_t>({kCtasPerSm * kAssumedSms / tiles, slabs / kMinChunk, kMaxChunks, fit, K * elem_bytes / (16 * M)});
   chunks = std::max<int64_t>(chunks, 1);
@@ -387,7 +402,7 @@ int launch_stream(const Problem& p, int splits, float* partial, const DeviceInfo
   if (ctas > 0x7fffffff) return fail(IXK_UNIMPLEMENTED, "too many tiles");
   // Shared memory for as many CTAs per SM as one wave takes (the ring of a lone CTA is as deep as there is room), three
   // at most, and no more than tensor memory has columns for.
-  const int per_sm = ctas <= dev.sm_count ? 1 : ctas > kCtasPerSm * dev.sm_count && a.tmem_cols <= 128 ? 3 : kCtasPerSm;
+  const int per_sm = ctas <= dev.sm_count ? 1 : ctas > kCtasPerSm * dev.sm_count && a.tmem_cols <= 128 ? kMaxCtasPerSm : kCtasPerSm;
   const int stage_bytes = kWeightBytes + a.x_bytes;
   a.stages = std::min<int>(kMaxStages, ((228 * 1024) / per_sm - 2 * 1024 - kTailBytes) / stage_bytes);
   const size_t smem = static_cast<size_t>(a.stages) * stage_bytes + kTailBytes + 1024;
