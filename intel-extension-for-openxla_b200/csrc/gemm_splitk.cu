@@ -69,16 +69,20 @@ __device__ __forceinline__ void reduce_epilogue_store(const ReduceArgs& a, int m
   store_from_f32(a.d, static_cast<int64_t>(m) * a.ldd + n, a.out_dtype, v);
 }
 
-// Four consecutive columns of one row summed over the chunks, in chunk order, with the loads of eight chunks in flight
-// together: a decode step's reduce is a few dozen threads whose time is the number of trips to L2.
+// Four consecutive columns of one row summed over the chunks, in chunk order, with the loads of up to eight chunks in
+// flight together: a decode step's reduce is a few dozen threads whose time is the number of trips to L2.  kHeld is no more
+// than there are chunks, up to a power of two: room for eight in every thread left a pass over one or two large planes with
+// too few threads (GeGLU, us, four one by one, eight, and as many as there are: 128 x 42992 x 768 28.9, 29.8, 24.8; 112 x
+// 54512 x 640 27.2, 31.0, 25.6).
+template <int kHeld>
 __device__ __forceinline__ float4 sum_chunks(const float4* src, int64_t plane4, int splits) {
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s0 = 0; s0 < splits; s0 += 8) {
-    float4 v[8];
+  for (int s0 = 0; s0 < splits; s0 += kHeld) {
+    float4 v[kHeld];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = s0 + i < splits ? src[(s0 + i) * plane4] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < kHeld; ++i) v[i] = s0 + i < splits ? src[(s0 + i) * plane4] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < kHeld; ++i) {
       acc.x += v[i].x;
       acc.y += v[i].y;
       acc.z += v[i].z;
@@ -87,7 +91,7 @@ __device__ __forceinline__ float4 sum_chunks(const float4* src, int64_t plane4, 
   }
   return acc;
 }
-// (kVec: N is a multiple of 4, so the partial planes can be read 16 bytes at a time; otherwise one element per thread.)
+// (N is a multiple of 4, so the partial planes can be read 16 bytes at a time; otherwise one element per thread.)
 __device__ __forceinline__ float round_to(float v, int dtype) {
   if (dtype == IXK_BF16) return __bfloat162float(__float2bfloat16_rn(v));
   if (dtype == IXK_F16) return __half2float(__float2half_rn(v));
@@ -97,6 +101,7 @@ __device__ __forceinline__ float round_to(float v, int dtype) {
 // GeGLU over the two halves of a [M, 2 N'] product: thread = four consecutive output columns; the
 // gate is activated and rounded, the up half rounded, then multiplied (the values a gate GEMM with
 // a GELU epilogue, an up GEMM and an elementwise product would have produced one after the other).
+template <int kHeld>
 __global__ void splitk_reduce_geglu_kernel(const ReduceArgs a) {
   ptx::grid_dependency_sync();
   const int half = a.N / 2, h4 = half / 4;
@@ -108,7 +113,7 @@ __global__ void splitk_reduce_geglu_kernel(const ReduceArgs a) {
     const int n = static_cast<int>(i - static_cast<int64_t>(m) * h4) * 4;
     const float4* gsrc = reinterpret_cast<const float4*>(a.partial) + (static_cast<int64_t>(m) * a.N + n) / 4;
     const float4* usrc = gsrc + h4;
-    const float4 g = sum_chunks(gsrc, plane4, a.splits), u = sum_chunks(usrc, plane4, a.splits);
+    const float4 g = sum_chunks<kHeld>(gsrc, plane4, a.splits), u = sum_chunks<kHeld>(usrc, plane4, a.splits);
     const float gs[4] = {g.x, g.y, g.z, g.w}, us[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e)
@@ -117,18 +122,18 @@ __global__ void splitk_reduce_geglu_kernel(const ReduceArgs a) {
   }
 }
 
-template <bool kVec>
+template <int kHeld>   // 0: N is not a multiple of 4
 __global__ void splitk_reduce_kernel(const ReduceArgs a) {
   ptx::grid_dependency_sync();
   const int64_t plane = static_cast<int64_t>(a.M) * a.N;
-  if constexpr (kVec) {
+  if constexpr (kHeld > 0) {
     const int64_t total = plane / 4;
     const int n4 = a.N / 4;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
       const int m = static_cast<int>(i / n4);
       const int n = static_cast<int>(i - static_cast<int64_t>(m) * n4) * 4;
-      const float4 acc = sum_chunks(reinterpret_cast<const float4*>(a.partial) + i, plane / 4, a.splits);
+      const float4 acc = sum_chunks<kHeld>(reinterpret_cast<const float4*>(a.partial) + i, plane / 4, a.splits);
       reduce_epilogue_store(a, m, n, acc.x);
       reduce_epilogue_store(a, m, n + 1, acc.y);
       reduce_epilogue_store(a, m, n + 2, acc.z);
@@ -186,7 +191,7 @@ int split_k_factor(int64_t M, int64_t N, int64_t K, int64_t batch, bool fp8) {
 
 // Problems whose tiles leave half of the SMs or more without work.  An estimate of both ways; cut where that is a tenth
 // shorter.  Whole -> cut, us: bf16 300 x 512 x 8192 31.7 -> 13.6, 500 x 512 x 16384 60 -> 19, 2000 x 256 x 8192 32 -> 18,
-// 900 x 304 x 16000 59 -> 21; fp8 250 x 512 x 16384 72 -> 18, 256 x 4096 x 4096 38 -> 21.
+// 900 x 304 x 16000 59 -> 21; fp8 250 x 512 x 16384 72 -> 18.
 int tiled_splits(int64_t M, int64_t N, int64_t K, int64_t batch, int elem_bytes, size_t workspace_bytes) {
   const int64_t tiles = (M + 127) / 128 * ((N + 127) / 128), slabs = (K * elem_bytes + kSlabBytes - 1) / kSlabBytes;
   const int64_t plane = M * N * static_cast<int64_t>(sizeof(float));
@@ -240,12 +245,15 @@ int launch_split_k(const Problem& p, int splits, void* workspace, const DeviceIn
   if (geglu) {
     const int64_t total = p.M * (p.N / 8);
     const ReduceGrid g = reduce_grid(total, dev.sm_count);
-    return launch_overlapped(splitk_reduce_geglu_kernel, dim3(g.blocks), dim3(g.threads), 0, stream, r);
+    auto* fn = splits == 1 ? splitk_reduce_geglu_kernel<1> : splits == 2 ? splitk_reduce_geglu_kernel<2>
+             : splits <= 4 ? splitk_reduce_geglu_kernel<4> : splitk_reduce_geglu_kernel<8>;
+    return launch_overlapped(fn, dim3(g.blocks), dim3(g.threads), 0, stream, r);
   }
   const bool vec = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0;
   const int64_t total = vec ? p.M * p.N / 4 : p.M * p.N;
   const ReduceGrid g = reduce_grid(total, dev.sm_count);
-  return launch_overlapped(vec ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3(g.blocks), dim3(g.threads), 0, stream, r);
+  auto* fn = !vec ? splitk_reduce_kernel<0> : splits == 2 ? splitk_reduce_kernel<2> : splits <= 4 ? splitk_reduce_kernel<4> : splitk_reduce_kernel<8>;
+  return launch_overlapped(fn, dim3(g.blocks), dim3(g.threads), 0, stream, r);
 }
 
 }  // namespace gemm
