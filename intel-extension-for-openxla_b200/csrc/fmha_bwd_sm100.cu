@@ -697,9 +697,15 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 }
 
 // The three kernels start under one another where each is a few microseconds; of long ones the next one's early CTAs
-// only stand in the way (B8 N16 S2048 H128 causal, 14 rounds: forward and backward 708 us in order, 723).
+// only stand in the way (B8 N16 S2048 H128 causal, 14 rounds: forward and backward 708 us in order, 723).  At head sizes of
+// up to 64 two main CTAs fit on an SM, and those that start under the prepare kernel crowd on the SMs that it has left:
+// where they are many and long that costs more than the start gains (forward and backward, against all three in order, by
+// rows: up to 512 0.85 to 1.0; up to 1024 0.94 to 0.96 with up to 100 CTAs, 0.98 to 1.04 with more; beyond that 0.96 with
+// 20 CTAs, 0.97 to 1.12 with more: B3 N1 S2069 non-causal 65.7 and 70.3 us).
 bool bwd_overlaps(const Problem& p, const DeviceInfo& dev) {
-  return static_cast<int64_t>((p.T + kBlk - 1) / kBlk) * p.N * p.B <= 2 * dev.sm_count;
+  const int64_t ctas = static_cast<int64_t>((p.T + kBlk - 1) / kBlk) * p.N * p.B;
+  if (p.H <= 64 && p.F > 512 && ctas > (p.F <= 1024 ? 100 : 20)) return false;
+  return ctas <= 2 * dev.sm_count;
 }
 
 template <int kHeadDim, bool kBias, bool kBf16>
