@@ -191,7 +191,7 @@ int run(const ixk_gemm_desc* desc, const void* a, const void* b, const void* c, 
   p.out_dtype = tc;
   p.act = act;
   p.beta = desc->beta;
-  (void)swapped;
+  if (swapped) std::swap(p.a_fmt, p.b_fmt);   // (e4m3 and e5m2 operands may be mixed)
   if (aux_call) {
     // aux has the output's type, order and shape (after a column-major output has been rewritten
     // it is row-major [M,N] like D), its own pitch, and D's batch spacing rule: dense batches.

@@ -115,6 +115,22 @@ def test_bf16_operands_rejected_by_fp8_entry(pkg, cuda):
     assert e.value.status == pkg.IXK_INVALID_ARGUMENT
 
 
+@pytest.mark.parametrize("shape", [(40, 96, 17), (40, 96, 200), (300, 8208, 136), (1500, 256, 4608)], ids=lambda s: "M{}K{}N{}".format(*s))
+@pytest.mark.parametrize("a_dtype,b_dtype", [(torch.float8_e4m3fn, torch.float8_e5m2), (torch.float8_e5m2, torch.float8_e4m3fn)])
+def test_mixed_types_into_a_column_major_result(pkg, cuda, shape, a_dtype, b_dtype):
+    """The product is computed transposed then: each operand keeps its own type.  Few rows of the transposed product, tiles,
+    tiles cut along K (fp32 sums within (K + 16) * 2^-23 of the sum of magnitudes), CTA pairs."""
+    M, K, N = shape
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a = torch.randn(M, K, generator=g, device=cuda).to(a_dtype)
+    b = torch.randn(N, K, generator=g, device=cuda).to(b_dtype).t()
+    out = torch.empty(N, M, device=cuda).t()
+    ws = torch.empty(16 << 20, dtype=torch.uint8, device=cuda)
+    got = pkg.gemm_fp8(a, b, 0.5, 0.25, out=out, workspace=ws)
+    want, mag = a.double() @ b.double() * 0.125, a.double().abs() @ b.double().abs() * 0.125
+    assert ((got.double() - want).abs() <= (K + 16) * 2.0 ** -23 * mag + 2.0 ** -22 * want.abs()).all()
+
+
 FIRST_CALLS = """
 import sys
 sys.path.insert(0, sys.argv[1])
