@@ -251,23 +251,30 @@ __device__ __forceinline__ void epilogue_tile(const KernelArgs& args, const CUte
       // two passes earlier has read it.  Stored from registers, a warp's 16-byte stores land in
       // 32 different lines each; those requests queue in front of the producer's and the
       // issuer's barrier traffic and cost 8-11 % of the kernel.
+      // A TMA store writes whole 16-byte pieces: where N ends inside one it would put zeros into up to seven elements
+      // behind the row, which belong to somebody else.  The box with that end is stored from registers.
+      const bool odd_end = (args.N & 7) != 0;
 #pragma unroll 1
       for (int c0 = 0; c0 < width; c0 += 64) {
         const int n = n_first + c0;
         if (n >= args.N) break;  // warp-uniform
+        const bool plain = odd_end && n + 64 > args.N;
         uint32_t wv[32];
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           const int nh = n + 32 * half;
           if (nh < args.N) {  // warp-uniform
             float v[32];
-            chunk(c0 + 32 * half, nh, min(32, args.N - nh), v);
+            const int count = min(32, args.N - nh);
+            chunk(c0 + 32 * half, nh, count, v);
+            if (plain && row_ok) store_row(args.d, d_row + nh, args.out_dtype, count, vec_d, v);
             pack_row16(v, args.out_dtype, &wv[16 * half]);
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i) wv[16 * half + i] = 0u;
           }
         }
+        if (plain) break;   // (the row's last box)
         const uint32_t box = stage_smem + static_cast<uint32_t>((quarter * 2 + (n_store & 1)) * 4096);
         if (lane == 0) ptx::bulk_wait_group_read<1>();
         __syncwarp();

@@ -587,3 +587,25 @@ def test_few_tiles_long_k(pkg, cuda, shape, kind, la, lb):
     assert pkg.launch_count() - n0 == 2
     want = plain + c
     assert ((out.double() - want).abs().max() <= 1.01 * half * want.abs().max() + sums + 2.0 ** -22).item()
+
+
+@pytest.mark.parametrize("shape", [(24, 64, 3), (200, 72, 77), (130, 64, 8), (300, 128, 259), (1400, 256, 4611), (2, 40, 64, 13)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("la", ["row", "col"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float8_e4m3fn])
+def test_result_among_others_leaves_them_alone(pkg, cuda, shape, la, dtype):
+    """A result that is a slice of wider rows, which start on 16-byte boundaries and whose columns end anywhere: what lies
+    behind them stays.  One CTA, pairs, batches; K as short as the slices' few columns let a wrong store show."""
+    *batch, M, K, N = shape
+    g = torch.Generator(device="cuda").manual_seed(N)
+    pad = lambda n: (n + 15) // 16 * 16
+    x, w = (torch.randn(*batch, r, pad(c), generator=g, device=cuda).to(dtype)[..., :c] for r, c in (((M, K) if la == "row" else (K, M)), (K, N)))
+    x = x if la == "row" else x.transpose(-1, -2)
+    out_dtype = torch.bfloat16 if dtype == torch.float8_e4m3fn else dtype
+    wide = torch.full((*batch, M, (N + 23) // 8 * 8), 7.0, dtype=out_dtype, device=cuda)
+    out = wide[..., 8:8 + N]
+    got = pkg.gemm_fp8(x, w, 1.0, 1.0, out=out) if dtype == torch.float8_e4m3fn else pkg.gemm(x, w, out=out)
+    want, mag = x.double() @ w.double(), x.double().abs() @ w.double().abs()
+    half = 2.0 ** -11 if out_dtype == torch.float16 else 2.0 ** -8
+    assert ((got.double() - want).abs() <= 1.01 * half * want.abs() + (K + 16) * 2.0 ** -23 * mag + 2.0 ** -24).all()
+    assert (wide[..., :8] == 7.0).all() and (wide[..., 8 + N:] == 7.0).all()
