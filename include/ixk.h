@@ -181,9 +181,9 @@ int ixk_gemm_fp8(const ixk_gemm_desc* desc, const void* a, const void* b,
  * last; desc describes the [M, 2 N'] product (row-major, dense, 16-bit, DEFAULT epilogue, alpha 1,
  * beta 0, batch 1, M <= 128: decode); out [M, N'] receives
  *   round(gelu_tanh(gate)) * round(up)   rounded once more,
- * the bits of a gate GEMM with the GELU epilogue, an up GEMM and an elementwise product.  The
- * product itself (split along K where that helps) lives in the workspace, which must hold
- * ixk_gemm_geglu_workspace_bytes(desc) bytes.  Other shapes: IXK_UNIMPLEMENTED (use the calls above). */
+ * the roundings of a gate GEMM with the GELU epilogue, an up GEMM and an elementwise product (the
+ * sums of K agree within fp32 summation order: K is cut by the product's size and the scratch).  The
+ * product itself lives in the workspace, which must hold ixk_gemm_geglu_workspace_bytes(desc) bytes.  Other shapes: IXK_UNIMPLEMENTED (use the calls above). */
 int ixk_gemm_geglu(const ixk_gemm_desc* desc, const void* a, const void* b, void* out,
                    int64_t out_leading_dim_stride, void* workspace, size_t workspace_bytes,
                    void* cuda_stream);

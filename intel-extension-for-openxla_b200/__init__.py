@@ -221,7 +221,7 @@ def device_status() -> int:
     return word.value
 
 
-# A decode step is sixteen launches of a few microseconds, so what Python does for each call is part of
+# A decode step is fourteen launches of a few microseconds, so what Python does for each call is part of
 # its time: descriptors are packed in one go, pointers and the stream travel as plain integers (the
 # current stream's handle is read without a Stream object around it).
 _current_device = getattr(torch._C, "_cuda_getDevice", None)
@@ -323,7 +323,7 @@ def _launch_gemm(d: "_GemmDesc", lhs, rhs, add, output, bias, stream, inv_scale_
 
 
 def gemm_workspace_bytes(lhs: torch.Tensor, rhs: torch.Tensor, out_shape=None) -> int:
-    """Scratch bytes ixk_gemm can make use of for lhs @ rhs (0 unless the problem is skinny)."""
+    """Scratch bytes ixk_gemm can make use of for lhs @ rhs (0 where K is not cut: see run_gemm_custom_call)."""
     d = _GemmDesc()
     m, k = lhs.shape[-2], lhs.shape[-1]
     n = rhs.shape[-1]

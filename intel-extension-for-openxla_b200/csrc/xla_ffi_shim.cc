@@ -95,7 +95,7 @@ static ffi::Error LtMatmul(cudaStream_t stream, ffi::ScratchAllocator scratch, f
                       desc.output.leading_dim_stride, stream);
     return ToError(st);
   }
-  // Optional scratch: non-zero only for skinny (decode, M <= 128) problems, which then run split along K.
+  // Optional scratch, for problems that run split along K: few rows, or few tiles and a long K.
   size_t ws_bytes = ixk_gemm_workspace_bytes(&desc);
   void* ws = nullptr;
   if (ws_bytes != 0) {
